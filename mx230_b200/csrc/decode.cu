@@ -624,7 +624,12 @@ decode_q8_kernel(const DecodeParams P) {
 //            next MMA (thread (g, j) holds head g, keys 2j, 2j+1 of each 8-key group);
 //   values:  O[16 x 64] += (p vs)[16 x 16 keys] Vc[16 x 64], f16 x f16 -> f32 (m16n8k16).  The int8
 //            codes become f16 exactly (byte permutes onto the mantissa of 1024, minus 1152); p vs
-//            goes in as a high and a low f16 part, so the product carries ~22 bits.
+//            goes in as a high and a low f16 part, so the product carries ~22 bits.  The low parts are
+//            rows 8..15 of the same A tile, which a group of at most 8 heads leaves empty: one MMA does
+//            both products and every accumulator tile is four registers of its own.  (Two MMAs whose
+//            unused rows shared a pair of zero registers cost 153 register moves among 576 instructions
+//            per 32-key tile: 8 x 131072 keys, 4 K/V heads, 118 -> 99 us = 6.1 TB/s; the loop is bound by
+//            issue slots whenever it is not bound by HBM.)
 // ---------------------------------------------------------------------------
 constexpr int MG = 8;                               // heads per CTA (rows 8..15 of the tiles are padding)
 // Probabilities are taken against a running max that may lag by up to RAISE_MMA (natural-log units);
@@ -641,11 +646,11 @@ __device__ __forceinline__ void mma_s8(int (&c)[4], int a0, int a2, int b0, int 
                  : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
                  : "r"(a0), "r"(0), "r"(a2), "r"(0), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ void mma_f16(float &c0, float &c1, float &z0, float &z1, uint32_t a0, uint32_t a2,
-                                        uint32_t b0, uint32_t b1) {
+__device__ __forceinline__ void mma_f16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                        uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(c0), "+f"(c1), "+f"(z0), "+f"(z1)
-                 : "r"(a0), "r"(0u), "r"(a2), "r"(0u), "r"(b0), "r"(b1));
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 __device__ __forceinline__ uint32_t pack_f16(float lo, float hi) {
     uint32_t r;
@@ -802,10 +807,9 @@ decode_q8_mma_kernel(const DecodeParams P) {
     const float hq_g = hq[g], qsum_g = hq[MG + g];
 
     float m_run = -CUDART_INF_F, l_thr = 0.0f, b_thr = 0.0f;
-    float oacc[8][2];
-    float z0 = 0.0f, z1 = 0.0f;   // rows 8..15 of the output tiles: stay zero
+    float oacc[8][4];   // [0..1]: the high parts' products (row g), [2..3]: the low parts' (row g + 8)
 #pragma unroll
-    for (int t = 0; t < 8; ++t) oacc[t][0] = oacc[t][1] = 0.0f;
+    for (int t = 0; t < 8; ++t) oacc[t][0] = oacc[t][1] = oacc[t][2] = oacc[t][3] = 0.0f;
 
     const uint32_t MAGIC = 0x64646464u, BIAS = 0x64806480u;  // f16 1024 | byte, minus 1152
     for (int tile = 0; tile < n_tiles; ++tile) {
@@ -850,7 +854,7 @@ decode_q8_mma_kernel(const DecodeParams P) {
                 l_thr *= alpha;
                 b_thr *= alpha;
 #pragma unroll
-                for (int t = 0; t < 8; ++t) oacc[t][0] *= alpha, oacc[t][1] *= alpha;
+                for (int t = 0; t < 8; ++t) oacc[t][0] *= alpha, oacc[t][1] *= alpha, oacc[t][2] *= alpha, oacc[t][3] *= alpha;
                 m_run = m_new;
             }
             // ---- probabilities, weights (high + low f16 parts) ----
@@ -887,10 +891,7 @@ decode_q8_mma_kernel(const DecodeParams P) {
                 b[r][7] = hsub2(__byte_perm(zy23, MAGIC, 0x4342), BIAS);
             }
 #pragma unroll
-            for (int t = 0; t < 8; ++t) {
-                mma_f16(oacc[t][0], oacc[t][1], z0, z1, ah[0], ah[1], b[0][t], b[1][t]);
-                mma_f16(oacc[t][0], oacc[t][1], z0, z1, al[0], al[1], b[0][t], b[1][t]);
-            }
+            for (int t = 0; t < 8; ++t) mma_f16(oacc[t], ah[0], al[0], ah[1], al[1], b[0][t], b[1][t]);
         }
         __syncwarp();  // the ring slot is rewritten by the next iterations
     }
@@ -913,8 +914,8 @@ decode_q8_mma_kernel(const DecodeParams P) {
         // tile t, columns 2j, 2j+1 <-> dims 16j + t, 16j + 8 + t
 #pragma unroll
         for (int t = 0; t < 8; ++t) {
-            dst[4 + 16 * j + t] = oacc[t][0];
-            dst[4 + 16 * j + 8 + t] = oacc[t][1];
+            dst[4 + 16 * j + t] = oacc[t][0] + oacc[t][2];
+            dst[4 + 16 * j + 8 + t] = oacc[t][1] + oacc[t][3];
         }
     }
     __syncthreads();
