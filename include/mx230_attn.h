@@ -287,6 +287,23 @@ int mx230_attn_decode_q8_batched(mx230_handle *h, void *stream, float *out, cons
                                  const int *tables, int block_size, int n_log, int qkv_stride,
                                  int out_stride);
 
+/* The whole attention step of one decode token in one launch: RoPE at the token's position on the Q and K heads of the
+ * qkv row (use_rope != 0; rotated in place, as mx230_rope leaves it), the K and V heads written to the cache (fp32
+ * kcache / vcache when kq == NULL, else int8 quantize-on-write; kb == vb == NULL: absmax) and attention over keys
+ * 0..=pos -- what 03-llm-engine/src/gpu.rs:2570-2672 (and :2808-2918 with pos_ptr, the graph-captured form) does in
+ * three launches per layer.  Host position: the row written is write_row (the caller's phys_row); device position:
+ * through bt / bs, or pos itself without a table.  mx230_batched_step: the same for one token of each of n_seq
+ * sequences over packed block tables (gpu.rs:3530-3628).  Every result equals that of the separate entry points, which
+ * also run when a group has more than 8 query heads per K/V head or the int8 cache is scored on CUDA cores. */
+int mx230_decode_step(mx230_handle *h, void *stream, float *out, float *qkv, float *kcache, float *vcache,
+                      int8_t *kq, int8_t *vq, float *ks, float *vs, float *kb, float *vb, int pos,
+                      const int *pos_ptr, int write_row, int n_head, int n_kv_head, int head_dim, int use_rope,
+                      float theta, const int *bt, int bs);
+int mx230_batched_step(mx230_handle *h, void *stream, float *out, float *qkv, float *kcache, float *vcache,
+                       int8_t *kq, int8_t *vq, float *ks, float *vs, float *kb, float *vb, const int *pos,
+                       int n_seq, int n_head, int n_kv_head, int head_dim, int use_rope, float theta,
+                       const int *tables, int block_size, int n_log, int qkv_stride, int out_stride);
+
 /* Decode over an int8 cache without a handle and without any allocation (no counterpart in
  * the reference, whose kernels use no scratch memory at all).  For hosts that cannot call
  * cudaMalloc when they need attention -- all free HBM already given to their KV pool, or only

@@ -569,6 +569,61 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
     return r;
 }
 
+// ---- RoPE (HF rotate_half): the pair (d, d + 32) of a 64-value head at position `pos` ----
+// precise powf / sincosf: the reference's CPU path (03-llm-engine/src/cpu.rs:25-37); its GPU kernel uses the fast
+// intrinsics, which lose accuracy at large angles
+__device__ __forceinline__ void rope_angle(int pos, int d, int head_dim, float theta, float &cs, float &sn) {
+    const float freq = powf(theta, -2.0f * (float)d / (float)head_dim);
+    sincosf((float)pos * freq, &sn, &cs);
+}
+// one rounding order for every kernel that rotates, so that they all leave the same bits
+__device__ __forceinline__ void rope_pair(float &x1, float &x2, float cs, float sn) {
+    const float a = x1, b = x2;
+    x1 = __fmaf_rn(a, cs, -__fmul_rn(b, sn));
+    x2 = __fmaf_rn(a, sn, __fmul_rn(b, cs));
+}
+
+// ---- int8 quantize-on-write of one head's 64 values by one warp, two values per lane (any assignment of values to
+// lanes): IEEE division and round-to-nearest-even exactly as quant_affine (03-llm-engine/kernels/llm.cu:1137-1149), or
+// symmetric absmax / 127 when !affine (beta 0) ----
+__device__ __forceinline__ void quant_head_row(float x0, float x1, bool affine, int &c0, int &c1, float &scale, float &beta) {
+    auto wmax = [](float v) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
+        return v;
+    };
+    if (affine) {
+        const float hi = wmax(fmaxf(x0, x1));
+        const float lo = -wmax(fmaxf(-x0, -x1));
+        scale = (hi > lo) ? __fdiv_rn(hi - lo, 255.0f) : 1.0f;
+        beta = __fmaf_rn(128.0f, scale, lo);   // exact: 128*scale is a power-of-two scaling
+        c0 = max(-128, min(127, __float2int_rn(__fdiv_rn(x0 - beta, scale))));
+        c1 = max(-128, min(127, __float2int_rn(__fdiv_rn(x1 - beta, scale))));
+    } else {
+        const float amax = wmax(fmaxf(fabsf(x0), fabsf(x1)));
+        const float id = amax > 0.0f ? __fdiv_rn(127.0f, amax) : 0.0f;
+        c0 = max(-127, min(127, __float2int_rn(x0 * id)));
+        c1 = max(-127, min(127, __float2int_rn(x1 * id)));
+        scale = amax > 0.0f ? __fdiv_rn(amax, 127.0f) : 0.0f;
+        beta = 0.0f;
+    }
+}
+
+// ---- thread-block clusters: barrier and loads from the shared memory of the cluster's other CTAs ----
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t cluster_map(uint32_t saddr, int rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ float cluster_ld_f32(uint32_t addr) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+    return v;
+}
+
 // ---- {value, step} words of the split-KV exchange: 8-byte accesses are single-copy atomic, so a reader that
 // finds the current step number in a word also has that word's value ----
 __device__ __forceinline__ void st_words2(uint2 *p, float a, float b, unsigned step) {

@@ -5,13 +5,19 @@
 // 03-llm-engine/kernels/llm.cu:1246-1487 -- one block per QUERY head, three phases
 // (scores+max, exp+sum, PV), whole score row in shared s[2048].
 //
+// The step of one token (mx230_decode_step, mx230_batched_step) is ONE launch: the attention kernel rotates q, rotates,
+// quantises and writes the new K and V rows, and takes the new key from registers (host-launched step at 778 keys, fp32
+// cache: three launches 18.1 us of device time and 28 us per pass -> 9.0 and 11 us; 64 int8 sequences of up to 2048 keys:
+// 22.8 and 34 us -> 13.3 and 15 us).
+//
 // This design: one CTA per (key split, kv head, sequence) serves ALL query heads of
 // the kv head's group, so every cache byte leaves HBM once.  Inside the CTA every warp
 // streams its own key sub-range through a private cp.async shared-memory ring (memory
 // parallelism independent of register pressure, no block barrier in the loop) and keeps
 // a private online-softmax state, so the context length is unbounded; the warps are merged
-// by log-sum-exp at the end.  Split CTAs leave (m, l, acc) partials in the workspace; the
-// last CTA to arrive for a (sequence, kv head) merges them.  Three kernels share this
+// by log-sum-exp at the end.  Up to eight CTAs of a group form a thread-block cluster and
+// merge through distributed shared memory; several clusters leave (m, l, acc) partials in the
+// workspace, which the last CTA to arrive for a (sequence, kv head) merges (see plan_splits).  Three kernels share this
 // skeleton: fp32 cache on CUDA cores; int8 cache on CUDA cores (exact score mode); int8
 // cache with the GQA group on warp-level tensor-core tiles (reference score mode).
 #include <math_constants.h>
@@ -46,6 +52,17 @@ struct DecodeParams {
     int max_keys;        // capacity of one sequence (slab rows, or table entries x block) when positions come from the device; 0 = unknown
     int n_head, n_kv_head, group, head_groups;
     int score_mode;
+    // key splits of one (sequence, K/V head) group: grid.x = max_clusters clusters of cl_size CTAs (a power of two up to
+    // 8); a sequence of `len` keys uses the first ceil(len / cluster_keys) clusters (all of them when cluster_keys == 0),
+    // so that the split follows the length of each sequence and not only the largest one
+    int cl_size, max_clusters, cluster_keys;
+    int bs_shift;        // log2(bs) when bs is a power of two, else -1
+    // fused step (RoPE and KV write of the new token inside the attention kernel): keys [0, pos) come from the cache,
+    // key `pos` from the qkv row, whose K and V heads are written to cache row `write_row` (< 0: through the table)
+    float *qkv_rw;       // the same buffer as qkv, for the rotated q and k left in place; null = not fused
+    int use_rope;
+    float theta;
+    long long write_row;
     // partial mode with a push: the finished triples also go, as {value, step} words, into slot `push_rank` of every
     // rank's split-KV exchange region (table of `push_world` region bases in device memory)
     uint2 *const *push_regions;
@@ -86,19 +103,32 @@ __device__ __forceinline__ size_t cache_row(const DecodeParams &P, const int *ta
     if (table) return (size_t)(table[t / P.bs] * P.bs + t % P.bs);
     return (size_t)(base + t);
 }
+// the same for paged caches, with the division as a shift where the block size is a power of two
+__device__ __forceinline__ int paged_row(const DecodeParams &P, const int *table, int t) {
+    const int b = P.bs_shift >= 0 ? t >> P.bs_shift : t / P.bs;
+    return table[b] * P.bs + (t - b * P.bs);
+}
 
+__device__ __forceinline__ int seq_pos(const DecodeParams &P, int s) {
+    int p = P.pos_kind == 0 ? P.pos : (P.pos_kind == 1 ? *P.pos_dev : P.pos_dev[s]);
+    // a position read from device memory cannot be validated by the host: where the capacity of a sequence is
+    // known, a wild value (a caller's ordering bug) is kept inside it rather than turned into wild addresses
+    if (P.pos_kind == 2 && P.max_keys > 0) p = min(max(p, 0), P.max_keys - 1);
+    return p;
+}
 __device__ __forceinline__ void key_range(const DecodeParams &P, int s, int &kbeg, int &kend) {
     if (P.range_mode) {
         kbeg = P.t0;
         kend = P.t1;
     } else {
-        int p = P.pos_kind == 0 ? P.pos : (P.pos_kind == 1 ? *P.pos_dev : P.pos_dev[s]);
-        // a position read from device memory cannot be validated by the host: where the capacity of a sequence is
-        // known, a wild value (a caller's ordering bug) is kept inside it rather than turned into wild addresses
-        if (P.pos_kind == 2 && P.max_keys > 0) p = min(max(p, 0), P.max_keys - 1);
         kbeg = 0;
-        kend = p + 1;
+        kend = seq_pos(P, s) + 1;
     }
+}
+// clusters of a group that take part for a range of `len` keys
+__device__ __forceinline__ int active_clusters(const DecodeParams &P, int len) {
+    if (P.cluster_keys == 0) return P.max_clusters;
+    return max(1, min(P.max_clusters, (len + P.cluster_keys - 1) / P.cluster_keys));
 }
 
 // Split c of n covers a 32-aligned slice of [kbeg, kend).
@@ -240,6 +270,113 @@ __device__ void merge_and_store(const DecodeParams &P, int s, int head0, int gc,
         __syncthreads();
         if (threadIdx.x < gc) P.push_steps[(size_t)s * P.n_head + head0 + threadIdx.x] += 1u;
     }
+}
+
+// Merge of a CTA's warps, then of its cluster's CTAs, then (several clusters) of the clusters through the workspace.
+// mg: shared memory, [n_warps][G][68] = m (log2 domain), l, sum of p * V offset, pad, acc[64] per warp and head; the
+// CTA's own totals go behind it, [G][68], where the cluster's other CTAs read them: rank r finishes the heads
+// g = r (mod cl_size), so that the merge of up to eight CTAs costs one cluster barrier and one round of remote loads
+// instead of a fence, an atomic and a re-read of global memory (int8, one sequence of 2001 keys, 2 K/V heads: 16 splits
+// merged through the workspace 8.2 us, one cluster of 8 CTAs 5.3 us).
+// q_rot (fused step): rotated q, [G][64] in shared memory; it replaces the raw q in qkv once every CTA of the group
+// has read that.
+template <int G>
+__device__ void finish_group(const DecodeParams &P, float *mg, int n_warps, int s, int head0, int gc, int cl, int rank,
+                             int active, const float *q_rot, int *is_last) {
+    const int tid = threadIdx.x, nt = blockDim.x, C = P.cl_size;
+    const bool direct = active == 1 && P.fin_acc == nullptr;
+    float *cm = mg + n_warps * G * 68;
+    auto emit = [&](int g, int d, float m2, float l, float a) {
+        const int h = head0 + g;
+        if (direct) {
+            P.out[(size_t)s * P.out_stride + h * 64 + d] = a / l;
+        } else {   // partial triples carry the max in natural-log units, as the split-KV interface states
+            const size_t pi = ((size_t)s * P.n_head + h) * active + cl;
+            P.ws_acc[pi * 64 + d] = a;
+            if (d == 0) {
+                P.ws_m[pi] = m2 * 0.6931471805599453f;
+                P.ws_l[pi] = l;
+            }
+        }
+    };
+    auto put_q = [&](int g, int d) { P.qkv_rw[(size_t)s * P.qkv_stride + (head0 + g) * 64 + d] = q_rot[g * 64 + d]; };
+    for (int i = tid; i < gc * 64; i += nt) {
+        const int g = i >> 6, d = i & 63;
+        float mm = -CUDART_INF_F;
+        for (int w = 0; w < n_warps; ++w) mm = fmaxf(mm, mg[(w * G + g) * 68]);
+        float lt = 0.0f, a = 0.0f;
+        for (int w = 0; w < n_warps; ++w) {
+            const float *src = mg + (w * G + g) * 68;
+            const float wgt = (src[0] == -CUDART_INF_F) ? 0.0f : mx::ex2(src[0] - mm);
+            lt += src[1] * wgt;
+            a += (src[4 + d] + src[2]) * wgt;  // V's affine offset sum_j p_j vb_j folds into every dim
+        }
+        if (C == 1) {
+            emit(g, d, mm, lt, a);
+            if (q_rot && active == 1) put_q(g, d);
+        } else {
+            cm[g * 68 + 4 + d] = a;
+            if (d == 0) cm[g * 68] = mm, cm[g * 68 + 1] = lt;
+        }
+    }
+    if (C > 1) {
+        mx::cluster_sync();
+        const uint32_t cm_u32 = mx::smem_u32(cm);
+        for (int i = tid; (i >> 6) * C + rank < gc; i += nt) {
+            const int g = (i >> 6) * C + rank, d = i & 63;
+            float mp[8], lp[8], ap[8];
+#pragma unroll
+            for (int p = 0; p < 8; ++p) {
+                mp[p] = -CUDART_INF_F, lp[p] = ap[p] = 0.0f;
+                if (p < C) {
+                    const uint32_t src = mx::cluster_map(cm_u32 + g * 68 * 4, p);
+                    mp[p] = mx::cluster_ld_f32(src);
+                    lp[p] = mx::cluster_ld_f32(src + 4);
+                    ap[p] = mx::cluster_ld_f32(src + 16 + d * 4);
+                }
+            }
+            float mm = mp[0];
+#pragma unroll
+            for (int p = 1; p < 8; ++p) mm = fmaxf(mm, mp[p]);
+            float lt = 0.0f, a = 0.0f;
+#pragma unroll
+            for (int p = 0; p < 8; ++p) {
+                const float wgt = (mp[p] == -CUDART_INF_F) ? 0.0f : mx::ex2(mp[p] - mm);
+                lt += lp[p] * wgt;
+                a += ap[p] * wgt;
+            }
+            emit(g, d, mm, lt, a);
+            if (q_rot && active == 1) put_q(g, d);
+        }
+        mx::cluster_sync();   // nobody leaves while its totals may still be read
+    }
+    if (direct) return;
+
+    // ---- the group's last CTA merges the clusters ----
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) {
+        const unsigned n = (unsigned)(active * C);
+        *is_last = atomicInc(&P.counters[(size_t)s * gridDim.y + blockIdx.y], n - 1) == n - 1;
+    }
+    __syncthreads();
+    if (!*is_last) return;
+    __threadfence();
+    if (q_rot && active > 1)
+        for (int i = tid; i < gc * 64; i += nt) put_q(i >> 6, i & 63);
+    merge_and_store<G>(P, s, head0, gc, active, nt);
+}
+
+// Fused step: the new token's K or V head as fp32 pairs (lane, lane + 32), K rotated in place in qkv.
+__device__ __forceinline__ float2 new_kv_pair(const DecodeParams &P, int s, int kvh, int which, int lane, float cs, float sn) {
+    float *src = P.qkv_rw + (size_t)s * P.qkv_stride + (P.n_head + which * P.n_kv_head + kvh) * 64;
+    float2 x = make_float2(src[lane], src[lane + 32]);
+    if (which == 0 && P.use_rope) {
+        mx::rope_pair(x.x, x.y, cs, sn);
+        src[lane] = x.x;
+        src[lane + 32] = x.y;
+    }
+    return x;
 }
 
 // ---------------------------------------------------------------------------
@@ -671,20 +808,21 @@ __device__ __forceinline__ uint32_t hsub2(uint32_t a, uint32_t b) {
 struct Q8MmaSmem {
     static constexpr int Q_BYTES = MG * 64 * 4 + MG * 16 * 4 + 2 * MG * 4 + 64;
     static constexpr int PER_WARP = MMA_STAGES * WT_STAGE;
-    static constexpr int MERGE = Q8_WARPS * MG * 68 * 4;
-    static constexpr int TOTAL = ((Q_BYTES + 127) & ~127) + (Q8_WARPS * PER_WARP > MERGE ? Q8_WARPS * PER_WARP : MERGE);
+    static constexpr int MERGE = (Q8_WARPS + 1) * MG * 68 * 4;
+    static constexpr int TOTAL = ((Q_BYTES + 127) & ~127) + WT_STAGE + (Q8_WARPS * PER_WARP > MERGE ? Q8_WARPS * PER_WARP : MERGE);
 };
 
-template <bool PAGED>
+template <bool PAGED, bool FUSED>
 __global__ void __launch_bounds__(Q8_THREADS, 2)
 decode_q8_mma_kernel(const DecodeParams P) {
     using SM = Q8MmaSmem;
     constexpr float LOG2E = 1.4426950408889634f;
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    float *qf = (float *)smem_raw;                        // [8][64]
+    float *qf = (float *)smem_raw;                        // [8][64] rotated q (fused step only)
     int *qq = (int *)(qf + MG * 64);                      // [8][16] int8 codes
     float *hq = (float *)(qq + MG * 16);                  // [2][8]: score scale (log2 domain), sum of q codes
-    unsigned char *warp_base = smem_raw + ((SM::Q_BYTES + 127) & ~127);
+    unsigned char *extra = smem_raw + ((SM::Q_BYTES + 127) & ~127);   // fused step: the new token as a one-key tile
+    unsigned char *warp_base = extra + WT_STAGE;
     __shared__ int is_last;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -693,11 +831,16 @@ decode_q8_mma_kernel(const DecodeParams P) {
     const int hg = blockIdx.y - kvh * P.head_groups;
     const int head0 = kvh * P.group + hg * 8;
     const int gc = min(MG, P.group - hg * 8);
-    const int n_splits = gridDim.x;
     const int nkv = P.n_kv_head, kvd = nkv * 64;
+    const int cl = blockIdx.x / P.cl_size, rank = blockIdx.x - cl * P.cl_size;
 
     int kbeg, kend, ka, kb_;
     key_range(P, s, kbeg, kend);
+    const int pos = kend - 1;                             // fused step: the new token's position
+    if (FUSED) kend = pos;
+    const int active = active_clusters(P, kend - kbeg);
+    if (cl >= active) return;
+    const int n_splits = active * P.cl_size;
     split_range(kbeg, kend, blockIdx.x, n_splits, ka, kb_);
     const int *table = PAGED ? P.tables + (P.pos_kind == 2 ? (size_t)s * P.n_log : 0) : nullptr;
     const long long base = PAGED ? 0 : (long long)s * P.seq_rows;
@@ -735,11 +878,35 @@ decode_q8_mma_kernel(const DecodeParams P) {
         s_vb = affine ? P.vb + sd : P.vs + sd;
     }
     const size_t it_stride = (size_t)8 * kvd, tile_stride = (size_t)WT_KEYS * kvd;
+    // paged caches: lane l looks up the row of key l of the NEXT tile to be issued one tile ahead, so that the table
+    // read is off the chain of dependent loads and every key costs one division and one lookup
+    auto row_ahead = [&](int tile) {
+        const int t = wa + tile * WT_KEYS + lane;
+        return paged_row(P, table, t < wb ? t : wa);
+    };
+    int row_l = 0;
+    if (PAGED && n_tiles > 0) row_l = row_ahead(0);
 
     auto issue = [&](int tile) {
         const uint32_t dst = ring_u32 + (tile % MMA_STAGES) * WT_STAGE;
         const int key0 = wa + tile * WT_KEYS;
-        if (!PAGED && key0 + WT_KEYS <= wb) {  // full tile of a linear cache: no predicates, no lookups
+        if (PAGED) {
+#pragma unroll
+            for (int it = 0; it < 4; ++it) {
+                const size_t off = (size_t)__shfl_sync(0xFFFFFFFFu, row_l, it * 8 + pk) * kvd + kvh * 64 + pp * 16;
+                const int n = key0 + it * 8 + pk < wb ? 16 : 0;
+                cp_async16(dst + dk0 + it * 512, P.kq + off, n);
+                cp_async16(dst + v_dst(it * 8 + pk), P.vq + off, n);
+            }
+            const size_t sd = (size_t)row_l * nkv + kvh;
+            cp_async4(dst + ds0, P.ks + sd);
+            cp_async4(dst + ds0 + 128, affine ? P.kb + sd : P.ks + sd);
+            cp_async4(dst + ds0 + 256, P.vs + sd);
+            cp_async4(dst + ds0 + 384, affine ? P.vb + sd : P.vs + sd);
+            if (tile + 1 < n_tiles) row_l = row_ahead(tile + 1);
+            return;
+        }
+        if (key0 + WT_KEYS <= wb) {  // full tile of a linear cache: no predicates
 #pragma unroll
             for (int it = 0; it < 4; ++it) {
                 cp_async16(dst + dk0 + it * 512, ksrc + it * it_stride, 16);
@@ -752,23 +919,21 @@ decode_q8_mma_kernel(const DecodeParams P) {
         } else {
 #pragma unroll
             for (int it = 0; it < 4; ++it) {
-                int t = key0 + it * 8 + pk;
-                bool ok = t < wb;
-                size_t row = cache_row(P, table, base, ok ? t : wa);
-                cp_async16(dst + dk0 + it * 512, P.kq + row * kvd + kvh * 64 + pp * 16, ok ? 16 : 0);
-                cp_async16(dst + v_dst(it * 8 + pk), P.vq + row * kvd + kvh * 64 + pp * 16, ok ? 16 : 0);
+                const int t = key0 + it * 8 + pk;
+                const bool ok = t < wb;
+                const size_t off = (size_t)(base + (ok ? t : wa)) * kvd + kvh * 64 + pp * 16;
+                cp_async16(dst + dk0 + it * 512, P.kq + off, ok ? 16 : 0);
+                cp_async16(dst + v_dst(it * 8 + pk), P.vq + off, ok ? 16 : 0);
             }
-            int t = key0 + lane;
-            size_t sd = cache_row(P, table, base, t < wb ? t : wa) * nkv + kvh;
+            const int t = key0 + lane;
+            const size_t sd = (size_t)(base + (t < wb ? t : wa)) * nkv + kvh;
             cp_async4(dst + ds0, P.ks + sd);
             cp_async4(dst + ds0 + 128, affine ? P.kb + sd : P.ks + sd);
             cp_async4(dst + ds0 + 256, P.vs + sd);
             cp_async4(dst + ds0 + 384, affine ? P.vb + sd : P.vs + sd);
         }
-        if (!PAGED) {
-            ksrc += tile_stride, vsrc += tile_stride;
-            s_ks += WT_KEYS * nkv, s_kb += WT_KEYS * nkv, s_vs += WT_KEYS * nkv, s_vb += WT_KEYS * nkv;
-        }
+        ksrc += tile_stride, vsrc += tile_stride;
+        s_ks += WT_KEYS * nkv, s_kb += WT_KEYS * nkv, s_vs += WT_KEYS * nkv, s_vb += WT_KEYS * nkv;
     };
 
     // the first tiles are requested before anything else: their HBM latency then covers the q prologue below
@@ -779,12 +944,39 @@ decode_q8_mma_kernel(const DecodeParams P) {
     }
 
     // ---- q: per-head int8 codes as the reference kernel forms them (padding heads: zeros) ----
-    const float *qrow = P.qkv + (size_t)s * P.qkv_stride + head0 * 64;
-    for (int i = tid; i < MG * 64; i += Q8_THREADS) qf[i] = (i / 64 < gc) ? qrow[i] : 0.0f;
-    __syncthreads();
+    const bool owner = FUSED && (int)blockIdx.x == n_splits - 1;   // the CTA that takes the new token's own key
     {
         const int g = warp;  // Q8_WARPS == MG
-        float a = qf[g * 64 + lane], b = qf[g * 64 + 32 + lane];
+        const float *qrow = P.qkv + (size_t)s * P.qkv_stride + (head0 + g) * 64;
+        float a = 0.0f, b = 0.0f;
+        if (g < gc) a = qrow[lane], b = qrow[32 + lane];
+        if (FUSED) {
+            float cs = 1.0f, sn = 0.0f;
+            if (P.use_rope) {
+                mx::rope_angle(pos, lane, 64, P.theta, cs, sn);
+                mx::rope_pair(a, b, cs, sn);
+            }
+            qf[g * 64 + lane] = a, qf[g * 64 + 32 + lane] = b;
+            if (owner && warp < 2) {   // warp 0: the K head, warp 1: the V head -> the cache and the one-key tile
+                const float2 x = new_kv_pair(P, s, kvh, warp, lane, cs, sn);
+                int c0, c1;
+                float sc, be;
+                mx::quant_head_row(x.x, x.y, affine, c0, c1, sc, be);
+                const size_t row = P.write_row >= 0 ? (size_t)P.write_row
+                                                    : (PAGED ? (size_t)paged_row(P, table, pos) : (size_t)(base + pos));
+                int8_t *dst = (int8_t *)(warp ? P.vq : P.kq) + row * kvd + kvh * 64;
+                dst[lane] = (int8_t)c0, dst[lane + 32] = (int8_t)c1;
+                int8_t *tile = (int8_t *)extra + warp * WT_KEYS * 64;   // key 0: first 64 bytes of K, first line of V
+                tile[lane] = (int8_t)c0, tile[lane + 32] = (int8_t)c1;
+                float *side = (float *)(extra + 2 * WT_KEYS * 64) + warp * 64;
+                side[lane] = sc, side[32 + lane] = be;
+                if (lane == 0) {
+                    float *gsc = (float *)(warp ? P.vs : P.ks), *gbe = (float *)(warp ? P.vb : P.kb);
+                    gsc[row * nkv + kvh] = sc;
+                    if (affine) gbe[row * nkv + kvh] = be;
+                }
+            }
+        }
         float qmax = warp_max_f(fmaxf(fabsf(a), fabsf(b)));
         float qid = qmax > 0.0f ? __fdiv_rn(127.0f, qmax) : 0.0f;
         int ca = max(-127, min(127, __float2int_rn(a * qid)));
@@ -812,14 +1004,17 @@ decode_q8_mma_kernel(const DecodeParams P) {
     for (int t = 0; t < 8; ++t) oacc[t][0] = oacc[t][1] = oacc[t][2] = oacc[t][3] = 0.0f;
 
     const uint32_t MAGIC = 0x64646464u, BIAS = 0x64806480u;  // f16 1024 | byte, minus 1152
-    for (int tile = 0; tile < n_tiles; ++tile) {
+    // the last warp of the owning CTA (the one with the fewest keys) takes the new token's one-key tile at the end
+    const int n_loop = n_tiles + (FUSED && owner && warp == Q8_WARPS - 1 ? 1 : 0);
+    for (int tile = 0; tile < n_loop; ++tile) {
         if (tile + MMA_STAGES - 1 < n_tiles) issue(tile + MMA_STAGES - 1);
         cp_async_commit();
         cp_async_wait<MMA_STAGES - 1>();
         __syncwarp();
-        const unsigned char *st = ring + (tile % MMA_STAGES) * WT_STAGE;
+        const bool own_key = FUSED && tile == n_tiles;
+        const unsigned char *st = own_key ? extra : ring + (tile % MMA_STAGES) * WT_STAGE;
         const float *side = (const float *)(st + 2 * WT_KEYS * 64);
-        const int key_lim = wb - (wa + tile * WT_KEYS);  // valid keys in this tile
+        const int key_lim = own_key ? 1 : wb - (wa + tile * WT_KEYS);  // valid keys in this tile
 #pragma unroll
         for (int blk = 0; blk < 2; ++blk) {
             // ---- scores (log2 domain): two 8-key groups ----
@@ -919,47 +1114,7 @@ decode_q8_mma_kernel(const DecodeParams P) {
         }
     }
     __syncthreads();
-
-    const bool direct = (n_splits == 1) && (P.fin_acc == nullptr);
-    for (int i = tid; i < gc * 64; i += Q8_THREADS) {
-        const int gg = i >> 6, d = i & 63;
-        float mm = -CUDART_INF_F;
-#pragma unroll
-        for (int w = 0; w < Q8_WARPS; ++w) mm = fmaxf(mm, mg[(w * MG + gg) * 68]);
-        float lt = 0.0f, a = 0.0f;
-#pragma unroll
-        for (int w = 0; w < Q8_WARPS; ++w) {
-            const float *src = mg + (w * MG + gg) * 68;
-            const float wgt = (src[0] == -CUDART_INF_F) ? 0.0f : mx::ex2(src[0] - mm);
-            lt += src[1] * wgt;
-            a += (src[4 + d] + src[2]) * wgt;  // V's affine offset sum_j p_j vb_j folds into every dim
-        }
-        const int h = head0 + gg;
-        if (direct) {
-            P.out[(size_t)s * P.out_stride + h * 64 + d] = a / lt;
-        } else {
-            // partial triples carry the max in natural-log units, as the split-KV interface states
-            size_t pi = ((size_t)s * P.n_head + h) * n_splits + blockIdx.x;
-            P.ws_acc[pi * 64 + d] = a;
-            if (d == 0) {
-                P.ws_m[pi] = mm * 0.6931471805599453f;
-                P.ws_l[pi] = lt;
-            }
-        }
-    }
-    if (direct) return;
-
-    // ---- last CTA of this (sequence, kv head group) merges the splits ----
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) {
-        unsigned prev = atomicInc(&P.counters[(size_t)s * gridDim.y + blockIdx.y], n_splits - 1);
-        is_last = (prev == (unsigned)(n_splits - 1));
-    }
-    __syncthreads();
-    if (!is_last) return;
-    __threadfence();
-    merge_and_store<MG>(P, s, head0, gc, n_splits, Q8_THREADS);
+    finish_group<MG>(P, mg, Q8_WARPS, s, head0, gc, cl, rank, active, FUSED ? qf : nullptr, &is_last);
 }
 
 // ---------------------------------------------------------------------------
@@ -986,11 +1141,11 @@ struct F32Smem {
     static constexpr int Q_BYTES = G * 64 * 4;
     static constexpr int WBUF = FT_KEYS * GP * 4;
     static constexpr int PER_WARP = FT_STAGES * FT_STAGE + WBUF;
-    static constexpr int MERGE = F32_WARPS * G * 68 * 4;
+    static constexpr int MERGE = (F32_WARPS + 1) * G * 68 * 4;
     static constexpr int TOTAL = ((Q_BYTES + 127) & ~127) + (F32_WARPS * PER_WARP > MERGE ? F32_WARPS * PER_WARP : MERGE);
 };
 
-template <int G, bool PAGED>
+template <int G, bool PAGED, bool FUSED>
 __global__ void __launch_bounds__(F32_THREADS, 3)
 decode_f32_ring_kernel(const DecodeParams P) {
     using SM = F32Smem<G>;
@@ -999,6 +1154,7 @@ decode_f32_ring_kernel(const DecodeParams P) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     float *qf = (float *)smem_raw;                        // [G][64]
     unsigned char *warp_base = smem_raw + ((SM::Q_BYTES + 127) & ~127);
+    __shared__ float new_k[64], new_v[64];                // fused step: the new token's rows (owning CTA)
     __shared__ int is_last;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1007,19 +1163,20 @@ decode_f32_ring_kernel(const DecodeParams P) {
     const int hg = blockIdx.y - kvh * P.head_groups;
     const int head0 = kvh * P.group + hg * 8;
     const int gc = min(G, P.group - hg * 8);
-    const int n_splits = gridDim.x;
     const int nkv = P.n_kv_head, kvd = nkv * 64;
+    const int cl = blockIdx.x / P.cl_size, rank = blockIdx.x - cl * P.cl_size;
 
     int kbeg, kend, ka, kb_;
     key_range(P, s, kbeg, kend);
+    const int pos = kend - 1;                             // fused step: the new token's position
+    if (FUSED) kend = pos;
+    const int active = active_clusters(P, kend - kbeg);
+    if (cl >= active) return;
+    const int n_splits = active * P.cl_size;
     split_range(kbeg, kend, blockIdx.x, n_splits, ka, kb_);
     const int *table = PAGED ? P.tables + (P.pos_kind == 2 ? (size_t)s * P.n_log : 0) : nullptr;
     const long long base = PAGED ? 0 : (long long)s * P.seq_rows;
     const float scale = 0.125f * LOG2E;  // scores are kept in the log2 domain
-
-    const float *qrow = P.qkv + (size_t)s * P.qkv_stride + head0 * 64;
-    for (int i = tid; i < G * 64; i += F32_THREADS) qf[i] = (i / 64 < gc) ? qrow[i] : 0.0f;
-    __syncthreads();
 
     // ---- this warp's key sub-range ----
     const int n_keys = kb_ - ka;
@@ -1043,11 +1200,30 @@ decode_f32_ring_kernel(const DecodeParams P) {
         vsrc = P.vcache + (r0 + pk) * kvd + kvh * 64 + pc * 4;
     }
     const size_t it_stride = (size_t)2 * kvd, tile_stride = (size_t)FT_KEYS * kvd;
+    // paged caches: lane l looks up the row of key l (mod 16) of the next tile one tile ahead, as in the int8 kernel
+    auto row_ahead = [&](int tile) {
+        const int t = wa + tile * FT_KEYS + pc;
+        return paged_row(P, table, t < wb ? t : wa);
+    };
+    int row_l = 0;
+    if (PAGED && n_tiles > 0) row_l = row_ahead(0);
 
     auto issue = [&](int tile) {
         const uint32_t dst = ring_u32 + (tile % FT_STAGES) * FT_STAGE;
         const int key0 = wa + tile * FT_KEYS;
-        if (!PAGED && key0 + FT_KEYS <= wb) {  // full tile of a linear cache: no predicates, no lookups
+        if (PAGED) {
+#pragma unroll
+            for (int it = 0; it < 8; ++it) {
+                const int key = it * 2 + pk;
+                const size_t off = (size_t)__shfl_sync(0xFFFFFFFFu, row_l, key) * kvd + kvh * 64 + pc * 4;
+                const int n = key0 + key < wb ? 16 : 0;
+                cp_async16(dst + k_off(key), P.kcache + off, n);
+                cp_async16(dst + FT_KEYS * 256 + key * 256 + v_chunk, P.vcache + off, n);
+            }
+            if (tile + 1 < n_tiles) row_l = row_ahead(tile + 1);
+            return;
+        }
+        if (key0 + FT_KEYS <= wb) {  // full tile of a linear cache: no predicates
 #pragma unroll
             for (int it = 0; it < 8; ++it) {
                 const int key = it * 2 + pk;
@@ -1060,14 +1236,40 @@ decode_f32_ring_kernel(const DecodeParams P) {
                 const int key = it * 2 + pk;
                 const int t = key0 + key;
                 const bool ok = t < wb;
-                const size_t row = cache_row(P, table, base, ok ? t : wa);
-                cp_async16(dst + k_off(key), P.kcache + row * kvd + kvh * 64 + pc * 4, ok ? 16 : 0);
-                cp_async16(dst + FT_KEYS * 256 + key * 256 + v_chunk, P.vcache + row * kvd + kvh * 64 + pc * 4,
-                           ok ? 16 : 0);
+                const size_t off = (size_t)(base + (ok ? t : wa)) * kvd + kvh * 64 + pc * 4;
+                cp_async16(dst + k_off(key), P.kcache + off, ok ? 16 : 0);
+                cp_async16(dst + FT_KEYS * 256 + key * 256 + v_chunk, P.vcache + off, ok ? 16 : 0);
             }
         }
-        if (!PAGED) ksrc += tile_stride, vsrc += tile_stride;
+        ksrc += tile_stride, vsrc += tile_stride;
     };
+
+    // the first tile is requested before the q prologue, whose latency then runs under it
+    if (n_tiles > 0) issue(0);
+    cp_async_commit();
+
+    const bool owner = FUSED && (int)blockIdx.x == n_splits - 1;   // the CTA that takes the new token's own key
+    {
+        float cs = 1.0f, sn = 0.0f;
+        if (FUSED && P.use_rope) mx::rope_angle(pos, lane, 64, P.theta, cs, sn);
+        for (int g = warp; g < G; g += F32_WARPS) {
+            const float *qrow = P.qkv + (size_t)s * P.qkv_stride + (head0 + g) * 64;
+            float a = 0.0f, b = 0.0f;
+            if (g < gc) a = qrow[lane], b = qrow[32 + lane];
+            if (FUSED && P.use_rope) mx::rope_pair(a, b, cs, sn);
+            qf[g * 64 + lane] = a, qf[g * 64 + 32 + lane] = b;
+        }
+        if (owner && warp < 2) {   // warp 0: the K head, warp 1: the V head -> the cache and shared memory
+            const float2 x = new_kv_pair(P, s, kvh, warp, lane, cs, sn);
+            const size_t row = P.write_row >= 0 ? (size_t)P.write_row
+                                                : (PAGED ? (size_t)paged_row(P, table, pos) : (size_t)(base + pos));
+            float *dst = (float *)(warp ? P.vcache : P.kcache) + row * kvd + kvh * 64;
+            dst[lane] = x.x, dst[lane + 32] = x.y;
+            float *keep = warp ? new_v : new_k;
+            keep[lane] = x.x, keep[lane + 32] = x.y;
+        }
+    }
+    __syncthreads();
 
     float m_run[G], l_thr[G];
     float acc[G][8];
@@ -1079,8 +1281,6 @@ decode_f32_ring_kernel(const DecodeParams P) {
         for (int j = 0; j < 8; ++j) acc[g][j] = 0.0f;
     }
 
-    if (n_tiles > 0) issue(0);
-    cp_async_commit();
     const int sk = lane & 15, sh = lane >> 4;          // scores: key, dim half
     const int kl = lane >> 3, dsl = lane & 7;          // values: key lane, 8-dim slice
     const uint32_t vo0 = (uint32_t)(((2 * dsl) ^ ((2 * dsl) >> 3)) << 4);
@@ -1162,6 +1362,21 @@ decode_f32_ring_kernel(const DecodeParams P) {
     }
     cp_async_wait<0>();
 
+    // ---- fused step: the new token's own key, by the owning CTA's last warp (the one with the fewest keys) ----
+    if (FUSED && owner && warp == F32_WARPS - 1) {
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            const float sg = warp_sum_f(fmaf(qf[g * 64 + lane], new_k[lane], qf[g * 64 + 32 + lane] * new_k[lane + 32])) * scale;
+            const float m_new = fmaxf(m_run[g], sg);
+            const float alpha = (m_run[g] == -CUDART_INF_F) ? 0.0f : mx::ex2(m_run[g] - m_new);
+            const float p = mx::ex2(sg - m_new);
+            m_run[g] = m_new;
+            l_thr[g] = l_thr[g] * alpha + (lane == 0 ? p : 0.0f);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) acc[g][j] = acc[g][j] * alpha + (kl == 0 ? p * new_v[dsl * 8 + j] : 0.0f);
+        }
+    }
+
     // ---- warp totals, then the CTA-level log-sum-exp merge of the warps ----
 #pragma unroll
     for (int g = 0; g < G; ++g) {
@@ -1175,13 +1390,14 @@ decode_f32_ring_kernel(const DecodeParams P) {
         }
     }
     __syncthreads();  // every warp is done with its ring: reuse the memory for the merge
-    float *mg = (float *)warp_base;  // [warp][g][68]: m (log2 domain), l, pad, pad, acc[64]
+    float *mg = (float *)warp_base;  // [warp][g][68]: m (log2 domain), l, 0, pad, acc[64]
 #pragma unroll
     for (int g = 0; g < G; ++g) {
         float *dst = mg + (warp * G + g) * 68;
         if (lane == 0) {
             dst[0] = m_run[g];
             dst[1] = l_thr[g];
+            dst[2] = 0.0f;
         }
         if (lane < 8) {
             *(float4 *)(dst + 4 + lane * 8) = make_float4(acc[g][0], acc[g][1], acc[g][2], acc[g][3]);
@@ -1189,47 +1405,7 @@ decode_f32_ring_kernel(const DecodeParams P) {
         }
     }
     __syncthreads();
-
-    const bool direct = (n_splits == 1) && (P.fin_acc == nullptr);
-    for (int i = tid; i < gc * 64; i += F32_THREADS) {
-        const int g = i >> 6, d = i & 63;
-        float mm = -CUDART_INF_F;
-#pragma unroll
-        for (int w = 0; w < F32_WARPS; ++w) mm = fmaxf(mm, mg[(w * G + g) * 68]);
-        float lt = 0.0f, a = 0.0f;
-#pragma unroll
-        for (int w = 0; w < F32_WARPS; ++w) {
-            const float *src = mg + (w * G + g) * 68;
-            const float wgt = (src[0] == -CUDART_INF_F) ? 0.0f : mx::ex2(src[0] - mm);
-            lt += src[1] * wgt;
-            a += src[4 + d] * wgt;
-        }
-        const int h = head0 + g;
-        if (direct) {
-            P.out[(size_t)s * P.out_stride + h * 64 + d] = a / lt;
-        } else {
-            // partial triples carry the max in natural-log units, as the split-KV interface states
-            size_t pi = ((size_t)s * P.n_head + h) * n_splits + blockIdx.x;
-            P.ws_acc[pi * 64 + d] = a;
-            if (d == 0) {
-                P.ws_m[pi] = mm * 0.6931471805599453f;
-                P.ws_l[pi] = lt;
-            }
-        }
-    }
-    if (direct) return;
-
-    // ---- last CTA of this (sequence, kv head group) merges the splits ----
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) {
-        unsigned prev = atomicInc(&P.counters[(size_t)s * gridDim.y + blockIdx.y], n_splits - 1);
-        is_last = (prev == (unsigned)(n_splits - 1));
-    }
-    __syncthreads();
-    if (!is_last) return;
-    __threadfence();
-    merge_and_store<G>(P, s, head0, gc, n_splits, F32_THREADS);
+    finish_group<G>(P, mg, F32_WARPS, s, head0, gc, cl, rank, active, FUSED ? qf : nullptr, &is_last);
 }
 
 // Log-sum-exp merge of gathered partial triples: one thread per (row, 4 dims).
@@ -1261,20 +1437,54 @@ size_t q8_smem_bytes() {
     return (size_t)Q8Smem<G>::TOTAL;
 }
 
+// Kernel launch with the cluster size as a launch attribute.
+template <typename... KArgs, typename... Args>
+cudaError_t launch_clusters(void (*kernel)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t st, int cl_size,
+                            Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = cl_size, at[0].val.clusterDim.y = 1, at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = cl_size > 1 ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+template <bool PAGED, bool FUSED>
+int launch_q8_mma(mx230_handle *h, cudaStream_t st, const DecodeParams &P, dim3 grid) {
+    const size_t sm = (size_t)Q8MmaSmem::TOTAL;
+    MX_SMEM_ATTR_ONCE(h->device, (decode_q8_mma_kernel<PAGED, FUSED>), sm);
+    MX_LAUNCH(h, st, MX230_K_DECODE_Q8,
+              launch_clusters(decode_q8_mma_kernel<PAGED, FUSED>, grid, Q8_THREADS, sm, st, P.cl_size, P));
+    return MX230_OK;
+}
+template <int G, bool PAGED, bool FUSED>
+int launch_f32(mx230_handle *h, cudaStream_t st, const DecodeParams &P, dim3 grid) {
+    const size_t sm = (size_t)F32Smem<G>::TOTAL;
+    MX_SMEM_ATTR_ONCE(h->device, (decode_f32_ring_kernel<G, PAGED, FUSED>), sm);
+    MX_LAUNCH(h, st, MX230_K_DECODE_F32,
+              launch_clusters(decode_f32_ring_kernel<G, PAGED, FUSED>, grid, F32_THREADS, sm, st, P.cl_size, P));
+    return MX230_OK;
+}
+
+// int8 cache in the reference score mode: the tensor-core kernel serves any group size up to 8 per CTA
+bool uses_q8_mma(const mx230_handle *h, const DecodeParams &P) {
+    return P.kq != nullptr && P.score_mode == MX230_Q8_SCORE_REF && h->decode_tensor;
+}
+
 template <int G>
-int launch_g(mx230_handle *h, cudaStream_t st, const DecodeParams &P, dim3 grid, bool q8) {
-    if (q8 && P.score_mode == MX230_Q8_SCORE_REF && h->decode_tensor) {
-        // reference score mode: the tensor-core kernel serves any group size up to 8 per CTA
-        size_t sm = (size_t)Q8MmaSmem::TOTAL;
-        if (P.tables) {
-            MX_SMEM_ATTR_ONCE(h->device, (decode_q8_mma_kernel<true>), sm);
-            MX_LAUNCH(h, st, MX230_K_DECODE_Q8, (decode_q8_mma_kernel<true><<<grid, Q8_THREADS, sm, st>>>(P)));
-        } else {
-            MX_SMEM_ATTR_ONCE(h->device, (decode_q8_mma_kernel<false>), sm);
-            MX_LAUNCH(h, st, MX230_K_DECODE_Q8, (decode_q8_mma_kernel<false><<<grid, Q8_THREADS, sm, st>>>(P)));
-        }
-    } else if (q8) {
-        size_t sm = q8_smem_bytes<G>();
+int launch_g(mx230_handle *h, cudaStream_t st, const DecodeParams &P, dim3 grid) {
+    const bool fused = P.qkv_rw != nullptr;
+    if (uses_q8_mma(h, P)) {
+        if (P.tables) return fused ? launch_q8_mma<true, true>(h, st, P, grid) : launch_q8_mma<true, false>(h, st, P, grid);
+        return fused ? launch_q8_mma<false, true>(h, st, P, grid) : launch_q8_mma<false, false>(h, st, P, grid);
+    }
+    if (P.kq) {
+        const size_t sm = q8_smem_bytes<G>();
         if (P.tables) {
             MX_SMEM_ATTR_ONCE(h->device, (decode_q8_kernel<G, true>), sm);
             MX_LAUNCH(h, st, MX230_K_DECODE_Q8, (decode_q8_kernel<G, true><<<grid, Q8_THREADS, sm, st>>>(P)));
@@ -1282,17 +1492,41 @@ int launch_g(mx230_handle *h, cudaStream_t st, const DecodeParams &P, dim3 grid,
             MX_SMEM_ATTR_ONCE(h->device, (decode_q8_kernel<G, false>), sm);
             MX_LAUNCH(h, st, MX230_K_DECODE_Q8, (decode_q8_kernel<G, false><<<grid, Q8_THREADS, sm, st>>>(P)));
         }
-    } else {
-        size_t sm = (size_t)F32Smem<G>::TOTAL;
-        if (P.tables) {
-            MX_SMEM_ATTR_ONCE(h->device, (decode_f32_ring_kernel<G, true>), sm);
-            MX_LAUNCH(h, st, MX230_K_DECODE_F32, (decode_f32_ring_kernel<G, true><<<grid, F32_THREADS, sm, st>>>(P)));
-        } else {
-            MX_SMEM_ATTR_ONCE(h->device, (decode_f32_ring_kernel<G, false>), sm);
-            MX_LAUNCH(h, st, MX230_K_DECODE_F32, (decode_f32_ring_kernel<G, false><<<grid, F32_THREADS, sm, st>>>(P)));
-        }
+        return MX230_OK;
     }
-    return MX230_OK;
+    if (P.tables) return fused ? launch_f32<G, true, true>(h, st, P, grid) : launch_f32<G, true, false>(h, st, P, grid);
+    return fused ? launch_f32<G, false, true>(h, st, P, grid) : launch_f32<G, false, false>(h, st, P, grid);
+}
+
+// How a group's keys are split over CTAs.  slots: CTAs of the kernel that are resident at once; groups: (sequence, K/V
+// head group) pairs; keys: largest number of keys of a sequence, 0 = unknown (position on the device).
+//  * whole grid resident at once: cl_size * max_clusters * groups <= slots (a partial second wave would nearly double
+//    the time);
+//  * up to 8 CTAs of a group form a cluster, whose merge costs one cluster barrier; pass_keys = keys that a CTA's warps
+//    take in one tile each: a CTA is not given less than one such pass;
+//  * further clusters join in (merge through global memory, about 2 us) only for sequences with more than 4 passes per
+//    CTA of the first; the kernel decides that per sequence from its actual length;
+//  * ranges of many tiles per CTA use clusters of one: any number of splits then fits the machine (9 per group fill
+//    296 slots where 8 would leave a tenth of them empty), and the merge is small against the stream.
+void plan_splits(DecodeParams &P, long long slots, long long groups, long long keys, int pass_keys) {
+    long long want = slots / groups;
+    if (want < 1) want = 1;
+    if (want > 256) want = 256;
+    const bool known = keys > 0;
+    if (known && keys / want >= 8LL * pass_keys) {
+        P.cl_size = 1;
+        P.max_clusters = (int)want;
+        P.cluster_keys = pass_keys;
+        return;
+    }
+    int c = 1;
+    while (c < 8 && 2 * c <= want && (!known || (long long)c * pass_keys < keys)) c *= 2;
+    P.cl_size = c;
+    P.cluster_keys = 4 * c * pass_keys;
+    long long k = want / c;
+    if (known && k > (keys + P.cluster_keys - 1) / P.cluster_keys) k = (keys + P.cluster_keys - 1) / P.cluster_keys;
+    if (!known && k > 4) k = 4;
+    P.max_clusters = (int)(k < 1 ? 1 : k);
 }
 
 // `known_keys`: host-known upper bound of keys per sequence (<= 0 when the position
@@ -1333,10 +1567,7 @@ int launch_decode(mx230_handle *h, void *stream, DecodeParams P, int n_seq, int 
     MX_REQUIRE((size_t)n_seq * gy <= h->n_counters, MX230_ERR_UNSUPPORTED,
                "attn_decode: n_seq*n_kv_head %lld exceeds %zu", (long long)n_seq * gy, h->n_counters);
 
-    // how many key splits: fill the machine (2 resident CTAs per SM for the int8 kernel, 3 for
-    // the fp32 one) but keep >= 256 keys each
-    // (rounded down so that the whole grid is resident at once: a partial second wave would
-    // nearly double the time)
+    // how many key splits: fill the machine (2 resident CTAs per SM for the int8 kernels, 3 for the fp32 one)
     long long base_ctas = (long long)n_seq * gy;
     // One-kernel split-KV step: the CTA that finishes a group waits there for the other ranks.  At most one CTA per
     // group ever waits, so with fewer groups than SMs a slot always stays free for the CTAs that still have keys to
@@ -1344,21 +1575,24 @@ int launch_decode(mx230_handle *h, void *stream, DecodeParams P, int n_seq, int 
     // groups the wait moves into a kernel of its own behind this one.
     float *merge_after = nullptr;
     if (P.push_out && base_ctas >= h->sm_count) merge_after = P.push_out, P.push_out = nullptr;
-    int want = (int)(((q8 ? 2LL : 3LL) * h->sm_count) / base_ctas);
-    int n_splits;
-    if (h->decode_chunk > 0 && known_keys > 0) {
-        n_splits = (int)((known_keys + h->decode_chunk - 1) / h->decode_chunk);
+    const bool mma = uses_q8_mma(h, P);
+    const long long slots = (q8 ? 2LL : 3LL) * h->sm_count;
+    if (h->decode_chunk > 0 && known_keys > 0) {   // fixed chunks: the split depends on the capacity alone
+        P.cl_size = 1, P.cluster_keys = 0;
+        P.max_clusters = (int)((known_keys + h->decode_chunk - 1) / h->decode_chunk);
+        if (P.max_clusters > 256) P.max_clusters = 256;
+    } else if ((q8 && !mma) || P.range_mode) {
+        // the CUDA-core int8 kernel splits by the grid; the forms of a split-KV step all split alike (they agree bit for
+        // bit), and the one that waits for peers must not hold a cluster
+        const long long keys = known_keys > 0 ? known_keys : 4096;
+        long long n = slots / base_ctas, by_len = (keys + 255) / 256;
+        if (n > by_len) n = by_len;
+        P.cl_size = 1, P.cluster_keys = 0;
+        P.max_clusters = (int)(n < 1 ? 1 : n > 256 ? 256 : n);
     } else {
-        long long keys = known_keys > 0 ? known_keys : 4096;
-        int max_by_len = (int)((keys + 255) / 256);
-        n_splits = want < 1 ? 1 : want;
-        if (n_splits > max_by_len) n_splits = max_by_len;
-        // a second split is not worth its merge pass when one CTA per (sequence, kv head) already
-        // covers most of the SMs and the contexts are short (measured: batch 64 x 2048 keys, 19.7 vs 22.3 us)
-        if (n_splits == 2 && base_ctas * 5 >= (long long)h->sm_count * 4 && keys <= 4096) n_splits = 1;
+        plan_splits(P, slots, base_ctas, known_keys, mma ? Q8_WARPS * WT_KEYS : F32_WARPS * FT_KEYS);
     }
-    if (n_splits < 1) n_splits = 1;
-    if (n_splits > 256) n_splits = 256;
+    const int n_splits = P.max_clusters;   // partial triples per row in the workspace
     if (n_splits > 1 || P.fin_acc) {
         size_t need = (size_t)n_seq * P.n_head * n_splits * 66 * sizeof(float);
         MX_REQUIRE(h->ws && need <= h->ws_bytes, MX230_ERR_WORKSPACE,
@@ -1373,15 +1607,16 @@ int launch_decode(mx230_handle *h, void *stream, DecodeParams P, int n_seq, int 
     P.counters = h->counters;
 
     mx230_device_guard guard(h->device);
-    dim3 grid(n_splits, gy, n_seq);
+    dim3 grid(P.cl_size * P.max_clusters, gy, n_seq);
     cudaStream_t st = (cudaStream_t)stream;
+    P.bs_shift = P.tables && (P.bs & (P.bs - 1)) == 0 ? __builtin_ctz((unsigned)P.bs) : -1;
     int g = P.group > 8 ? 8 : P.group;
     int rc;
-    if (g == 1) rc = launch_g<1>(h, st, P, grid, q8);
-    else if (g == 2) rc = launch_g<2>(h, st, P, grid, q8);
-    else if (g <= 4) rc = launch_g<4>(h, st, P, grid, q8);
-    else if (g <= 7) rc = launch_g<7>(h, st, P, grid, q8);
-    else rc = launch_g<8>(h, st, P, grid, q8);
+    if (g == 1) rc = launch_g<1>(h, st, P, grid);
+    else if (g == 2) rc = launch_g<2>(h, st, P, grid);
+    else if (g <= 4) rc = launch_g<4>(h, st, P, grid);
+    else if (g <= 7) rc = launch_g<7>(h, st, P, grid);
+    else rc = launch_g<8>(h, st, P, grid);
     if (rc == MX230_OK && merge_after) rc = mx230_splitkv_wait_merge(comm, stream, merge_after);
     return rc;
 }
@@ -1510,6 +1745,81 @@ extern "C" int mx230_attn_decode_q8_batched(mx230_handle *h, void *stream, float
     set_q8(P, Q8_ARGS);
     P.pos_kind = 2, P.pos_dev = pos, P.tables = tables, P.bs = block_size, P.n_log = n_log;
     return launch_decode(h, stream, P, n_seq, head_dim, (long long)n_log * block_size);
+}
+
+// ---- the whole step of one token: RoPE, KV write and attention in one launch ----
+// Group sizes above 8 (several CTAs would rotate and write the same K row) and the CUDA-core int8 kernel take the three
+// launches of the separate entry points.
+static bool step_is_fused(const mx230_handle *h, const int8_t *kq, int n_head, int n_kv_head) {
+    return n_kv_head > 0 && n_head / n_kv_head <= 8 &&
+           (kq == nullptr || (h->decode_tensor && h->q8_score_mode == MX230_Q8_SCORE_REF));
+}
+
+extern "C" int mx230_decode_step(mx230_handle *h, void *stream, float *out, float *qkv, float *kcache, float *vcache,
+                                 int8_t *kq, int8_t *vq, float *ks, float *vs, float *kb, float *vb, int pos,
+                                 const int *pos_ptr, int write_row, int n_head, int n_kv_head, int head_dim, int use_rope,
+                                 float theta, const int *bt, int bs) {
+    MX_REQUIRE(h && qkv, MX230_ERR_INVALID_ARG, "decode_step: null argument");
+    MX_REQUIRE(pos_ptr || pos >= 0, MX230_ERR_INVALID_ARG, "decode_step: negative position %d", pos);
+    if (step_is_fused(h, kq, n_head, n_kv_head)) {
+        DecodeParams P = base_params(out, n_head * 64, qkv, 0, n_head, n_kv_head);
+        P.kcache = kcache, P.vcache = vcache;
+        set_q8(P, Q8_ARGS);
+        P.pos_kind = pos_ptr ? 1 : 0, P.pos = pos, P.pos_dev = pos_ptr, P.tables = bt, P.bs = bs;
+        P.qkv_rw = qkv, P.use_rope = use_rope, P.theta = theta, P.write_row = pos_ptr ? -1 : write_row;
+        return launch_decode(h, stream, P, 1, head_dim, pos_ptr ? 0 : (pos > 0 ? pos : 1));
+    }
+    const int q_dim = n_head * head_dim, kv_dim = n_kv_head * head_dim;
+    int rc = MX230_OK;
+    if (pos_ptr) {
+        if (use_rope) rc = mx230_rope_dyn(h, stream, qkv, pos_ptr, n_head, n_kv_head, head_dim, theta);
+        if (rc) return rc;
+        if (kq) rc = bt ? mx230_quantize_kv_paged_dyn(h, stream, Q8_ARGS, qkv, pos_ptr, q_dim, n_kv_head, head_dim, bt, bs)
+                        : mx230_quantize_kv_dyn(h, stream, Q8_ARGS, qkv, pos_ptr, q_dim, n_kv_head, head_dim);
+        else rc = bt ? mx230_copy_kv_paged_dyn(h, stream, kcache, vcache, qkv, pos_ptr, q_dim, kv_dim, bt, bs)
+                     : mx230_copy_kv_dyn(h, stream, kcache, vcache, qkv, pos_ptr, q_dim, kv_dim);
+        if (rc) return rc;
+        if (kq) return bt ? mx230_attn_decode_q8_paged_dyn(h, stream, out, qkv, Q8_ARGS, pos_ptr, n_head, n_kv_head, head_dim, bt, bs)
+                          : mx230_attn_decode_q8_dyn(h, stream, out, qkv, Q8_ARGS, pos_ptr, n_head, n_kv_head, head_dim);
+        return bt ? mx230_attn_decode_paged_dyn(h, stream, out, qkv, kcache, vcache, pos_ptr, n_head, n_kv_head, head_dim, bt, bs)
+                  : mx230_attn_decode_dyn(h, stream, out, qkv, kcache, vcache, pos_ptr, n_head, n_kv_head, head_dim);
+    }
+    if (use_rope) rc = mx230_rope(h, stream, qkv, pos, n_head, n_kv_head, head_dim, theta);
+    if (rc) return rc;
+    rc = kq ? mx230_quantize_kv(h, stream, Q8_ARGS, qkv, write_row, q_dim, n_kv_head, head_dim)
+            : mx230_copy_kv(h, stream, kcache, vcache, qkv, write_row, q_dim, kv_dim);
+    if (rc) return rc;
+    if (kq) return bt ? mx230_attn_decode_q8_paged(h, stream, out, qkv, Q8_ARGS, pos, n_head, n_kv_head, head_dim, bt, bs)
+                      : mx230_attn_decode_q8(h, stream, out, qkv, Q8_ARGS, pos, n_head, n_kv_head, head_dim);
+    return bt ? mx230_attn_decode_paged(h, stream, out, qkv, kcache, vcache, pos, n_head, n_kv_head, head_dim, bt, bs)
+              : mx230_attn_decode(h, stream, out, qkv, kcache, vcache, pos, n_head, n_kv_head, head_dim);
+}
+
+extern "C" int mx230_batched_step(mx230_handle *h, void *stream, float *out, float *qkv, float *kcache, float *vcache,
+                                  int8_t *kq, int8_t *vq, float *ks, float *vs, float *kb, float *vb, const int *pos,
+                                  int n_seq, int n_head, int n_kv_head, int head_dim, int use_rope, float theta,
+                                  const int *tables, int block_size, int n_log, int qkv_stride, int out_stride) {
+    MX_REQUIRE(h && qkv && pos && tables, MX230_ERR_INVALID_ARG, "batched_step: null argument");
+    MX_REQUIRE(block_size > 0 && n_log > 0, MX230_ERR_INVALID_ARG, "batched_step: bad table");
+    if (step_is_fused(h, kq, n_head, n_kv_head)) {
+        DecodeParams P = base_params(out, out_stride, qkv, qkv_stride, n_head, n_kv_head);
+        P.kcache = kcache, P.vcache = vcache;
+        set_q8(P, Q8_ARGS);
+        P.pos_kind = 2, P.pos_dev = pos, P.tables = tables, P.bs = block_size, P.n_log = n_log;
+        P.qkv_rw = qkv, P.use_rope = use_rope, P.theta = theta, P.write_row = -1;
+        return launch_decode(h, stream, P, n_seq, head_dim, (long long)n_log * block_size);
+    }
+    const int q_dim = n_head * head_dim, kv_dim = n_kv_head * head_dim;
+    int rc = use_rope ? mx230_rope_seqpos(h, stream, qkv, pos, n_seq, n_head, n_kv_head, head_dim, qkv_stride, theta) : MX230_OK;
+    if (rc) return rc;
+    rc = kq ? mx230_quantize_kv_seqpos(h, stream, Q8_ARGS, qkv, pos, n_seq, q_dim, n_kv_head, head_dim, qkv_stride, tables,
+                                       block_size, n_log)
+            : mx230_copy_kv_seqpos(h, stream, kcache, vcache, qkv, pos, n_seq, q_dim, kv_dim, qkv_stride, tables, block_size, n_log);
+    if (rc) return rc;
+    return kq ? mx230_attn_decode_q8_batched(h, stream, out, qkv, Q8_ARGS, pos, n_seq, n_head, n_kv_head, head_dim, tables,
+                                             block_size, n_log, qkv_stride, out_stride)
+              : mx230_attn_decode_batched(h, stream, out, qkv, kcache, vcache, pos, n_seq, n_head, n_kv_head, head_dim, tables,
+                                          block_size, n_log, qkv_stride, out_stride);
 }
 
 // ---- contiguous per-sequence slabs, and split-KV partials ----

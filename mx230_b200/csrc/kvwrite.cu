@@ -48,14 +48,12 @@ __global__ void rope_kernel(float *qkv, RowPos rp, int n_rows, int n_head, int n
     int h = i / half;
     int d = i - h * half;
     float *base = qkv + (size_t)r * stride + h * head_dim;
-    // precise powf / sincosf: the reference's CPU path (03-llm-engine/src/cpu.rs:25-37);
-    // its GPU kernel uses the fast intrinsics, which lose accuracy at large angles
-    float freq = powf(theta, -2.0f * (float)d / (float)head_dim);
-    float sn, cs;
-    sincosf((float)row_position(rp, r) * freq, &sn, &cs);
+    float cs, sn;
+    mx::rope_angle(row_position(rp, r), d, head_dim, theta, cs, sn);
     float x1 = base[d], x2 = base[d + half];
-    base[d] = x1 * cs - x2 * sn;
-    base[d + half] = x1 * sn + x2 * cs;
+    mx::rope_pair(x1, x2, cs, sn);
+    base[d] = x1;
+    base[d + half] = x2;
 }
 
 __global__ void copy_kv_kernel(float *kcache, float *vcache, const float *qkv, RowPos rp,
@@ -69,14 +67,8 @@ __global__ void copy_kv_kernel(float *kcache, float *vcache, const float *qkv, R
     *(float4 *)(vcache + row + i) = *(const float4 *)(src + kv_dim + i);
 }
 
-__device__ __forceinline__ float warp_max(float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
-    return v;
-}
-
 // One warp quantises one 64-value head row (K or V) of one qkv row: lane l owns
-// elements 2l, 2l+1.  IEEE division and round-to-nearest-even exactly as quant_affine.
+// elements 2l, 2l+1.
 __global__ void quantize_kv_kernel(int8_t *kq, int8_t *vq, float *ks, float *vs, float *kb,
                                    float *vb, const float *qkv, RowPos rp, int n_rows, int q_dim,
                                    int n_kv_head, int stride) {
@@ -96,23 +88,11 @@ __global__ void quantize_kv_kernel(int8_t *kq, int8_t *vq, float *ks, float *vs,
     float *be = which ? vb : kb;
     size_t sd = pr * n_kv_head + h;
     int c0, c1;
-    if (be != nullptr) {
-        float hi = warp_max(fmaxf(x.x, x.y));
-        float lo = -warp_max(fmaxf(-x.x, -x.y));
-        float scale = (hi > lo) ? __fdiv_rn(hi - lo, 255.0f) : 1.0f;
-        float beta = __fmaf_rn(128.0f, scale, lo);  // exact: 128*scale is a power-of-two scaling
-        c0 = max(-128, min(127, __float2int_rn(__fdiv_rn(x.x - beta, scale))));
-        c1 = max(-128, min(127, __float2int_rn(__fdiv_rn(x.y - beta, scale))));
-        if (lane == 0) {
-            sc[sd] = scale;
-            be[sd] = beta;
-        }
-    } else {
-        float amax = warp_max(fmaxf(fabsf(x.x), fabsf(x.y)));
-        float id = amax > 0.0f ? __fdiv_rn(127.0f, amax) : 0.0f;
-        c0 = max(-127, min(127, __float2int_rn(x.x * id)));
-        c1 = max(-127, min(127, __float2int_rn(x.y * id)));
-        if (lane == 0) sc[sd] = amax > 0.0f ? __fdiv_rn(amax, 127.0f) : 0.0f;
+    float scale, beta;
+    mx::quant_head_row(x.x, x.y, be != nullptr, c0, c1, scale, beta);
+    if (lane == 0) {
+        sc[sd] = scale;
+        if (be != nullptr) be[sd] = beta;
     }
     unsigned short packed = (unsigned short)((c0 & 0xFF) | ((c1 & 0xFF) << 8));
     *(unsigned short *)(dst + 2 * lane) = packed;

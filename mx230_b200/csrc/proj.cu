@@ -65,12 +65,6 @@ __device__ __forceinline__ float4 load_w4(const __half *w, size_t idx) {
     return make_float4(a.x, a.y, c.x, c.y);
 }
 
-__device__ __forceinline__ float wmax(float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
-    return v;
-}
-
 template <typename WT>
 __global__ void __launch_bounds__(PJ_THREADS)
 gemv_heads_kernel(const GemvParams P) {
@@ -183,13 +177,9 @@ gemv_heads_kernel(const GemvParams P) {
     const bool is_v = hb >= E.n_head + E.n_kv_head;
     if (tid < 32) {   // one warp: lane l owns the rotation pair (l, l + 32), then elements 2l, 2l+1
         if (!is_v) {
-            // HF rotate_half RoPE with precise powf / sincosf (the reference's CPU semantics, cpu.rs:25-37)
-            const float freq = powf(E.theta, -2.0f * (float)tid / 64.0f);
-            float sn, cs;
-            sincosf((float)pos * freq, &sn, &cs);
-            const float x1 = val[tid], x2 = val[tid + 32];
-            val[tid] = x1 * cs - x2 * sn;
-            val[tid + 32] = x1 * sn + x2 * cs;
+            float cs, sn;
+            mx::rope_angle(pos, tid, 64, E.theta, cs, sn);
+            mx::rope_pair(val[tid], val[tid + 32], cs, sn);
         }
         __syncwarp();
         const float2 xv = make_float2(val[2 * tid], val[2 * tid + 1]);
@@ -206,20 +196,11 @@ gemv_heads_kernel(const GemvParams P) {
                 float *sc = is_v ? E.vs : E.ks, *be = is_v ? E.vb : E.kb;
                 const size_t sd = row * E.n_kv_head + kvh;
                 int c0, c1;
-                if (be != nullptr) {   // affine, IEEE division and round-to-nearest-even as quant_affine
-                    const float hi = wmax(fmaxf(xv.x, xv.y));
-                    const float lo = -wmax(fmaxf(-xv.x, -xv.y));
-                    const float scale = (hi > lo) ? __fdiv_rn(hi - lo, 255.0f) : 1.0f;
-                    const float beta = __fmaf_rn(128.0f, scale, lo);
-                    c0 = max(-128, min(127, __float2int_rn(__fdiv_rn(xv.x - beta, scale))));
-                    c1 = max(-128, min(127, __float2int_rn(__fdiv_rn(xv.y - beta, scale))));
-                    if (tid == 0) sc[sd] = scale, be[sd] = beta;
-                } else {               // symmetric absmax
-                    const float amax = wmax(fmaxf(fabsf(xv.x), fabsf(xv.y)));
-                    const float id = amax > 0.0f ? __fdiv_rn(127.0f, amax) : 0.0f;
-                    c0 = max(-127, min(127, __float2int_rn(xv.x * id)));
-                    c1 = max(-127, min(127, __float2int_rn(xv.y * id)));
-                    if (tid == 0) sc[sd] = amax > 0.0f ? __fdiv_rn(amax, 127.0f) : 0.0f;
+                float scale, beta;
+                mx::quant_head_row(xv.x, xv.y, be != nullptr, c0, c1, scale, beta);
+                if (tid == 0) {
+                    sc[sd] = scale;
+                    if (be != nullptr) be[sd] = beta;
                 }
                 *(unsigned short *)(dst + 2 * tid) = (unsigned short)((c0 & 0xFF) | ((c1 & 0xFF) << 8));
             }

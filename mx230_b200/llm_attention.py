@@ -214,6 +214,10 @@ def _cache_args(c: KvCache):
     return (ptr(c.k), ptr(c.v), None, None, None, None, None, None)
 
 
+def _table_args(pg: Paging | None):
+    return (None, 0) if pg is None else (ptr(pg.table_dev), pg.block_size)
+
+
 def attn_decode_slab(h: Handle, out, qkv, c: KvCache, pos, n_seq, n_head, n_kv_head, head_dim,
                      seq_rows, qkv_stride, out_stride, stream=None):
     """Batched decode over contiguous per-sequence cache slabs of `seq_rows` rows."""
@@ -260,49 +264,25 @@ def merge_partials_packed(h: Handle, out, gathered, parts, rows, head_dim=64, st
 def decode_step(h: Handle, out, qkv, c: KvCache, pos: int, n_head, n_kv_head, head_dim, theta,
                 pg: Paging | None = None, host_table=None, use_rope=True, stream=None):
     """One token of one sequence, as forward_layers does per layer (gpu.rs:2570-2672):
-    RoPE, KV write at the host-resolved physical row, then attention over 0..=pos."""
-    q_dim, kv_dim = n_head * head_dim, n_kv_head * head_dim
-    if use_rope:
-        rope(h, qkv, pos, n_head, n_kv_head, head_dim, theta, stream)
+    RoPE, KV write at the host-resolved physical row, then attention over 0..=pos -- one launch."""
     phys = pos if pg is None else pg.phys_row(host_table, pos)
-    if c.quant:
-        quantize_kv(h, c, qkv, phys, q_dim, n_kv_head, head_dim, stream)
-    else:
-        copy_kv(h, c, qkv, phys, q_dim, kv_dim, stream)
-    attn_decode(h, out, qkv, c, pos, n_head, n_kv_head, head_dim, pg, stream)
+    check(lib().mx230_decode_step(h._h, stream_ptr(stream), ptr(out), ptr(qkv), *_cache_args(c), pos, None, phys, n_head,
+                                  n_kv_head, head_dim, int(use_rope), theta, *_table_args(pg)))
 
 
 def decode_step_dyn(h: Handle, out, qkv, c: KvCache, pos_ptr, n_head, n_kv_head, head_dim, theta,
                     pg: Paging | None = None, use_rope=True, stream=None):
     """The graph-capturable step of forward_body_dyn (gpu.rs:2808-2918)."""
-    q_dim, kv_dim = n_head * head_dim, n_kv_head * head_dim
-    if use_rope:
-        rope_dyn(h, qkv, pos_ptr, n_head, n_kv_head, head_dim, theta, stream)
-    if c.quant:
-        if pg is None:
-            quantize_kv_dyn(h, c, qkv, pos_ptr, q_dim, n_kv_head, head_dim, stream)
-        else:
-            quantize_kv_paged_dyn(h, c, qkv, pos_ptr, q_dim, n_kv_head, head_dim, pg, stream)
-    else:
-        if pg is None:
-            copy_kv_dyn(h, c, qkv, pos_ptr, q_dim, kv_dim, stream)
-        else:
-            copy_kv_paged_dyn(h, c, qkv, pos_ptr, q_dim, kv_dim, pg, stream)
-    attn_decode_dyn(h, out, qkv, c, pos_ptr, n_head, n_kv_head, head_dim, pg, stream)
+    check(lib().mx230_decode_step(h._h, stream_ptr(stream), ptr(out), ptr(qkv), *_cache_args(c), 0, ptr(pos_ptr), 0, n_head,
+                                  n_kv_head, head_dim, int(use_rope), theta, *_table_args(pg)))
 
 
 def batched_step(h: Handle, out, qkv, c: KvCache, pos, n_seq, n_head, n_kv_head, head_dim, theta,
                  pg: Paging, qkv_stride, out_stride, use_rope=True, stream=None):
     """One token for each of n_seq sequences, as forward_batched (gpu.rs:3530-3628)."""
-    q_dim, kv_dim = n_head * head_dim, n_kv_head * head_dim
-    if use_rope:
-        rope_seqpos(h, qkv, pos, n_seq, n_head, n_kv_head, head_dim, qkv_stride, theta, stream)
-    if c.quant:
-        quantize_kv_seqpos(h, c, qkv, pos, n_seq, q_dim, n_kv_head, head_dim, qkv_stride, pg, stream)
-    else:
-        copy_kv_seqpos(h, c, qkv, pos, n_seq, q_dim, kv_dim, qkv_stride, pg, stream)
-    attn_decode_batched(h, out, qkv, c, pos, n_seq, n_head, n_kv_head, head_dim, pg, qkv_stride,
-                        out_stride, stream)
+    check(lib().mx230_batched_step(h._h, stream_ptr(stream), ptr(out), ptr(qkv), *_cache_args(c), ptr(pos), n_seq, n_head,
+                                   n_kv_head, head_dim, int(use_rope), theta, ptr(pg.table_dev), pg.block_size, pg.n_log,
+                                   qkv_stride, out_stride))
 
 
 # ---------------------------------------------------------------- prefill attention
