@@ -111,6 +111,33 @@ int mx230_fail(int code, const char *fmt, ...);
         (h)->launches++;                                                                    \
     } while (0)
 
+// Kernel launch with a cluster size along x (1 = none) and, with `pdl`, the attribute that lets the kernel start while
+// the stream's previous kernel drains.  Such a kernel must call mx::pdl_wait() before it touches global memory.
+template <typename... KArgs, typename... Args>
+cudaError_t mx_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, int cluster_x, bool pdl,
+                      Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[2];
+    int n = 0;
+    if (cluster_x > 1) {
+        at[n].id = cudaLaunchAttributeClusterDimension;
+        at[n].val.clusterDim.x = cluster_x, at[n].val.clusterDim.y = 1, at[n].val.clusterDim.z = 1;
+        ++n;
+    }
+    if (pdl) {
+        at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[n].val.programmaticStreamSerializationAllowed = 1;
+        ++n;
+    }
+    cfg.attrs = at;
+    cfg.numAttrs = n;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 // RAII-free "make this handle's device current" used at the top of every entry point.
 struct mx230_device_guard {
     int prev;
@@ -609,7 +636,18 @@ __device__ __forceinline__ void quant_head_row(float x0, float x1, bool affine, 
     }
 }
 
+// ---- programmatic dependent launch ----
+// A kernel that calls pdl_trigger() lets the next kernel of the stream (if that was launched with the attribute, see
+// mx_launch) take up free SM slots while this one still runs; pdl_wait() returns once every earlier kernel has completed
+// and its writes are visible.  Before the wait a kernel may set up shared memory and prefetch into L2 (which is coherent:
+// a line that an earlier kernel still writes is simply updated there); it must not load or write anything else.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // ---- thread-block clusters: barrier and loads from the shared memory of the cluster's other CTAs ----
+__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
@@ -617,6 +655,9 @@ __device__ __forceinline__ uint32_t cluster_map(uint32_t saddr, int rank) {
     uint32_t r;
     asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
     return r;
+}
+__device__ __forceinline__ void cluster_st_f32(uint32_t addr, float v) {
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
 }
 __device__ __forceinline__ float cluster_ld_f32(uint32_t addr) {
     float v;

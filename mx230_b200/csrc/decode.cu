@@ -834,6 +834,11 @@ decode_q8_mma_kernel(const DecodeParams P) {
     const int nkv = P.n_kv_head, kvd = nkv * 64;
     const int cl = blockIdx.x / P.cl_size, rank = blockIdx.x - cl * P.cl_size;
 
+    // programmatic launch on both sides (never in a split-KV step, whose CTAs wait for other ranks)
+    if (P.push_regions == nullptr) {
+        mx::pdl_trigger();
+        mx::pdl_wait();
+    }
     int kbeg, kend, ka, kb_;
     key_range(P, s, kbeg, kend);
     const int pos = kend - 1;                             // fused step: the new token's position
@@ -1166,6 +1171,11 @@ decode_f32_ring_kernel(const DecodeParams P) {
     const int nkv = P.n_kv_head, kvd = nkv * 64;
     const int cl = blockIdx.x / P.cl_size, rank = blockIdx.x - cl * P.cl_size;
 
+    // programmatic launch on both sides (never in a split-KV step, whose CTAs wait for other ranks)
+    if (P.push_regions == nullptr) {
+        mx::pdl_trigger();
+        mx::pdl_wait();
+    }
     int kbeg, kend, ka, kb_;
     key_range(P, s, kbeg, kend);
     const int pos = kend - 1;                             // fused step: the new token's position
@@ -1437,29 +1447,12 @@ size_t q8_smem_bytes() {
     return (size_t)Q8Smem<G>::TOTAL;
 }
 
-// Kernel launch with the cluster size as a launch attribute.
-template <typename... KArgs, typename... Args>
-cudaError_t launch_clusters(void (*kernel)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t st, int cl_size,
-                            Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = cl_size, at[0].val.clusterDim.y = 1, at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = cl_size > 1 ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
 template <bool PAGED, bool FUSED>
 int launch_q8_mma(mx230_handle *h, cudaStream_t st, const DecodeParams &P, dim3 grid) {
     const size_t sm = (size_t)Q8MmaSmem::TOTAL;
     MX_SMEM_ATTR_ONCE(h->device, (decode_q8_mma_kernel<PAGED, FUSED>), sm);
     MX_LAUNCH(h, st, MX230_K_DECODE_Q8,
-              launch_clusters(decode_q8_mma_kernel<PAGED, FUSED>, grid, Q8_THREADS, sm, st, P.cl_size, P));
+              mx_launch(decode_q8_mma_kernel<PAGED, FUSED>, grid, Q8_THREADS, sm, st, P.cl_size, P.push_regions == nullptr, P));
     return MX230_OK;
 }
 template <int G, bool PAGED, bool FUSED>
@@ -1467,7 +1460,7 @@ int launch_f32(mx230_handle *h, cudaStream_t st, const DecodeParams &P, dim3 gri
     const size_t sm = (size_t)F32Smem<G>::TOTAL;
     MX_SMEM_ATTR_ONCE(h->device, (decode_f32_ring_kernel<G, PAGED, FUSED>), sm);
     MX_LAUNCH(h, st, MX230_K_DECODE_F32,
-              launch_clusters(decode_f32_ring_kernel<G, PAGED, FUSED>, grid, F32_THREADS, sm, st, P.cl_size, P));
+              mx_launch(decode_f32_ring_kernel<G, PAGED, FUSED>, grid, F32_THREADS, sm, st, P.cl_size, P.push_regions == nullptr, P));
     return MX230_OK;
 }
 

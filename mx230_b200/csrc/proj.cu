@@ -12,24 +12,25 @@
 //                    even), weights are int32 words of four consecutive input rows, w32[(i/4)*n_out + o],
 //                    integer dots by dp4a, one float multiply-add per group, one scale per output column.
 //
-// HBM-bound on the weight matrix (n_in x n_out fp32, fp16 or int8, each byte read once).  The reference
-// gives one thread a whole output column, which leaves most of a B200 idle for a 1152-column
-// matrix; here a CTA owns a 64-column block (one attention head) and a slice of the input rows, so
-// that the grid covers the machine: 16 lanes x 128-bit loads across the columns, 8 row lanes down
-// the slice.  Slices leave partial sums in the workspace; the last CTA to arrive for a column block
-// adds them in slice order (deterministic), adds the bias and runs the epilogue on its 64 values.
+// The floor is HBM on the weight matrix (n_in x n_out fp32, fp16 or int8, each byte read once); at a decode token's
+// sizes (2 MB) the time is latency instead: launch, one memory round trip, the merge of the partial sums.  The reference
+// gives one thread a whole output column.  Here a 64-column block (one attention head) belongs to a thread-block cluster
+// of up to eight CTAs, each with a slice of the input rows small enough that a thread's loads are all in flight at once;
+// the CTAs push their 64 sums into the first one's shared memory, which adds them in slice order (deterministic), adds
+// the bias and runs the epilogue.  Only matrices whose slices would get long (or that have few columns) use several
+// clusters per block, merged through the workspace by the last one to arrive.  The kernel is launched programmatically:
+// its slice of the weights is on its way into L2 while the kernel before it still runs.
 #include <cuda_fp16.h>
 
 #include "common.cuh"
 
 namespace {
 
-constexpr int PJ_THREADS = 128;
+constexpr int PJ_THREADS = 256;
+constexpr int PJ_WARPS = PJ_THREADS / 32;
 constexpr int PJ_COLS = 64;     // columns per CTA = one head
-constexpr int PJ_ROWLANES = 8;
-#ifndef PJ_CTAS_PER_SM
-#define PJ_CTAS_PER_SM 6
-#endif
+constexpr int PJ_CLUSTER = 8;   // most CTAs of a column block that merge through shared memory
+constexpr int PJ_MAX_ROWS = 4096;   // input rows per CTA at most (bounds the int8 path's shared memory)
 
 struct QkvEpilogue {
     int enabled;
@@ -52,38 +53,131 @@ struct GemvParams {
     int n_in, n_out, accum;
     const float *scales;     // int8 weights: one scale per output column
     int ag;                  // int8 weights: activations are quantised in groups of `ag` values (4 or 8)
-    int rows_per_slice;
-    float *partials;         // [n_slices][n_out]
+    int rows_per_slice, n_slices, cl_size;   // n_slices = clusters per block x cl_size
+    float *partials;         // [clusters per block][n_out]
     unsigned *counters;      // one per column block, self-resetting
     QkvEpilogue e;
 };
 
-__device__ __forceinline__ float4 load_w4(const float *w, size_t idx) { return *(const float4 *)(w + idx); }
-__device__ __forceinline__ float4 load_w4(const __half *w, size_t idx) {
-    const uint2 raw = *(const uint2 *)(w + idx);
-    const float2 a = __half22float2(*(const __half2 *)&raw.x), c = __half22float2(*(const __half2 *)&raw.y);
-    return make_float4(a.x, a.y, c.x, c.y);
+// CPT consecutive columns of one weight row: fp32 (4), fp16 (8, or 4 where rows are only 8-byte aligned) or packed int8
+// words (4)
+template <typename WT, int CPT>
+struct WeightRow;
+template <>
+struct WeightRow<float, 4> {
+    float4 r;
+    __device__ __forceinline__ void load(const void *w, size_t i) { r = *(const float4 *)((const float *)w + i); }
+    __device__ __forceinline__ void zero() { r = make_float4(0.f, 0.f, 0.f, 0.f); }
+    __device__ __forceinline__ void fma(float x, float (&a)[4]) const {
+        a[0] = fmaf(x, r.x, a[0]), a[1] = fmaf(x, r.y, a[1]), a[2] = fmaf(x, r.z, a[2]), a[3] = fmaf(x, r.w, a[3]);
+    }
+};
+__device__ __forceinline__ void fma_half2(float x, uint32_t raw, float &a, float &b) {
+    const float2 w = __half22float2(*(const __half2 *)&raw);
+    a = fmaf(x, w.x, a), b = fmaf(x, w.y, b);
 }
+template <>
+struct WeightRow<__half, 8> {
+    uint4 r;
+    __device__ __forceinline__ void load(const void *w, size_t i) { r = *(const uint4 *)((const __half *)w + i); }
+    __device__ __forceinline__ void zero() { r = make_uint4(0, 0, 0, 0); }
+    __device__ __forceinline__ void fma(float x, float (&a)[8]) const {
+        fma_half2(x, r.x, a[0], a[1]), fma_half2(x, r.y, a[2], a[3]), fma_half2(x, r.z, a[4], a[5]), fma_half2(x, r.w, a[6], a[7]);
+    }
+};
+template <>
+struct WeightRow<__half, 4> {
+    uint2 r;
+    __device__ __forceinline__ void load(const void *w, size_t i) { r = *(const uint2 *)((const __half *)w + i); }
+    __device__ __forceinline__ void zero() { r = make_uint2(0, 0); }
+    __device__ __forceinline__ void fma(float x, float (&a)[4]) const {
+        fma_half2(x, r.x, a[0], a[1]), fma_half2(x, r.y, a[2], a[3]);
+    }
+};
+template <>
+struct WeightRow<int8_t, 4> {
+    int4 r;
+    __device__ __forceinline__ void load(const void *w, size_t i) { r = *(const int4 *)((const int *)w + i); }
+    __device__ __forceinline__ void zero() { r = make_int4(0, 0, 0, 0); }
+    __device__ __forceinline__ void fma(int xq, float sx, float (&a)[4]) const {
+        a[0] = fmaf((float)__dp4a(r.x, xq, 0), sx, a[0]), a[1] = fmaf((float)__dp4a(r.y, xq, 0), sx, a[1]);
+        a[2] = fmaf((float)__dp4a(r.z, xq, 0), sx, a[2]), a[3] = fmaf((float)__dp4a(r.w, xq, 0), sx, a[3]);
+    }
+};
 
-template <typename WT>
+// Grid: column blocks x n_slices, slices fastest; a cluster holds cl_size consecutive slices of one block.
+template <typename WT, int CPT>
 __global__ void __launch_bounds__(PJ_THREADS)
 gemv_heads_kernel(const GemvParams P) {
-    __shared__ float red[PJ_ROWLANES][PJ_COLS];
+    constexpr bool I8 = sizeof(WT) == 1;
+    constexpr int TPR = PJ_COLS / CPT;              // threads across a weight row
+    constexpr int RL = PJ_THREADS / TPR;            // weight rows per pass
+    constexpr int BATCH = 4;                        // passes whose loads are issued together
+    constexpr int ELT = I8 ? 4 : (int)sizeof(WT);   // bytes of a stored weight word
+    constexpr int IN_PER_ROW = I8 ? 4 : 1;          // input rows in one stored row
+    __shared__ float red[PJ_WARPS][PJ_COLS];
+    __shared__ float parts[PJ_CLUSTER][PJ_COLS];    // first CTA of the cluster: the sums of every CTA
     __shared__ float val[PJ_COLS];
     __shared__ int is_last;
-    extern __shared__ float xs[];                      // this slice of x (int8: packed codes, then group scales)
-    constexpr bool I8 = sizeof(WT) == 1;
-    const int tid = threadIdx.x;
-    const int col0 = blockIdx.x * PJ_COLS;
-    const int k0 = blockIdx.y * P.rows_per_slice;
-    const int k1 = min(P.n_in, k0 + P.rows_per_slice);
-    int *xq = (int *)xs;                               // int8: (k1 - k0) / 4 words
-    float *xsc = xs + P.rows_per_slice / 4;            // int8: (k1 - k0) / ag scales
-    if (!I8) {
-        for (int i = tid; i < k1 - k0; i += PJ_THREADS) xs[i] = P.x[k0 + i];
-    } else {
+    extern __shared__ float xs[];                   // int8: this slice of x as packed codes, then group scales
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, C = P.cl_size;
+    const int blk = blockIdx.x / P.n_slices, slice = blockIdx.x - blk * P.n_slices;
+    const int cl = slice / C, rank = slice - cl * C;
+    const int col0 = blk * PJ_COLS;
+    const int k0 = min(P.n_in, slice * P.rows_per_slice), k1 = min(P.n_in, k0 + P.rows_per_slice);
+    const int r0 = k0 / IN_PER_ROW, r1 = k1 / IN_PER_ROW;   // stored rows of this slice
+
+    mx::pdl_trigger();
+    if (C > 1) mx::cluster_arrive_relaxed();        // waited for before the first access to another CTA's memory
+    // start of the slice into L2 under the previous kernel's tail
+    for (int r = r0 + tid; r < min(r1, r0 + 2 * PJ_THREADS); r += PJ_THREADS) {
+        const char *line = (const char *)P.w + ((size_t)r * P.n_out + col0) * ELT;
+        mx::prefetch_l2(line);
+        if (ELT == 4 && col0 + 32 < P.n_out) mx::prefetch_l2(line + 128);
+    }
+    mx::pdl_wait();
+
+    const int cq = tid % TPR, rl = tid / TPR;
+    const int col = col0 + CPT * cq;
+    const bool live = col < P.n_out;                // n_out is a multiple of CPT
+    float acc[CPT];
+#pragma unroll
+    for (int c = 0; c < CPT; ++c) acc[c] = 0.0f;
+    WeightRow<WT, CPT> w[BATCH];
+    float xv[BATCH];
+    auto load = [&](int r) {
+#pragma unroll
+        for (int u = 0; u < BATCH; ++u) {
+            const int i = r + u * RL;
+            const bool in = live && i < r1;
+            if (in) w[u].load(P.w, (size_t)i * P.n_out + col);
+            else w[u].zero();
+            if (!I8) xv[u] = in ? P.x[i] : 0.0f;
+        }
+    };
+    load(r0 + rl);
+    // what the epilogue of the cluster's first CTA needs, under the weight loads
+    const QkvEpilogue &E = P.e;
+    const bool is_v = blk >= E.n_head + E.n_kv_head;
+    float bias = 0.0f, scale_o = 1.0f, y_old = 0.0f, cs = 1.0f, sn = 0.0f;
+    int pos = 0;
+    size_t row = 0;
+    if (rank == 0 && tid < PJ_COLS && col0 + tid < P.n_out) {
+        const int o = col0 + tid;
+        if (P.b) bias = P.b[o];
+        if (I8) scale_o = P.scales[o];
+        if (P.accum) y_old = P.y[o];
+        if (E.enabled && tid < 32) {
+            pos = E.pos_dev ? *E.pos_dev : E.pos;
+            row = E.bt && blk >= E.n_head ? (size_t)(E.bt[pos / E.bs] * E.bs + pos % E.bs) : (size_t)pos;
+            if (!is_v) mx::rope_angle(pos, tid, 64, E.theta, cs, sn);
+        }
+    }
+    if constexpr (I8) {
         // quantise this slice of the activations exactly as the reference kernel does
         const int ag = P.ag;
+        int *xq = (int *)xs;                        // (k1 - k0) / 4 words
+        float *xsc = xs + P.rows_per_slice / 4;     // (k1 - k0) / ag scales
         for (int g = tid; g < (k1 - k0) / ag; g += PJ_THREADS) {
             const float *xg = P.x + k0 + g * ag;
             float amax = 0.0f;
@@ -99,105 +193,87 @@ gemv_heads_kernel(const GemvParams P) {
             }
             xsc[g] = amax > 0.0f ? __fdiv_rn(amax, 127.0f) : 1.0f;
         }
-    }
-    __syncthreads();
-
-    const int cq = tid & 15, rl = tid >> 4;
-    const int col = col0 + 4 * cq;
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (col + 3 < P.n_out) {
-        if constexpr (!I8) {
-            const WT *w = (const WT *)P.w;
-#pragma unroll 8
-            for (int i = k0 + rl; i < k1; i += PJ_ROWLANES) {
-                const float4 w4 = load_w4(w, (size_t)i * P.n_out + col);
-                const float xv = xs[i - k0];
-                acc.x = fmaf(xv, w4.x, acc.x);
-                acc.y = fmaf(xv, w4.y, acc.y);
-                acc.z = fmaf(xv, w4.z, acc.z);
-                acc.w = fmaf(xv, w4.w, acc.w);
-            }
-        } else {
-            // word q holds input rows 4q .. 4q+3 of a column; its group scale is xsc[q / (ag / 4)]
-            const int *w32 = (const int *)P.w;
-            const int wpg = P.ag / 4;
-#pragma unroll 8
-            for (int q = k0 / 4 + rl; q < k1 / 4; q += PJ_ROWLANES) {
-                const int4 wv = *(const int4 *)(w32 + (size_t)q * P.n_out + col);
-                const int xv = xq[q - k0 / 4];
-                const float sx = xsc[(q - k0 / 4) / wpg];
-                acc.x = fmaf((float)__dp4a(wv.x, xv, 0), sx, acc.x);
-                acc.y = fmaf((float)__dp4a(wv.y, xv, 0), sx, acc.y);
-                acc.z = fmaf((float)__dp4a(wv.z, xv, 0), sx, acc.z);
-                acc.w = fmaf((float)__dp4a(wv.w, xv, 0), sx, acc.w);
+        __syncthreads();
+        const int wpg = ag / 4;   // word q holds input rows 4q .. 4q+3; its group scale is xsc[q / wpg]
+        for (int r = r0 + rl; r < r1; r += BATCH * RL) {
+            if (r != r0 + rl) load(r);
+#pragma unroll
+            for (int u = 0; u < BATCH; ++u) {
+                const int q = r + u * RL - r0;
+                if (q < r1 - r0) w[u].fma(xq[q], xsc[q / wpg], acc);
             }
         }
-    }
-    *(float4 *)&red[rl][4 * cq] = acc;
-    __syncthreads();
-    const int n_slices = gridDim.y;
-    if (tid < PJ_COLS) {
-        float s = 0.0f;
+    } else {
+        for (int r = r0 + rl; r < r1; r += BATCH * RL) {
+            if (r != r0 + rl) load(r);
 #pragma unroll
-        for (int r = 0; r < PJ_ROWLANES; ++r) s += red[r][tid];
-        if (n_slices == 1) val[tid] = s;
-        else if (col0 + tid < P.n_out) P.partials[(size_t)blockIdx.y * P.n_out + col0 + tid] = s;
+            for (int u = 0; u < BATCH; ++u) w[u].fma(xv[u], acc);
+        }
     }
-    if (n_slices > 1) {
+    // ---- CTA, then cluster, then (several clusters) block totals ----
+#pragma unroll
+    for (int c = 0; c < CPT; ++c) {
+#pragma unroll
+        for (int o = TPR; o < 32; o <<= 1) acc[c] += __shfl_xor_sync(0xFFFFFFFFu, acc[c], o);
+        if (lane < TPR) red[warp][CPT * cq + c] = acc[c];
+    }
+    __syncthreads();
+    float sum = 0.0f;
+    if (tid < PJ_COLS) {
+#pragma unroll
+        for (int r = 0; r < PJ_WARPS; ++r) sum += red[r][tid];
+    }
+    if (C > 1) {
+        mx::cluster_wait();       // every CTA of the cluster runs
+        if (tid < PJ_COLS) mx::cluster_st_f32(mx::cluster_map(mx::smem_u32(&parts[rank][tid]), 0), sum);
+        mx::cluster_sync();
+        if (rank != 0) return;
+        if (tid < PJ_COLS) {
+            sum = 0.0f;
+            for (int r = 0; r < C; ++r) sum += parts[r][tid];
+        }
+    }
+    const int n_cl = P.n_slices / C;
+    if (n_cl > 1) {
+        if (tid < PJ_COLS && col0 + tid < P.n_out) P.partials[(size_t)cl * P.n_out + col0 + tid] = sum;
         __threadfence();
         __syncthreads();
-        if (tid == 0) is_last = atomicInc(&P.counters[blockIdx.x], n_slices - 1) == (unsigned)(n_slices - 1);
+        if (tid == 0) is_last = atomicInc(&P.counters[blk], n_cl - 1) == (unsigned)(n_cl - 1);
         __syncthreads();
         if (!is_last) return;
         __threadfence();
         if (tid < PJ_COLS && col0 + tid < P.n_out) {
-            float s = 0.0f;
-            for (int sl = 0; sl < n_slices; ++sl) s += P.partials[(size_t)sl * P.n_out + col0 + tid];
-            val[tid] = s;
+            sum = 0.0f;
+            for (int r = 0; r < n_cl; ++r) sum += __ldcg(P.partials + (size_t)r * P.n_out + col0 + tid);
         }
     }
-    __syncthreads();
     // ---- epilogue on the 64 finished sums of this column block ----
-    if (tid < PJ_COLS) {
-        const int o = col0 + tid;
-        if (o < P.n_out) val[tid] = (I8 ? val[tid] * P.scales[o] : val[tid]) + (P.b ? P.b[o] : 0.0f);
-    }
+    if (tid < PJ_COLS) val[tid] = (I8 ? sum * scale_o : sum) + bias;
     __syncthreads();
-    if (!P.e.enabled) {
-        if (tid < PJ_COLS && col0 + tid < P.n_out) {
-            const int o = col0 + tid;
-            P.y[o] = P.accum ? P.y[o] + val[tid] : val[tid];
-        }
+    if (!E.enabled) {
+        if (tid < PJ_COLS && col0 + tid < P.n_out) P.y[col0 + tid] = P.accum ? y_old + val[tid] : val[tid];
         return;
     }
     // qkv step: this block is head `hb` of the row [Q heads | K heads | V heads]
-    const QkvEpilogue &E = P.e;
-    const int hb = blockIdx.x;
-    const int pos = E.pos_dev ? *E.pos_dev : E.pos;
-    const bool is_v = hb >= E.n_head + E.n_kv_head;
+    const int hb = blk;
     if (tid < 32) {   // one warp: lane l owns the rotation pair (l, l + 32), then elements 2l, 2l+1
-        if (!is_v) {
-            float cs, sn;
-            mx::rope_angle(pos, tid, 64, E.theta, cs, sn);
-            mx::rope_pair(val[tid], val[tid + 32], cs, sn);
-        }
+        if (!is_v) mx::rope_pair(val[tid], val[tid + 32], cs, sn);
         __syncwarp();
-        const float2 xv = make_float2(val[2 * tid], val[2 * tid + 1]);
-        *(float2 *)(P.y + (size_t)hb * 64 + 2 * tid) = xv;
+        const float2 x2 = make_float2(val[2 * tid], val[2 * tid + 1]);
+        *(float2 *)(P.y + (size_t)hb * 64 + 2 * tid) = x2;
         if (hb >= E.n_head) {   // K or V head: the cache row of this position
             const int kvh = is_v ? hb - E.n_head - E.n_kv_head : hb - E.n_head;
-            const size_t row = E.bt ? (size_t)(E.bt[pos / E.bs] * E.bs + pos % E.bs) : (size_t)pos;
             const int kvd = E.n_kv_head * 64;
             if (E.kq == nullptr) {
                 float *dst = (is_v ? E.vcache : E.kcache) + row * kvd + kvh * 64;
-                *(float2 *)(dst + 2 * tid) = xv;
+                *(float2 *)(dst + 2 * tid) = x2;
             } else {
                 int8_t *dst = (is_v ? E.vq : E.kq) + row * kvd + kvh * 64;
                 float *sc = is_v ? E.vs : E.ks, *be = is_v ? E.vb : E.kb;
                 const size_t sd = row * E.n_kv_head + kvh;
                 int c0, c1;
                 float scale, beta;
-                mx::quant_head_row(xv.x, xv.y, be != nullptr, c0, c1, scale, beta);
+                mx::quant_head_row(x2.x, x2.y, be != nullptr, c0, c1, scale, beta);
                 if (tid == 0) {
                     sc[sd] = scale;
                     if (be != nullptr) be[sd] = beta;
@@ -214,23 +290,31 @@ int launch_gemv(mx230_handle *h, void *stream, GemvParams P, int w_kind, const c
     MX_REQUIRE(P.n_in > 0 && P.n_out > 0 && P.n_out % 4 == 0, MX230_ERR_INVALID_ARG,
                "%s: n_in %d, n_out %d (n_out must be a positive multiple of 4)", who, P.n_in, P.n_out);
     MX_REQUIRE((((uintptr_t)P.w | (uintptr_t)P.y) & 15) == 0, MX230_ERR_INVALID_ARG, "%s: y and w must be 16-byte aligned", who);
-    const int n_blocks = (P.n_out + PJ_COLS - 1) / PJ_COLS;
-    // enough input slices for PJ_CTAS_PER_SM CTAs on every SM (bytes in flight, not arithmetic, set the
-    // pace), at least 16 rows each
-    int n_slices = (PJ_CTAS_PER_SM * h->sm_count + n_blocks - 1) / n_blocks;
-    const int max_slices = (P.n_in + 15) / 16;
-    if (n_slices > max_slices) n_slices = max_slices;
-    if (n_slices < 1) n_slices = 1;
-    // int8: a slice holds whole activation groups and whole passes of the eight row lanes over 4-row words
-    const int gran = w_kind == 2 ? 4 * PJ_ROWLANES : PJ_ROWLANES;
     if (w_kind == 2) {
         MX_REQUIRE(P.scales && (P.ag == 4 || P.ag == 8) && P.n_in % 8 == 0, MX230_ERR_INVALID_ARG,
                    "%s: int8 weights need scales, an activation group of 4 or 8 and n_in %% 8 == 0 (n_in %d)", who, P.n_in);
     }
-    P.rows_per_slice = ((P.n_in + n_slices - 1) / n_slices + gran - 1) / gran * gran;
-    n_slices = (P.n_in + P.rows_per_slice - 1) / P.rows_per_slice;
-    if (n_slices > 1) {
-        const size_t need = (size_t)n_slices * P.n_out * sizeof(float);
+    const int n_blocks = (P.n_out + PJ_COLS - 1) / PJ_COLS;
+    const bool wide = w_kind == 1 && P.n_out % 8 == 0;   // fp16 rows of whole 16-byte pieces
+    const int pass = (wide ? 32 : 16) * (w_kind == 2 ? 4 : 1);   // input rows that a CTA takes in one load per thread
+    // Measured on one token through 24 layers (fp16 896 x 1152 and 896 x 896, int8 cache of 2001 keys, one graph): with 38 and
+    // 56 slices merged through the workspace 10.5 and 9.4 us per launch, 536 us per token; one cluster of eight per block
+    // and programmatic launches of this kernel and the attention kernel, 247 us.
+    // One cluster per column block, of as many CTAs (up to 8) as have a pass of rows each.  Further clusters (a merge
+    // through global memory, about 2 us) only where the blocks alone leave SMs idle and every CTA still gets four passes,
+    // or where a slice would exceed PJ_MAX_ROWS.
+    int c = (P.n_in + pass - 1) / pass;
+    P.cl_size = c < PJ_CLUSTER ? c : PJ_CLUSTER;
+    long long n_cl = (2ll * h->sm_count + n_blocks * P.cl_size - 1) / ((long long)n_blocks * P.cl_size);
+    const long long by_rows = P.n_in / ((long long)P.cl_size * 4 * pass);
+    if (n_cl > by_rows) n_cl = by_rows;
+    const long long at_least = (P.n_in + (long long)P.cl_size * PJ_MAX_ROWS - 1) / ((long long)P.cl_size * PJ_MAX_ROWS);
+    if (n_cl < at_least) n_cl = at_least;
+    P.n_slices = (int)n_cl * P.cl_size;
+    const int gran = w_kind == 2 ? 8 : 1;   // int8: a slice holds whole activation groups
+    P.rows_per_slice = ((P.n_in + P.n_slices - 1) / P.n_slices + gran - 1) / gran * gran;
+    if (n_cl > 1) {
+        const size_t need = (size_t)n_cl * P.n_out * sizeof(float);
         MX_REQUIRE(h->ws && need <= h->ws_bytes, MX230_ERR_WORKSPACE, "%s: workspace %zu B < %zu B needed", who,
                    h->ws_bytes, need);
         MX_REQUIRE((size_t)n_blocks <= h->n_counters, MX230_ERR_UNSUPPORTED, "%s: %d column blocks exceed %zu counters",
@@ -241,11 +325,13 @@ int launch_gemv(mx230_handle *h, void *stream, GemvParams P, int w_kind, const c
     }
     mx230_device_guard guard(h->device);
     cudaStream_t st = (cudaStream_t)stream;
-    dim3 grid(n_blocks, n_slices);
-    const size_t sm = (size_t)P.rows_per_slice * sizeof(float);   // int8: n/4 words + n/ag scales <= n floats
-    if (w_kind == 2) MX_LAUNCH(h, st, MX230_K_GEMV, (gemv_heads_kernel<int8_t><<<grid, PJ_THREADS, sm, st>>>(P)));
-    else if (w_kind == 1) MX_LAUNCH(h, st, MX230_K_GEMV, (gemv_heads_kernel<__half><<<grid, PJ_THREADS, sm, st>>>(P)));
-    else MX_LAUNCH(h, st, MX230_K_GEMV, (gemv_heads_kernel<float><<<grid, PJ_THREADS, sm, st>>>(P)));
+    const dim3 grid((unsigned)(n_blocks * P.n_slices));
+    const size_t sm = w_kind == 2 ? (size_t)P.rows_per_slice * sizeof(float) / 2 : 0;   // rows/4 words + rows/ag scales
+    const int cx = P.cl_size;
+    if (w_kind == 2) MX_LAUNCH(h, st, MX230_K_GEMV, mx_launch(gemv_heads_kernel<int8_t, 4>, grid, PJ_THREADS, sm, st, cx, true, P));
+    else if (wide) MX_LAUNCH(h, st, MX230_K_GEMV, mx_launch(gemv_heads_kernel<__half, 8>, grid, PJ_THREADS, sm, st, cx, true, P));
+    else if (w_kind == 1) MX_LAUNCH(h, st, MX230_K_GEMV, mx_launch(gemv_heads_kernel<__half, 4>, grid, PJ_THREADS, sm, st, cx, true, P));
+    else MX_LAUNCH(h, st, MX230_K_GEMV, mx_launch(gemv_heads_kernel<float, 4>, grid, PJ_THREADS, sm, st, cx, true, P));
     return MX230_OK;
 }
 

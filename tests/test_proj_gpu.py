@@ -128,3 +128,55 @@ def test_gemv_rejects_bad_arguments(handle):
     from mx230_b200._lib import Mx230Error
     with pytest.raises(Mx230Error):
         la.gemv(handle, torch.zeros(6, device="cuda"), torch.zeros(8, device="cuda"), torch.zeros(8, 6, device="cuda"))
+
+
+@pytest.mark.parametrize("n_in,n_out,kind", [
+    (8, 64, "int8"), (40, 68, "fp16"), (33, 132, "fp32"), (264, 72, "int8"),      # a cluster of one to five CTAs, short slices
+    (4104, 64, "fp16"), (8200, 12, "fp32"), (16392, 64, "int8"),                  # several clusters per column block
+    (70000, 8, "fp16"),                                                           # slices bounded by their largest length
+])
+def test_gemv_slices_and_clusters(handle, n_in, n_out, kind):
+    """Edges of the split over CTAs and clusters.  fp32 sums of n_in products of size 0.05 in any order: the error of a
+    sum stays below n_in * 2^-24 times the sum of the products' magnitudes (about 0.03 n_in), a random walk of it in
+    practice: sqrt(n_in) * 0.05 * log2(n_in) * 2^-23 with a factor of 8 to spare."""
+    x = oracle.normal((n_in,), 640, 0)
+    if kind == "int8":
+        codes = np.random.default_rng(3).integers(-127, 128, (n_in, n_out), dtype=np.int8)
+        scales = np.full(n_out, 0.05 / 64, np.float32)
+        words = codes.reshape(n_in // 4, 4, n_out).astype(np.int64) & 0xff
+        packed = (words[:, 0] | words[:, 1] << 8 | words[:, 2] << 16 | words[:, 3] << 24).astype(np.uint32).view(np.int32)
+        y = torch.zeros(n_out, device="cuda")
+        la.gemv_int8(handle, y, dev(x), dev(packed), dev(scales), act_group=8)
+        g = x.reshape(-1, 8)
+        amax = np.abs(g).max(1, keepdims=True)
+        q = np.clip(np.rint(g * (np.float32(127) / amax)), -127, 127)
+        want = ((q * (amax / np.float32(127)).astype(np.float32)).astype(np.float64).reshape(-1) @ codes.astype(np.float64)) * scales[0]
+    else:
+        w = (oracle.normal((n_in, n_out), 641, 0) * 0.05).astype(np.float16 if kind == "fp16" else np.float32)
+        y = torch.zeros(n_out, device="cuda")
+        la.gemv(handle, y, dev(x), dev(w))
+        want = x.astype(np.float64) @ w.astype(np.float64)
+    handle.check_status()
+    tol = 8 * np.sqrt(n_in) * 0.05 * max(1.0, np.log2(n_in)) * 2.0 ** -23
+    assert np.abs(y.cpu().numpy() - want).max() <= tol
+
+
+def test_chain_of_dependent_launches(handle):
+    """gemv -> gemv -> gemv on one stream, each launch allowed to start before the previous one has drained: the values are
+    those of the launches with a synchronisation after each."""
+    n = 896
+    w = dev((oracle.normal((n, n), 650, 0) * 0.03).astype(np.float16))
+    x = dev(oracle.normal((n,), 651, 0))
+    bufs = [torch.empty(n, device="cuda") for _ in range(24)]
+    prev = x
+    for b in bufs:
+        la.gemv(handle, b, prev, w)
+        prev = b
+    torch.cuda.synchronize()
+    prev = x
+    for b in bufs:
+        want = torch.empty_like(b)
+        la.gemv(handle, want, prev, w)
+        torch.cuda.synchronize()
+        assert torch.equal(want, b)
+        prev = want
