@@ -304,6 +304,17 @@ int mx230_batched_step(mx230_handle *h, void *stream, float *out, float *qkv, fl
                        int n_seq, int n_head, int n_kv_head, int head_dim, int use_rope, float theta,
                        const int *tables, int block_size, int n_log, int qkv_stride, int out_stride);
 
+/* The prefill attention step of a chunk of n_tok tokens at positions pos0.. (what gpu.rs:3204-3347 does per layer): RoPE
+ * on the Q and K heads of the qkv rows (use_rope != 0; rotated in place), their K and V heads written to the cache (fp32
+ * kcache / vcache when kq == NULL, else int8 quantize-on-write; kb == vb == NULL: absmax; rows through bt / bs, or the
+ * positions themselves without a table), then causal attention of the n_tok rows over keys 0..pos0+n_tok.  Every result
+ * equals that of mx230_rope_batch, mx230_copy_kv_batch / mx230_quantize_kv_batch and mx230_attn_prefill in turn; the work
+ * in front of attention is one launch. */
+int mx230_prefill_step(mx230_handle *h, void *stream, float *out, float *qkv, float *kcache, float *vcache,
+                       int8_t *kq, int8_t *vq, float *ks, float *vs, float *kb, float *vb, int pos0, int n_tok,
+                       int n_head, int n_kv_head, int head_dim, int use_rope, float theta, int qkv_stride,
+                       int out_stride, const int *bt, int bs);
+
 /* Decode over an int8 cache without a handle and without any allocation (no counterpart in
  * the reference, whose kernels use no scratch memory at all).  For hosts that cannot call
  * cudaMalloc when they need attention -- all free HBM already given to their KV pool, or only

@@ -206,10 +206,10 @@ inline size_t mx230_flash_norm_bytes(int batch_heads) {
 // [heads / kv_group][n_k][64]; causal row r sees keys <= r + q_off; output row r of head h at
 // O + h*o_head_stride + r*o_row_stride.  q_prescaled: Qb holds Q * MX230_QK_LOG2_SCALE.  q_norm2 / k_norm2 (both or
 // neither): largest squared row norm per head of the unscaled Q [heads][MX230_NORM_PARTS] and of K
-// [heads / kv_group][MX230_NORM_PARTS]; with them (and q_prescaled) a head whose scores are provably small takes the
-// kernel's max-free softmax loop.  row_a / row_qsum / col_kskb (all or none; with them q_prescaled must be 0 and Qb, Kb
+// [heads / kv_group][MX230_NORM_PARTS] (int8 score mode: of the dequantised rows); with them a head whose scores are
+// provably small takes the kernel's max-free softmax loop.  row_a / row_qsum / col_kskb (all or none; with them q_prescaled must be 0 and Qb, Kb
 // hold int8 codes as bf16): the int8 score mode -- score = row_a[h][i] * (dot * ks[j] + row_qsum[h][i] * kb[j]), with
-// col_kskb [heads / kv_group][n_k rounded up to 128] pairs (ks, kb).
+// col_kskb [heads / kv_group][tiles of 128 keys][ks of the 128 keys, then their kb], 16-byte aligned.
 int mx230_launch_flash_fwd_ex(mx230_handle *h, cudaStream_t st, const void *Qb, const void *Kb,
                               const void *Vb, float *O, float *L, int heads, int n_q, int n_k, int q_off,
                               int kv_group, long long o_head_stride, long long o_row_stride, int causal,
@@ -342,6 +342,12 @@ __device__ __forceinline__ void tma_store_3d(const CUtensorMap *tmap, uint32_t s
         "cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4}], [%1];"
         ::"l"(tmap), "r"(src), "r"(x), "r"(y), "r"(z)
         : "memory");
+}
+// Untiled copy into this CTA's shared memory: both addresses 16-byte aligned, size a multiple of 16.
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"(src), "r"(bytes), "r"(bar)
+                 : "memory");
 }
 __device__ __forceinline__ void bulk_commit_group() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // all but the newest `N` groups of this thread have finished READING their shared-memory source
@@ -546,6 +552,11 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
 __device__ __forceinline__ uint64_t add2_rm(uint64_t a, uint64_t b) {   // round towards minus infinity
     uint64_t r;
     asm("add.rm.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
@@ -647,6 +658,7 @@ __device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefe
 
 // ---- thread-block clusters: barrier and loads from the shared memory of the cluster's other CTAs ----
 __device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_arrive_release() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -658,6 +670,9 @@ __device__ __forceinline__ uint32_t cluster_map(uint32_t saddr, int rank) {
 }
 __device__ __forceinline__ void cluster_st_f32(uint32_t addr, float v) {
     asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+}
+__device__ __forceinline__ void cluster_red_max(uint32_t addr, int v) {
+    asm volatile("red.relaxed.cluster.shared::cluster.max.s32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
 __device__ __forceinline__ float cluster_ld_f32(uint32_t addr) {
     float v;

@@ -7,7 +7,8 @@
 // when causal, any N, natural-log L) and maps the two contractions onto the 5th-gen
 // tensor cores:
 //
-//   * a work item is 256 query rows of one head as two 128-row tiles; the kernel is persistent:
+//   * a work item is 256 query rows of one head as two 128-row tiles (or, for calls that would fill the SMs unevenly, one
+//     tile with its key tiles split between the softmax groups: KEY_SPLIT below); the kernel is persistent:
 //     one CTA per SM walks a fixed share of the items (heaviest first, dealt out in snake order so
 //     that every CTA gets the same number of key tiles), and every role runs ahead into the next
 //     item on its own, so the next item's Q / K loads and first Q K^T run under the current
@@ -67,29 +68,22 @@ static_assert(SOFT_WARPS * FWD_REGS_SOFTMAX + 4 * FWD_REGS_SERVICE <= (SOFT_WARP
 #ifndef FWD_POLY_DEN
 #define FWD_POLY_DEN 4
 #endif
-#ifndef FWD_ADD2
-#define FWD_ADD2 1        // row sums with packed f32x2 adds
-#endif
-
-#ifndef FWD_UNIFORM_ISSUE
-#define FWD_UNIFORM_ISSUE 1   // MMA issuer warps run warp-uniform with one elected lane (0: a lone lane in a divergent branch)
-#endif
-#if FWD_UNIFORM_ISSUE
+// The MMA issuer warps run warp-uniformly (waits included) with one elected lane issuing.
 #define ISSUER_WAIT(w) __all_sync(0xFFFFFFFFu, (w))
 #define ISSUER_LANE mx::elect_one()
-#else
-#define ISSUER_WAIT(w) (w)
-#define ISSUER_LANE true
-#endif
 
 constexpr int Q_BUFS = 2;                // Q of the next item lands while the current one is in use
 constexpr int SMEM_Q = 0;
 constexpr int SMEM_K = SMEM_Q + Q_BUFS * QT * TILE_BYTES;
 constexpr int SMEM_V = SMEM_K + KV_STAGES * TILE_BYTES;
 constexpr int SMEM_BAR = SMEM_V + KV_STAGES * TILE_BYTES;
-constexpr int SMEM_XCH = SMEM_BAR + 512;   // [2 item parities][QT][2][BM] floats: row sums handed from the second half of a tile to the first
-constexpr int SMEM_XMAX = SMEM_XCH + 2 * QT * 2 * BM * 4;   // [QT][2 tile parities][HALVES][BM] floats: row-max parts of the general mode
-constexpr int SMEM_TOTAL = SMEM_XMAX + QT * 2 * HALVES * BM * 4;
+constexpr int XCH_PUBS = 3;                // groups that hand their row sums over (one per query tile; three in the key-split form)
+constexpr int SMEM_XCH = SMEM_BAR + 512;   // [2 item parities][XCH_PUBS][3][BM] floats: row sums (and max) handed to the group that does the epilogue
+constexpr int SMEM_XMAX = SMEM_XCH + 2 * XCH_PUBS * 3 * BM * 4;   // [QT][2 tile parities][HALVES][BM] floats: row-max parts of the general mode
+constexpr int KSKB_SLOTS = 8;              // int8 scores: ring of the key tiles' scales and offsets
+constexpr int KSKB_BYTES = 2 * BN * 4;     // ks[BN], kb[BN]
+constexpr int SMEM_KSKB = SMEM_XMAX + QT * 2 * HALVES * BM * 4;
+constexpr int SMEM_TOTAL = SMEM_KSKB + KSKB_SLOTS * KSKB_BYTES;
 constexpr int SMEM_ALLOC = SMEM_TOTAL + 1024;  // slack for 1024-byte alignment
 
 // barrier slots (8 bytes each) inside SMEM_BAR
@@ -103,9 +97,11 @@ constexpr int BAR_S_FULL = BAR_V_EMPTY + KV_STAGES;  // [QT] MMA -> softmax: S_t
 constexpr int BAR_S_FREE = BAR_S_FULL + QT;          // [QT] softmax -> MMA: S_t copied to registers
 constexpr int BAR_P_FULL = BAR_S_FREE + QT;          // [QT] softmax -> MMA: P_t written
 constexpr int BAR_O_DONE = BAR_P_FULL + QT;          // [QT] MMA -> softmax: O_t += P_t V complete
-constexpr int BAR_XCH = BAR_O_DONE + QT;             // [QT] second half of tile t -> first half: its row sums are published
+constexpr int BAR_XCH = BAR_O_DONE + QT;             // [QT] row sums are published (key-split form: [0] only, by three groups)
 constexpr int BAR_XMAX = BAR_XCH + QT;               // [QT] general mode: both halves of tile t have published their part of the row max
-constexpr int N_BARS = BAR_XMAX + QT;                // 32
+constexpr int BAR_O1_READ = BAR_XMAX + QT;           // key-split form: O_1 of the item has been read by the epilogue
+constexpr int N_BARS = BAR_O1_READ + 1;
+static_assert(8 * N_BARS + 16 <= 512, "barrier area");
 
 // tensor-memory columns: nothing aliases, so S_t(j+1) can be produced while P_t(j) is consumed
 constexpr int TM_S = 0;     // S_t at TM_S + t*128, fp32
@@ -132,7 +128,6 @@ struct FwdParams {
     int n_qblocks;        // blocks of item_tiles*BM query rows per head
     int n_items;          // heads * n_qblocks
     int tma_out;          // O leaves through staged TMA stores (strides and base 16-byte aligned) or per-thread stores
-    int prescaled;        // Q was staged multiplied by scale * log2(e): the scores arrive in log2 units
     const float *q_norm2; // [heads][MX230_NORM_PARTS] largest squared row norm of the unscaled Q per head and part, or null
     const float *k_norm2; // [heads / kv_group][MX230_NORM_PARTS] the same for K
     int test_drop_tile;   // test hook: K/V tile (counted over the CTA's items) that CTA 0's producer never requests; -1 = off
@@ -141,8 +136,8 @@ struct FwdParams {
     // row_a[i] * (dot * ks[j] + row_qsum[i] * kb[j]) in log2 units (03-llm-engine/kernels/llm.cu:3774-3782)
     const float *row_a;      // [heads][n_q]   q scale * 1/sqrt(64) * log2(e), or null = mode off
     const float *row_qsum;   // [heads][n_q]   sum of the row's q codes
-    const float2 *col_kskb;  // [heads / kv_group][n_k_pad] (scale, offset) of every key
-    int n_k_pad;             // n_k rounded up to a multiple of BN
+    const float *col_kskb;   // [heads / kv_group][key tiles][ks[BN], kb[BN]]: scale and offset of every key
+    int n_k_tiles;           // key tiles of BN keys
     int *status;
 };
 
@@ -171,6 +166,27 @@ __device__ __forceinline__ int fwd_tile_iters(const FwdParams &P, int q0, int t)
     return P.causal ? min(n_kv_total, (r0 + BM - 1 + P.q_off) / BN + 1) : n_kv_total;
 }
 
+// Whether every score of head `bh` is bounded by 80 in log2 units (see the softmax loop); whole-warp call.
+__device__ __forceinline__ bool fwd_fast_head(const FwdParams &P, int bh, int lane) {
+    if (!FWD_FAST || P.q_norm2 == nullptr) return false;
+    static_assert(MX230_NORM_PARTS == 32, "one part per lane");
+    // norms are >= 0 or NaN: as integers they order like that, with NaN the largest
+    const int nq = __reduce_max_sync(0xFFFFFFFFu, __float_as_int(P.q_norm2[(size_t)bh * MX230_NORM_PARTS + lane]) & 0x7FFFFFFF);
+    const int nk = __reduce_max_sync(0xFFFFFFFFu, __float_as_int(P.k_norm2[(size_t)(bh / P.kv_group) * MX230_NORM_PARTS + lane]) & 0x7FFFFFFF);
+    // the norms are those of the fp32 values; rounding to bf16 moves a norm by less than 0.4 %
+    return __int_as_float(nq) * __int_as_float(nk) * (MX230_QK_LOG2_SCALE * MX230_QK_LOG2_SCALE) <= 80.0f * 80.0f;
+}
+
+// Where scores come from: Q staged times scale * log2(e) (they arrive in log2 units), Q and K as the caller gave them, or
+// int8 codes of both (exact integer dots, see FwdParams::row_a).
+enum { SRC_PRE = 0, SRC_RAW = 1, SRC_I8 = 2 };
+
+// KEY_SPLIT: an item is ONE query tile whose even key tiles belong to softmax groups 0, 1 and whose odd ones to groups 2, 3,
+// each pair with its own S and P in tensor memory, so that both pairs of groups work on every item and items are half as
+// large (fwd_key_split says when).  Without a row max P V of all key tiles is summed into one O in key order, and both
+// forms sum a row's probabilities over even and odd key tiles apart: a head's result has the same bits in either form.
+// With a row max each pair of groups has its own max and its own O, which the first group joins at the end.
+template <int SRC, bool KEY_SPLIT>
 __global__ void __launch_bounds__(FWD_THREADS, 1)
 flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                  const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO,
@@ -202,9 +218,10 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             mx::mbar_init(bar(BAR_S_FREE + t), HALVES * BM / 32);  // one elected lane per warp of the tile's groups arrives
             mx::mbar_init(bar(BAR_P_FULL + t), HALVES * BM / 32);
             mx::mbar_init(bar(BAR_O_DONE + t), 1);
-            mx::mbar_init(bar(BAR_XCH + t), BM / 32);
+            mx::mbar_init(bar(BAR_XCH + t), (KEY_SPLIT ? XCH_PUBS : 1) * BM / 32);
             mx::mbar_init(bar(BAR_XMAX + t), HALVES * BM / 32);
         }
+        mx::mbar_init(bar(BAR_O1_READ), BM / 32);
         *abort_flag = 0;
         mx::mbar_fence_init();
     }
@@ -213,6 +230,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     __syncthreads();
     mx::tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    mx::pdl_wait();
 
     // register budget: a softmax thread holds 64 score values and their packed probabilities, the
     // service warpgroup (TMA, two MMA issuers, one idle warp) needs few
@@ -228,7 +246,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             uint32_t g = 0;  // K/V tiles loaded so far, over all items: ring slot g % KV_STAGES, use g / KV_STAGES
             int bh, q0;
             for (int it = 0; ok && fwd_item(P, it, bh, q0); ++it) {
-                const int n_it1 = fwd_tile_iters(P, q0, 1);
+                const int n_it1 = KEY_SPLIT ? 0 : fwd_tile_iters(P, q0, 1);
                 const int n_max = max(fwd_tile_iters(P, q0, 0), n_it1);
                 const int qbuf = it & 1;
                 // the buffer's previous item (two items ago) must have staged its last O piece out of it
@@ -246,9 +264,16 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                     if (r > 0) ok = mx::mbar_wait(bar(BAR_K_EMPTY + s), (r - 1) & 1, abort_flag, P.status);
                     if (!ok) break;
                     if (P.test_drop_tile == (int)g && blockIdx.x == 0) continue;   // test hook: this tile never arrives
-                    mx::mbar_expect_tx(bar(BAR_K_FULL + s), TILE_BYTES);
+                    mx::mbar_expect_tx(bar(BAR_K_FULL + s), TILE_BYTES + (SRC == SRC_I8 ? KSKB_BYTES : 0));
                     mx::tma_load_3d(smem_base + SMEM_K + s * TILE_BYTES, &tmK, bar(BAR_K_FULL + s), 0,
                                     j * BN, kvh);
+                    // The tile's scales and offsets land before its scores exist.  Slot g % 8 is free: the load of tile g
+                    // is issued after the Q K^T of tile g - 4, which waited for the softmax groups to have taken their
+                    // previous tile (g - 5; g - 6 in the key-split form) into registers, so every group is done with
+                    // tile g - 8.
+                    if (SRC == SRC_I8)
+                        mx::bulk_load(smem_base + SMEM_KSKB + (g % KSKB_SLOTS) * KSKB_BYTES,
+                                      P.col_kskb + ((size_t)kvh * P.n_k_tiles + j) * 2 * BN, KSKB_BYTES, bar(BAR_K_FULL + s));
                     if (r > 0) ok = mx::mbar_wait(bar(BAR_V_EMPTY + s), (r - 1) & 1, abort_flag, P.status);
                     if (!ok) break;
                     mx::mbar_expect_tx(bar(BAR_V_FULL + s), TILE_BYTES);
@@ -263,7 +288,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         // The whole warp runs the loop and the waits; one elected lane issues.  Control flow and descriptor
         // arithmetic stay warp-uniform that way (a lone thread inside a divergent branch pays several dependent
         // instructions per tcgen05.mma to move its operands to the uniform registers the instruction reads).
-        if (FWD_UNIFORM_ISSUE || lane == 0) {
+        {
             constexpr uint32_t IDESC_S = mx::mma_idesc_bf16(BM, BN, false, false);
             bool ok = true;
             uint32_t g = 0;            // K/V tiles consumed so far, over all items
@@ -272,7 +297,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             for (int it = 0; ok && fwd_item(P, it, bh, q0); ++it) {
                 int n_it[QT];
 #pragma unroll
-                for (int t = 0; t < QT; ++t) n_it[t] = fwd_tile_iters(P, q0, t);
+                for (int t = 0; t < QT; ++t) n_it[t] = fwd_tile_iters(P, q0, KEY_SPLIT ? 0 : t);
                 const int n_max = max(n_it[0], n_it[1]);
                 const int qbuf = it & 1;
                 ok = ISSUER_WAIT(mx::mbar_wait(bar(BAR_Q_FULL + qbuf), (it >> 1) & 1, abort_flag, P.status));
@@ -282,13 +307,13 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                     const uint64_t b = mx::smem_desc_sw128(smem_base + SMEM_K + s * TILE_BYTES);
 #pragma unroll
                     for (int t = 0; t < QT; ++t) {
-                        if (!ok || j >= n_it[t]) continue;
+                        if (!ok || j >= n_it[t] || (KEY_SPLIT && (j & 1) != t)) continue;
                         // next scores as soon as the softmax group holds the previous ones in registers (the
                         // previous ones may be the last of the item before: this is where the items overlap)
                         if (cs[t] > 0) ok = ISSUER_WAIT(mx::mbar_wait(bar(BAR_S_FREE + t), (cs[t] - 1) & 1, abort_flag, P.status));
                         if (!ok) continue;
                         mx::tc_fence_after();
-                        const uint64_t a = mx::smem_desc_sw128(smem_base + SMEM_Q + (qbuf * QT + t) * TILE_BYTES);
+                        const uint64_t a = mx::smem_desc_sw128(smem_base + SMEM_Q + (qbuf * QT + (KEY_SPLIT ? 0 : t)) * TILE_BYTES);
                         if (ISSUER_LANE) {
 #pragma unroll
                             for (int k = 0; k < HD / 16; ++k)  // 32 bytes per 16-element step inside the swizzle span
@@ -305,7 +330,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         __syncwarp();
         } else if (warp == SOFT_WARPS + 2) {
         // ------------------------- MMA issuer 2: O_t += P_t V -----------
-        if (FWD_UNIFORM_ISSUE || lane == 0) {
+        {
             constexpr uint32_t IDESC_O = mx::mma_idesc_bf16(BM, HD, false, true);
             bool ok = true;
             uint32_t g = 0;            // K/V tiles consumed so far, over all items
@@ -314,15 +339,16 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             for (int it = 0; ok && fwd_item(P, it, bh, q0); ++it) {
                 int n_it[QT];
 #pragma unroll
-                for (int t = 0; t < QT; ++t) n_it[t] = fwd_tile_iters(P, q0, t);
+                for (int t = 0; t < QT; ++t) n_it[t] = fwd_tile_iters(P, q0, KEY_SPLIT ? 0 : t);
                 const int n_max = max(n_it[0], n_it[1]);
+                const bool own_o = !KEY_SPLIT || !fwd_fast_head(P, bh, lane);   // each pair of groups sums into an O of its own
                 for (int j = 0; j < n_max && ok; ++j, ++g) {
                     const int s = g % KV_STAGES;
                     ok = ISSUER_WAIT(mx::mbar_wait(bar(BAR_V_FULL + s), (g / KV_STAGES) & 1, abort_flag, P.status));
                     const uint64_t b = mx::smem_desc_sw128(smem_base + SMEM_V + s * TILE_BYTES);
 #pragma unroll
                     for (int t = 0; t < QT; ++t) {
-                        if (!ok || j >= n_it[t]) continue;
+                        if (!ok || j >= n_it[t] || (KEY_SPLIT && (j & 1) != t)) continue;
                         // an item's first P_t is written after the softmax group has taken the previous item's
                         // O_t out of tensor memory, so overwriting O_t (j == 0) needs no barrier of its own
                         ok = ISSUER_WAIT(mx::mbar_wait(bar(BAR_P_FULL + t), cp[t] & 1, abort_flag, P.status));
@@ -331,8 +357,8 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                         if (ISSUER_LANE) {
 #pragma unroll
                             for (int k = 0; k < BN / 16; ++k)  // 16 keys: 8 packed columns of P, 2048 bytes of V
-                                mx::mma_ts(tmem + TM_O + t * HD, tmem + TM_P + t * (BN / 2) + 8 * k, b + 128 * k,
-                                           IDESC_O, (j > 0 || k > 0));
+                                mx::mma_ts(tmem + TM_O + (own_o ? t * HD : 0), tmem + TM_P + t * (BN / 2) + 8 * k, b + 128 * k,
+                                           IDESC_O, (j > (KEY_SPLIT && own_o ? t : 0) || k > 0));
                             mx::mma_commit(bar(BAR_O_DONE + t));
                         }
                         ++cp[t];
@@ -351,7 +377,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         // latencies; without a row max (the usual mode) the halves never talk to each other inside the loop, and the
         // general mode has each half compute the full row's max redundantly rather than exchange it.
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(FWD_REGS_SOFTMAX));
-        const int t = warp >> 3;             // query tile of this group
+        const int t = warp >> 3;             // query tile of this group (key-split form: parity of its key tiles)
         const int half = (warp >> 2) & 1;    // which 64 key columns of every tile
         const int row_in_tile = (warp & 3) * 32 + lane;
         const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
@@ -359,18 +385,39 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         const uint32_t tm_s = tm_s_tile + half * (BN / 2);
         const uint32_t tm_p = tmem + lane_off + TM_P + t * (BN / 2) + half * (BN / 4);
         const uint32_t tm_o = tmem + lane_off + TM_O + t * HD;
-        // Scores arrive in log2 units when Q was staged pre-multiplied by scale * log2(e) (c = 1), else raw (c = scale * log2(e)).
-        const bool i8_scores = P.row_a != nullptr;   // scores rebuilt from integer dots: already in log2 units
-        const float c = (P.prescaled || i8_scores) ? 1.0f : 0.125f * 1.4426950408889634f;
-        const float l_scale = (P.prescaled || i8_scores) ? 0.6931471805599453f : 0.125f;   // running max -> natural-log units
+        // Scores arrive in log2 units when Q was staged pre-multiplied by scale * log2(e) or when they are rebuilt from
+        // integer dots (c = 1), else raw (c = scale * log2(e)).
+        constexpr float c = SRC == SRC_RAW ? MX230_QK_LOG2_SCALE : 1.0f;
+        constexpr float l_scale = SRC == SRC_RAW ? 0.125f : 0.6931471805599453f;   // running max -> natural-log units
         bool ok = true;
         uint32_t cnt = 0;  // score tiles this group has taken so far, over all items
+        uint32_t cnt1 = 0; // key-split form: odd key tiles so far (what groups 2, 3 count in cnt)
+        uint32_t g0 = 0;   // key tiles of the items so far (int8 scores: ring position)
         uint32_t xmc = 0;  // row-max exchanges this group has made so far (general-mode tiles only)
         int bh, q0;
         for (int it = 0; ok && fwd_item(P, it, bh, q0); ++it) {
-        const int n_t = fwd_tile_iters(P, q0, t);
-        const int row = q0 + t * BM + row_in_tile;
+        const int n_all = KEY_SPLIT ? fwd_tile_iters(P, q0, 0) : 0;
+        const int n_t = KEY_SPLIT ? (n_all + 1 - t) >> 1 : fwd_tile_iters(P, q0, t);
+        const int row0 = q0 + (KEY_SPLIT ? 0 : t * BM);   // first row of this group's query tile
+        const int row = row0 + row_in_tile;
         const int qbuf = it & 1;
+        auto key_tile = [&](int j) { return KEY_SPLIT ? 2 * j + t : j; };
+        float row_a = 0.0f, row_qsum = 0.0f;
+        if (SRC == SRC_I8 && row < NQ) {
+            row_a = P.row_a[(size_t)bh * NQ + row];
+            row_qsum = P.row_qsum[(size_t)bh * NQ + row];
+        }
+        // int8 scores: ks (and BN floats further kb) of this half's columns of the group's j-th key tile
+        auto kskb_of = [&](int j) {
+            return (const float *)(smem + SMEM_KSKB + ((g0 + (uint32_t)key_tile(j)) % KSKB_SLOTS) * KSKB_BYTES) + half * (BN / 2);
+        };
+        // key-split form: O_1 of the previous item has been read (asked once per item by both halves of tile 1, so that
+        // they stay in step with the reader)
+        auto o1_free = [&]() {
+            if (KEY_SPLIT && t == 1 && it > 0)
+                return (bool)__all_sync(0xFFFFFFFFu, mx::mbar_wait(bar(BAR_O1_READ), (it - 1) & 1, abort_flag, P.status));
+            return true;
+        };
         const int last = P.causal ? min(N - 1, row + P.q_off) : N - 1;  // last visible key of this row
         // Fixed-reference mode, chosen per head: when |q . k| * scale * log2(e) <= 80 for every row pair of the head --
         // by Cauchy-Schwarz from the largest row norms of Q and K that the staging pass left -- the probabilities are
@@ -378,32 +425,50 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         // fp32 sums carry the same relative precision at 2^-80 .. 2^80 as around 1, every row sum stays inside
         // [2^-80, N 2^80], and the result is that of the max-subtracted form.  Heads with larger scores (and calls
         // without the norms) take the general path: running max, lazy rescale.
-        bool fast = false;
-        if (FWD_FAST && P.q_norm2 != nullptr) {
-            float nq = 0.0f, nk = 0.0f;
-            if (lane < MX230_NORM_PARTS) {
-                nq = P.q_norm2[(size_t)bh * MX230_NORM_PARTS + lane];
-                nk = P.k_norm2[(size_t)(bh / P.kv_group) * MX230_NORM_PARTS + lane];
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                nq = fmaxf(nq, __shfl_xor_sync(0xFFFFFFFFu, nq, o));
-                nk = fmaxf(nk, __shfl_xor_sync(0xFFFFFFFFu, nk, o));
-            }
-            // the norms are those of the fp32 values; rounding to bf16 moves a norm by less than 0.4 %
-            fast = nq * nk * (MX230_QK_LOG2_SCALE * MX230_QK_LOG2_SCALE) <= 80.0f * 80.0f;
-        }
-        float m = fast ? 0.0f : -CUDART_INF_F, l = 0.0f;   // l: this half's share of the row sum
-        float l_norm = 0.0f;   // what O is divided by (fast mode: see below; general mode: l)
+        const bool fast = fwd_fast_head(P, bh, lane);
+        float m = fast ? 0.0f : -CUDART_INF_F, l = 0.0f;   // l: this group's share of the row sum
+        float l_odd = 0.0f;    // pair form, fast mode: the sum over odd key tiles, l being that over even ones
+        // Shares of the row sums, handed to the group that does the epilogue: [publisher][sum, second sum or max, correction].
+        // The correction (what the first key tile's rounding adds to the sum that O is divided by: fast mode, see below) is
+        // parked there from the first tile on, by the groups that publish nothing as well, instead of in a register.
+        float *xch = (float *)(smem + SMEM_XCH) + (it & 1) * XCH_PUBS * 3 * BM + row_in_tile;
+        float *slot = xch + (KEY_SPLIT ? 2 * t + half - 1 : t) * 3 * BM;
+        float *park = half == 1 || (KEY_SPLIT && t == 1) ? slot + 2 * BM : xch + (2 * 3 + (KEY_SPLIT ? 2 : t)) * BM;
         uint32_t va[32], vb[32];
+        // int8 scores: exact integer dots -> row_a * (dot * ks + qsum * kb), two keys per instruction
+        auto rebuild32 = [&](uint32_t *x, const float *kskb) {
+            const uint64_t qs2 = mx::pk2(row_qsum, row_qsum), ra2 = mx::pk2(row_a, row_a);
+#pragma unroll
+            for (int i = 0; i < 32; i += 4) {
+                const float4 k4 = *(const float4 *)(kskb + i), b4 = *(const float4 *)(kskb + BN + i);
+                const uint64_t u = mx::fma2(mx::pk2(__uint_as_float(x[i]), __uint_as_float(x[i + 1])), mx::pk2(k4.x, k4.y),
+                                            mx::mul2(qs2, mx::pk2(b4.x, b4.y)));
+                const uint64_t w = mx::fma2(mx::pk2(__uint_as_float(x[i + 2]), __uint_as_float(x[i + 3])), mx::pk2(k4.z, k4.w),
+                                            mx::mul2(qs2, mx::pk2(b4.z, b4.w)));
+                float a, b;
+                mx::upk2(mx::mul2(ra2, u), a, b);
+                x[i] = __float_as_uint(a), x[i + 1] = __float_as_uint(b);
+                mx::upk2(mx::mul2(ra2, w), a, b);
+                x[i + 2] = __float_as_uint(a), x[i + 3] = __float_as_uint(b);
+            }
+        };
         if (fast) {
         // ---- max-free loop: the group's second 32 columns land under the exponentials of the first 32
-        uint64_t rs2[2] = {0ull, 0ull};
-        float rs[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        auto exp32 = [&](const uint32_t *src, uint32_t *pk, int key_base, bool need_mask) {
+        uint64_t rs2;              // sum of one score tile
+        float l_other = 0.0f;      // pair form: l and l_other change places after every tile: sums over even and odd key tiles
+        auto exp32 = [&](const uint32_t *src, uint32_t *pk, int key_base, bool need_mask, const float *kskb, bool start) {
             uint32_t x[32];
 #pragma unroll
             for (int i = 0; i < 32; ++i) x[i] = src[i];
+            if (SRC == SRC_RAW) {
+#pragma unroll
+                for (int i = 0; i < 32; i += 2) {
+                    float a, b;
+                    mx::upk2(mx::mul2(mx::pk2(__uint_as_float(x[i]), __uint_as_float(x[i + 1])), mx::pk2(c, c)), a, b);
+                    x[i] = __float_as_uint(a), x[i + 1] = __float_as_uint(b);
+                }
+            }
+            if (SRC == SRC_I8) rebuild32(x, kskb);
             if (need_mask) {   // diagonal and ragged tiles only (a warp-uniform branch: full tiles pay nothing)
 #pragma unroll
                 for (int i = 0; i < 32; ++i)
@@ -419,12 +484,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                     p1 = mx::ex2(__uint_as_float(x[i + 1]));
                 }
                 pk[i >> 1] = mx::pack_bf16(p0, p1);
-                if (FWD_ADD2) {
-                    rs2[(i >> 1) & 1] = mx::add2(rs2[(i >> 1) & 1], mx::pk2(p0, p1));
-                } else {
-                    rs[i & 2] += p0;
-                    rs[(i & 2) + 1] += p1;
-                }
+                rs2 = start && i == 0 ? mx::pk2(p0, p1) : mx::add2(rs2, mx::pk2(p0, p1));
             }
         };
         // First key tile only: the sum of the ROUNDED probabilities as well.  Rows that see a handful of keys live
@@ -433,19 +493,14 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         // bf16(p) / p, or dO . O stops cancelling against dP in the backward.  Everywhere else a row sums so many
         // terms that the two sums differ far below the rounding of V itself, and the fp32 sum serves both uses.
         float rb[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        float l_first = 0.0f;   // fp32 sum of the first tile
         auto sum_rounded16 = [&](const uint32_t *pk) {
 #pragma unroll
             for (int w = 0; w < 16; ++w) mx::add_bf16x2(pk[w], rb[(w & 1) * 2], rb[(w & 1) * 2 + 1]);
         };
-        auto sum_now = [&]() {
-            if (FWD_ADD2) {
-                float a0, a1, a2, a3;
-                mx::upk2(rs2[0], a0, a1);
-                mx::upk2(rs2[1], a2, a3);
-                return (a0 + a1) + (a2 + a3);
-            }
-            return (rs[0] + rs[1]) + (rs[2] + rs[3]);
+        auto sum_of = [](uint64_t v) {
+            float a0, a1;
+            mx::upk2(v, a0, a1);
+            return a0 + a1;
         };
         // one score tile; FIRST (a compile-time flag: the loop below stays free of the first tile's extra work) also
         // takes the sums of the rounded probabilities
@@ -457,10 +512,11 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             mx::tmem_ld32(tm_s, va);
             mx::tmem_wait_ld();                                       // va is in registers
             mx::tmem_ld32(tm_s + 32, vb);                             // lands under the first exponentials
-            const int key0 = j * BN;
-            const bool need_mask = (key0 + BN > N) || (P.causal && key0 + BN - 1 > q0 + t * BM + P.q_off);
+            const int key0 = key_tile(j) * BN;
+            const bool need_mask = (key0 + BN > N) || (P.causal && key0 + BN - 1 > row0 + P.q_off);
+            const float *kskb = SRC == SRC_I8 ? kskb_of(j) : nullptr;
             uint32_t pk[16];
-            exp32(va, pk, key0 + half * (BN / 2), need_mask);
+            exp32(va, pk, key0 + half * (BN / 2), need_mask, kskb, true);
             mx::tmem_wait_ld();                                       // this group's columns have left S_t
             mx::tc_fence_before();
             __syncwarp();
@@ -474,17 +530,27 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 mx::tc_fence_after();
             }
             mx::tmem_st16(tm_p, pk);
-            if (FIRST) sum_rounded16(pk);
-            exp32(vb, pk, key0 + half * (BN / 2) + 32, need_mask);
+            if (FIRST && !(KEY_SPLIT && t == 1)) sum_rounded16(pk);
+            exp32(vb, pk, key0 + half * (BN / 2) + 32, need_mask, kskb + 32, false);
             mx::tmem_st16(tm_p + 16, pk);
             if (FIRST) {
-                sum_rounded16(pk);
-                l_first = sum_now();
+                if (!(KEY_SPLIT && t == 1)) {
+                    sum_rounded16(pk);
+                    *park = ((rb[0] + rb[1]) + (rb[2] + rb[3])) - sum_of(rs2);
+                }
+                if (!o1_free()) return false;
             }
             mx::tmem_wait_st();
             mx::tc_fence_before();
             __syncwarp();
             if (lane == 0) mx::mbar_arrive(bar(BAR_P_FULL + t));
+            const float l_new = l + sum_of(rs2);
+            if (KEY_SPLIT) {
+                l = l_new;
+            } else {   // the next key tile has the other parity
+                l = l_other;
+                l_other = l_new;
+            }
             return true;
         };
         if (n_t > 0) {
@@ -495,17 +561,14 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 ++cnt;
             }
         }
-        l = sum_now();
-        l_norm = l - l_first + ((rb[0] + rb[1]) + (rb[2] + rb[3]));
+        if (!KEY_SPLIT) {
+            l_odd = (n_t & 1) ? l : l_other;
+            if (n_t & 1) l = l_other;
+        }
         } else {
         // ---- general loop: running row max, raised lazily.  Each half takes the max of its own 64 columns and the two
         // exchange them through shared memory (one bounded barrier per tile and query tile); both then hold the same
         // row max and take the same decisions, exponentiate their own columns and rescale their own 32 columns of O.
-        float row_a = 0.0f, row_qsum = 0.0f;
-        if (i8_scores && row < NQ) {
-            row_a = P.row_a[(size_t)bh * NQ + row];
-            row_qsum = P.row_qsum[(size_t)bh * NQ + row];
-        }
         float *xmax = (float *)(smem + SMEM_XMAX) + t * 2 * HALVES * BM;   // [2 tile parities][HALVES][BM]
         for (int j = 0; j < n_t; ++j, ++cnt) {
             ok = __all_sync(0xFFFFFFFFu, mx::mbar_wait(bar(BAR_S_FULL + t), cnt & 1, abort_flag, P.status));
@@ -517,18 +580,13 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             mx::tc_fence_before();
             __syncwarp();
             if (lane == 0) mx::mbar_arrive(bar(BAR_S_FREE + t));   // this group's columns have left S_t
-            const int key0 = j * BN, col0 = half * (BN / 2);
-            if (i8_scores) {
-                // the tile holds exact integer dots of int8 codes: the reference kernel's score for them
-                const float2 *cs = P.col_kskb + (size_t)(bh / P.kv_group) * P.n_k_pad + key0 + col0;
-#pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                    const float2 k0 = __ldg(cs + i), k1 = __ldg(cs + 32 + i);
-                    va[i] = __float_as_uint(row_a * fmaf(__uint_as_float(va[i]), k0.x, row_qsum * k0.y));
-                    vb[i] = __float_as_uint(row_a * fmaf(__uint_as_float(vb[i]), k1.x, row_qsum * k1.y));
-                }
+            const int key0 = key_tile(j) * BN, col0 = half * (BN / 2);
+            if (SRC == SRC_I8) {   // the tile holds exact integer dots of int8 codes: the reference kernel's score for them
+                const float *kskb = kskb_of(j);
+                rebuild32(va, kskb);
+                rebuild32(vb, kskb + 32);
             }
-            if ((key0 + BN > N) || (P.causal && key0 + BN - 1 > q0 + t * BM + P.q_off)) {
+            if ((key0 + BN > N) || (P.causal && key0 + BN - 1 > row0 + P.q_off)) {
 #pragma unroll
                 for (int i = 0; i < 32; ++i) {
                     if (key0 + col0 + i > last) va[i] = 0xFF800000u;  // -inf
@@ -557,7 +615,8 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             const bool raise = (j == 0) || ((mx_ - m) * c > RESCALE_LOG2);
             const float m_new = raise ? mx_ : m;
             const float alpha = (raise && j > 0) ? mx::ex2((m - m_new) * c) : 1.0f;
-            const float nmc = -m_new * c;
+            // (key-split form: a row may see none of the group's first key tiles; its max is still -inf then)
+            const float nmc = KEY_SPLIT && m_new == -CUDART_INF_F ? 0.0f : -m_new * c;
             if (j > 0) {
                 // P_t and O_t are stable once the previous P V has completed
                 ok = __all_sync(0xFFFFFFFFu,
@@ -598,51 +657,88 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             mx::tmem_st16(tm_p + 16, pk);
             l = l * alpha + ((rs[0] + rs[1]) + (rs[2] + rs[3]));
             m = m_new;
+            if (KEY_SPLIT && j == 0) {
+                ok = o1_free();
+                if (!ok) break;
+            }
             mx::tmem_wait_st();
             mx::tc_fence_before();
             __syncwarp();
             if (lane == 0) mx::mbar_arrive(bar(BAR_P_FULL + t));
         }
-        l_norm = l;
         }
-        // The two halves of a row add their sums: half 1 publishes its pair and goes on to the next item, half 0 waits
-        // for it (and for the tile's last P V) and does the tile's epilogue.
-        float *xch = (float *)(smem + SMEM_XCH) + ((it & 1) * QT + t) * 2 * BM;
-        if (half == 1) {
+        if (KEY_SPLIT && n_t == 0 && ok) ok = o1_free();
+        // The groups of a row add their sums: half 1 (key-split form: every group but the first) publishes its share and
+        // goes on to the next item; the first group waits for it, and for the last P V, and does the tile's epilogue.
+        float l_norm = 0.0f;             // what O is divided by
+        float w0 = 1.0f, w1 = 1.0f;      // key-split form, general mode: weights of O_0 and O_1
+        if (half == 1 || (KEY_SPLIT && t == 1)) {
             // (the tile's last P V must have read this group's share of P_t before the next item's first tile overwrites it)
             if (ok && n_t > 0)
                 ok = __all_sync(0xFFFFFFFFu, mx::mbar_wait(bar(BAR_O_DONE + t), (cnt - 1) & 1, abort_flag, P.status));
             if (ok) {
-                xch[row_in_tile] = l;
-                xch[BM + row_in_tile] = l_norm;
+                slot[0] = l;
+                slot[BM] = KEY_SPLIT ? m : l_odd;
                 __syncwarp();
-                if (lane == 0) mx::mbar_arrive(bar(BAR_XCH + t));
+                if (lane == 0) mx::mbar_arrive(bar(BAR_XCH + (KEY_SPLIT ? 0 : t)));
             }
         } else if (ok) {
             ok = __all_sync(0xFFFFFFFFu, mx::mbar_wait(bar(BAR_XCH + t), it & 1, abort_flag, P.status));
             if (ok) {
-                l += xch[row_in_tile];
-                l_norm += xch[BM + row_in_tile];
+                const float *other = xch + (KEY_SPLIT ? 0 : t) * 3 * BM;   // half 1 of this tile
+                l += other[0];
+                const float corr = fast ? *park + other[2 * BM] : 0.0f;
+                if (KEY_SPLIT) {
+                    l_odd = other[3 * BM] + other[6 * BM];
+                    if (!fast) {
+                        const float m1 = other[4 * BM], mm = fmaxf(m, m1);
+                        w0 = mx::ex2((m - mm) * c);   // m is finite: key tile 0 has a key that every row sees
+                        w1 = mx::ex2((m1 - mm) * c);
+                        l *= w0, l_odd *= w1;
+                        m = mm;
+                    }
+                } else {
+                    l_odd += other[BM];
+                }
+                l += l_odd;
+                l_norm = l + corr;
             }
         }
+        if (KEY_SPLIT) cnt1 += (uint32_t)(n_all >> 1);
         // epilogue: O / l and the log-sum-exp
-        if (ok && n_t > 0 && half == 0) {
+        if (ok && n_t > 0 && half == 0 && !(KEY_SPLIT && t == 1)) {
+            const bool odd = KEY_SPLIT && n_all > 1, two = odd && !fast;   // O_1 holds something
             ok = __all_sync(0xFFFFFFFFu,
                             mx::mbar_wait(bar(BAR_O_DONE + t), (cnt - 1) & 1, abort_flag, P.status));
+            if (ok && odd) ok = __all_sync(0xFFFFFFFFu, mx::mbar_wait(bar(BAR_O_DONE + 1), (cnt1 - 1) & 1, abort_flag, P.status));
             if (ok) {
                 mx::tc_fence_after();
                 const float inv = 1.0f / l_norm;
+                auto load_o = [&](int cc) {   // 32 columns of the row's sum into va
+                    mx::tmem_ld32(tm_o + cc * 32, va);
+                    if (two) mx::tmem_ld32(tm_o + HD + cc * 32, vb);
+                    mx::tmem_wait_ld();
+                    if (two) {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i)
+                            va[i] = __float_as_uint(__uint_as_float(va[i]) * w0 + __uint_as_float(vb[i]) * w1);
+                    }
+                    if (KEY_SPLIT && cc == HD / 32 - 1) {   // O_1 has been read: the odd groups may go on to the next item
+                        mx::tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mx::mbar_arrive(bar(BAR_O1_READ));
+                    }
+                };
                 float *orow = P.O + (size_t)bh * P.o_head_stride + (size_t)row * P.o_row_stride;
                 if (P.tma_out) {
                     // each warp stages its 32 rows, 32 columns at a time, in a swizzled 4 KB piece of this tile's Q
                     // buffer (its last Q K^T has completed) and hands it to the TMA unit, which clips rows past the
                     // end: 16-byte stores from lane = row registers each touch a sector of their own
-                    const int wrow0 = q0 + t * BM + (warp & 3) * 32;
+                    const int wrow0 = row0 + (warp & 3) * 32;
                     const int st_off = SMEM_Q + (qbuf * QT + t) * TILE_BYTES + (warp & 3) * 4096;
 #pragma unroll 1
                     for (int cc = 0; cc < HD / 32; ++cc) {
-                        mx::tmem_ld32(tm_o + cc * 32, va);
-                        mx::tmem_wait_ld();
+                        load_o(cc);
                         unsigned char *srow = smem + st_off + lane * 128;
 #pragma unroll
                         for (int cch = 0; cch < 8; ++cch)
@@ -661,8 +757,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 } else
 #pragma unroll 1
                 for (int cc = 0; cc < HD / 32; ++cc) {
-                    mx::tmem_ld32(tm_o + cc * 32, va);
-                    mx::tmem_wait_ld();
+                    load_o(cc);
                     if (row < NQ) {
 #pragma unroll
                         for (int i = 0; i < 32; i += 4) {
@@ -678,6 +773,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         // this warp no longer touches the item's Q buffer (operand of its tile's Q K^T, then staging space)
         __syncwarp();
         if (ok && lane == 0) mx::mbar_arrive(bar(BAR_Q_EMPTY + qbuf));
+        g0 += KEY_SPLIT ? n_all : max(fwd_tile_iters(P, q0, 0), fwd_tile_iters(P, q0, 1));
         }  // items
     }
 
@@ -685,6 +781,10 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     mx::tc_fence_before();
     __syncthreads();
     mx::tc_fence_after();
+    // The next kernel may move in from here on, when every warp is done.  Not earlier: what follows a long kernel would
+    // fill the SMs that finish first with all of its blocks and find them unevenly spread when it may start (48 x 4096
+    // rows, next call's cast: 9 us slower with the trigger at the top).
+    mx::pdl_trigger();
     if (warp == SOFT_WARPS + 1) mx::tmem_dealloc(tmem, TM_COLS);
 }
 
@@ -704,6 +804,8 @@ struct CastParams {
 // the bf16 copies, which the attention kernels read next, out of L2), 8-byte stores.  A row of 64 values is 16
 // neighbouring lanes, so its squared norm costs four shuffles on a kernel that waits for memory anyway.
 __global__ void __launch_bounds__(256) cast_bf16_kernel(const CastParams P) {
+    mx::pdl_trigger();
+    mx::pdl_wait();
     const size_t n4 = P.per_head4;
     const size_t base = (size_t)blockIdx.z * n4;
     const size_t step = (size_t)gridDim.x * blockDim.x;
@@ -787,9 +889,55 @@ int mx230_launch_cast(mx230_handle *h, cudaStream_t st, const float *const *src,
     if (parts < 1) parts = 1;
     if (norm2 != nullptr && parts > MX230_NORM_PARTS) parts = MX230_NORM_PARTS;
     if (parts > 65535) parts = 65535;
-    MX_LAUNCH(h, st, MX230_K_CAST, (cast_bf16_kernel<<<dim3((unsigned)parts, slices, heads), 256, 0, st>>>(P)));
+    MX_LAUNCH(h, st, MX230_K_CAST, mx_launch(cast_bf16_kernel, dim3((unsigned)parts, slices, heads), 256, 0, st, 1, true, P));
     return MX230_OK;
 }
+
+namespace {
+
+// Which form a call takes.  Work is counted in 128 x 128 score tiles; the items of a form go to the SMs heaviest first in
+// snake order, and the call takes as long as the fullest SM.  A pair item (two query tiles) costs the tiles of both (one and
+// a half times the tiles where it has only one: half the softmax groups idle), a key-split item 1.2 times those of its query
+// tile (it reads every K/V tile for one query tile only) plus one.  Key-split items are half as large, so they even out
+// calls with few items.  Measured (us a call, pair / key-split; 12 heads unless given): 1000 rows causal 20.8 / 15.7, 2048
+// rows causal 33.7 / 25.4, 1 x 8192 rows 87 / 54, 24 x 4096 rows causal 101 / 111, 96 x 4096 rows causal 352 / 411.
+bool fwd_key_split(int heads, int n_q, int n_k, int q_off, int causal, int sms) {
+    const int tiles = (n_q + BM - 1) / BM, pairs = (tiles + 1) / 2, n_kv = (n_k + BN - 1) / BN;
+    if (sms > 256 || (long long)pairs * heads > 4LL * sms) return false;
+    auto iters = [&](int t) {
+        if (!causal) return n_kv;
+        const long long k = ((long long)t * BM + BM - 1 + q_off) / BN + 1;
+        return (int)(k < n_kv ? k : n_kv);
+    };
+    auto fullest = [&](bool split) {
+        long long load[256] = {}, most = 0;
+        const int blocks = split ? tiles : pairs;
+        for (int rank = 0, i = 0; rank < blocks; ++rank) {
+            const int b = causal ? blocks - 1 - rank : rank;
+            long long cost;   // in tenths of a tile
+            if (split) cost = 12LL * iters(b) + 10;
+            else cost = 2 * b + 1 < tiles ? 10LL * (iters(2 * b) + iters(2 * b + 1)) : 15LL * iters(2 * b);
+            for (int h = 0; h < heads; ++h, ++i) {
+                const int r = i / sms, c = (r & 1) ? sms - 1 - i % sms : i % sms;
+                load[c] += cost;
+                most = load[c] > most ? load[c] : most;
+            }
+        }
+        return most;
+    };
+    return fullest(true) < fullest(false);
+}
+
+template <int SRC, bool KEY_SPLIT>
+int launch_variant(mx230_handle *h, cudaStream_t st, dim3 grid, const CUtensorMap &tq, const CUtensorMap &tk,
+                   const CUtensorMap &tv, const CUtensorMap &to, const FwdParams &P) {
+    MX_SMEM_ATTR_ONCE(h->device, (flash_fwd_kernel<SRC, KEY_SPLIT>), SMEM_ALLOC);
+    MX_LAUNCH(h, st, MX230_K_FLASH_FWD,
+              mx_launch(flash_fwd_kernel<SRC, KEY_SPLIT>, grid, FWD_THREADS, SMEM_ALLOC, st, 1, true, tq, tk, tv, to, P));
+    return MX230_OK;
+}
+
+}  // namespace
 
 // General launcher.  Q: bf16 [heads][n_q][64]; K, V: bf16 [heads / kv_group][n_k][64].
 int mx230_launch_flash_fwd_ex(mx230_handle *h, cudaStream_t st, const void *Qb, const void *Kb,
@@ -812,14 +960,6 @@ int mx230_launch_flash_fwd_ex(mx230_handle *h, cudaStream_t st, const void *Qb, 
     if ((rc = mx230_make_tmap_bf16(h, &tq, Qb, n_q, heads, rs, (uint64_t)n_q * HD * 2, BM))) return rc;
     if ((rc = mx230_make_tmap_bf16(h, &tk, Kb, n_k, heads / kv_group, rs, (uint64_t)n_k * HD * 2, BN))) return rc;
     if ((rc = mx230_make_tmap_bf16(h, &tv, Vb, n_k, heads / kv_group, rs, (uint64_t)n_k * HD * 2, BN))) return rc;
-    // function attributes are per device: one handle per GPU may live in the same process
-    static bool attr_set[64] = {};
-    MX_REQUIRE(h->device >= 0 && h->device < 64, MX230_ERR_UNSUPPORTED, "flash forward: device index %d", h->device);
-    if (!attr_set[h->device]) {
-        MX_CHECK_CUDA(cudaFuncSetAttribute(flash_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           SMEM_ALLOC));
-        attr_set[h->device] = true;
-    }
     FwdParams P;
     P.O = O;
     P.L = L;
@@ -831,29 +971,28 @@ int mx230_launch_flash_fwd_ex(mx230_handle *h, cudaStream_t st, const void *Qb, 
     P.kv_group = kv_group;
     P.causal = causal ? 1 : 0;
     P.heads = heads;
-    // Two query tiles per item keep both softmax groups of a CTA busy; a call so small that every 128-row tile can have
-    // an SM of its own is cut into single-tile items instead (the second group idles, but twice as many SMs work).
-    // With more tiles than SMs the single-tile form would need a second round at two thirds of the two-tile pace per
-    // tile (measured: one head of 32768 rows, 0.51 ms against 0.37).
-    P.item_tiles = ((long long)heads * ((n_q + BM - 1) / BM) <= h->sm_count) ? 1 : QT;
+    const bool key_split = fwd_key_split(heads, n_q, n_k, q_off, causal, h->sm_count);
+    P.item_tiles = key_split ? 1 : QT;
     P.n_qblocks = (n_q + P.item_tiles * BM - 1) / (P.item_tiles * BM);
     MX_REQUIRE((long long)heads * P.n_qblocks <= 0x7FFFFFFF, MX230_ERR_UNSUPPORTED, "flash forward: too many query blocks");
     P.n_items = heads * P.n_qblocks;
     P.tma_out = tma_out ? 1 : 0;
-    P.prescaled = q_prescaled ? 1 : 0;
-    P.q_norm2 = (q_prescaled && q_norm2 && k_norm2) ? q_norm2 : nullptr;
+    P.q_norm2 = (q_norm2 && k_norm2) ? q_norm2 : nullptr;
     P.k_norm2 = P.q_norm2 ? k_norm2 : nullptr;
     P.test_drop_tile = h->test_drop_tile;
-    P.row_a = (row_a && row_qsum && col_kskb) ? row_a : nullptr;
-    P.row_qsum = P.row_a ? row_qsum : nullptr;
-    P.col_kskb = P.row_a ? (const float2 *)col_kskb : nullptr;
-    P.n_k_pad = (n_k + BN - 1) / BN * BN;
+    P.row_a = row_a;
+    P.row_qsum = row_qsum;
+    P.col_kskb = col_kskb;
+    P.n_k_tiles = (n_k + BN - 1) / BN;
     P.status = h->status_dev;
     // persistent: one CTA per SM (the kernel holds all of an SM's tensor memory), each walking its share of the items
     dim3 grid((unsigned)(P.n_items < h->sm_count ? P.n_items : h->sm_count));
-    MX_LAUNCH(h, st, MX230_K_FLASH_FWD,
-              (flash_fwd_kernel<<<grid, FWD_THREADS, SMEM_ALLOC, st>>>(tq, tk, tv, to, P)));
-    return MX230_OK;
+    if (row_a) return key_split ? launch_variant<SRC_I8, true>(h, st, grid, tq, tk, tv, to, P)
+                                : launch_variant<SRC_I8, false>(h, st, grid, tq, tk, tv, to, P);
+    if (q_prescaled) return key_split ? launch_variant<SRC_PRE, true>(h, st, grid, tq, tk, tv, to, P)
+                                      : launch_variant<SRC_PRE, false>(h, st, grid, tq, tk, tv, to, P);
+    return key_split ? launch_variant<SRC_RAW, true>(h, st, grid, tq, tk, tv, to, P)
+                     : launch_variant<SRC_RAW, false>(h, st, grid, tq, tk, tv, to, P);
 }
 
 int mx230_launch_flash_fwd(mx230_handle *h, cudaStream_t st, const void *Qb, const void *Kb,

@@ -7,221 +7,270 @@
 // cache (so under an int8 cache a token attends the *quantised* K/V of itself and of
 // its batch-mates, exactly as decode does).
 //
-// This design: two HBM-bound staging kernels bring the operands into the bf16 head-major
-// layout of the tcgen05 forward kernel (Q gathered from the strided qkv rows; K and V
-// gathered from the cache through the optional block table, int8 codes dequantised as
-// code*scale + beta first), then the same tensor-core flash kernel as the stage-2 forward
-// runs with the GQA head mapping (K/V head = h / group), the causal offset pos0 and the
-// reference's strided output layout.  KIND 2 of the reference (scores through on-the-fly
-// int8 K, an opt-in speed approximation on sm_61) is served by the exact-score path.
+// This design: one staging kernel, then the tensor-core flash kernel of the stage-2 forward with the GQA head mapping (K/V
+// head = h / group), the causal offset pos0 and the reference's strided output layout.  The staging kernel brings the
+// operands into that kernel's bf16 head-major layout (Q gathered from the strided qkv rows, K and V from the cache through
+// the optional block table) and, in the prefill step, does the work in front of attention in the same pass: RoPE on the
+// new rows, their K and V written to the cache (fp32 copy or int8 quantize-on-write) and staged from registers.
+// KIND 2 of the reference (scores through on-the-fly int8 K, an opt-in speed approximation on sm_61) is served over an
+// fp32 cache by quantising K while it is staged.
 #include "common.cuh"
 
 namespace {
 
 constexpr int HD = 64;
 
-// Largest value of `v` over the block (v >= 0), returned to thread 0
-__device__ __forceinline__ float block_max256(float v) {
-    __shared__ float part[8];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
-    __syncthreads();
-    if (threadIdx.x < 8) {
-        v = part[threadIdx.x];
-#pragma unroll
-        for (int o = 4; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xFFu, v, o));
-    }
-    return v;
+struct StageParams {
+    // operands of the attention kernel
+    __nv_bfloat16 *qout;             // [n_head][n_tok][64]
+    __nv_bfloat16 *kout, *vout;      // [n_kv_head][n_keys][64]
+    float *q_norm2, *k_norm2;        // [heads][MX230_NORM_PARTS] largest squared norm of the (dequantised) rows of each part
+    float *row_a, *row_qsum, *kskb;  // int8 scores: per-row factor and code sum; per-key scale and offset by tiles of 128
+    int i8_scores, n_k_tiles;
+    // inputs
+    float *qkv;
+    int stride, n_tok, pos0, n_keys, n_head, n_kv_head;
+    float *kcache, *vcache;          // fp32 cache, or
+    int8_t *kq, *vq;                 // int8 cache with
+    float *ks, *vs, *kb, *vb;        // per-(row, head) scale and (optional) beta
+    const int *bt;
+    int bs;
+    // the step's work in front of attention
+    int write_kv;                    // the new rows' K and V come from qkv and go to the cache (else they are in it)
+    int rope;
+    float theta;
+};
+
+constexpr int ST_THREADS = 512;
+constexpr int ST_CLUSTER = 4;        // CTAs that share one norm part
+constexpr int ST_GRID = MX230_NORM_PARTS * ST_CLUSTER;
+constexpr int ST_SUBS = 4;           // warps that share a token (they take its heads in turn)
+
+__device__ __forceinline__ size_t stage_row(const StageParams &P, int t) {
+    return P.bt ? (size_t)(P.bt[t / P.bs] * P.bs + t % P.bs) : (size_t)t;
+}
+__device__ __forceinline__ float *stage_kskb(const StageParams &P, int h, int t) {
+    return P.kskb + ((size_t)h * P.n_k_tiles + (t >> 7)) * 256 + (t & 127);
 }
 
-// out[h][r][0..63] (bf16) <- qkv[r*stride + h*64 + 0..63] * 1/sqrt(64) * log2(e), so that the attention
-// kernel's scores arrive in log2 units (one rounding, from the fp32 product).  Grid (MX230_NORM_PARTS, n_head): block
-// (p, h) stages the rows r = p (mod 32) of head h, eight threads per row, and leaves the largest squared norm of its
-// (unscaled) rows in norm2[h][p]: with the keys' norms that bounds every score of the head, which lets the attention
-// kernel run without a row max.
-__global__ void stage_q_kernel(__nv_bfloat16 *out, float *norm2, const float *qkv, int n_tok, int n_head, int stride) {
-    const int p = blockIdx.x, h = blockIdx.y;
-    const int c = threadIdx.x & 7, slot = threadIdx.x >> 3;
-    const float sc = MX230_QK_LOG2_SCALE;
-    float best = 0.0f;
-    for (int r0 = p; r0 < n_tok; r0 += MX230_NORM_PARTS * 32) {
-        const int r = r0 + MX230_NORM_PARTS * slot;
-        float ss = 0.0f;
-        if (r < n_tok) {
-            const float4 *src = (const float4 *)(qkv + (size_t)r * stride + h * HD + c * 8);
-            const float4 a = src[0], b = src[1];
-            ss = a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w + b.x * b.x + b.y * b.y + b.z * b.z + b.w * b.w;
-            uint4 o;
-            o.x = mx::pack_bf16(a.x * sc, a.y * sc);
-            o.y = mx::pack_bf16(a.z * sc, a.w * sc);
-            o.z = mx::pack_bf16(b.x * sc, b.y * sc);
-            o.w = mx::pack_bf16(b.z * sc, b.w * sc);
-            *(uint4 *)(out + ((size_t)h * n_tok + r) * HD + c * 8) = o;
+// 128 CTAs whatever the size: the kernel is a few microseconds of latency (launch, one or two memory round trips), so what
+// counts is that it is ONE launch and that every thread's loads are issued together.  In its place stood rope 5.4 us,
+// quantise 4, two staging kernels 3.8 + 4 (512 tokens over 1536 cached keys, int8), and 11.7 + 5 + 4.7 + 5 (1900 tokens,
+// fp32).  New tokens: four warps per token, lane l holds dims l and l + 32 of a head, so RoPE's angle is computed once
+// per token and warp and a head's quantiser is a warp reduction.  Cached keys: eight threads per key and head, eight dims
+// each.  Row norms go through shared memory and, per cluster of four CTAs, into one of MX230_NORM_PARTS parts: with Q's
+// and K's the attention kernel bounds every score of a head and, where the bound is small, runs without a row max.
+__global__ void __launch_bounds__(ST_THREADS) prefill_stage_kernel(const StageParams P) {
+    extern __shared__ int smax[];    // [n_head + n_kv_head] squared norms as ordered integers (NaN largest)
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int n_max = P.n_head + P.n_kv_head;
+    mx::pdl_trigger();
+    for (int i = tid; i < n_max; i += ST_THREADS) smax[i] = 0;
+    __syncthreads();
+    mx::cluster_arrive_release();    // waited for before this CTA adds to the first one's maxima
+    mx::pdl_wait();
+    auto raise = [&](int head, float norm2) { atomicMax(&smax[head], __float_as_int(norm2) & 0x7FFFFFFF); };
+    const size_t kvd = (size_t)P.n_kv_head * HD;
+
+    // ---- new tokens ----
+    const int n_units = P.n_head + (P.write_kv ? 2 * P.n_kv_head : 0);
+    const int sub = warp & (ST_SUBS - 1);
+    for (int tok = blockIdx.x + ST_GRID * (warp / ST_SUBS); tok < P.n_tok; tok += ST_GRID * (ST_THREADS / 32 / ST_SUBS)) {
+        const int pos = P.pos0 + tok;
+        float *row = P.qkv + (size_t)tok * P.stride;
+        const size_t crow = P.write_kv ? stage_row(P, pos) : 0;
+        float cs = 1.0f, sn = 0.0f;
+        bool have_angle = false;
+        for (int u0 = sub; u0 < n_units; u0 += 4 * ST_SUBS) {
+            float va[4], vb[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int u = u0 + i * ST_SUBS;
+                if (u < n_units) va[i] = row[u * HD + lane], vb[i] = row[u * HD + 32 + lane];
+            }
+            if (P.rope && !have_angle) {
+                mx::rope_angle(pos, lane, HD, P.theta, cs, sn);
+                have_angle = true;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int u = u0 + i * ST_SUBS;
+                if (u >= n_units) break;
+                float a = va[i], b = vb[i];
+                if (P.rope && u < n_max) {   // Q and K heads
+                    mx::rope_pair(a, b, cs, sn);
+                    row[u * HD + lane] = a, row[u * HD + 32 + lane] = b;
+                }
+                if (u < P.n_head) {
+                    __nv_bfloat16 *dst = P.qout + ((size_t)u * P.n_tok + tok) * HD;
+                    if (P.i8_scores) {
+                        // q row -> int8 codes per (row, head): id = 127 / amax, code = clamp(rne(q * id), +-127); the
+                        // codes go out as bf16 (exact), with the row's score factor (amax / 127) * 1/sqrt(64) * log2(e)
+                        // and the sum of its codes (the reference's own arithmetic, llm.cu:3700-3716)
+                        float amax = fmaxf(fabsf(a), fabsf(b));
+#pragma unroll
+                        for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
+                        const float id = amax > 0.0f ? __fdiv_rn(127.0f, amax) : 0.0f;
+                        const int ca = max(-127, min(127, __float2int_rn(a * id))), cb = max(-127, min(127, __float2int_rn(b * id)));
+                        const int sum = __reduce_add_sync(0xFFFFFFFFu, ca + cb), sq = __reduce_add_sync(0xFFFFFFFFu, ca * ca + cb * cb);
+                        dst[lane] = __float2bfloat16((float)ca);
+                        dst[lane + 32] = __float2bfloat16((float)cb);
+                        if (lane == 0) {
+                            const float qs = amax > 0.0f ? __fdiv_rn(amax, 127.0f) : 0.0f;
+                            P.row_a[(size_t)u * P.n_tok + tok] = qs * 0.125f * 1.4426950408889634f;
+                            P.row_qsum[(size_t)u * P.n_tok + tok] = (float)sum;
+                            raise(u, qs * qs * (float)sq);
+                        }
+                    } else {
+                        // values times 1/sqrt(64) * log2(e), one rounding: the scores arrive in log2 units
+                        dst[lane] = __float2bfloat16_rn(a * MX230_QK_LOG2_SCALE);
+                        dst[lane + 32] = __float2bfloat16_rn(b * MX230_QK_LOG2_SCALE);
+                        float ss = a * a + b * b;
+#pragma unroll
+                        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, o);
+                        if (lane == 0) raise(u, ss);
+                    }
+                    continue;
+                }
+                const bool is_v = u >= n_max;
+                const int h = is_v ? u - n_max : u - P.n_head;
+                __nv_bfloat16 *dst = (is_v ? P.vout : P.kout) + ((size_t)h * P.n_keys + pos) * HD;
+                float x0 = a, x1 = b;   // what attention sees
+                if (P.kq) {
+                    int8_t *cdst = (is_v ? P.vq : P.kq) + crow * kvd + h * HD;
+                    float *sc = is_v ? P.vs : P.ks, *be = is_v ? P.vb : P.kb;
+                    int c0, c1;
+                    float scale, beta;
+                    mx::quant_head_row(a, b, be != nullptr, c0, c1, scale, beta);
+                    cdst[lane] = (int8_t)c0, cdst[lane + 32] = (int8_t)c1;
+                    if (lane == 0) {
+                        sc[crow * P.n_kv_head + h] = scale;
+                        if (be) be[crow * P.n_kv_head + h] = beta;
+                    }
+                    x0 = (float)c0 * scale + beta, x1 = (float)c1 * scale + beta;
+                    a = x0, b = x1;
+                    if (P.i8_scores && !is_v) {
+                        x0 = (float)c0, x1 = (float)c1;
+                        if (lane == 0) {
+                            float *kk = stage_kskb(P, h, pos);
+                            kk[0] = scale, kk[128] = beta;
+                        }
+                    }
+                } else {
+                    float *cdst = (is_v ? P.vcache : P.kcache) + crow * kvd + h * HD;
+                    cdst[lane] = a, cdst[lane + 32] = b;
+                }
+                dst[lane] = __float2bfloat16_rn(x0);
+                dst[lane + 32] = __float2bfloat16_rn(x1);
+                if (!is_v) {
+                    float ss = a * a + b * b;
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, o);
+                    if (lane == 0) raise(P.n_head + h, ss);
+                }
+            }
+        }
+    }
+
+    // ---- cached keys [0, n_old) ----
+    const int n_old = P.write_kv ? P.pos0 : P.n_keys;
+    const size_t total = (size_t)n_old * P.n_kv_head * 8;
+    for (size_t base = (size_t)blockIdx.x * ST_THREADS; base < total; base += (size_t)ST_GRID * ST_THREADS) {
+        const bool live = base + tid < total;
+        const size_t idx = live ? base + tid : total - 1;   // keep the row's lanes together for the shuffles below
+        const int c = (int)(idx & 7);
+        const size_t th = idx >> 3;
+        const int t = (int)(th / P.n_kv_head), h = (int)(th - (size_t)t * P.n_kv_head);
+        const size_t row = stage_row(P, t);
+        const size_t dst = ((size_t)h * P.n_keys + t) * HD + c * 8;
+        float k[8], v[8], ksc = 0.0f, kbe = 0.0f, ss = 0.0f;
+        if (P.kq) {
+            const int2 kw = *(const int2 *)(P.kq + row * kvd + h * HD + c * 8);
+            const int2 vw = *(const int2 *)(P.vq + row * kvd + h * HD + c * 8);
+            ksc = P.ks[row * P.n_kv_head + h];
+            kbe = P.kb ? P.kb[row * P.n_kv_head + h] : 0.0f;
+            const float vsc = P.vs[row * P.n_kv_head + h], vbe = P.vb ? P.vb[row * P.n_kv_head + h] : 0.0f;
+            const int kk[2] = {kw.x, kw.y}, vv[2] = {vw.x, vw.y};
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                // dequantise as the reference does into its V tile: code * scale + beta (llm.cu:3759-3764)
+                const float code = (float)(int8_t)((kk[i >> 2] >> (8 * (i & 3))) & 0xFF);
+                const float val = code * ksc + kbe;
+                ss += val * val;
+                k[i] = P.i8_scores ? code : val;
+                v[i] = (float)(int8_t)((vv[i >> 2] >> (8 * (i & 3))) & 0xFF) * vsc + vbe;
+            }
+        } else {
+            const float4 *kp = (const float4 *)(P.kcache + row * kvd + h * HD + c * 8);
+            const float4 *vp = (const float4 *)(P.vcache + row * kvd + h * HD + c * 8);
+            const float4 a = kp[0], b = kp[1], e = vp[0], f = vp[1];
+            k[0] = a.x, k[1] = a.y, k[2] = a.z, k[3] = a.w, k[4] = b.x, k[5] = b.y, k[6] = b.z, k[7] = b.w;
+            v[0] = e.x, v[1] = e.y, v[2] = e.z, v[3] = e.w, v[4] = f.x, v[5] = f.y, v[6] = f.z, v[7] = f.w;
+            if (P.i8_scores) {   // K quantised on the fly, symmetric absmax per row (the reference's attn_prefill_dp4a)
+                float amax = 0.0f;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(k[i]));
+#pragma unroll
+                for (int o = 4; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
+                const float id = amax > 0.0f ? __fdiv_rn(127.0f, amax) : 0.0f;
+                ksc = amax > 0.0f ? __fdiv_rn(amax, 127.0f) : 0.0f;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    k[i] = (float)max(-127, min(127, __float2int_rn(k[i] * id)));
+                    ss += k[i] * ksc * (k[i] * ksc);
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) ss += k[i] * k[i];
+            }
         }
 #pragma unroll
         for (int o = 4; o > 0; o >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, o);   // the row's eight threads
-        best = fmaxf(best, ss);
-    }
-    best = block_max256(best);
-    if (threadIdx.x == 0) norm2[h * MX230_NORM_PARTS + p] = best;
-}
-
-struct StageKv {
-    __nv_bfloat16 *kout, *vout;      // [n_kv_head][n_keys][64]
-    const float *kcache, *vcache;    // fp32 cache, or
-    const int8_t *kq, *vq;           // int8 cache with
-    const float *ks, *vs, *kb, *vb;  // per-(row, head) scale and (optional) beta
-    const int *bt;
-    int bs;
-    int n_keys, n_kv_head;
-};
-
-// Grid (MX230_NORM_PARTS, n_kv_head): block (p, h) stages the keys t = p (mod 32) of K/V head h, eight threads per key (8
-// consecutive dims of K and of V each), and leaves the largest squared norm of its staged K rows in norm2[h][p].
-__global__ void stage_kv_kernel(const StageKv P, float *norm2) {
-    const int p = blockIdx.x, h = blockIdx.y;
-    const int c = threadIdx.x & 7, slot = threadIdx.x >> 3;
-    const size_t kvd = (size_t)P.n_kv_head * HD;
-    float best = 0.0f;
-    for (int t0 = p; t0 < P.n_keys; t0 += MX230_NORM_PARTS * 32) {
-        const int t = t0 + MX230_NORM_PARTS * slot;
-        float ss = 0.0f;
-        if (t < P.n_keys) {
-            const size_t row = P.bt ? (size_t)(P.bt[t / P.bs] * P.bs + t % P.bs) : (size_t)t;
-            const size_t dst = ((size_t)h * P.n_keys + t) * HD + c * 8;
-            float k[8], v[8];
-            if (P.kq) {
-                int2 kw = *(const int2 *)(P.kq + row * kvd + h * HD + c * 8);
-                int2 vw = *(const int2 *)(P.vq + row * kvd + h * HD + c * 8);
-                float ksc = P.ks[row * P.n_kv_head + h], vsc = P.vs[row * P.n_kv_head + h];
-                float kbe = P.kb ? P.kb[row * P.n_kv_head + h] : 0.0f, vbe = P.vb ? P.vb[row * P.n_kv_head + h] : 0.0f;
-                const int kk[2] = {kw.x, kw.y}, vv[2] = {vw.x, vw.y};
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    // dequantise as the reference does into its V tile: code * scale + beta (llm.cu:3759-3764)
-                    k[i] = (float)(int8_t)((kk[i >> 2] >> (8 * (i & 3))) & 0xFF) * ksc + kbe;
-                    v[i] = (float)(int8_t)((vv[i >> 2] >> (8 * (i & 3))) & 0xFF) * vsc + vbe;
-                }
-            } else {
-                const float4 *kp = (const float4 *)(P.kcache + row * kvd + h * HD + c * 8);
-                const float4 *vp = (const float4 *)(P.vcache + row * kvd + h * HD + c * 8);
-                float4 a = kp[0], b = kp[1], e = vp[0], f = vp[1];
-                k[0] = a.x, k[1] = a.y, k[2] = a.z, k[3] = a.w, k[4] = b.x, k[5] = b.y, k[6] = b.z, k[7] = b.w;
-                v[0] = e.x, v[1] = e.y, v[2] = e.z, v[3] = e.w, v[4] = f.x, v[5] = f.y, v[6] = f.z, v[7] = f.w;
+        if (!live) continue;
+        uint4 ko, vo;
+        ko.x = mx::pack_bf16(k[0], k[1]), ko.y = mx::pack_bf16(k[2], k[3]);
+        ko.z = mx::pack_bf16(k[4], k[5]), ko.w = mx::pack_bf16(k[6], k[7]);
+        vo.x = mx::pack_bf16(v[0], v[1]), vo.y = mx::pack_bf16(v[2], v[3]);
+        vo.z = mx::pack_bf16(v[4], v[5]), vo.w = mx::pack_bf16(v[6], v[7]);
+        *(uint4 *)(P.kout + dst) = ko;
+        *(uint4 *)(P.vout + dst) = vo;
+        if (c == 0) {
+            if (P.i8_scores) {
+                float *kk = stage_kskb(P, h, t);
+                kk[0] = ksc, kk[128] = kbe;
             }
-#pragma unroll
-            for (int i = 0; i < 8; ++i) ss += k[i] * k[i];
-            uint4 ko, vo;
-            ko.x = mx::pack_bf16(k[0], k[1]), ko.y = mx::pack_bf16(k[2], k[3]);
-            ko.z = mx::pack_bf16(k[4], k[5]), ko.w = mx::pack_bf16(k[6], k[7]);
-            vo.x = mx::pack_bf16(v[0], v[1]), vo.y = mx::pack_bf16(v[2], v[3]);
-            vo.z = mx::pack_bf16(v[4], v[5]), vo.w = mx::pack_bf16(v[6], v[7]);
-            *(uint4 *)(P.kout + dst) = ko;
-            *(uint4 *)(P.vout + dst) = vo;
+            raise(P.n_head + h, ss);
         }
-#pragma unroll
-        for (int o = 4; o > 0; o >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, o);   // the key's eight threads
-        best = fmaxf(best, ss);
     }
-    best = block_max256(best);
-    if (threadIdx.x == 0) norm2[h * MX230_NORM_PARTS + p] = best;
-}
 
-// ---- int8 score mode (the reference kernels' own arithmetic, llm.cu:3700-3716,3737-3754,3774-3782) ----
-// q row -> int8 codes per (row, head): id = 127 / amax, code = clamp(rne(q * id), +-127); the codes go out as bf16
-// (exact), with the row's score factor (amax / 127) * 1/sqrt(64) * log2(e) and the sum of its codes.
-// One warp per (head, row); lane l holds dims l and l + 32.
-__global__ void stage_q_codes_kernel(__nv_bfloat16 *out, float *row_a, float *row_qsum, const float *qkv, int n_tok,
-                                     int n_head, int stride) {
-    const int w = (int)(((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-    if (w >= n_head * n_tok) return;
-    const int h = w / n_tok, r = w - h * n_tok;
-    const float *src = qkv + (size_t)r * stride + h * HD;
-    const float a = src[lane], b = src[lane + 32];
-    float amax = fmaxf(fabsf(a), fabsf(b));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
-    const float id = amax > 0.0f ? __fdiv_rn(127.0f, amax) : 0.0f;
-    const int ca = max(-127, min(127, __float2int_rn(a * id))), cb = max(-127, min(127, __float2int_rn(b * id)));
-    int sum = ca + cb;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
-    __nv_bfloat16 *dst = out + ((size_t)h * n_tok + r) * HD;
-    dst[lane] = __float2bfloat16((float)ca);
-    dst[lane + 32] = __float2bfloat16((float)cb);
-    if (lane == 0) {
-        const float qs = amax > 0.0f ? __fdiv_rn(amax, 127.0f) : 0.0f;
-        row_a[(size_t)h * n_tok + r] = qs * 0.125f * 1.4426950408889634f;
-        row_qsum[(size_t)h * n_tok + r] = (float)sum;
+    // ---- the cluster's maxima -> its part ----
+    const int part = blockIdx.x / ST_CLUSTER, rank = blockIdx.x % ST_CLUSTER;
+    __syncthreads();
+    mx::cluster_wait();
+    if (rank != 0)
+        for (int i = tid; i < n_max; i += ST_THREADS) mx::cluster_red_max(mx::cluster_map(mx::smem_u32(&smax[i]), 0), smax[i]);
+    mx::cluster_sync();
+    if (rank != 0) return;
+    for (int i = tid; i < n_max; i += ST_THREADS) {
+        float *dst = i < P.n_head ? P.q_norm2 + (size_t)i * MX230_NORM_PARTS : P.k_norm2 + (size_t)(i - P.n_head) * MX230_NORM_PARTS;
+        dst[part] = __int_as_float(smax[i]);
     }
 }
 
-// K as int8 codes in bf16 (exact) with its per-key (scale, offset) pair, V dequantised to bf16.  Over an int8
-// cache the codes and pairs are the cache's own (absmax format: offset 0); over an fp32 cache (the reference's
-// opt-in attn_prefill_dp4a) every K row is quantised on the fly, symmetric absmax, and V is the fp32 row.
-// One thread stages 8 consecutive dims of one (key, kv head); the 8 threads of a row are neighbouring lanes.
-__global__ void stage_kv_codes_kernel(const StageKv P, float2 *kskb, int n_k_pad) {
-    size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;  // over n_keys*n_kv_head*8
-    size_t total = (size_t)P.n_keys * P.n_kv_head * 8;
-    const bool live = idx < total;
-    if (!live) idx = total - 1;   // keep the row's lanes together for the shuffles below
-    int c = (int)(idx & 7);
-    size_t th = idx >> 3;
-    int h = (int)(th % P.n_kv_head);
-    int t = (int)(th / P.n_kv_head);
-    size_t row = P.bt ? (size_t)(P.bt[t / P.bs] * P.bs + t % P.bs) : (size_t)t;
-    size_t kvd = (size_t)P.n_kv_head * HD;
-    size_t dst = ((size_t)h * P.n_keys + t) * HD + c * 8;
-    float k[8], v[8];
-    float ksc, kbe;
-    if (P.kq) {
-        int2 kw = *(const int2 *)(P.kq + row * kvd + h * HD + c * 8);
-        int2 vw = *(const int2 *)(P.vq + row * kvd + h * HD + c * 8);
-        ksc = P.ks[row * P.n_kv_head + h];
-        kbe = P.kb ? P.kb[row * P.n_kv_head + h] : 0.0f;
-        float vsc = P.vs[row * P.n_kv_head + h], vbe = P.vb ? P.vb[row * P.n_kv_head + h] : 0.0f;
-        const int kk[2] = {kw.x, kw.y}, vv[2] = {vw.x, vw.y};
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            k[i] = (float)(int8_t)((kk[i >> 2] >> (8 * (i & 3))) & 0xFF);
-            v[i] = (float)(int8_t)((vv[i >> 2] >> (8 * (i & 3))) & 0xFF) * vsc + vbe;
-        }
-    } else {
-        const float4 *kp = (const float4 *)(P.kcache + row * kvd + h * HD + c * 8);
-        const float4 *vp = (const float4 *)(P.vcache + row * kvd + h * HD + c * 8);
-        float4 a = kp[0], b = kp[1], e = vp[0], f = vp[1];
-        k[0] = a.x, k[1] = a.y, k[2] = a.z, k[3] = a.w, k[4] = b.x, k[5] = b.y, k[6] = b.z, k[7] = b.w;
-        v[0] = e.x, v[1] = e.y, v[2] = e.z, v[3] = e.w, v[4] = f.x, v[5] = f.y, v[6] = f.z, v[7] = f.w;
-        float amax = 0.0f;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(k[i]));
-        const unsigned m8 = 0xFFu << ((threadIdx.x & 31) & ~7);   // the 8 lanes of this row
-#pragma unroll
-        for (int o = 4; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(m8, amax, o));
-        const float id = amax > 0.0f ? __fdiv_rn(127.0f, amax) : 0.0f;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) k[i] = (float)max(-127, min(127, __float2int_rn(k[i] * id)));
-        ksc = amax > 0.0f ? __fdiv_rn(amax, 127.0f) : 0.0f;
-        kbe = 0.0f;
-    }
-    if (!live) return;
-    uint4 ko, vo;
-    ko.x = mx::pack_bf16(k[0], k[1]), ko.y = mx::pack_bf16(k[2], k[3]);
-    ko.z = mx::pack_bf16(k[4], k[5]), ko.w = mx::pack_bf16(k[6], k[7]);
-    vo.x = mx::pack_bf16(v[0], v[1]), vo.y = mx::pack_bf16(v[2], v[3]);
-    vo.z = mx::pack_bf16(v[4], v[5]), vo.w = mx::pack_bf16(v[6], v[7]);
-    *(uint4 *)(P.kout + dst) = ko;
-    *(uint4 *)(P.vout + dst) = vo;
-    if (c == 0) kskb[(size_t)h * n_k_pad + t] = make_float2(ksc, kbe);
-}
+// What the prefill step adds to plain prefill attention
+struct StepArgs {
+    bool write_kv;
+    int rope;
+    float theta;
+};
 
 size_t align1k(size_t x) { return (x + 1023) & ~(size_t)1023; }
 
+// With a step, qkv and the cache are written as well (the entry point that asks for one takes them non-const).
 int prefill(mx230_handle *h, void *stream, float *out, const float *qkv, const float *kcache,
             const float *vcache, const int8_t *kq, const int8_t *vq, const float *ks, const float *vs,
             const float *kb, const float *vb, int pos0, int n_tok, int n_head, int n_kv_head, int qkv_stride,
-            int out_stride, const int *bt, int bs, const char *who, bool dp4a = false) {
+            int out_stride, const int *bt, int bs, const char *who, bool dp4a = false, StepArgs step = {}) {
     MX_REQUIRE(h != nullptr, MX230_ERR_INVALID_ARG, "%s: null handle", who);
     MX_REQUIRE(pos0 >= 0 && n_tok >= 0, MX230_ERR_INVALID_ARG, "%s: negative pos0/n_tok", who);
     if (n_tok == 0) return MX230_OK;
@@ -256,33 +305,30 @@ int prefill(mx230_handle *h, void *stream, float *out, const float *qkv, const f
     __nv_bfloat16 *vbuf = (__nv_bfloat16 *)((char *)h->ws + qbytes + kbytes);
     float *row_a = (float *)((char *)h->ws + qbytes + 2 * kbytes);
     float *row_qsum = (float *)((char *)row_a + rbytes);
-    float2 *kskb = (float2 *)((char *)row_qsum + rbytes);
+    float *kskb = (float *)((char *)row_qsum + rbytes);
     float *q_norm2 = (float *)((char *)kskb + cbytes);
     float *k_norm2 = q_norm2 + (size_t)n_head * MX230_NORM_PARTS;
-    StageKv S{kbuf, vbuf, kcache, vcache, kq, vq, ks, vs, kb, vb, bt, bs, n_keys, n_kv_head};
-    size_t tk = (size_t)n_keys * n_kv_head * 8;
     // Which score arithmetic: over an int8 cache the handle's MX230_OPT_Q8_SCORE_MODE decides, as for decode
     // (REF, the default: q quantised per (row, head) to int8 and integer dots, what attn_prefill_q8 computes;
     // EXACT: fp32 q against dequantised K); the _dp4a entry points are the reference's int8-score approximation
     // over an fp32 cache by definition.
     const bool i8_scores = dp4a || (kq && h->q8_score_mode == MX230_Q8_SCORE_REF);
-    if (i8_scores) {
-        size_t warps = (size_t)n_head * n_tok;
-        MX_LAUNCH(h, st, MX230_K_PREFILL,
-                  (stage_q_codes_kernel<<<(unsigned)((warps * 32 + 255) / 256), 256, 0, st>>>(qb, row_a, row_qsum, qkv, n_tok,
-                                                                                              n_head, qkv_stride)));
-        MX_LAUNCH(h, st, MX230_K_PREFILL, (stage_kv_codes_kernel<<<(unsigned)((tk + 255) / 256), 256, 0, st>>>(S, kskb, n_k_pad)));
-        return mx230_launch_flash_fwd_ex(h, st, qb, kbuf, vbuf, out, nullptr, n_head, n_tok, n_keys, pos0,
-                                         n_head / n_kv_head, HD, out_stride, 1, 0, nullptr, nullptr, row_a, row_qsum,
-                                         (const float *)kskb);
-    }
-    // values (fp32 cache, or an int8 cache in the exact score mode): the staging kernels also leave the row norms that
-    // let the attention kernel take its max-free path whenever the head's scores are bounded
-    MX_LAUNCH(h, st, MX230_K_PREFILL,
-              (stage_q_kernel<<<dim3(MX230_NORM_PARTS, n_head), 256, 0, st>>>(qb, q_norm2, qkv, n_tok, n_head, qkv_stride)));
-    MX_LAUNCH(h, st, MX230_K_PREFILL, (stage_kv_kernel<<<dim3(MX230_NORM_PARTS, n_kv_head), 256, 0, st>>>(S, k_norm2)));
-    return mx230_launch_flash_fwd_ex(h, st, qb, kbuf, vbuf, out, nullptr, n_head, n_tok, n_keys, pos0,
-                                     n_head / n_kv_head, HD, out_stride, 1, 1, q_norm2, k_norm2, nullptr, nullptr, nullptr);
+    StageParams S;
+    S.qout = qb, S.kout = kbuf, S.vout = vbuf, S.q_norm2 = q_norm2, S.k_norm2 = k_norm2;
+    S.row_a = row_a, S.row_qsum = row_qsum, S.kskb = kskb, S.i8_scores = i8_scores, S.n_k_tiles = n_k_pad / 128;
+    S.qkv = const_cast<float *>(qkv), S.stride = qkv_stride, S.n_tok = n_tok, S.pos0 = pos0, S.n_keys = n_keys;
+    S.n_head = n_head, S.n_kv_head = n_kv_head;
+    S.kcache = const_cast<float *>(kcache), S.vcache = const_cast<float *>(vcache);
+    S.kq = const_cast<int8_t *>(kq), S.vq = const_cast<int8_t *>(vq);
+    S.ks = const_cast<float *>(ks), S.vs = const_cast<float *>(vs), S.kb = const_cast<float *>(kb), S.vb = const_cast<float *>(vb);
+    S.bt = bt, S.bs = bs;
+    S.write_kv = step.write_kv, S.rope = step.rope, S.theta = step.theta;
+    const size_t sm = (size_t)(n_head + n_kv_head) * sizeof(int);
+    MX_REQUIRE(sm <= 48 * 1024, MX230_ERR_UNSUPPORTED, "%s: %d heads", who, n_head + n_kv_head);
+    MX_LAUNCH(h, st, MX230_K_PREFILL, mx_launch(prefill_stage_kernel, ST_GRID, ST_THREADS, sm, st, ST_CLUSTER, true, S));
+    return mx230_launch_flash_fwd_ex(h, st, qb, kbuf, vbuf, out, nullptr, n_head, n_tok, n_keys, pos0, n_head / n_kv_head, HD,
+                                     out_stride, 1, i8_scores ? 0 : 1, q_norm2, k_norm2, i8_scores ? row_a : nullptr,
+                                     i8_scores ? row_qsum : nullptr, i8_scores ? kskb : nullptr);
 }
 
 }  // namespace
@@ -339,4 +385,13 @@ extern "C" int mx230_attn_prefill_dp4a_paged(mx230_handle *h, void *stream, floa
     MX_REQUIRE(bt, MX230_ERR_INVALID_ARG, "attn_prefill_dp4a_paged: null block table");
     return prefill(h, stream, out, qkv, kcache, vcache, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
                    pos0, n_tok, n_head, n_kv_head, qkv_stride, out_stride, bt, bs, "attn_prefill_dp4a_paged", true);
+}
+
+extern "C" int mx230_prefill_step(mx230_handle *h, void *stream, float *out, float *qkv, float *kcache, float *vcache,
+                                  int8_t *kq, int8_t *vq, float *ks, float *vs, float *kb, float *vb, int pos0, int n_tok,
+                                  int n_head, int n_kv_head, int head_dim, int use_rope, float theta, int qkv_stride,
+                                  int out_stride, const int *bt, int bs) {
+    MX_REQUIRE(head_dim == HD, MX230_ERR_UNSUPPORTED, "prefill_step: head_dim %d unsupported (must be 64)", head_dim);
+    return prefill(h, stream, out, qkv, kcache, vcache, kq, vq, ks, vs, kb, vb, pos0, n_tok, n_head, n_kv_head, qkv_stride,
+                   out_stride, bt, bs, "prefill_step", false, StepArgs{true, use_rope, theta});
 }

@@ -317,15 +317,18 @@ def attn_prefill(h: Handle, out, qkv, c: KvCache, pos0, n_tok, n_head, n_kv_head
 def prefill_step(h: Handle, out, qkv, c: KvCache, pos0, n_tok, n_head, n_kv_head, head_dim, theta,
                  qkv_stride, out_stride, pg: Paging | None = None, use_rope=True, stream=None):
     """The prefill attention step of batch_body_from (gpu.rs:3204-3347): RoPE on the n_tok rows,
-    KV write of all of them, then causal attention over the cache."""
-    q_dim, kv_dim = n_head * head_dim, n_kv_head * head_dim
-    if use_rope:
-        rope_batch(h, qkv, pos0, n_tok, n_head, n_kv_head, head_dim, qkv_stride, theta, stream)
-    if c.quant:
-        quantize_kv_batch(h, c, qkv, pos0, n_tok, q_dim, n_kv_head, head_dim, qkv_stride, pg, stream)
-    else:
-        copy_kv_batch(h, c, qkv, pos0, n_tok, q_dim, kv_dim, qkv_stride, pg, stream)
-    attn_prefill(h, out, qkv, c, pos0, n_tok, n_head, n_kv_head, qkv_stride, out_stride, pg, stream)
+    KV write of all of them, then causal attention over the cache -- two launches."""
+    if head_dim != 64:   # the fused entry point knows 64 only; the separate ones decide what they take
+        q_dim, kv_dim = n_head * head_dim, n_kv_head * head_dim
+        if use_rope:
+            rope_batch(h, qkv, pos0, n_tok, n_head, n_kv_head, head_dim, qkv_stride, theta, stream)
+        if c.quant:
+            quantize_kv_batch(h, c, qkv, pos0, n_tok, q_dim, n_kv_head, head_dim, qkv_stride, pg, stream)
+        else:
+            copy_kv_batch(h, c, qkv, pos0, n_tok, q_dim, kv_dim, qkv_stride, pg, stream)
+        return attn_prefill(h, out, qkv, c, pos0, n_tok, n_head, n_kv_head, qkv_stride, out_stride, pg, stream)
+    check(lib().mx230_prefill_step(h._h, stream_ptr(stream), ptr(out), ptr(qkv), *_cache_args(c), pos0, n_tok, n_head,
+                                   n_kv_head, head_dim, int(use_rope), theta, qkv_stride, out_stride, *_table_args(pg)))
 
 
 def attn_decode_q8_noalloc(out, qkv, c: KvCache, t_cur: int, n_head, n_kv_head, head_dim, stream=None):
