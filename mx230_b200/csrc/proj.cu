@@ -14,23 +14,23 @@
 //
 // The floor is HBM on the weight matrix (n_in x n_out fp32, fp16 or int8, each byte read once); at a decode token's
 // sizes (2 MB) the time is latency instead: launch, one memory round trip, the merge of the partial sums.  The reference
-// gives one thread a whole output column.  Here a 64-column block (one attention head) belongs to a thread-block cluster
-// of up to eight CTAs, each with a slice of the input rows small enough that a thread's loads are all in flight at once;
-// the CTAs push their 64 sums into the first one's shared memory, which adds them in slice order (deterministic), adds
-// the bias and runs the epilogue.  Only matrices whose slices would get long (or that have few columns) use several
-// clusters per block, merged through the workspace by the last one to arrive.  The kernel is launched programmatically:
-// its slice of the weights is on its way into L2 while the kernel before it still runs.
+// gives one thread a whole output column.  Here a 64-column block (one attention head) is summed in slices of the input
+// rows, eight row lanes per slice, lanes and slices added in a fixed order that depends on the sizes alone (a rotated q is
+// quantised to int8 downstream, where another last bit can move a code).  Up to 64 slices belong to one thread-block
+// cluster of up to eight CTAs, which push their slices' sums into the first one's shared memory, where the epilogue runs;
+// more slices go through the workspace, merged by the last CTA to arrive.  The kernel is launched programmatically: its
+// slices of the weights are on their way into L2 while the kernel before it still runs.
 #include <cuda_fp16.h>
 
 #include "common.cuh"
 
 namespace {
 
-constexpr int PJ_THREADS = 256;
-constexpr int PJ_WARPS = PJ_THREADS / 32;
-constexpr int PJ_COLS = 64;     // columns per CTA = one head
-constexpr int PJ_CLUSTER = 8;   // most CTAs of a column block that merge through shared memory
-constexpr int PJ_MAX_ROWS = 4096;   // input rows per CTA at most (bounds the int8 path's shared memory)
+constexpr int PJ_COLS = 64;       // columns per CTA = one head
+constexpr int PJ_ROWLANES = 8;    // row lanes of a slice: lane l sums rows l, l + 8, ...
+constexpr int PJ_CLUSTER = 8;     // most CTAs of a column block that merge through shared memory
+constexpr int PJ_SLOTS = 8;       // most slices of a CTA
+constexpr int PJ_SLICES_PER_SM = 6;   // slices, over all column blocks, that the split aims at
 
 struct QkvEpilogue {
     int enabled;
@@ -53,8 +53,9 @@ struct GemvParams {
     int n_in, n_out, accum;
     const float *scales;     // int8 weights: one scale per output column
     int ag;                  // int8 weights: activations are quantised in groups of `ag` values (4 or 8)
-    int rows_per_slice, n_slices, cl_size;   // n_slices = clusters per block x cl_size
-    float *partials;         // [clusters per block][n_out]
+    int rows_per_slice, n_slices;   // per column block
+    int slots, ctas, cl_size;       // slices per CTA, CTAs per column block; cl_size = ctas, or 1: merge through the workspace
+    float *partials;                // [n_slices][n_out]
     unsigned *counters;      // one per column block, self-resetting
     QkvEpilogue e;
 };
@@ -105,39 +106,42 @@ struct WeightRow<int8_t, 4> {
     }
 };
 
-// Grid: column blocks x n_slices, slices fastest; a cluster holds cl_size consecutive slices of one block.
+// Grid: column blocks x CTAs, the CTAs of a block next to each other.  A slice takes 64 / CPT * 8 threads.
 template <typename WT, int CPT>
-__global__ void __launch_bounds__(PJ_THREADS)
+__global__ void __launch_bounds__(PJ_SLOTS * PJ_COLS / CPT * PJ_ROWLANES)
 gemv_heads_kernel(const GemvParams P) {
     constexpr bool I8 = sizeof(WT) == 1;
     constexpr int TPR = PJ_COLS / CPT;              // threads across a weight row
-    constexpr int RL = PJ_THREADS / TPR;            // weight rows per pass
+    constexpr int TPS = TPR * PJ_ROWLANES;          // threads of a slice
     constexpr int BATCH = 4;                        // passes whose loads are issued together
     constexpr int ELT = I8 ? 4 : (int)sizeof(WT);   // bytes of a stored weight word
     constexpr int IN_PER_ROW = I8 ? 4 : 1;          // input rows in one stored row
-    __shared__ float red[PJ_WARPS][PJ_COLS];
-    __shared__ float parts[PJ_CLUSTER][PJ_COLS];    // first CTA of the cluster: the sums of every CTA
+    __shared__ float red[PJ_SLOTS][PJ_ROWLANES][PJ_COLS];
+    __shared__ float parts[PJ_CLUSTER * PJ_SLOTS][PJ_COLS];   // first CTA of the cluster: the sums of every slice
     __shared__ float val[PJ_COLS];
     __shared__ int is_last;
-    extern __shared__ float xs[];                   // int8: this slice of x as packed codes, then group scales
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, C = P.cl_size;
-    const int blk = blockIdx.x / P.n_slices, slice = blockIdx.x - blk * P.n_slices;
-    const int cl = slice / C, rank = slice - cl * C;
+    extern __shared__ float xs[];                   // int8: the CTA's part of x as packed codes, then group scales
+    const int tid = threadIdx.x, nt = blockDim.x, C = P.cl_size;
+    const int blk = blockIdx.x / P.ctas, rank = blockIdx.x - blk * P.ctas;
     const int col0 = blk * PJ_COLS;
-    const int k0 = min(P.n_in, slice * P.rows_per_slice), k1 = min(P.n_in, k0 + P.rows_per_slice);
-    const int r0 = k0 / IN_PER_ROW, r1 = k1 / IN_PER_ROW;   // stored rows of this slice
+    const int slot = tid / TPS, tl = tid - slot * TPS;
+    const int slice = rank * P.slots + slot;
+    // input rows of the CTA and of this thread's slice
+    const int c0 = min(P.n_in, rank * P.slots * P.rows_per_slice), c1 = min(P.n_in, c0 + P.slots * P.rows_per_slice);
+    const int r0 = min(P.n_in, slice * P.rows_per_slice) / IN_PER_ROW;
+    const int r1 = min(P.n_in, (slice + 1) * P.rows_per_slice) / IN_PER_ROW;
 
     mx::pdl_trigger();
     if (C > 1) mx::cluster_arrive_relaxed();        // waited for before the first access to another CTA's memory
-    // start of the slice into L2 under the previous kernel's tail
-    for (int r = r0 + tid; r < min(r1, r0 + 2 * PJ_THREADS); r += PJ_THREADS) {
+    // start of the CTA's rows into L2 under the previous kernel's tail
+    for (int r = c0 / IN_PER_ROW + tid, n = 0; r < c1 / IN_PER_ROW && n < 2; r += nt, ++n) {
         const char *line = (const char *)P.w + ((size_t)r * P.n_out + col0) * ELT;
         mx::prefetch_l2(line);
         if (ELT == 4 && col0 + 32 < P.n_out) mx::prefetch_l2(line + 128);
     }
     mx::pdl_wait();
 
-    const int cq = tid % TPR, rl = tid / TPR;
+    const int cq = tl % TPR, rl = tl / TPR;
     const int col = col0 + CPT * cq;
     const bool live = col < P.n_out;                // n_out is a multiple of CPT
     float acc[CPT];
@@ -148,7 +152,7 @@ gemv_heads_kernel(const GemvParams P) {
     auto load = [&](int r) {
 #pragma unroll
         for (int u = 0; u < BATCH; ++u) {
-            const int i = r + u * RL;
+            const int i = r + u * PJ_ROWLANES;
             const bool in = live && i < r1;
             if (in) w[u].load(P.w, (size_t)i * P.n_out + col);
             else w[u].zero();
@@ -156,13 +160,13 @@ gemv_heads_kernel(const GemvParams P) {
         }
     };
     load(r0 + rl);
-    // what the epilogue of the cluster's first CTA needs, under the weight loads
+    // what the epilogue needs, under the weight loads
     const QkvEpilogue &E = P.e;
     const bool is_v = blk >= E.n_head + E.n_kv_head;
     float bias = 0.0f, scale_o = 1.0f, y_old = 0.0f, cs = 1.0f, sn = 0.0f;
     int pos = 0;
     size_t row = 0;
-    if (rank == 0 && tid < PJ_COLS && col0 + tid < P.n_out) {
+    if ((rank == 0 || C == 1) && tid < PJ_COLS && col0 + tid < P.n_out) {
         const int o = col0 + tid;
         if (P.b) bias = P.b[o];
         if (I8) scale_o = P.scales[o];
@@ -174,12 +178,12 @@ gemv_heads_kernel(const GemvParams P) {
         }
     }
     if constexpr (I8) {
-        // quantise this slice of the activations exactly as the reference kernel does
+        // quantise the CTA's part of the activations exactly as the reference kernel does
         const int ag = P.ag;
-        int *xq = (int *)xs;                        // (k1 - k0) / 4 words
-        float *xsc = xs + P.rows_per_slice / 4;     // (k1 - k0) / ag scales
-        for (int g = tid; g < (k1 - k0) / ag; g += PJ_THREADS) {
-            const float *xg = P.x + k0 + g * ag;
+        int *xq = (int *)xs;                                  // (c1 - c0) / 4 words
+        float *xsc = xs + P.slots * P.rows_per_slice / 4;     // (c1 - c0) / ag scales
+        for (int g = tid; g < (c1 - c0) / ag; g += nt) {
+            const float *xg = P.x + c0 + g * ag;
             float amax = 0.0f;
             for (int j = 0; j < ag; ++j) amax = fmaxf(amax, fabsf(xg[j]));
             const float id = amax > 0.0f ? __fdiv_rn(127.0f, amax) : 0.0f;
@@ -195,60 +199,64 @@ gemv_heads_kernel(const GemvParams P) {
         }
         __syncthreads();
         const int wpg = ag / 4;   // word q holds input rows 4q .. 4q+3; its group scale is xsc[q / wpg]
-        for (int r = r0 + rl; r < r1; r += BATCH * RL) {
+        for (int r = r0 + rl; r < r1; r += BATCH * PJ_ROWLANES) {
             if (r != r0 + rl) load(r);
 #pragma unroll
             for (int u = 0; u < BATCH; ++u) {
-                const int q = r + u * RL - r0;
-                if (q < r1 - r0) w[u].fma(xq[q], xsc[q / wpg], acc);
+                const int q = r + u * PJ_ROWLANES;
+                if (q < r1) w[u].fma(xq[q - c0 / 4], xsc[(q - c0 / 4) / wpg], acc);
             }
         }
     } else {
-        for (int r = r0 + rl; r < r1; r += BATCH * RL) {
+        for (int r = r0 + rl; r < r1; r += BATCH * PJ_ROWLANES) {
             if (r != r0 + rl) load(r);
 #pragma unroll
-            for (int u = 0; u < BATCH; ++u) w[u].fma(xv[u], acc);
+            for (int u = 0; u < BATCH; ++u)
+                if (r + u * PJ_ROWLANES < r1) w[u].fma(xv[u], acc);
         }
     }
-    // ---- CTA, then cluster, then (several clusters) block totals ----
 #pragma unroll
-    for (int c = 0; c < CPT; ++c) {
-#pragma unroll
-        for (int o = TPR; o < 32; o <<= 1) acc[c] += __shfl_xor_sync(0xFFFFFFFFu, acc[c], o);
-        if (lane < TPR) red[warp][CPT * cq + c] = acc[c];
-    }
+    for (int c = 0; c < CPT; c += 4) *(float4 *)&red[slot][rl][CPT * cq + c] = make_float4(acc[c], acc[c + 1], acc[c + 2], acc[c + 3]);
     __syncthreads();
-    float sum = 0.0f;
-    if (tid < PJ_COLS) {
+    // ---- lanes -> slices -> block, each in index order ----
+    if (C > 1) mx::cluster_wait();   // every CTA of the cluster runs
+    for (int i = tid; i < P.slots * PJ_COLS; i += nt) {
+        const int sl = i / PJ_COLS, c = i - sl * PJ_COLS, g = rank * P.slots + sl;
+        if (g >= P.n_slices) break;
+        float sum = 0.0f;
 #pragma unroll
-        for (int r = 0; r < PJ_WARPS; ++r) sum += red[r][tid];
+        for (int r = 0; r < PJ_ROWLANES; ++r) sum += red[sl][r][c];
+        if (C > 1) mx::cluster_st_f32(mx::cluster_map(mx::smem_u32(&parts[g][c]), 0), sum);
+        else if (P.ctas == 1) parts[g][c] = sum;
+        else if (col0 + c < P.n_out) P.partials[(size_t)g * P.n_out + col0 + c] = sum;
     }
     if (C > 1) {
-        mx::cluster_wait();       // every CTA of the cluster runs
-        if (tid < PJ_COLS) mx::cluster_st_f32(mx::cluster_map(mx::smem_u32(&parts[rank][tid]), 0), sum);
         mx::cluster_sync();
         if (rank != 0) return;
-        if (tid < PJ_COLS) {
-            sum = 0.0f;
-            for (int r = 0; r < C; ++r) sum += parts[r][tid];
-        }
-    }
-    const int n_cl = P.n_slices / C;
-    if (n_cl > 1) {
-        if (tid < PJ_COLS && col0 + tid < P.n_out) P.partials[(size_t)cl * P.n_out + col0 + tid] = sum;
+    } else if (P.ctas > 1) {
         __threadfence();
         __syncthreads();
-        if (tid == 0) is_last = atomicInc(&P.counters[blk], n_cl - 1) == (unsigned)(n_cl - 1);
+        if (tid == 0) is_last = atomicInc(&P.counters[blk], P.ctas - 1) == (unsigned)(P.ctas - 1);
         __syncthreads();
         if (!is_last) return;
         __threadfence();
-        if (tid < PJ_COLS && col0 + tid < P.n_out) {
-            sum = 0.0f;
-            for (int r = 0; r < n_cl; ++r) sum += __ldcg(P.partials + (size_t)r * P.n_out + col0 + tid);
-        }
+    } else {
+        __syncthreads();
     }
     // ---- epilogue on the 64 finished sums of this column block ----
-    if (tid < PJ_COLS) val[tid] = (I8 ? sum * scale_o : sum) + bias;
+    if (tid < PJ_COLS) {
+        float sum = 0.0f;
+        if (P.n_slices == 1) {
+            sum = parts[0][tid];
+        } else if (C == 1 && P.ctas > 1) {
+            if (col0 + tid < P.n_out)
+                for (int g = 0; g < P.n_slices; ++g) sum += __ldcg(P.partials + (size_t)g * P.n_out + col0 + tid);
+        } else {
+#pragma unroll 8
+            for (int g = 0; g < P.n_slices; ++g) sum += parts[g][tid];
+        }
+        val[tid] = (I8 ? sum * scale_o : sum) + bias;
+    }
     __syncthreads();
     if (!E.enabled) {
         if (tid < PJ_COLS && col0 + tid < P.n_out) P.y[col0 + tid] = P.accum ? y_old + val[tid] : val[tid];
@@ -295,26 +303,28 @@ int launch_gemv(mx230_handle *h, void *stream, GemvParams P, int w_kind, const c
                    "%s: int8 weights need scales, an activation group of 4 or 8 and n_in %% 8 == 0 (n_in %d)", who, P.n_in);
     }
     const int n_blocks = (P.n_out + PJ_COLS - 1) / PJ_COLS;
+    // Slices: PJ_SLICES_PER_SM of them per SM over all blocks, at least 16 rows each (int8: whole activation groups and whole
+    // passes of the eight row lanes over 4-row words).  This fixes the order of the sums.
+    int n_slices = (PJ_SLICES_PER_SM * h->sm_count + n_blocks - 1) / n_blocks;
+    const int max_slices = (P.n_in + 15) / 16;
+    if (n_slices > max_slices) n_slices = max_slices;
+    const int gran = w_kind == 2 ? 4 * PJ_ROWLANES : PJ_ROWLANES;
+    P.rows_per_slice = ((P.n_in + n_slices - 1) / n_slices + gran - 1) / gran * gran;
+    P.n_slices = n_slices = (P.n_in + P.rows_per_slice - 1) / P.rows_per_slice;
+    // CTAs: up to 64 slices are one cluster per block, a few slices per CTA; the merge is then a cluster barrier.  Measured
+    // on one token through 24 layers (fp16 896 x 1152 and 896 x 896, 38 and 56 slices, int8 cache of 2001 keys, one graph):
+    // a CTA per slice and a merge through the workspace 10.5 and 9.4 us per launch, 536 us per token; this and programmatic
+    // launches of this kernel and the attention kernel, 268 us.  More slices (few columns, many rows) are merged
+    // through the workspace.
     const bool wide = w_kind == 1 && P.n_out % 8 == 0;   // fp16 rows of whole 16-byte pieces
-    const int pass = (wide ? 32 : 16) * (w_kind == 2 ? 4 : 1);   // input rows that a CTA takes in one load per thread
-    // Measured on one token through 24 layers (fp16 896 x 1152 and 896 x 896, int8 cache of 2001 keys, one graph): with 38 and
-    // 56 slices merged through the workspace 10.5 and 9.4 us per launch, 536 us per token; one cluster of eight per block
-    // and programmatic launches of this kernel and the attention kernel, 247 us.
-    // One cluster per column block, of as many CTAs (up to 8) as have a pass of rows each.  Further clusters (a merge
-    // through global memory, about 2 us) only where the blocks alone leave SMs idle and every CTA still gets four passes,
-    // or where a slice would exceed PJ_MAX_ROWS.
-    int c = (P.n_in + pass - 1) / pass;
-    P.cl_size = c < PJ_CLUSTER ? c : PJ_CLUSTER;
-    long long n_cl = (2ll * h->sm_count + n_blocks * P.cl_size - 1) / ((long long)n_blocks * P.cl_size);
-    const long long by_rows = P.n_in / ((long long)P.cl_size * 4 * pass);
-    if (n_cl > by_rows) n_cl = by_rows;
-    const long long at_least = (P.n_in + (long long)P.cl_size * PJ_MAX_ROWS - 1) / ((long long)P.cl_size * PJ_MAX_ROWS);
-    if (n_cl < at_least) n_cl = at_least;
-    P.n_slices = (int)n_cl * P.cl_size;
-    const int gran = w_kind == 2 ? 8 : 1;   // int8: a slice holds whole activation groups
-    P.rows_per_slice = ((P.n_in + P.n_slices - 1) / P.n_slices + gran - 1) / gran * gran;
-    if (n_cl > 1) {
-        const size_t need = (size_t)n_cl * P.n_out * sizeof(float);
+    if (n_slices <= PJ_CLUSTER * PJ_SLOTS) {
+        P.slots = (n_slices + PJ_CLUSTER - 1) / PJ_CLUSTER;
+        P.ctas = P.cl_size = (n_slices + P.slots - 1) / P.slots;
+    } else {
+        P.slots = wide ? 4 : 2;
+        P.ctas = (n_slices + P.slots - 1) / P.slots;
+        P.cl_size = 1;
+        const size_t need = (size_t)n_slices * P.n_out * sizeof(float);
         MX_REQUIRE(h->ws && need <= h->ws_bytes, MX230_ERR_WORKSPACE, "%s: workspace %zu B < %zu B needed", who,
                    h->ws_bytes, need);
         MX_REQUIRE((size_t)n_blocks <= h->n_counters, MX230_ERR_UNSUPPORTED, "%s: %d column blocks exceed %zu counters",
@@ -325,13 +335,17 @@ int launch_gemv(mx230_handle *h, void *stream, GemvParams P, int w_kind, const c
     }
     mx230_device_guard guard(h->device);
     cudaStream_t st = (cudaStream_t)stream;
-    const dim3 grid((unsigned)(n_blocks * P.n_slices));
-    const size_t sm = w_kind == 2 ? (size_t)P.rows_per_slice * sizeof(float) / 2 : 0;   // rows/4 words + rows/ag scales
+    const dim3 grid((unsigned)(n_blocks * P.ctas));
+    const int threads = P.slots * PJ_ROWLANES * PJ_COLS / (wide ? 8 : 4);
+    // rows/4 words + rows/ag scales; up to 12288 rows per slice fit
+    const size_t sm = w_kind == 2 ? (size_t)P.slots * P.rows_per_slice * sizeof(float) / 2 : 0;
     const int cx = P.cl_size;
-    if (w_kind == 2) MX_LAUNCH(h, st, MX230_K_GEMV, mx_launch(gemv_heads_kernel<int8_t, 4>, grid, PJ_THREADS, sm, st, cx, true, P));
-    else if (wide) MX_LAUNCH(h, st, MX230_K_GEMV, mx_launch(gemv_heads_kernel<__half, 8>, grid, PJ_THREADS, sm, st, cx, true, P));
-    else if (w_kind == 1) MX_LAUNCH(h, st, MX230_K_GEMV, mx_launch(gemv_heads_kernel<__half, 4>, grid, PJ_THREADS, sm, st, cx, true, P));
-    else MX_LAUNCH(h, st, MX230_K_GEMV, mx_launch(gemv_heads_kernel<float, 4>, grid, PJ_THREADS, sm, st, cx, true, P));
+    if (w_kind == 2) {
+        MX_SMEM_ATTR_ONCE(h->device, (gemv_heads_kernel<int8_t, 4>), 192 * 1024);
+        MX_LAUNCH(h, st, MX230_K_GEMV, mx_launch(gemv_heads_kernel<int8_t, 4>, grid, threads, sm, st, cx, true, P));
+    } else if (wide) MX_LAUNCH(h, st, MX230_K_GEMV, mx_launch(gemv_heads_kernel<__half, 8>, grid, threads, sm, st, cx, true, P));
+    else if (w_kind == 1) MX_LAUNCH(h, st, MX230_K_GEMV, mx_launch(gemv_heads_kernel<__half, 4>, grid, threads, sm, st, cx, true, P));
+    else MX_LAUNCH(h, st, MX230_K_GEMV, mx_launch(gemv_heads_kernel<float, 4>, grid, threads, sm, st, cx, true, P));
     return MX230_OK;
 }
 
