@@ -47,15 +47,10 @@ constexpr int KV_STAGES = 4;
 constexpr int TILE_BYTES = BN * HD * 2;  // 16 KB
 constexpr int HALVES = 2;               // softmax groups per query tile: each takes half of the tile's key columns
 constexpr int SOFT_WARPS = QT * HALVES * 4;   // 16
-constexpr int FWD_THREADS = (SOFT_WARPS + 4) * 32;   // 640: four softmax warpgroups + {TMA, 2 MMA issuers, idle}
-// setmaxnreg moves registers only inside the CTA's launch-time allocation (96 per thread for 640
-// threads): what the softmax warps gain must have been released by the service warpgroup, or the
-// increase would block for ever.
-#ifndef FWD_REGS_SOFTMAX
-#define FWD_REGS_SOFTMAX 104
-#define FWD_REGS_SERVICE 64
-#endif
-static_assert(SOFT_WARPS * FWD_REGS_SOFTMAX + 4 * FWD_REGS_SERVICE <= (SOFT_WARPS + 4) * 96, "setmaxnreg budget exceeds the launch-time register allocation");
+constexpr int FWD_THREADS = (SOFT_WARPS + 3) * 32;   // 608: four softmax warpgroups + {TMA, 2 MMA issuers}
+// No 20th, idle warp and no register moves between warps: every warp runs at the 96 registers per thread of the launch.
+// (640 threads, 104 for the softmax warps and 64 for the others by setmaxnreg: 48 x 4096 rows causal 170.8 us a call against
+// 166.1, no mask 284.6 against 270.0, bf16 operands 396 against 361, 8 x 8192 rows 176.7 against 164.3.)
 
 // build-time knobs of the softmax loop
 #ifndef FWD_FAST
@@ -232,10 +227,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     const uint32_t tmem = *tmem_slot;
     mx::pdl_wait();
 
-    // register budget: a softmax thread holds 64 score values and their packed probabilities, the
-    // service warpgroup (TMA, two MMA issuers, one idle warp) needs few
     if (warp >= SOFT_WARPS) {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(FWD_REGS_SERVICE));
         if (warp == SOFT_WARPS) {
         // ------------------------- TMA producer -------------------------
         if (lane == 0) {
@@ -341,7 +333,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 #pragma unroll
                 for (int t = 0; t < QT; ++t) n_it[t] = fwd_tile_iters(P, q0, KEY_SPLIT ? 0 : t);
                 const int n_max = max(n_it[0], n_it[1]);
-                const bool own_o = !KEY_SPLIT || !fwd_fast_head(P, bh, lane);   // each pair of groups sums into an O of its own
+                const bool own_o = !KEY_SPLIT || SRC == SRC_RAW || !fwd_fast_head(P, bh, lane);   // each pair of groups sums into an O of its own
                 for (int j = 0; j < n_max && ok; ++j, ++g) {
                     const int s = g % KV_STAGES;
                     ok = ISSUER_WAIT(mx::mbar_wait(bar(BAR_V_FULL + s), (g / KV_STAGES) & 1, abort_flag, P.status));
@@ -376,7 +368,6 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         // per query row and half).  Four softmax warps per scheduler instead of two hide each other's dependent-issue
         // latencies; without a row max (the usual mode) the halves never talk to each other inside the loop, and the
         // general mode has each half compute the full row's max redundantly rather than exchange it.
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(FWD_REGS_SOFTMAX));
         const int t = warp >> 3;             // query tile of this group (key-split form: parity of its key tiles)
         const int half = (warp >> 2) & 1;    // which 64 key columns of every tile
         const int row_in_tile = (warp & 3) * 32 + lane;
@@ -425,15 +416,20 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         // fp32 sums carry the same relative precision at 2^-80 .. 2^80 as around 1, every row sum stays inside
         // [2^-80, N 2^80], and the result is that of the max-subtracted form.  Heads with larger scores (and calls
         // without the norms) take the general path: running max, lazy rescale.
-        const bool fast = fwd_fast_head(P, bh, lane);
+        const bool fast = SRC != SRC_RAW && fwd_fast_head(P, bh, lane);   // (operands the caller staged come without norms)
         float m = fast ? 0.0f : -CUDART_INF_F, l = 0.0f;   // l: this group's share of the row sum
         float l_odd = 0.0f;    // pair form, fast mode: the sum over odd key tiles, l being that over even ones
         // Shares of the row sums, handed to the group that does the epilogue: [publisher][sum, second sum or max, correction].
         // The correction (what the first key tile's rounding adds to the sum that O is divided by: fast mode, see below) is
         // parked there from the first tile on, by the groups that publish nothing as well, instead of in a register.
-        float *xch = (float *)(smem + SMEM_XCH) + (it & 1) * XCH_PUBS * 3 * BM + row_in_tile;
-        float *slot = xch + (KEY_SPLIT ? 2 * t + half - 1 : t) * 3 * BM;
-        float *park = half == 1 || (KEY_SPLIT && t == 1) ? slot + 2 * BM : xch + (2 * 3 + (KEY_SPLIT ? 2 : t)) * BM;
+        // (addresses are formed where they are used: pointers kept over the loop cost registers it needs)
+        auto xch = [&](int pub, int what) -> float & {
+            return ((float *)(smem + SMEM_XCH))[(((it & 1) * XCH_PUBS + pub) * 3 + what) * BM + row_in_tile];
+        };
+        const int my_pub = KEY_SPLIT ? 2 * t + half - 1 : t;
+        auto park = [&]() -> float & {
+            return half == 1 || (KEY_SPLIT && t == 1) ? xch(my_pub, 2) : xch(2, KEY_SPLIT ? 2 : t);
+        };
         uint32_t va[32], vb[32];
         // int8 scores: exact integer dots -> row_a * (dot * ks + qsum * kb), two keys per instruction
         auto rebuild32 = [&](uint32_t *x, const float *kskb) {
@@ -454,30 +450,23 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         };
         if (fast) {
         // ---- max-free loop: the group's second 32 columns land under the exponentials of the first 32
+        constexpr int POLY = SRC == SRC_PRE ? FWD_POLY : 0;   // (the rebuilt int8 scores leave the exp unit time enough)
         uint64_t rs2;              // sum of one score tile
         float l_other = 0.0f;      // pair form: l and l_other change places after every tile: sums over even and odd key tiles
         auto exp32 = [&](const uint32_t *src, uint32_t *pk, int key_base, bool need_mask, const float *kskb, bool start) {
             uint32_t x[32];
 #pragma unroll
             for (int i = 0; i < 32; ++i) x[i] = src[i];
-            if (SRC == SRC_RAW) {
-#pragma unroll
-                for (int i = 0; i < 32; i += 2) {
-                    float a, b;
-                    mx::upk2(mx::mul2(mx::pk2(__uint_as_float(x[i]), __uint_as_float(x[i + 1])), mx::pk2(c, c)), a, b);
-                    x[i] = __float_as_uint(a), x[i + 1] = __float_as_uint(b);
-                }
-            }
             if (SRC == SRC_I8) rebuild32(x, kskb);
             if (need_mask) {   // diagonal and ragged tiles only (a warp-uniform branch: full tiles pay nothing)
 #pragma unroll
                 for (int i = 0; i < 32; ++i)
-                    if (key_base + i > last) x[i] = (FWD_POLY > 0) ? 0xC2FC0000u : 0xFF800000u;  // -126 (2^-126 against sums >= 2^-80) | -inf
+                    if (key_base + i > last) x[i] = (POLY > 0) ? 0xC2FC0000u : 0xFF800000u;  // -126 (2^-126 against sums >= 2^-80) | -inf
             }
 #pragma unroll
             for (int i = 0; i < 32; i += 2) {
                 float p0, p1;
-                if (((i >> 1) % FWD_POLY_DEN) < FWD_POLY) {
+                if (((i >> 1) % FWD_POLY_DEN) < POLY) {
                     mx::ex2_poly2<false>(__uint_as_float(x[i]), __uint_as_float(x[i + 1]), p0, p1);
                 } else {
                     p0 = mx::ex2(__uint_as_float(x[i]));
@@ -536,7 +525,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             if (FIRST) {
                 if (!(KEY_SPLIT && t == 1)) {
                     sum_rounded16(pk);
-                    *park = ((rb[0] + rb[1]) + (rb[2] + rb[3])) - sum_of(rs2);
+                    park() = ((rb[0] + rb[1]) + (rb[2] + rb[3])) - sum_of(rs2);
                 }
                 if (!o1_free()) return false;
             }
@@ -677,28 +666,28 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             if (ok && n_t > 0)
                 ok = __all_sync(0xFFFFFFFFu, mx::mbar_wait(bar(BAR_O_DONE + t), (cnt - 1) & 1, abort_flag, P.status));
             if (ok) {
-                slot[0] = l;
-                slot[BM] = KEY_SPLIT ? m : l_odd;
+                xch(my_pub, 0) = l;
+                xch(my_pub, 1) = KEY_SPLIT ? m : l_odd;
                 __syncwarp();
                 if (lane == 0) mx::mbar_arrive(bar(BAR_XCH + (KEY_SPLIT ? 0 : t)));
             }
         } else if (ok) {
             ok = __all_sync(0xFFFFFFFFu, mx::mbar_wait(bar(BAR_XCH + t), it & 1, abort_flag, P.status));
             if (ok) {
-                const float *other = xch + (KEY_SPLIT ? 0 : t) * 3 * BM;   // half 1 of this tile
-                l += other[0];
-                const float corr = fast ? *park + other[2 * BM] : 0.0f;
+                const int other = KEY_SPLIT ? 0 : t;   // half 1 of this tile
+                l += xch(other, 0);
+                const float corr = fast ? park() + xch(other, 2) : 0.0f;
                 if (KEY_SPLIT) {
-                    l_odd = other[3 * BM] + other[6 * BM];
+                    l_odd = xch(1, 0) + xch(2, 0);
                     if (!fast) {
-                        const float m1 = other[4 * BM], mm = fmaxf(m, m1);
+                        const float m1 = xch(1, 1), mm = fmaxf(m, m1);
                         w0 = mx::ex2((m - mm) * c);   // m is finite: key tile 0 has a key that every row sees
                         w1 = mx::ex2((m1 - mm) * c);
                         l *= w0, l_odd *= w1;
                         m = mm;
                     }
                 } else {
-                    l_odd += other[BM];
+                    l_odd += xch(other, 1);
                 }
                 l += l_odd;
                 l_norm = l + corr;
