@@ -9,23 +9,29 @@
 //   * fp32 weights would lose their low mantissa bits in one 16-bit operand, so both sides are staged as a
 //     (high, low) pair of bf16 values, x = hi + lo to 16 bits of mantissa, and three products are accumulated:
 //     A_hi W_hi + A_hi W_lo + A_lo W_hi.  The tensor cores have the time: these GEMMs are launch-bound.
-// CTA = one 128 x 64 tile of C; k in steps of 64 through a 4-stage TMA ring (out-of-range rows and columns are
-// zero-filled by the TMA unit, so m, n, k need no padding); one TMA warp, one MMA-issuing warp, four epilogue
-// warps that add the bias and store fp32 rows.
+// CTA = one 128 x 128 tile of C (128 x 64 where that leaves SMs idle, see mx230_gemm); k in steps of 64 through a 4-stage
+// TMA ring (out-of-range rows and columns are zero-filled by the TMA unit, so m, n, k need no padding); one TMA warp, one
+// MMA-issuing warp, eight epilogue warps that add the bias and hand fp32 pieces to the TMA unit.
+// What bounds it at these sizes is the operands' way from L2 into shared memory (1900 x 896 x 1152: 90 MB with 64-column
+// tiles, 60 MB with 128-column ones) and the launches around it.
+#include <cstring>
+
 #include "common.cuh"
 
 namespace {
 
-constexpr int GM = 128, GN = 64, GK = 64;
-constexpr int STAGES = 4;
+constexpr int GM = 128, GK = 64;
 constexpr int A_TILE = GM * GK * 2;   // 16 KB
-constexpr int W_TILE = GK * GN * 2;   // 8 KB
-constexpr int THREADS = 256;
+constexpr int W_CHUNK = GK * 64 * 2;  // 8 KB: 64 columns (one 128-byte swizzle span) of a weight tile
+constexpr int EPI_WARPS = 8;
+constexpr int THREADS = (4 + EPI_WARPS) * 32;
 
-template <bool SPLIT>
+template <bool SPLIT, int GN>
 struct Smem {
     static constexpr int PARTS = SPLIT ? 2 : 1;
+    static constexpr int W_TILE = GN / 64 * W_CHUNK;
     static constexpr int STAGE = PARTS * (A_TILE + W_TILE);
+    static constexpr int STAGES = SPLIT && GN == 128 ? 3 : 4;   // 96 .. 192 KB
     static constexpr int BAR = STAGES * STAGE;
     static constexpr int TOTAL = BAR + 128;
     static constexpr int ALLOC = TOTAL + 1024;
@@ -35,20 +41,23 @@ struct GemmParams {
     float *C;
     const float *bias;
     int m, n, k;
+    int tma_out;   // C leaves through staged TMA stores (n a multiple of 64)
     int *status;
 };
 
 // kind::f16 instruction descriptor: fp32 accumulate, A K-major, B MN-major, both operands fp16 or both bf16
-__host__ __device__ constexpr uint32_t idesc(bool bf16) {
+__host__ __device__ constexpr uint32_t idesc(bool bf16, int GN) {
     return (1u << 4) | ((bf16 ? 1u : 0u) << 7) | ((bf16 ? 1u : 0u) << 10) | (0u << 15) | (1u << 16) |
            ((uint32_t)(GN >> 3) << 17) | ((uint32_t)(GM >> 4) << 24);
 }
 
-template <bool SPLIT>
+template <bool SPLIT, int GN>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmA1,
-            const __grid_constant__ CUtensorMap tmW0, const __grid_constant__ CUtensorMap tmW1, const GemmParams P) {
-    using S = Smem<SPLIT>;
+            const __grid_constant__ CUtensorMap tmW0, const __grid_constant__ CUtensorMap tmW1,
+            const __grid_constant__ CUtensorMap tmC, const GemmParams P) {
+    using S = Smem<SPLIT, GN>;
+    constexpr int STAGES = S::STAGES, W_TILE = S::W_TILE;
     extern __shared__ unsigned char smem_dyn[];
     const uint32_t smem_base = (mx::smem_u32(smem_dyn) + 1023u) & ~1023u;
     unsigned char *smem = smem_dyn + (smem_base - mx::smem_u32(smem_dyn));
@@ -74,6 +83,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CU
     __syncthreads();
     mx::tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    mx::pdl_wait();
 
     if (warp == 0) {
         // ------------------------- TMA producer -------------------------
@@ -88,17 +98,18 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CU
                 const uint32_t base = smem_base + s * S::STAGE;
                 mx::mbar_expect_tx(bar(s), S::STAGE);
                 mx::tma_load_3d(base, &tmA0, bar(s), i * GK, m0, 0);
-                mx::tma_load_3d(base + S::PARTS * A_TILE, &tmW0, bar(s), n0, i * GK, 0);
-                if (SPLIT) {
-                    mx::tma_load_3d(base + A_TILE, &tmA1, bar(s), i * GK, m0, 0);
-                    mx::tma_load_3d(base + 2 * A_TILE + W_TILE, &tmW1, bar(s), n0, i * GK, 0);
+                if (SPLIT) mx::tma_load_3d(base + A_TILE, &tmA1, bar(s), i * GK, m0, 0);
+#pragma unroll
+                for (int c = 0; c < GN / 64; ++c) {   // (a chunk past the last column is all zero fill)
+                    mx::tma_load_3d(base + S::PARTS * A_TILE + c * W_CHUNK, &tmW0, bar(s), n0 + 64 * c, i * GK, 0);
+                    if (SPLIT) mx::tma_load_3d(base + 2 * A_TILE + W_TILE + c * W_CHUNK, &tmW1, bar(s), n0 + 64 * c, i * GK, 0);
                 }
             }
         }
         __syncwarp();
     } else if (warp == 1) {
         // ------------------------- MMA issuer (warp-uniform, one elected lane issues) --------------------
-        constexpr uint32_t IDESC = idesc(SPLIT);
+        constexpr uint32_t IDESC = idesc(SPLIT, GN);
         bool ok = true;
         for (int i = 0; i < n_steps && ok; ++i) {
             const int s = i % STAGES;
@@ -106,8 +117,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CU
             if (!ok) break;
             mx::tc_fence_after();
             const uint32_t base = smem_base + s * S::STAGE;
-            const uint64_t a0 = mx::smem_desc_sw128(base), w0 = mx::smem_desc_sw128(base + S::PARTS * A_TILE);
-            const uint64_t a1 = mx::smem_desc_sw128(base + A_TILE), w1 = mx::smem_desc_sw128(base + 2 * A_TILE + W_TILE);
+            const uint64_t a0 = mx::smem_desc_sw128(base), w0 = mx::smem_desc_sw128_mn(base + S::PARTS * A_TILE, W_CHUNK);
+            const uint64_t a1 = mx::smem_desc_sw128(base + A_TILE), w1 = mx::smem_desc_sw128_mn(base + 2 * A_TILE + W_TILE, W_CHUNK);
             if (mx::elect_one()) {
 #pragma unroll
                 for (int kk = 0; kk < GK / 16; ++kk) {   // A: 32 bytes per 16-element step inside the swizzle span; W: 16 rows of 128 bytes
@@ -124,35 +135,53 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CU
         }
     } else if (warp >= 4) {
         // ------------------------- epilogue: bias, fp32 rows out -------------------------
-        const int q = warp & 3;
+        // warp: 32 rows (its tensor-memory lanes), half of the tile's columns
+        const int q = warp & 3, colh = ((warp - 4) >> 2) * (GN / 2);
         bool ok = __all_sync(0xFFFFFFFFu, mx::mbar_wait(bar(2 * STAGES), 0, abort_flag, P.status));
         if (ok) {
             mx::tc_fence_after();
             const int row = m0 + q * 32 + lane;
             const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16);
+            // pieces of 32 x 32 go through 4 KB each of the ring's first stage or two (every MMA has read them) and the TMA
+            // unit, which clips rows past the end: 16-byte stores from lane = row registers each touch a sector of their own
+            const int st_off = (warp - 4) * 4096;
 #pragma unroll
-            for (int half = 0; half < 2; ++half) {
+            for (int part = 0; part < GN / 64; ++part) {
+                const int col0 = n0 + colh + part * 32;
+                if (col0 >= P.n) break;
                 uint32_t v[32];
-                mx::tmem_ld32(ta + half * 32, v);
+                mx::tmem_ld32(ta + colh + part * 32, v);
                 mx::tmem_wait_ld();
-                if (row < P.m) {
-                    float *crow = P.C + (size_t)row * P.n + n0 + half * 32;
+                if (part > 0 && P.tma_out) {
+                    if (lane == 0) mx::bulk_wait_group_read<0>();
+                    __syncwarp();
+                }
+                float *crow = P.tma_out ? (float *)(smem + st_off + lane * 128) : P.C + (size_t)row * P.n + col0;
 #pragma unroll
-                    for (int c = 0; c < 32; c += 4) {
-                        const int col = n0 + half * 32 + c;
-                        if (col < P.n) {   // n is a multiple of 4: a float4 is inside or outside as a whole
-                            float4 b4 = P.bias ? *(const float4 *)(P.bias + col) : make_float4(0.f, 0.f, 0.f, 0.f);
-                            *(float4 *)(crow + c) = make_float4(__uint_as_float(v[c]) + b4.x, __uint_as_float(v[c + 1]) + b4.y,
-                                                                __uint_as_float(v[c + 2]) + b4.z, __uint_as_float(v[c + 3]) + b4.w);
-                        }
+                for (int c = 0; c < 32; c += 4) {
+                    if (col0 + c >= P.n) break;   // n is a multiple of 4: a float4 is inside or outside as a whole
+                    const float4 b4 = P.bias ? *(const float4 *)(P.bias + col0 + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    const float4 o4 = make_float4(__uint_as_float(v[c]) + b4.x, __uint_as_float(v[c + 1]) + b4.y,
+                                                  __uint_as_float(v[c + 2]) + b4.z, __uint_as_float(v[c + 3]) + b4.w);
+                    if (P.tma_out) *(float4 *)((unsigned char *)crow + (((c >> 2) ^ (lane & 7)) << 4)) = o4;
+                    else if (row < P.m) *(float4 *)(crow + c) = o4;
+                }
+                if (P.tma_out) {
+                    mx::fence_proxy_async_smem();
+                    __syncwarp();
+                    if (lane == 0 && m0 + q * 32 < P.m) {
+                        mx::tma_store_3d(&tmC, smem_base + st_off, col0 & 63, m0 + q * 32, col0 >> 6);
+                        mx::bulk_commit_group();
                     }
                 }
             }
+            if (P.tma_out && lane == 0) mx::bulk_wait_group_read<0>();   // the pieces must outlive the reads
         }
     }
     mx::tc_fence_before();
     __syncthreads();
     mx::tc_fence_after();
+    mx::pdl_trigger();   // (here, when the tensor memory is no longer wanted: the next kernel may need all of it)
     if (warp == 1) mx::tmem_dealloc(tmem, GN);
 }
 
@@ -167,6 +196,8 @@ struct StageParams {
 
 template <bool SPLIT>
 __global__ void gemm_stage_kernel(StageParams P) {
+    mx::pdl_trigger();
+    mx::pdl_wait();
     const int t = blockIdx.y;
     const float4 *src = (const float4 *)P.src[t];
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < P.n4[t]; i += (size_t)gridDim.x * blockDim.x) {
@@ -190,6 +221,16 @@ __global__ void gemm_stage_kernel(StageParams P) {
 }
 
 size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
+
+template <bool SPLIT, int GN>
+int launch_tiles(mx230_handle *h, cudaStream_t st, const CUtensorMap &tA0, const CUtensorMap &tA1, const CUtensorMap &tW0,
+                 const CUtensorMap &tW1, const CUtensorMap &tC, const GemmParams &P) {
+    const dim3 grid((unsigned)((P.n + GN - 1) / GN), (unsigned)((P.m + GM - 1) / GM));
+    MX_SMEM_ATTR_ONCE(h->device, (gemm_kernel<SPLIT, GN>), (Smem<SPLIT, GN>::ALLOC));
+    MX_LAUNCH(h, st, MX230_K_GEMV, mx_launch(gemm_kernel<SPLIT, GN>, grid, THREADS, Smem<SPLIT, GN>::ALLOC, st, 1, true, tA0, tA1,
+                                             tW0, tW1, tC, P));
+    return MX230_OK;
+}
 
 }  // namespace
 
@@ -226,9 +267,9 @@ extern "C" int mx230_gemm(mx230_handle *h, void *stream, float *C, const float *
     unsigned blocks = (unsigned)((big + 255) / 256);
     if (blocks > (unsigned)h->sm_count * 8) blocks = (unsigned)h->sm_count * 8;
     if (split) {
-        MX_LAUNCH(h, st, MX230_K_CAST, (gemm_stage_kernel<true><<<dim3(blocks, 2), 256, 0, st>>>(SP)));
+        MX_LAUNCH(h, st, MX230_K_CAST, mx_launch(gemm_stage_kernel<true>, dim3(blocks, 2), 256, 0, st, 1, true, SP));
     } else {
-        MX_LAUNCH(h, st, MX230_K_CAST, (gemm_stage_kernel<false><<<dim3(blocks, 1), 256, 0, st>>>(SP)));
+        MX_LAUNCH(h, st, MX230_K_CAST, mx_launch(gemm_stage_kernel<false>, dim3(blocks, 1), 256, 0, st, 1, true, SP));
     }
 
     CUtensorMap tA0, tA1, tW0, tW1;
@@ -237,21 +278,26 @@ extern "C" int mx230_gemm(mx230_handle *h, void *stream, float *C, const float *
     if (rc) return rc;
     rc = mx230_make_tmap_2d_16bit(h, &tA1, split ? a_lo : a_hi, f16, (uint64_t)k, (uint64_t)m, (uint64_t)k * 2, GK, GM);
     if (rc) return rc;
-    rc = mx230_make_tmap_2d_16bit(h, &tW0, split ? w_hi : W_fp16, f16, (uint64_t)n, (uint64_t)k, (uint64_t)n * 2, GN, GK);
+    rc = mx230_make_tmap_2d_16bit(h, &tW0, split ? w_hi : W_fp16, f16, (uint64_t)n, (uint64_t)k, (uint64_t)n * 2, 64, GK);
     if (rc) return rc;
-    rc = mx230_make_tmap_2d_16bit(h, &tW1, split ? w_lo : W_fp16, f16, (uint64_t)n, (uint64_t)k, (uint64_t)n * 2, GN, GK);
+    rc = mx230_make_tmap_2d_16bit(h, &tW1, split ? w_lo : W_fp16, f16, (uint64_t)n, (uint64_t)k, (uint64_t)n * 2, 64, GK);
     if (rc) return rc;
 
     GemmParams P;
     P.C = C, P.bias = bias, P.m = m, P.n = n, P.k = k, P.status = h->status_dev;
-    dim3 grid((unsigned)((n + GN - 1) / GN), (unsigned)((m + GM - 1) / GM));
-    if (split) {
-        MX_SMEM_ATTR_ONCE(h->device, (gemm_kernel<true>), Smem<true>::ALLOC);
-        MX_LAUNCH(h, st, MX230_K_GEMV, (gemm_kernel<true><<<grid, THREADS, Smem<true>::ALLOC, st>>>(tA0, tA1, tW0, tW1, P)));
-    } else {
-        MX_SMEM_ATTR_ONCE(h->device, (gemm_kernel<false>), Smem<false>::ALLOC);
-        MX_LAUNCH(h, st, MX230_K_GEMV, (gemm_kernel<false><<<grid, THREADS, Smem<false>::ALLOC, st>>>(tA0, tA1, tW0, tW1, P)));
-    }
+    // C [m][n] as [n / 64][m][64]: the store map of the attention kernels
+    CUtensorMap tC;
+    memset(&tC, 0, sizeof(tC));
+    P.tma_out = n % 64 == 0;
+    if (P.tma_out && (rc = mx230_make_tmap_f32_half_rows_strided(h, &tC, C, (uint64_t)m, (uint64_t)(n / 64), (uint64_t)n * 4, 256)))
+        return rc;
+    // 128-column tiles move two thirds of the bytes per CTA step that two 64-column ones do; they are taken when there are
+    // enough of them for two thirds of the SMs.  (Attention half of a layer, 1900 tokens, fp16 896 x 1152 and 896 x 896: these
+    // tiles, the TMA epilogue and programmatic launches of staging and GEMM 69.6 -> 55.2 us.)
+    const bool wide = (long long)((n + 127) / 128) * ((m + GM - 1) / GM) * 3 >= 2ll * h->sm_count;
+    if (split) rc = wide ? launch_tiles<true, 128>(h, st, tA0, tA1, tW0, tW1, tC, P) : launch_tiles<true, 64>(h, st, tA0, tA1, tW0, tW1, tC, P);
+    else rc = wide ? launch_tiles<false, 128>(h, st, tA0, tA1, tW0, tW1, tC, P) : launch_tiles<false, 64>(h, st, tA0, tA1, tW0, tW1, tC, P);
+    if (rc) return rc;
     MX_CHECK_CUDA(cudaGetLastError());
     return MX230_OK;
 }

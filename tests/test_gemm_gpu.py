@@ -101,3 +101,23 @@ def test_prefill_layer_attention_with_projections(handle, quant):
     assert_close(attn[pos0:].cpu().numpy(), want_attn, "attention rows")
     want_y = oracle.gemm(attn[pos0:].cpu().numpy(), w_proj, b_proj)
     assert_close(y[pos0:].cpu().numpy(), want_y, "output projection", max_abs=2e-4, mean_rel=2e-5)
+
+
+@pytest.mark.parametrize("fp16", [False, True])
+@pytest.mark.parametrize("m,n,k", [
+    (1900, 1152, 896),   # 128-column tiles, ragged rows
+    (1665, 1096, 48),    # the last tile 72 columns wide (its second 64-column chunk ragged, plain stores), one partial k step
+    (12700, 200, 144),   # the last tile's second 64-column chunk ragged
+    (12801, 64, 64),     # half of every tile past the last column
+])
+def test_wide_tiles(handle, m, n, k, fp16):
+    """128-column tiles against 64-bit sums; tolerances as at the top (k <= 896)."""
+    a = dev(oracle.normal((m, k), 731, 0))
+    w = dev((oracle.normal((k, n), 732, 1) / np.sqrt(k)).astype(np.float16 if fp16 else np.float32))
+    b = dev(oracle.normal((n,), 733, 2))
+    c = torch.full((m, n), float("nan"), device="cuda")
+    la.gemm(handle, c, a, w, b)
+    handle.check_status()
+    want = (a.double() @ w.double() + b.double()).cpu().numpy()
+    tol = dict(max_abs=5e-3, mean_rel=1e-3) if fp16 else dict(max_abs=2e-4, mean_rel=2e-5)
+    assert_close(c.cpu().numpy(), want, f"gemm {m}x{n}x{k} fp16={fp16}", **tol)
