@@ -52,8 +52,7 @@ struct DecodeParams {
     int max_keys;        // capacity of one sequence (slab rows, or table entries x block) when positions come from the device; 0 = unknown
     int n_head, n_kv_head, group, head_groups;
     int score_mode;
-    // key splits of one (sequence, K/V head) group: grid.x = max_clusters clusters of cl_size CTAs (a power of two up to
-    // 8); a sequence of `len` keys uses the first ceil(len / cluster_keys) clusters (all of them when cluster_keys == 0),
+    // key splits of one (sequence, K/V head) group: grid.x = max_clusters clusters of cl_size CTAs (up to 8); a sequence of `len` keys uses the first ceil(len / cluster_keys) clusters (all of them when cluster_keys == 0),
     // so that the split follows the length of each sequence and not only the largest one
     int cl_size, max_clusters, cluster_keys;
     // Let the next kernel of the stream in once this one's loops are done: only a grid that leaves SMs free.  After a larger
@@ -1494,7 +1493,8 @@ int launch_g(mx230_handle *h, cudaStream_t st, const DecodeParams &P, dim3 grid)
 // head group) pairs; keys: largest number of keys of a sequence, 0 = unknown (position on the device).
 //  * whole grid resident at once: cl_size * max_clusters * groups <= slots (a partial second wave would nearly double
 //    the time);
-//  * up to 8 CTAs of a group form a cluster, whose merge costs one cluster barrier; pass_keys = keys that a CTA's warps
+//  * up to 8 CTAs of a group (any number, so that 6 per group fill 444 slots where 4 would leave a third of them empty) form
+//    a cluster, whose merge costs one cluster barrier; pass_keys = keys that a CTA's warps
 //    take in one tile each: a CTA is not given less than one such pass;
 //  * further clusters join in (merge through global memory, about 2 us) only for sequences with more than 4 passes per
 //    CTA of the first; the kernel decides that per sequence from its actual length;
@@ -1511,8 +1511,8 @@ void plan_splits(DecodeParams &P, long long slots, long long groups, long long k
         P.cluster_keys = pass_keys;
         return;
     }
-    int c = 1;
-    while (c < 8 && 2 * c <= want && (!known || (long long)c * pass_keys < keys)) c *= 2;
+    int c = want < 8 ? (int)want : 8;
+    if (known && c > (keys + pass_keys - 1) / pass_keys) c = (int)((keys + pass_keys - 1) / pass_keys);
     P.cl_size = c;
     P.cluster_keys = 4 * c * pass_keys;
     long long k = want / c;
