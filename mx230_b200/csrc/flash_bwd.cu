@@ -208,6 +208,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmOwnA, const __grid_constant__ C
     __syncthreads();
     mx::tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    mx::pdl_wait();   // (launched programmatically: the set-up above runs under the previous kernel's tail)
 
     if (warp >= 8) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS_SERVICE));
@@ -738,12 +739,15 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmOwnA, const __grid_constant__ C
     mx::tc_fence_before();
     __syncthreads();
     mx::tc_fence_after();
+    mx::pdl_trigger();   // (at the very end: what follows would otherwise fill the SMs that finish first)
     if (warp == 9) mx::tmem_dealloc(tmem, TM_COLS);
 }
 
 // Delta_i = sum_x dO[i,x] O[i,x]; 16 threads per row, one float4 each.  With `dOb` the bf16 copy of dO that the
 // backward's tensor-core passes read is written on the way (the values are in registers here anyway).
 __global__ void bwd_preprocess_kernel(const float *dO, const float *O, float *Delta, size_t rows, __nv_bfloat16 *dOb) {
+    mx::pdl_trigger();
+    mx::pdl_wait();
     size_t gid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     size_t row = gid >> 4;
     int part = (int)(gid & 15);
@@ -813,12 +817,10 @@ int launch_dq(mx230_handle *h, cudaStream_t st, const Maps &m, const float *L, c
     dim3 grid((unsigned)set_items(P, batch_heads, n));   // one item per CTA
     if (pre)
         MX_LAUNCH(h, st, MX230_K_BWD_DQ,
-                  (bwd_kernel<0, true><<<grid, BWD_THREADS, SM_ALLOC, st>>>(m.box128[0], m.box128[3], m.box128[1], m.box128[2],
-                                                                            m.box128[0], m.box128[0], m.box128[0], P)));
+                  mx_launch(bwd_kernel<0, true>, grid, BWD_THREADS, SM_ALLOC, st, 1, true, m.box128[0], m.box128[3], m.box128[1], m.box128[2], m.box128[0], m.box128[0], m.box128[0], P));
     else
         MX_LAUNCH(h, st, MX230_K_BWD_DQ,
-                  (bwd_kernel<0, false><<<grid, BWD_THREADS, SM_ALLOC, st>>>(m.box128[0], m.box128[3], m.box128[1], m.box128[2],
-                                                                             m.box128[0], m.box128[0], m.box128[0], P)));
+                  mx_launch(bwd_kernel<0, false>, grid, BWD_THREADS, SM_ALLOC, st, 1, true, m.box128[0], m.box128[3], m.box128[1], m.box128[2], m.box128[0], m.box128[0], m.box128[0], P));
     return MX230_OK;
 }
 
@@ -828,12 +830,10 @@ int launch_dkv(mx230_handle *h, cudaStream_t st, const Maps &m, const float *L, 
     dim3 grid((unsigned)set_items(P, batch_heads, n));   // one item per CTA
     if (pre)
         MX_LAUNCH(h, st, MX230_K_BWD_DKV,
-                  (bwd_kernel<1, true><<<grid, BWD_THREADS, SM_ALLOC, st>>>(m.box128[1], m.box128[2], m.box128[0], m.box128[3],
-                                                                            m.box128[0], m.box128[0], m.box128[0], P)));
+                  mx_launch(bwd_kernel<1, true>, grid, BWD_THREADS, SM_ALLOC, st, 1, true, m.box128[1], m.box128[2], m.box128[0], m.box128[3], m.box128[0], m.box128[0], m.box128[0], P));
     else
         MX_LAUNCH(h, st, MX230_K_BWD_DKV,
-                  (bwd_kernel<1, false><<<grid, BWD_THREADS, SM_ALLOC, st>>>(m.box128[1], m.box128[2], m.box128[0], m.box128[3],
-                                                                             m.box128[0], m.box128[0], m.box128[0], P)));
+                  mx_launch(bwd_kernel<1, false>, grid, BWD_THREADS, SM_ALLOC, st, 1, true, m.box128[1], m.box128[2], m.box128[0], m.box128[3], m.box128[0], m.box128[0], m.box128[0], P));
     return MX230_OK;
 }
 
@@ -856,12 +856,10 @@ int launch_fused(mx230_handle *h, cudaStream_t st, const Maps &m, const float *L
     dim3 grid((unsigned)(n_items < h->sm_count ? n_items : h->sm_count));
     if (pre)
         MX_LAUNCH(h, st, MX230_K_BWD_FUSED,
-                  (bwd_kernel<2, true><<<grid, BWD_THREADS, SM_ALLOC, st>>>(m.box128[1], m.box128[2], m.box128[0], m.box128[3],
-                                                                            tm_dq, tm_dk, tm_dv, P)));
+                  mx_launch(bwd_kernel<2, true>, grid, BWD_THREADS, SM_ALLOC, st, 1, true, m.box128[1], m.box128[2], m.box128[0], m.box128[3], tm_dq, tm_dk, tm_dv, P));
     else
         MX_LAUNCH(h, st, MX230_K_BWD_FUSED,
-                  (bwd_kernel<2, false><<<grid, BWD_THREADS, SM_ALLOC, st>>>(m.box128[1], m.box128[2], m.box128[0], m.box128[3],
-                                                                             tm_dq, tm_dk, tm_dv, P)));
+                  mx_launch(bwd_kernel<2, false>, grid, BWD_THREADS, SM_ALLOC, st, 1, true, m.box128[1], m.box128[2], m.box128[0], m.box128[3], tm_dq, tm_dk, tm_dv, P));
     return MX230_OK;
 }
 
@@ -958,7 +956,7 @@ extern "C" int mx230_attn_bwd_preprocess(mx230_handle *h, void *stream, const fl
         h->staged.d_o = nullptr;
     }
     MX_LAUNCH(h, st, MX230_K_BWD_PREPROCESS,
-              (bwd_preprocess_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(dO, O, Delta, rows, dOb)));
+              mx_launch(bwd_preprocess_kernel, (unsigned)((threads + 255) / 256), 256, 0, st, 1, true, dO, O, Delta, rows, dOb));
     if (dOb) h->staged.d_o = dO;
     return MX230_OK;
 }
