@@ -161,20 +161,29 @@ __device__ __forceinline__ int fwd_tile_iters(const FwdParams &P, int q0, int t)
     return P.causal ? min(n_kv_total, (r0 + BM - 1 + P.q_off) / BN + 1) : n_kv_total;
 }
 
-// Whether every score of head `bh` is bounded by 80 in log2 units (see the softmax loop); whole-warp call.
-__device__ __forceinline__ bool fwd_fast_head(const FwdParams &P, int bh, int lane) {
+// Largest score, in log2 units, of a head that takes the max-free loop: against the reference 0, or (SRC_RAW_BOUND, SRC_I8) against
+// a row's max over the first key tile, from which a score may be twice as far (probabilities stay below 2^80 either way).
+constexpr float FAST_BOUND = 80.0f, FAST_BOUND_REF = 40.0f;
+// Whether every score of head `bh` is within `bound` (see the softmax loop); whole-warp call.  Operands the
+// caller staged: from the bound that raw_bounds_kernel left in L at the first row of every query tile (`row0`: the tile's),
+// read before that tile's epilogue, which overwrites it and which waits for every warp that reads it.
+__device__ __forceinline__ bool fwd_fast_raw(const FwdParams &P, int bh, int row0) {
+    return FWD_FAST && row0 < P.n_q && *(const volatile float *)(P.L + (size_t)bh * P.n_q + row0) <= FAST_BOUND_REF * FAST_BOUND_REF;
+}
+__device__ __forceinline__ bool fwd_fast_head(const FwdParams &P, int bh, int lane, float bound) {
     if (!FWD_FAST || P.q_norm2 == nullptr) return false;
     static_assert(MX230_NORM_PARTS == 32, "one part per lane");
     // norms are >= 0 or NaN: as integers they order like that, with NaN the largest
     const int nq = __reduce_max_sync(0xFFFFFFFFu, __float_as_int(P.q_norm2[(size_t)bh * MX230_NORM_PARTS + lane]) & 0x7FFFFFFF);
     const int nk = __reduce_max_sync(0xFFFFFFFFu, __float_as_int(P.k_norm2[(size_t)(bh / P.kv_group) * MX230_NORM_PARTS + lane]) & 0x7FFFFFFF);
     // the norms are those of the fp32 values; rounding to bf16 moves a norm by less than 0.4 %
-    return __int_as_float(nq) * __int_as_float(nk) * (MX230_QK_LOG2_SCALE * MX230_QK_LOG2_SCALE) <= 80.0f * 80.0f;
+    return __int_as_float(nq) * __int_as_float(nk) * (MX230_QK_LOG2_SCALE * MX230_QK_LOG2_SCALE) <= bound * bound;
 }
 
-// Where scores come from: Q staged times scale * log2(e) (they arrive in log2 units), Q and K as the caller gave them, or
-// int8 codes of both (exact integer dots, see FwdParams::row_a).
-enum { SRC_PRE = 0, SRC_RAW = 1, SRC_I8 = 2 };
+// Where scores come from: Q staged times scale * log2(e) (they arrive in log2 units), Q and K as the caller gave them
+// (general loop only), the same with a bound in L, or int8 codes of both (exact integer dots, see FwdParams::row_a).
+// (A kernel of its own for RAW without a bound: with the max-free loop beside it the general one is 5 % slower.)
+enum { SRC_PRE = 0, SRC_RAW = 1, SRC_RAW_BOUND = 2, SRC_I8 = 3 };
 
 // KEY_SPLIT: an item is ONE query tile whose even key tiles belong to softmax groups 0, 1 and whose odd ones to groups 2, 3,
 // each pair with its own S and P in tensor memory, so that both pairs of groups work on every item and items are half as
@@ -333,7 +342,9 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 #pragma unroll
                 for (int t = 0; t < QT; ++t) n_it[t] = fwd_tile_iters(P, q0, KEY_SPLIT ? 0 : t);
                 const int n_max = max(n_it[0], n_it[1]);
-                const bool own_o = !KEY_SPLIT || SRC == SRC_RAW || !fwd_fast_head(P, bh, lane);   // each pair of groups sums into an O of its own
+                const bool own_o = !KEY_SPLIT || SRC == SRC_RAW ||
+                                   !(SRC == SRC_RAW_BOUND ? fwd_fast_raw(P, bh, q0)
+                                                          : fwd_fast_head(P, bh, lane, SRC == SRC_I8 ? FAST_BOUND_REF : FAST_BOUND));   // each pair of groups sums into an O of its own
                 for (int j = 0; j < n_max && ok; ++j, ++g) {
                     const int s = g % KV_STAGES;
                     ok = ISSUER_WAIT(mx::mbar_wait(bar(BAR_V_FULL + s), (g / KV_STAGES) & 1, abort_flag, P.status));
@@ -378,13 +389,19 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         const uint32_t tm_o = tmem + lane_off + TM_O + t * HD;
         // Scores arrive in log2 units when Q was staged pre-multiplied by scale * log2(e) or when they are rebuilt from
         // integer dots (c = 1), else raw (c = scale * log2(e)).
-        constexpr float c = SRC == SRC_RAW ? MX230_QK_LOG2_SCALE : 1.0f;
-        constexpr float l_scale = SRC == SRC_RAW ? 0.125f : 0.6931471805599453f;   // running max -> natural-log units
+        constexpr bool RAW = SRC == SRC_RAW || SRC == SRC_RAW_BOUND;
+        constexpr float c = RAW ? MX230_QK_LOG2_SCALE : 1.0f;
+        constexpr float l_scale = RAW ? 0.125f : 0.6931471805599453f;   // running max -> natural-log units
+        // These sources need a multiply per score anyway, which subtracts a reference for free: the max-free loop then takes
+        // probabilities against the row's max over the first key tile, as the general loop does until a later tile raises
+        // it (against 0 the leading probability is rounded like any other: 1 to 8 % more error with int8 scores).
+        constexpr bool REF = SRC != SRC_PRE;
         bool ok = true;
         uint32_t cnt = 0;  // score tiles this group has taken so far, over all items
         uint32_t cnt1 = 0; // key-split form: odd key tiles so far (what groups 2, 3 count in cnt)
         uint32_t g0 = 0;   // key tiles of the items so far (int8 scores: ring position)
-        uint32_t xmc = 0;  // row-max exchanges this group has made so far (general-mode tiles only)
+        uint32_t xmc = 0;  // row-max exchanges this tile's groups have made so far
+        uint32_t xmc0 = 0; // key-split form, odd groups: those of the even ones
         int bh, q0;
         for (int it = 0; ok && fwd_item(P, it, bh, q0); ++it) {
         const int n_all = KEY_SPLIT ? fwd_tile_iters(P, q0, 0) : 0;
@@ -416,7 +433,9 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         // fp32 sums carry the same relative precision at 2^-80 .. 2^80 as around 1, every row sum stays inside
         // [2^-80, N 2^80], and the result is that of the max-subtracted form.  Heads with larger scores (and calls
         // without the norms) take the general path: running max, lazy rescale.
-        const bool fast = SRC != SRC_RAW && fwd_fast_head(P, bh, lane);   // (operands the caller staged come without norms)
+        const bool fast = SRC == SRC_RAW ? false
+                          : SRC == SRC_RAW_BOUND ? fwd_fast_raw(P, bh, row0)
+                                                 : fwd_fast_head(P, bh, lane, REF ? FAST_BOUND_REF : FAST_BOUND);
         float m = fast ? 0.0f : -CUDART_INF_F, l = 0.0f;   // l: this group's share of the row sum
         float l_odd = 0.0f;    // pair form, fast mode: the sum over odd key tiles, l being that over even ones
         // Shares of the row sums, handed to the group that does the epilogue: [publisher][sum, second sum or max, correction].
@@ -431,8 +450,9 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             return half == 1 || (KEY_SPLIT && t == 1) ? xch(my_pub, 2) : xch(2, KEY_SPLIT ? 2 : t);
         };
         uint32_t va[32], vb[32];
-        // int8 scores: exact integer dots -> row_a * (dot * ks + qsum * kb), two keys per instruction
-        auto rebuild32 = [&](uint32_t *x, const float *kskb) {
+        // int8 scores: exact integer dots -> row_a * (dot * ks + qsum * kb) + add, two keys per instruction
+        auto rebuild32 = [&](uint32_t *x, const float *kskb, float add) {
+            const uint64_t add_2 = mx::pk2(add, add);
             const uint64_t qs2 = mx::pk2(row_qsum, row_qsum), ra2 = mx::pk2(row_a, row_a);
 #pragma unroll
             for (int i = 0; i < 32; i += 4) {
@@ -442,23 +462,62 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 const uint64_t w = mx::fma2(mx::pk2(__uint_as_float(x[i + 2]), __uint_as_float(x[i + 3])), mx::pk2(k4.z, k4.w),
                                             mx::mul2(qs2, mx::pk2(b4.z, b4.w)));
                 float a, b;
-                mx::upk2(mx::mul2(ra2, u), a, b);
+                mx::upk2(mx::fma2(ra2, u, add_2), a, b);
                 x[i] = __float_as_uint(a), x[i + 1] = __float_as_uint(b);
-                mx::upk2(mx::mul2(ra2, w), a, b);
+                mx::upk2(mx::fma2(ra2, w, add_2), a, b);
                 x[i + 2] = __float_as_uint(a), x[i + 3] = __float_as_uint(b);
             }
         };
+        // the halves of a row exchange their maxima of one score tile through shared memory (one bounded barrier)
+        float *xmax = (float *)(smem + SMEM_XMAX) + row_in_tile;   // [QT][2 exchange parities][HALVES][BM]
+        auto row_max = [&](float own) -> float {
+            float *xm = xmax + (t * 2 + (xmc & 1)) * HALVES * BM;
+            xm[half * BM] = own;
+            __syncwarp();
+            if (lane == 0) mx::mbar_arrive(bar(BAR_XMAX + t));
+            ok = __all_sync(0xFFFFFFFFu, mx::mbar_wait(bar(BAR_XMAX + t), xmc & 1, abort_flag, P.status));
+            ++xmc;
+            return fmaxf(own, xm[(1 - half) * BM]);
+        };
+        // this half's maximum of a score tile in va, vb: four independent chains (a single one would serialise on the latency)
+        auto max64 = [&]() {
+            float mx4[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) mx4[u] = fmaxf(__uint_as_float(va[u]), __uint_as_float(vb[u]));
+#pragma unroll
+            for (int i = 4; i < 32; i += 4)
+#pragma unroll
+                for (int u = 0; u < 4; ++u) mx4[u] = fmax3(mx4[u], __uint_as_float(va[i + u]), __uint_as_float(vb[i + u]));
+            return fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+        };
+        auto mask64 = [&](int key_base) {   // keys this row does not see
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+                if (key_base + i > last) va[i] = 0xFF800000u;  // -inf
+                if (key_base + 32 + i > last) vb[i] = 0xFF800000u;
+            }
+        };
         if (fast) {
+        float nmc = 0.0f;   // REF: minus the reference, in log2 units
         // ---- max-free loop: the group's second 32 columns land under the exponentials of the first 32
         constexpr int POLY = SRC == SRC_PRE ? FWD_POLY : 0;   // (the rebuilt int8 scores leave the exp unit time enough)
         uint64_t rs2;              // sum of one score tile
         float l_other = 0.0f;      // pair form: l and l_other change places after every tile: sums over even and odd key tiles
-        auto exp32 = [&](const uint32_t *src, uint32_t *pk, int key_base, bool need_mask, const float *kskb, bool start) {
+        auto exp32 = [&](const uint32_t *src, uint32_t *pk, int key_base, bool need_mask, const float *kskb, bool start, bool scores) {
             uint32_t x[32];
 #pragma unroll
             for (int i = 0; i < 32; ++i) x[i] = src[i];
-            if (SRC == SRC_I8) rebuild32(x, kskb);
-            if (need_mask) {   // diagonal and ragged tiles only (a warp-uniform branch: full tiles pay nothing)
+            if (RAW || (REF && scores)) {   // to log2 units, against the reference
+#pragma unroll
+                for (int i = 0; i < 32; i += 2) {
+                    float a, b;
+                    mx::upk2(mx::fma2(mx::pk2(__uint_as_float(x[i]), __uint_as_float(x[i + 1])), mx::pk2(c, c), mx::pk2(nmc, nmc)), a, b);
+                    x[i] = __float_as_uint(a), x[i + 1] = __float_as_uint(b);
+                }
+            } else if (SRC == SRC_I8) {
+                rebuild32(x, kskb, nmc);
+            }
+            if (need_mask && !scores) {   // diagonal and ragged tiles only (a warp-uniform branch: full tiles pay nothing)
 #pragma unroll
                 for (int i = 0; i < 32; ++i)
                     if (key_base + i > last) x[i] = (POLY > 0) ? 0xC2FC0000u : 0xFF800000u;  // -126 (2^-126 against sums >= 2^-80) | -inf
@@ -505,7 +564,22 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             const bool need_mask = (key0 + BN > N) || (P.causal && key0 + BN - 1 > row0 + P.q_off);
             const float *kskb = SRC == SRC_I8 ? kskb_of(j) : nullptr;
             uint32_t pk[16];
-            exp32(va, pk, key0 + half * (BN / 2), need_mask, kskb, true);
+            constexpr bool LEAD = REF && FIRST;
+            const bool scores = LEAD && !(KEY_SPLIT && t == 1);   // va, vb hold masked scores already
+            if (scores) {   // the reference: the row's max over its first key tile
+                mx::tmem_wait_ld();
+                if (SRC == SRC_I8) rebuild32(va, kskb, 0.0f), rebuild32(vb, kskb + 32, 0.0f);
+                if (need_mask) mask64(key0 + half * (BN / 2));
+                m = row_max(max64());
+                if (!ok) return false;
+            } else if (LEAD) {   // odd key tiles of the key-split form: that of the even ones
+                good = __all_sync(0xFFFFFFFFu, mx::mbar_wait(bar(BAR_XMAX), xmc0 & 1, abort_flag, P.status));
+                if (!good) return false;
+                const float *xm = xmax + (xmc0 & 1) * HALVES * BM;
+                m = fmaxf(xm[0], xm[BM]);
+            }
+            if (LEAD) nmc = -m * c;
+            exp32(va, pk, key0 + half * (BN / 2), need_mask, kskb, true, scores);
             mx::tmem_wait_ld();                                       // this group's columns have left S_t
             mx::tc_fence_before();
             __syncwarp();
@@ -520,7 +594,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             }
             mx::tmem_st16(tm_p, pk);
             if (FIRST && !(KEY_SPLIT && t == 1)) sum_rounded16(pk);
-            exp32(vb, pk, key0 + half * (BN / 2) + 32, need_mask, kskb + 32, false);
+            exp32(vb, pk, key0 + half * (BN / 2) + 32, need_mask, kskb + 32, false, scores);
             mx::tmem_st16(tm_p + 16, pk);
             if (FIRST) {
                 if (!(KEY_SPLIT && t == 1)) {
@@ -558,7 +632,6 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         // ---- general loop: running row max, raised lazily.  Each half takes the max of its own 64 columns and the two
         // exchange them through shared memory (one bounded barrier per tile and query tile); both then hold the same
         // row max and take the same decisions, exponentiate their own columns and rescale their own 32 columns of O.
-        float *xmax = (float *)(smem + SMEM_XMAX) + t * 2 * HALVES * BM;   // [2 tile parities][HALVES][BM]
         for (int j = 0; j < n_t; ++j, ++cnt) {
             ok = __all_sync(0xFFFFFFFFu, mx::mbar_wait(bar(BAR_S_FULL + t), cnt & 1, abort_flag, P.status));
             if (!ok) break;
@@ -572,34 +645,12 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             const int key0 = key_tile(j) * BN, col0 = half * (BN / 2);
             if (SRC == SRC_I8) {   // the tile holds exact integer dots of int8 codes: the reference kernel's score for them
                 const float *kskb = kskb_of(j);
-                rebuild32(va, kskb);
-                rebuild32(vb, kskb + 32);
+                rebuild32(va, kskb, 0.0f);
+                rebuild32(vb, kskb + 32, 0.0f);
             }
-            if ((key0 + BN > N) || (P.causal && key0 + BN - 1 > row0 + P.q_off)) {
-#pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                    if (key0 + col0 + i > last) va[i] = 0xFF800000u;  // -inf
-                    if (key0 + col0 + 32 + i > last) vb[i] = 0xFF800000u;
-                }
-            }
-            // four independent max chains (a single chain would serialise on the ALU latency)
-            float mx4[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) mx4[u] = fmaxf(__uint_as_float(va[u]), __uint_as_float(vb[u]));
-#pragma unroll
-            for (int i = 4; i < 32; i += 4)
-#pragma unroll
-                for (int u = 0; u < 4; ++u) mx4[u] = fmax3(mx4[u], __uint_as_float(va[i + u]), __uint_as_float(vb[i + u]));
-            float mx_ = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-            // exchange with the other half of the row
-            float *xm = xmax + (cnt & 1) * HALVES * BM;
-            xm[half * BM + row_in_tile] = mx_;
-            __syncwarp();
-            if (lane == 0) mx::mbar_arrive(bar(BAR_XMAX + t));
-            ok = __all_sync(0xFFFFFFFFu, mx::mbar_wait(bar(BAR_XMAX + t), xmc & 1, abort_flag, P.status));
-            ++xmc;
+            if ((key0 + BN > N) || (P.causal && key0 + BN - 1 > row0 + P.q_off)) mask64(key0 + col0);
+            const float mx_ = row_max(max64());
             if (!ok) break;
-            mx_ = fmaxf(mx_, xm[(1 - half) * BM + row_in_tile]);
             // raise the running max only when it pays (always on the first tile)
             const bool raise = (j == 0) || ((mx_ - m) * c > RESCALE_LOG2);
             const float m_new = raise ? mx_ : m;
@@ -694,6 +745,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             }
         }
         if (KEY_SPLIT) cnt1 += (uint32_t)(n_all >> 1);
+        if (KEY_SPLIT && t == 1) xmc0 += fast ? (REF ? 1u : 0u) : (uint32_t)((n_all + 1) >> 1);
         // epilogue: O / l and the log-sum-exp
         if (ok && n_t > 0 && half == 0 && !(KEY_SPLIT && t == 1)) {
             const bool odd = KEY_SPLIT && n_all > 1, two = odd && !fast;   // O_1 holds something
@@ -775,6 +827,59 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     // rows, next call's cast: 9 us slower with the trigger at the top).
     mx::pdl_trigger();
     if (warp == SOFT_WARPS + 1) mx::tmem_dealloc(tmem, TM_COLS);
+}
+
+// Largest |q|^2 |k|^2 scale^2 log2(e)^2 over the rows of a head of bf16 Q and K -> L[head][first row of every query tile],
+// where flash_fwd_kernel looks for it (its own scratch would be shared by the streams of a handle; L is the call's).  A
+// cluster per head, eight threads per row; bound by the latency of its loads (24 heads of 2048 rows: about 4 us).
+constexpr int RB_THREADS = 256, RB_CLUSTER = 8;
+__global__ void __launch_bounds__(RB_THREADS) raw_bounds_kernel(const uint4 *Q, const uint4 *K, float *L, int n) {
+    __shared__ int most[2];
+    const int tid = threadIdx.x, rank = blockIdx.x, bh = blockIdx.y;
+    mx::pdl_trigger();
+    if (tid < 2) most[tid] = 0;
+    __syncthreads();
+    mx::cluster_arrive_release();
+    mx::pdl_wait();
+    const size_t base = (size_t)bh * n * 8;   // uint4s of 8 values
+    const int c = tid & 7;
+    int best[2] = {0, 0};   // squared norms as ordered integers (NaN largest)
+    auto norm2 = [&](const uint4 &v) {
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+        float ss = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float a = __uint_as_float(w[i] << 16), b = __uint_as_float(w[i] & 0xFFFF0000u);
+            ss = fmaf(a, a, fmaf(b, b, ss));
+        }
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, o);   // the row's eight threads
+        return __float_as_int(ss) & 0x7FFFFFFF;
+    };
+    constexpr int STEP = RB_CLUSTER * RB_THREADS / 8, U = 4;   // rows per pass, passes in flight
+    for (int r0 = 0; r0 < n; r0 += U * STEP) {
+        uint4 q[U], k[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int r = r0 + u * STEP + rank * (RB_THREADS / 8) + (tid >> 3);
+            q[u] = k[u] = make_uint4(0, 0, 0, 0);
+            if (r < n) q[u] = Q[base + (size_t)r * 8 + c], k[u] = K[base + (size_t)r * 8 + c];
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) best[0] = max(best[0], norm2(q[u])), best[1] = max(best[1], norm2(k[u]));
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        best[i] = __reduce_max_sync(0xFFFFFFFFu, best[i]);
+        if ((tid & 31) == 0) atomicMax(&most[i], best[i]);
+    }
+    __syncthreads();
+    mx::cluster_wait();
+    if (rank != 0 && tid < 2) mx::cluster_red_max(mx::cluster_map(mx::smem_u32(&most[tid]), 0), most[tid]);
+    mx::cluster_sync();
+    if (rank != 0) return;
+    const float bound = __int_as_float(most[0]) * __int_as_float(most[1]) * (MX230_QK_LOG2_SCALE * MX230_QK_LOG2_SCALE);
+    for (int r = tid * BM; r < n; r += RB_THREADS * BM) L[(size_t)bh * n + r] = bound;
 }
 
 // fp32 -> bf16 (round to nearest even) for up to four equally sized tensors of `heads` x `per_head4` float4s.
@@ -887,9 +992,10 @@ namespace {
 // Which form a call takes.  Work is counted in 128 x 128 score tiles; the items of a form go to the SMs heaviest first in
 // snake order, and the call takes as long as the fullest SM.  A pair item (two query tiles) costs the tiles of both (one and
 // a half times the tiles where it has only one: half the softmax groups idle), a key-split item 1.2 times those of its query
-// tile (it reads every K/V tile for one query tile only) plus one.  Key-split items are half as large, so they even out
-// calls with few items.  Measured (us a call, pair / key-split; 12 heads unless given): 1000 rows causal 20.8 / 15.7, 2048
-// rows causal 33.7 / 25.4, 1 x 8192 rows 87 / 54, 24 x 4096 rows causal 101 / 111, 96 x 4096 rows causal 352 / 411.
+// tile (it reads every K/V tile for one query tile only) plus two.  Key-split items are half as large, so they even out
+// calls with few items.  Measured (us a call, pair / key-split; 12 heads unless given): 1000 rows causal 18.7 / 15.7, 2048
+// rows causal 30.3 / 24.4, 1 x 8192 rows 76 / 51, 4096 rows causal 52.6 / 57.4, 24 x 4096 rows causal 93 / 108, 48 x 4096 rows
+// causal 165 / 198.  Over 110 such pairs of timings the rule costs 0.1 % on average, 6 % at most.
 bool fwd_key_split(int heads, int n_q, int n_k, int q_off, int causal, int sms) {
     const int tiles = (n_q + BM - 1) / BM, pairs = (tiles + 1) / 2, n_kv = (n_k + BN - 1) / BN;
     if (sms > 256 || (long long)pairs * heads > 4LL * sms) return false;
@@ -904,7 +1010,7 @@ bool fwd_key_split(int heads, int n_q, int n_k, int q_off, int causal, int sms) 
         for (int rank = 0, i = 0; rank < blocks; ++rank) {
             const int b = causal ? blocks - 1 - rank : rank;
             long long cost;   // in tenths of a tile
-            if (split) cost = 12LL * iters(b) + 10;
+            if (split) cost = 12LL * iters(b) + 20;
             else cost = 2 * b + 1 < tiles ? 10LL * (iters(2 * b) + iters(2 * b + 1)) : 15LL * iters(2 * b);
             for (int h = 0; h < heads; ++h, ++i) {
                 const int r = i / sms, c = (r & 1) ? sms - 1 - i % sms : i % sms;
@@ -969,6 +1075,13 @@ int mx230_launch_flash_fwd_ex(mx230_handle *h, cudaStream_t st, const void *Qb, 
     P.q_norm2 = (q_norm2 && k_norm2) ? q_norm2 : nullptr;
     P.k_norm2 = P.q_norm2 ? k_norm2 : nullptr;
     P.test_drop_tile = h->test_drop_tile;
+    // Operands the caller staged come without norms; with L at hand a pass over Q and K bounds the scores.  It is worth its
+    // launch from 16 key tiles per row on (a head's row count decides, not the number of heads: a head's bits do not
+    // depend on the heads beside it).
+    const bool raw_bounds = !row_a && !q_prescaled && L != nullptr && kv_group == 1 && n_q == n_k && n_k > 15 * BN;
+    if (raw_bounds)
+        MX_LAUNCH(h, st, MX230_K_CAST, mx_launch(raw_bounds_kernel, dim3(RB_CLUSTER, heads), RB_THREADS, 0, st, RB_CLUSTER, true,
+                                                 (const uint4 *)Qb, (const uint4 *)Kb, L, n_q));
     P.row_a = row_a;
     P.row_qsum = row_qsum;
     P.col_kskb = col_kskb;
@@ -980,6 +1093,8 @@ int mx230_launch_flash_fwd_ex(mx230_handle *h, cudaStream_t st, const void *Qb, 
                                 : launch_variant<SRC_I8, false>(h, st, grid, tq, tk, tv, to, P);
     if (q_prescaled) return key_split ? launch_variant<SRC_PRE, true>(h, st, grid, tq, tk, tv, to, P)
                                       : launch_variant<SRC_PRE, false>(h, st, grid, tq, tk, tv, to, P);
+    if (raw_bounds) return key_split ? launch_variant<SRC_RAW_BOUND, true>(h, st, grid, tq, tk, tv, to, P)
+                                     : launch_variant<SRC_RAW_BOUND, false>(h, st, grid, tq, tk, tv, to, P);
     return key_split ? launch_variant<SRC_RAW, true>(h, st, grid, tq, tk, tv, to, P)
                      : launch_variant<SRC_RAW, false>(h, st, grid, tq, tk, tv, to, P);
 }

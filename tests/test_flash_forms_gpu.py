@@ -1,0 +1,54 @@
+"""Forward over operands the caller staged (bf16): the form of the kernel, its max-free loop (from 16 key tiles per row on,
+where a pass over Q and K bounds a head's scores) and its general loop, mixed among the heads of one call."""
+import pytest
+import torch
+
+from mx230_b200 import flash_attention as fa
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("heads,n", [(3, 1920), (3, 1921), (3, 2177), (1, 4096), (40, 2050)])   # 40: pair form
+def test_bf16_forward_modes(handle, heads, n, causal):
+    """bf16 operands are exact, so scores differ from 64 bits by fp32 rounding only (2^-24 * 64 * |q||k|/8 < 2e-3 at the
+    largest scale here, below 1e-5 at scale 1): what remains is P in bf16, 2^-9 relative per probability, which moves a row by
+    less than 2 * 2^-9 * max|v| (max|v| < 5.5), and ln of an fp32 sum."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(5)
+    q, k, v = (torch.randn(heads, n, 64, device="cuda", generator=g) for _ in range(3))
+    q[1::3] *= 30          # scores beyond the bound: these heads take the general loop
+    q, k, v = q.bfloat16(), k.bfloat16(), v.bfloat16()
+    o, l = torch.empty(heads, n, 64, device="cuda"), torch.full((heads, n), float("nan"), device="cuda")
+    fa.run_flash_bf16(handle, q, k, v, o, l, n, causal)
+    o2, l2 = torch.empty_like(o), torch.empty_like(l)
+    fa.run_flash_bf16(handle, q, k, v, o2, l2, n, causal)
+    handle.check_status()
+    assert torch.equal(o, o2) and torch.equal(l, l2)
+    for h in range(min(heads, 5)):
+        s = q[h].double() @ k[h].double().T * 0.125
+        if causal:
+            s = s.masked_fill(torch.triu(torch.ones(n, n, dtype=torch.bool, device="cuda"), 1), -float("inf"))
+        assert (o[h].double() - torch.softmax(s, -1) @ v[h].double()).abs().max() <= 2.2e-2
+        assert (l[h].double() - torch.logsumexp(s, -1)).abs().max() <= (2e-3 if h % 3 == 1 else 1e-5)
+        one, l_one = torch.empty(n, 64, device="cuda"), torch.empty(n, device="cuda")
+        fa.run_flash_bf16(handle, q[h], k[h], v[h], one, l_one, n, causal)
+        if h % 3 != 1:     # the max-free loop gives a head the same bits in either form of the kernel
+            if n > 1920:
+                assert torch.equal(one, o[h]) and torch.equal(l_one, l[h])
+
+
+def test_bf16_forward_non_finite_operand(handle):
+    """A NaN in one head leaves the other heads alone and reaches every row of its own head that sees it."""
+    heads, n = 2, 2048
+    g = torch.Generator(device="cuda")
+    g.manual_seed(6)
+    q, k, v = (torch.randn(heads, n, 64, device="cuda", generator=g).bfloat16() for _ in range(3))
+    o, l = torch.empty(heads, n, 64, device="cuda"), torch.empty(heads, n, device="cuda")
+    fa.run_flash_bf16(handle, q, k, v, o, l, n, False)
+    k[1, 777, 5] = float("nan")
+    o2, l2 = torch.empty_like(o), torch.empty_like(l)
+    fa.run_flash_bf16(handle, q, k, v, o2, l2, n, False)
+    handle.check_status()
+    assert torch.equal(o[0], o2[0]) and torch.equal(l[0], l2[0])
+    assert torch.isnan(l2[1]).all()
