@@ -1498,24 +1498,28 @@ int launch_g(mx230_handle *h, cudaStream_t st, const DecodeParams &P, dim3 grid)
 //    take in one tile each: a CTA is not given less than one such pass;
 //  * further clusters join in (merge through global memory, about 2 us) only for sequences with more than 4 passes per
 //    CTA of the first; the kernel decides that per sequence from its actual length;
-//  * ranges of many tiles per CTA use clusters of one: any number of splits then fits the machine (9 per group fill
+//  * clusters of five to eight CTAs share one GPC and leave an eighth of its slots empty, so they are counted against 7/8
+//    of them (3 fp32 sequences of 32540 keys as 54 clusters of 8 took a second wave: 43 us against 36.5 as 74 splits);
+//  * ranges of four and more tiles per warp use clusters of one: any number of splits then fits the machine (9 per group fill
 //    296 slots where 8 would leave a tenth of them empty), and the merge is small against the stream.
 void plan_splits(DecodeParams &P, long long slots, long long groups, long long keys, int pass_keys) {
     long long want = slots / groups;
     if (want < 1) want = 1;
     if (want > 256) want = 256;
     const bool known = keys > 0;
-    if (known && keys / want >= 8LL * pass_keys) {
+    if (known && keys / want >= 4LL * pass_keys) {
         P.cl_size = 1;
         P.max_clusters = (int)want;
         P.cluster_keys = pass_keys;
         return;
     }
+    const long long fit = slots * 7 / 8;
     int c = want < 8 ? (int)want : 8;
+    if (c > 4) c = fit / groups > 8 ? 8 : fit / groups < 4 ? 4 : (int)(fit / groups);
     if (known && c > (keys + pass_keys - 1) / pass_keys) c = (int)((keys + pass_keys - 1) / pass_keys);
     P.cl_size = c;
     P.cluster_keys = 4 * c * pass_keys;
-    long long k = want / c;
+    long long k = (c > 4 ? fit / groups : want) / c;
     if (known && k > (keys + P.cluster_keys - 1) / P.cluster_keys) k = (keys + P.cluster_keys - 1) / P.cluster_keys;
     if (!known && k > 4) k = 4;
     P.max_clusters = (int)(k < 1 ? 1 : k);
