@@ -254,7 +254,7 @@ def prefill_bench(h, torch, la, n_tok=512, nh=14, nkv=2, reps=10):
             pairs = n_tok * pos0 + n_tok * (n_tok + 1) // 2
             out[f"{'int8' if quant else 'fp32'}_kv_pos0_{pos0}"] = {
                 "us": us, "tflops": 4.0 * 64 * pairs * nh / us / 1e6, "n_tok": n_tok, "n_keys": n_keys,
-                "heads": f"{nh}q/{nkv}kv", "launches_per_call": 3, "timing": "CUDA graph of 8 calls, 5 replays"}
+                "heads": f"{nh}q/{nkv}kv", "launches_per_call": 2, "timing": "CUDA graph of 8 calls, 5 replays"}
     # the projections either side (gpu.rs:3187-3198, 3354-3365): qkv = x W + b and y = attn W + b for the same chunk
     e = 896
     x = torch.randn(n_tok, e, device="cuda")

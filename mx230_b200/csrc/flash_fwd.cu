@@ -378,7 +378,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         // Four groups: tile t = warp / 8 has two, each taking 64 of the 128 key columns of every score tile (one thread
         // per query row and half).  Four softmax warps per scheduler instead of two hide each other's dependent-issue
         // latencies; without a row max (the usual mode) the halves never talk to each other inside the loop, and the
-        // general mode has each half compute the full row's max redundantly rather than exchange it.
+        // general mode has them exchange their part of the row max per score tile.
         const int t = warp >> 3;             // query tile of this group (key-split form: parity of its key tiles)
         const int half = (warp >> 2) & 1;    // which 64 key columns of every tile
         const int row_in_tile = (warp & 3) * 32 + lane;
