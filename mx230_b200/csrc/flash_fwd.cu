@@ -402,6 +402,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         uint32_t g0 = 0;   // key tiles of the items so far (int8 scores: ring position)
         uint32_t xmc = 0;  // row-max exchanges this tile's groups have made so far
         uint32_t xmc0 = 0; // key-split form, odd groups: those of the even ones
+        uint32_t turn = 0; // items this tile's groups have worked on
         int bh, q0;
         for (int it = 0; ok && fwd_item(P, it, bh, q0); ++it) {
         const int n_all = KEY_SPLIT ? fwd_tile_iters(P, q0, 0) : 0;
@@ -409,6 +410,15 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         const int row0 = q0 + (KEY_SPLIT ? 0 : t * BM);   // first row of this group's query tile
         const int row = row0 + row_in_tile;
         const int qbuf = it & 1;
+        // Pair form, the last rows of a head with an odd number of query tiles: there is no second tile, and its groups pass
+        // the item over; the first tile's arrive on the Q buffer's barrier in their place.  (Taking part without any work,
+        // they would run ahead of the first tile from one such item to the next, and a barrier that counts one item's
+        // arrivals cannot tell them from the next but one's.)
+        const bool lone = !KEY_SPLIT && q0 + BM >= NQ;
+        if (lone && t == 1) {
+            g0 += fwd_tile_iters(P, q0, 0);
+            continue;
+        }
         auto key_tile = [&](int j) { return KEY_SPLIT ? 2 * j + t : j; };
         float row_a = 0.0f, row_qsum = 0.0f;
         if (SRC == SRC_I8 && row < NQ) {
@@ -443,7 +453,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         // parked there from the first tile on, by the groups that publish nothing as well, instead of in a register.
         // (addresses are formed where they are used: pointers kept over the loop cost registers it needs)
         auto xch = [&](int pub, int what) -> float & {
-            return ((float *)(smem + SMEM_XCH))[(((it & 1) * XCH_PUBS + pub) * 3 + what) * BM + row_in_tile];
+            return ((float *)(smem + SMEM_XCH))[(((turn & 1) * XCH_PUBS + pub) * 3 + what) * BM + row_in_tile];
         };
         const int my_pub = KEY_SPLIT ? 2 * t + half - 1 : t;
         auto park = [&]() -> float & {
@@ -723,7 +733,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 if (lane == 0) mx::mbar_arrive(bar(BAR_XCH + (KEY_SPLIT ? 0 : t)));
             }
         } else if (ok) {
-            ok = __all_sync(0xFFFFFFFFu, mx::mbar_wait(bar(BAR_XCH + t), it & 1, abort_flag, P.status));
+            ok = __all_sync(0xFFFFFFFFu, mx::mbar_wait(bar(BAR_XCH + t), turn & 1, abort_flag, P.status));
             if (ok) {
                 const int other = KEY_SPLIT ? 0 : t;   // half 1 of this tile
                 l += xch(other, 0);
@@ -813,7 +823,11 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         }
         // this warp no longer touches the item's Q buffer (operand of its tile's Q K^T, then staging space)
         __syncwarp();
-        if (ok && lane == 0) mx::mbar_arrive(bar(BAR_Q_EMPTY + qbuf));
+        if (ok && lane == 0) {
+            mx::mbar_arrive(bar(BAR_Q_EMPTY + qbuf));
+            if (lone) mx::mbar_arrive(bar(BAR_Q_EMPTY + qbuf));
+        }
+        ++turn;
         g0 += KEY_SPLIT ? n_all : max(fwd_tile_iters(P, q0, 0), fwd_tile_iters(P, q0, 1));
         }  // items
     }

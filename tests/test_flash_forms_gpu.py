@@ -52,3 +52,33 @@ def test_bf16_forward_non_finite_operand(handle):
     handle.check_status()
     assert torch.equal(o[0], o2[0]) and torch.equal(l[0], l2[0])
     assert torch.isnan(l2[1]).all()
+
+
+@pytest.mark.parametrize("bf16", [False, True])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("heads,n", [(384, 64), (700, 128), (384, 300), (700, 300), (900, 129)])
+def test_many_heads_with_an_odd_number_of_query_tiles(handle, heads, n, causal, bf16):
+    """Pair form, several items per SM of which some or all have one query tile only, one after the other: the last rows of
+    every head.  Against 64-bit softmax with the bounds of the test above; fp32 operands: q and k are rounded to bf16 as well,
+    which moves a score by 1.6e-3 (sd; below 1.5e-2 over all of these), L by no more and a row by a quarter of twice that times
+    the spread of v (below 11).  The sharp check for those: the same bits as the head in a call of its own."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(7)
+    q, k, v = (torch.randn(heads, n, 64, device="cuda", generator=g) for _ in range(3))
+    if bf16:
+        q, k, v = q.bfloat16(), k.bfloat16(), v.bfloat16()
+    run = fa.run_flash_bf16 if bf16 else fa.run_flash_lse
+    handle.reserve(fa.workspace_bytes(heads, n, False))
+    o, l = torch.full((heads, n, 64), float("nan"), device="cuda"), torch.full((heads, n), float("nan"), device="cuda")
+    run(handle, q, k, v, o, l, n, causal)
+    handle.check_status()
+    s = q.double() @ k.double().transpose(1, 2) * 0.125
+    if causal:
+        s = s.masked_fill(torch.triu(torch.ones(n, n, dtype=torch.bool, device="cuda"), 1), -float("inf"))
+    assert (o.double() - torch.softmax(s, -1) @ v.double()).abs().max() <= (2.2e-2 if bf16 else 1e-1)
+    assert (l.double() - torch.logsumexp(s, -1)).abs().max() <= (1e-5 if bf16 else 1.5e-2)
+    if not bf16:
+        one, l_one = torch.empty(n, 64, device="cuda"), torch.empty(n, device="cuda")
+        for h in (0, 1, 147, 148, 295, 296, heads - 1):
+            run(handle, q[h], k[h], v[h], one, l_one, n, causal)
+            assert torch.equal(one, o[h]) and torch.equal(l_one, l[h]), f"head {h}"
