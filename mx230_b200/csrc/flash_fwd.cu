@@ -726,6 +726,15 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             // (the tile's last P V must have read this group's share of P_t before the next item's first tile overwrites it)
             if (ok && n_t > 0)
                 ok = __all_sync(0xFFFFFFFFu, mx::mbar_wait(bar(BAR_O_DONE + t), (cnt - 1) & 1, abort_flag, P.status));
+            // Key-split form, sources whose max-free loop takes its reference from the even groups' exchange: the odd groups
+            // see every item's last exchange complete before they go on, also where they take nothing from it.  A parity
+            // wait tells a phase from the one before, not from the one before that: with an exchange still open, the next
+            // item's wait would return on an older one and read another head's maxima.  (The exchange before the last is
+            // behind the P V that was waited for above, and none can follow the last before these groups have published.)
+            if (KEY_SPLIT && t == 1 && (SRC == SRC_RAW_BOUND || SRC == SRC_I8)) {
+                xmc0 += fast ? 1u : (uint32_t)((n_all + 1) >> 1);
+                if (ok) ok = __all_sync(0xFFFFFFFFu, mx::mbar_wait(bar(BAR_XMAX), (xmc0 - 1) & 1, abort_flag, P.status));
+            }
             if (ok) {
                 xch(my_pub, 0) = l;
                 xch(my_pub, 1) = KEY_SPLIT ? m : l_odd;
@@ -755,7 +764,6 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             }
         }
         if (KEY_SPLIT) cnt1 += (uint32_t)(n_all >> 1);
-        if (KEY_SPLIT && t == 1) xmc0 += fast ? (REF ? 1u : 0u) : (uint32_t)((n_all + 1) >> 1);
         // epilogue: O / l and the log-sum-exp
         if (ok && n_t > 0 && half == 0 && !(KEY_SPLIT && t == 1)) {
             const bool odd = KEY_SPLIT && n_all > 1, two = odd && !fast;   // O_1 holds something

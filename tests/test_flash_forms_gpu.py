@@ -82,3 +82,33 @@ def test_many_heads_with_an_odd_number_of_query_tiles(handle, heads, n, causal, 
         for h in (0, 1, 147, 148, 295, 296, heads - 1):
             run(handle, q[h], k[h], v[h], one, l_one, n, causal)
             assert torch.equal(one, o[h]) and torch.equal(l_one, l[h]), f"head {h}"
+
+
+@pytest.mark.parametrize("heads,n,causal", [(12, 2048, True), (14, 2177, True), (17, 2100, False)])   # key-split, over 148 items
+@pytest.mark.parametrize("every,first", [(3, 1), (2, 0), (5, 2)])
+def test_bf16_heads_inside_and_outside_the_bound_key_split(handle, heads, n, causal, every, first):
+    """Several items per SM, an item of the general loop followed by one of the max-free loop, whose odd groups take their
+    reference from the even ones' exchange: the bits of the head in a call of its own, and of every repetition."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(8)
+    q, k, v = (torch.randn(heads, n, 64, device="cuda", generator=g) for _ in range(3))
+    beyond = [h for h in range(heads) if h % every == first]
+    q[beyond] *= 30
+    q, k, v = q.bfloat16(), k.bfloat16(), v.bfloat16()
+    o, l = torch.empty(heads, n, 64, device="cuda"), torch.empty(heads, n, device="cuda")
+    o2, l2 = torch.empty_like(o), torch.empty_like(l)
+    fa.run_flash_bf16(handle, q, k, v, o, l, n, causal)
+    for _ in range(10):
+        fa.run_flash_bf16(handle, q, k, v, o2, l2, n, causal)
+        assert torch.equal(o, o2) and torch.equal(l, l2)
+    handle.check_status()
+    for h in range(heads):
+        s = q[h].double() @ k[h].double().T * 0.125
+        if causal:
+            s = s.masked_fill(torch.triu(torch.ones(n, n, dtype=torch.bool, device="cuda"), 1), -float("inf"))
+        assert (o[h].double() - torch.softmax(s, -1) @ v[h].double()).abs().max() <= 2.2e-2   # as above
+        if h not in beyond:
+            one, l_one = torch.empty(n, 64, device="cuda"), torch.empty(n, device="cuda")
+            fa.run_flash_bf16(handle, q[h], k[h], v[h], one, l_one, n, causal)
+            assert torch.equal(one, o[h]) and torch.equal(l_one, l[h]), f"head {h}"
+    handle.check_status()

@@ -112,3 +112,44 @@ def test_forms_and_edges(handle, quant, scale, nh, nkv, n_tok, pos0):
     else:
         lo, hi = v.amin(), v.amax()
         assert got.min() >= lo * (1 + 2.0 ** -7) and got.max() <= hi * (1 + 2.0 ** -7)
+
+
+@pytest.mark.parametrize("nh,nkv,n_tok,pos0", [(14, 2, 1900, 0), (14, 2, 1450, 500), (32, 4, 1024, 0)])   # key-split, over 148 items
+@pytest.mark.parametrize("every,first", [(3, 1), (2, 0), (5, 2)])
+def test_heads_inside_and_outside_the_bound_in_one_call(handle, nh, nkv, n_tok, pos0, every, first):
+    """int8 scores, several items per SM, some heads beyond the bound of the max-free loop: an SM goes from an item of one loop
+    to an item of the other.  Against 64-bit softmax (bounds of the test above), and a head inside the bound has the same
+    bits in a call of its own; every pass gives the same bits."""
+    n_keys, stride = pos0 + n_tok, (nh + 2 * nkv) * 64
+    c = filled_cache(handle, n_keys, nkv, True, True, 722)
+    qkv = dev(oracle.normal((n_tok, stride), 721, 0))
+    beyond = [h for h in range(nh) if h % every == first]
+    for h in beyond:
+        qkv[:, h * 64:(h + 1) * 64] *= 40
+    out, again = torch.empty(n_tok, nh * 64, device="cuda"), torch.empty(n_tok, nh * 64, device="cuda")
+    handle.reserve(la.prefill_workspace_bytes(n_tok, n_keys, nh, nkv))
+    la.attn_prefill(handle, out, qkv, c, pos0, n_tok, nh, nkv, stride, nh * 64)
+    for _ in range(10):
+        la.attn_prefill(handle, again, qkv, c, pos0, n_tok, nh, nkv, stride, nh * 64)
+        assert torch.equal(out, again)
+    handle.check_status()
+    mask = torch.arange(n_keys, device="cuda")[None, :] > torch.arange(n_tok, device="cuda")[:, None] + pos0
+    for g in range(nkv):
+        rep = nh // nkv
+        q = qkv[:, g * rep * 64:(g + 1) * rep * 64]
+        c1 = la.KvCache(n_keys, 1, 64, True)
+        for x in ("k", "v"):
+            getattr(c1, x).copy_(getattr(c, x)[:, g * 64:(g + 1) * 64])
+        for x in ("ks", "vs", "kb", "vb"):
+            getattr(c1, x).copy_(getattr(c, x)[:, g:g + 1])
+        s, v = scores64(q, c1, rep, 1, n_keys, True)
+        want = torch.einsum("htk,khd->thd", torch.softmax(s.masked_fill(mask, -float("inf")), -1), v).reshape(n_tok, rep * 64)
+        got = out[:, g * rep * 64:(g + 1) * rep * 64]
+        assert (got.double() - want).abs().max() <= 4e-2
+        assert (got.double() - want).abs().mean() / want.abs().mean() <= 6e-3
+        for h in range(rep):
+            if g * rep + h not in beyond:
+                one = torch.empty(n_tok, 64, device="cuda")
+                la.attn_prefill(handle, one, q[:, h * 64:(h + 1) * 64].contiguous(), c1, pos0, n_tok, 1, 1, 64, 64)
+                assert torch.equal(one, got[:, h * 64:(h + 1) * 64]), f"head {g * rep + h}"
+    handle.check_status()
