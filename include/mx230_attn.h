@@ -292,9 +292,13 @@ int mx230_attn_decode_q8_batched(mx230_handle *h, void *stream, float *out, cons
  * kcache / vcache when kq == NULL, else int8 quantize-on-write; kb == vb == NULL: absmax) and attention over keys
  * 0..=pos -- what 03-llm-engine/src/gpu.rs:2570-2672 (and :2808-2918 with pos_ptr, the graph-captured form) does in
  * three launches per layer.  Host position: the row written is write_row (the caller's phys_row); device position:
- * through bt / bs, or pos itself without a table.  mx230_batched_step: the same for one token of each of n_seq
- * sequences over packed block tables (gpu.rs:3530-3628).  Every result equals that of the separate entry points, which
- * also run when a group has more than 8 query heads per K/V head or the int8 cache is scored on CUDA cores. */
+ * through bt / bs, or pos itself without a table.  The table names a block once: no earlier position may share the new
+ * token's row.  The rotated row and the cache have the same bits as from the separate entry points, the attention row
+ * agrees with theirs to fp32 rounding (the new key is added last); those also run when a group has more than 8 query
+ * heads per K/V head or the int8 cache is scored on CUDA cores.
+ * mx230_batched_step: one token of each of n_seq sequences over packed block tables (gpu.rs:3530-3628), in two launches:
+ * every row is rotated and written before any is attended, so rows may belong to one sequence (consecutive positions,
+ * the same table) or to sequences that share blocks.  Every result has the bits of the separate entry points. */
 int mx230_decode_step(mx230_handle *h, void *stream, float *out, float *qkv, float *kcache, float *vcache,
                       int8_t *kq, int8_t *vq, float *ks, float *vs, float *kb, float *vb, int pos,
                       const int *pos_ptr, int write_row, int n_head, int n_kv_head, int head_dim, int use_rope,
@@ -307,7 +311,8 @@ int mx230_batched_step(mx230_handle *h, void *stream, float *out, float *qkv, fl
 /* The prefill attention step of a chunk of n_tok tokens at positions pos0.. (what gpu.rs:3204-3347 does per layer): RoPE
  * on the Q and K heads of the qkv rows (use_rope != 0; rotated in place), their K and V heads written to the cache (fp32
  * kcache / vcache when kq == NULL, else int8 quantize-on-write; kb == vb == NULL: absmax; rows through bt / bs, or the
- * positions themselves without a table), then causal attention of the n_tok rows over keys 0..pos0+n_tok.  Every result
+ * positions themselves without a table; the table names a block once), then causal attention of the n_tok rows over keys
+ * 0..pos0+n_tok.  Every result
  * equals that of mx230_rope_batch, mx230_copy_kv_batch / mx230_quantize_kv_batch and mx230_attn_prefill in turn; the work
  * in front of attention is one launch. */
 int mx230_prefill_step(mx230_handle *h, void *stream, float *out, float *qkv, float *kcache, float *vcache,

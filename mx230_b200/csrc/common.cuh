@@ -216,6 +216,12 @@ int mx230_launch_flash_fwd_ex(mx230_handle *h, cudaStream_t st, const void *Qb, 
                               int q_prescaled, const float *q_norm2, const float *k_norm2, const float *row_a,
                               const float *row_qsum, const float *col_kskb);
 
+// RoPE on the Q and K heads of one new row of each of n_seq sequences (use_rope != 0) and their K and V heads into the
+// paged cache (fp32 kcache / vcache when kq == NULL, else int8), in one launch (kvwrite.cu).
+int mx230_launch_seq_rows(mx230_handle *h, cudaStream_t st, float *qkv, float *kcache, float *vcache, int8_t *kq, int8_t *vq,
+                          float *ks, float *vs, float *kb, float *vb, const int *pos, int n_seq, int n_head, int n_kv_head,
+                          int use_rope, float theta, const int *tables, int block_size, int n_log, int qkv_stride);
+
 // ---------------------------------------------------------------------------
 // device
 // ---------------------------------------------------------------------------

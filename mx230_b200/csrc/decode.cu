@@ -5,10 +5,10 @@
 // 03-llm-engine/kernels/llm.cu:1246-1487 -- one block per QUERY head, three phases
 // (scores+max, exp+sum, PV), whole score row in shared s[2048].
 //
-// The step of one token (mx230_decode_step, mx230_batched_step) is ONE launch: the attention kernel rotates q, rotates,
-// quantises and writes the new K and V rows, and takes the new key from registers (host-launched step at 778 keys, fp32
-// cache: three launches 18.1 us of device time and 28 us per pass -> 9.0 and 11 us; 64 int8 sequences of up to 2048 keys:
-// 22.8 and 34 us -> 13.3 and 15 us).
+// The step of one token of one sequence (mx230_decode_step) is ONE launch: the attention kernel rotates q, rotates, quantises
+// and writes the new K and V rows, and takes the new key from registers (host-launched step at 778 keys, fp32 cache: three
+// launches 18.1 us of device time and 28 us per pass -> 9.0 and 11 us).  A batched step (mx230_batched_step) is two: its
+// rows may read one another's keys.
 //
 // This design: one CTA per (key split, kv head, sequence) serves ALL query heads of
 // the kv head's group, so every cache byte leaves HBM once.  Inside the CTA every warp
@@ -1798,20 +1798,11 @@ extern "C" int mx230_batched_step(mx230_handle *h, void *stream, float *out, flo
                                   const int *tables, int block_size, int n_log, int qkv_stride, int out_stride) {
     MX_REQUIRE(h && qkv && pos && tables, MX230_ERR_INVALID_ARG, "batched_step: null argument");
     MX_REQUIRE(block_size > 0 && n_log > 0, MX230_ERR_INVALID_ARG, "batched_step: bad table");
-    if (step_is_fused(h, kq, n_head, n_kv_head)) {
-        DecodeParams P = base_params(out, out_stride, qkv, qkv_stride, n_head, n_kv_head);
-        P.kcache = kcache, P.vcache = vcache;
-        set_q8(P, Q8_ARGS);
-        P.pos_kind = 2, P.pos_dev = pos, P.tables = tables, P.bs = block_size, P.n_log = n_log;
-        P.qkv_rw = qkv, P.use_rope = use_rope, P.theta = theta, P.write_row = -1;
-        return launch_decode(h, stream, P, n_seq, head_dim, (long long)n_log * block_size);
-    }
-    const int q_dim = n_head * head_dim, kv_dim = n_kv_head * head_dim;
-    int rc = use_rope ? mx230_rope_seqpos(h, stream, qkv, pos, n_seq, n_head, n_kv_head, head_dim, qkv_stride, theta) : MX230_OK;
-    if (rc) return rc;
-    rc = kq ? mx230_quantize_kv_seqpos(h, stream, Q8_ARGS, qkv, pos, n_seq, q_dim, n_kv_head, head_dim, qkv_stride, tables,
-                                       block_size, n_log)
-            : mx230_copy_kv_seqpos(h, stream, kcache, vcache, qkv, pos, n_seq, q_dim, kv_dim, qkv_stride, tables, block_size, n_log);
+    MX_REQUIRE(head_dim == 64, MX230_ERR_UNSUPPORTED, "batched_step: head_dim %d unsupported (must be 64)", head_dim);
+    // Two launches: the rows of one sequence (or of sequences that share blocks) may be in one call, and a row's keys are
+    // then being written by the same call.
+    const int rc = mx230_launch_seq_rows(h, (cudaStream_t)stream, qkv, kcache, vcache, Q8_ARGS, pos, n_seq, n_head, n_kv_head,
+                                         use_rope, theta, tables, block_size, n_log, qkv_stride);
     if (rc) return rc;
     return kq ? mx230_attn_decode_q8_batched(h, stream, out, qkv, Q8_ARGS, pos, n_seq, n_head, n_kv_head, head_dim, tables,
                                              block_size, n_log, qkv_stride, out_stride)

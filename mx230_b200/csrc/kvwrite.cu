@@ -67,6 +67,71 @@ __global__ void copy_kv_kernel(float *kcache, float *vcache, const float *qkv, R
     *(float4 *)(vcache + row + i) = *(const float4 *)(src + kv_dim + i);
 }
 
+struct SeqRows {
+    float *qkv, *kcache, *vcache;
+    int8_t *kq, *vq;
+    float *ks, *vs, *kb, *vb;
+    RowPos rp;
+    int n_head, n_kv_head, stride, use_rope, max_pos;
+    float theta;
+};
+
+// The work in front of a batched step's attention: a few microseconds of latency (the angle and two memory round trips), so
+// what counts is that it is one launch.  It is a launch of its own because sequences may share cache blocks (several rows of
+// one sequence, at consecutive positions): every row is written before any is read.  A warp takes two heads of a row,
+// lane l holding dims l and l + 32, their loads issued together; the angle is formed once per warp.
+// No early trigger: the attention kernel's clusters would take their places around this kernel's blocks and sit unevenly on
+// the SMs (16 fp32 sequences of 1500 keys, 32/4 heads: a pass 21.9 to 25.1 us with the trigger at the top, 19.2 without).
+// Against rows and attention in one launch, which cannot take rows that read one another, a batched step costs about 2 us
+// more (64 int8 sequences of up to 2048 keys, 14/2 heads: 15.5 us a pass against 13.4; the case above 18.9 / 17.3); three
+// separate launches took 33.3 and 32.0.
+constexpr int SR_WARPS = 8, SR_UNITS = 2;
+__global__ void __launch_bounds__(SR_WARPS * 32) seq_rows_kernel(const SeqRows P) {
+    mx::pdl_wait();
+    const int lane = threadIdx.x & 31, r = blockIdx.y;
+    const int n_rot = P.n_head + P.n_kv_head, n_units = n_rot + P.n_kv_head;
+    const int u0 = (P.use_rope ? 0 : P.n_head) + blockIdx.x * (SR_WARPS * SR_UNITS) + (threadIdx.x >> 5);
+    float *row = P.qkv + (size_t)r * P.stride;
+    float a[SR_UNITS], b[SR_UNITS];
+#pragma unroll
+    for (int i = 0; i < SR_UNITS; ++i) {
+        const int u = u0 + i * SR_WARPS;
+        if (u < n_units) a[i] = row[u * 64 + lane], b[i] = row[u * 64 + 32 + lane];
+    }
+    // (a position from device memory is kept inside the sequence's table, as in the attention kernel)
+    const int pos = min(max(row_position(P.rp, r), 0), P.max_pos);
+    const size_t crow = phys_row(P.rp, r, pos), kvd = (size_t)P.n_kv_head * 64;
+    float cs = 1.0f, sn = 0.0f;
+    if (P.use_rope && u0 < n_rot) mx::rope_angle(pos, lane, 64, P.theta, cs, sn);
+#pragma unroll
+    for (int i = 0; i < SR_UNITS; ++i) {
+        const int u = u0 + i * SR_WARPS;
+        if (u >= n_units) break;
+        if (P.use_rope && u < n_rot) {
+            mx::rope_pair(a[i], b[i], cs, sn);
+            row[u * 64 + lane] = a[i], row[u * 64 + 32 + lane] = b[i];
+        }
+        if (u < P.n_head) continue;
+        const bool is_v = u >= n_rot;
+        const int h = is_v ? u - n_rot : u - P.n_head;
+        if (P.kq == nullptr) {
+            float *dst = (is_v ? P.vcache : P.kcache) + crow * kvd + h * 64;
+            dst[lane] = a[i], dst[lane + 32] = b[i];
+        } else {
+            int8_t *dst = (is_v ? P.vq : P.kq) + crow * kvd + h * 64;
+            float *be = is_v ? P.vb : P.kb;
+            int c0, c1;
+            float scale, beta;
+            mx::quant_head_row(a[i], b[i], be != nullptr, c0, c1, scale, beta);
+            dst[lane] = (int8_t)c0, dst[lane + 32] = (int8_t)c1;
+            if (lane == 0) {
+                (is_v ? P.vs : P.ks)[crow * P.n_kv_head + h] = scale;
+                if (be != nullptr) be[crow * P.n_kv_head + h] = beta;
+            }
+        }
+    }
+}
+
 // One warp quantises one 64-value head row (K or V) of one qkv row: lane l owns
 // elements 2l, 2l+1.
 __global__ void quantize_kv_kernel(int8_t *kq, int8_t *vq, float *ks, float *vs, float *kb,
@@ -168,6 +233,24 @@ RowPos seq_pos(const int *p, const int *tables, int bs, int n_log) {
 }
 
 }  // namespace
+
+int mx230_launch_seq_rows(mx230_handle *h, cudaStream_t st, float *qkv, float *kcache, float *vcache, int8_t *kq, int8_t *vq,
+                          float *ks, float *vs, float *kb, float *vb, const int *pos, int n_seq, int n_head, int n_kv_head,
+                          int use_rope, float theta, const int *tables, int block_size, int n_log, int qkv_stride) {
+    if (kq) MX_REQUIRE(vq && ks && vs && (kb == nullptr) == (vb == nullptr), MX230_ERR_INVALID_ARG, "batched_step: missing cache array");
+    else MX_REQUIRE(kcache && vcache, MX230_ERR_INVALID_ARG, "batched_step: null cache");
+    MX_REQUIRE(n_head > 0 && n_kv_head > 0, MX230_ERR_INVALID_ARG, "batched_step: bad head counts %d/%d", n_head, n_kv_head);
+    MX_REQUIRE(n_seq >= 0 && n_seq <= 65535, n_seq < 0 ? MX230_ERR_INVALID_ARG : MX230_ERR_UNSUPPORTED, "batched_step: n_seq %d", n_seq);
+    if (n_seq == 0) return MX230_OK;
+    const long long slots = (long long)block_size * n_log;
+    SeqRows P{qkv, kcache, vcache, kq, vq, ks, vs, kb, vb, seq_pos(pos, tables, block_size, n_log), n_head, n_kv_head, qkv_stride,
+              use_rope, (int)((slots < 0x7FFFFFFF ? slots : 0x7FFFFFFF) - 1), theta};
+    mx230_device_guard guard(h->device);
+    const int units = (use_rope ? n_head : 0) + 2 * n_kv_head, per = SR_WARPS * SR_UNITS;
+    MX_LAUNCH(h, st, kq ? MX230_K_QUANTIZE_KV : MX230_K_COPY_KV,
+              mx_launch(seq_rows_kernel, dim3((units + per - 1) / per, n_seq), SR_WARPS * 32, 0, st, 1, true, P));
+    return MX230_OK;
+}
 
 // ---- rope ----
 extern "C" int mx230_rope(mx230_handle *h, void *stream, float *qkv, int pos, int n_head,

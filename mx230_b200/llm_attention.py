@@ -279,7 +279,8 @@ def decode_step_dyn(h: Handle, out, qkv, c: KvCache, pos_ptr, n_head, n_kv_head,
 
 def batched_step(h: Handle, out, qkv, c: KvCache, pos, n_seq, n_head, n_kv_head, head_dim, theta,
                  pg: Paging, qkv_stride, out_stride, use_rope=True, stream=None):
-    """One token for each of n_seq sequences, as forward_batched (gpu.rs:3530-3628)."""
+    """One token for each of n_seq sequences, as forward_batched (gpu.rs:3530-3628) -- two launches, so that rows of the same
+    sequence see one another."""
     check(lib().mx230_batched_step(h._h, stream_ptr(stream), ptr(out), ptr(qkv), *_cache_args(c), ptr(pos), n_seq, n_head,
                                    n_kv_head, head_dim, int(use_rope), theta, ptr(pg.table_dev), pg.block_size, pg.n_log,
                                    qkv_stride, out_stride))

@@ -110,11 +110,51 @@ def test_batched_step(handle, nh, nkv, n_seq, ctx, quant):
         la.copy_kv_seqpos(handle, cs, sep, posd, n_seq, qd, kvd, stride, pg)
     out = torch.zeros(n_seq, out_stride, device="cuda")
     la.batched_step(handle, out, fused, cf, posd, n_seq, nh, nkv, 64, THETA, pg, stride, out_stride)
-    assert torch.equal(fused, sep)
+    out_sep = torch.zeros_like(out)
+    la.attn_decode_batched(handle, out_sep, sep, cs, posd, n_seq, nh, nkv, 64, pg, stride, out_stride)
+    assert torch.equal(fused, sep) and torch.equal(out, out_sep)
     same_cache(cf, cs, "batched step")
     got, rows = out.cpu().numpy(), sep.cpu().numpy()
     assert (got[:, qd:] == 0).all()   # padding of the output rows is not touched
     for i in sorted({0, 1, n_seq // 2, n_seq - 1}):
         want = oracle_rows(cs, np.ascontiguousarray(rows[i]), int(pos[i]), nh, tables[i])
         assert_close(got[i, :qd], want, f"sequence {i} at {pos[i]}", **TOL)
+    handle.check_status()
+
+
+@pytest.mark.parametrize("quant,affine", [(False, True), (True, True), (True, False)])
+@pytest.mark.parametrize("nh,nkv", [(14, 2), (12, 12), (18, 1)])
+@pytest.mark.parametrize("rows,first", [(2, 0), (5, 30), (16, 500), (40, 1000)])
+def test_rows_of_one_sequence(handle, nh, nkv, quant, affine, rows, first):
+    """Consecutive positions of one sequence as rows of one batched step (a draft's verification, a chunk through the decode
+    path), beside a sequence that shares its first blocks: each row sees the keys that the call itself writes."""
+    qd, kvd = nh * 64, nkv * 64
+    stride = qd + 2 * kvd
+    n_log = (first + rows) // BS + 2
+    rng = np.random.default_rng(rows)
+    table = rng.permutation(2 * n_log).astype(np.int32)
+    other = table[n_log:].copy()
+    other[:first // BS] = table[:first // BS]
+    tables = np.concatenate([np.tile(table[:n_log], (rows, 1)), other[None]])
+    pos = np.concatenate([first + rng.permutation(rows), [first]]).astype(np.int32)
+    n_seq = rows + 1
+    pg, posd = la.Paging(torch.from_numpy(tables).cuda(), BS), torch.from_numpy(pos).cuda()
+    c0 = filled_cache(handle, 2 * n_log * BS, nkv, quant, affine)
+    raw = torch.from_numpy(oracle.normal((n_seq, stride), 78, rows)).cuda()
+    sep, cs = raw.clone(), copy_of(c0)
+    la.rope_seqpos(handle, sep, posd, n_seq, nh, nkv, 64, stride, THETA)
+    if quant:
+        la.quantize_kv_seqpos(handle, cs, sep, posd, n_seq, qd, nkv, 64, stride, pg)
+    else:
+        la.copy_kv_seqpos(handle, cs, sep, posd, n_seq, qd, kvd, stride, pg)
+    want = torch.empty(n_seq, qd, device="cuda")
+    la.attn_decode_batched(handle, want, sep, cs, posd, n_seq, nh, nkv, 64, pg, stride, qd)
+    for _ in range(5):
+        step, c, out = raw.clone(), copy_of(c0), torch.empty(n_seq, qd, device="cuda")
+        la.batched_step(handle, out, step, c, posd, n_seq, nh, nkv, 64, THETA, pg, stride, qd)
+        assert torch.equal(step, sep) and torch.equal(out, want)
+        same_cache(c, cs, "rows of one sequence")
+    for i in (0, rows - 1, rows):
+        w = oracle_rows(cs, np.ascontiguousarray(sep[i].cpu().numpy()), int(pos[i]), nh, tables[i])
+        assert_close(out[i].cpu().numpy(), w, f"row {i} at {pos[i]}", **TOL)
     handle.check_status()
