@@ -853,7 +853,11 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 
 // Largest |q|^2 |k|^2 scale^2 log2(e)^2 over the rows of a head of bf16 Q and K -> L[head][first row of every query tile],
 // where flash_fwd_kernel looks for it (its own scratch would be shared by the streams of a handle; L is the call's).  A
-// cluster per head, eight threads per row; bound by the latency of its loads (24 heads of 2048 rows: about 4 us).
+// cluster per head, eight threads per row; bound by the latency of its loads (24 heads of 2048 rows: about 4 us) or, from some
+// 20 MB on, by HBM.  A warp stops at the first pass that shows the head beyond the bound (what is left in L is then a part of
+// the product, beyond it as well).  Forward of heads beyond the bound, us a call, whole pass / stopping: 1 x 32768 rows
+// 554 / 523, 1 x 8192 83 / 77, 24 x 2048 67 / 66, 48 x 4096 causal 229 / 217, 96 x 2048 causal 131 / 127; without any bound pass
+// the general loop of an earlier build took 567, 103, 85, 215 and 123.  Heads inside it: 372, 62, 55, 151, 94 (557, 99, 79, 202, 117).
 constexpr int RB_THREADS = 256, RB_CLUSTER = 8;
 __global__ void __launch_bounds__(RB_THREADS) raw_bounds_kernel(const uint4 *Q, const uint4 *K, float *L, int n) {
     __shared__ int most[2];
@@ -889,6 +893,9 @@ __global__ void __launch_bounds__(RB_THREADS) raw_bounds_kernel(const uint4 *Q, 
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) best[0] = max(best[0], norm2(q[u])), best[1] = max(best[1], norm2(k[u]));
+        // beyond the bound already: the rest can only add to it, and the head takes the general loop
+        const float seen = __int_as_float(__reduce_max_sync(0xFFFFFFFFu, best[0])) * __int_as_float(__reduce_max_sync(0xFFFFFFFFu, best[1]));
+        if (!(seen * (MX230_QK_LOG2_SCALE * MX230_QK_LOG2_SCALE) <= FAST_BOUND_REF * FAST_BOUND_REF)) break;
     }
 #pragma unroll
     for (int i = 0; i < 2; ++i) {

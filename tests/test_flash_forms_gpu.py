@@ -112,3 +112,33 @@ def test_bf16_heads_inside_and_outside_the_bound_key_split(handle, heads, n, cau
             fa.run_flash_bf16(handle, q[h], k[h], v[h], one, l_one, n, causal)
             assert torch.equal(one, o[h]) and torch.equal(l_one, l[h]), f"head {h}"
     handle.check_status()
+
+
+@pytest.mark.parametrize("n", [1921, 4096, 5000])
+@pytest.mark.parametrize("where", ["first", "last", "apart", "swapped"])
+def test_bf16_bound_is_of_the_whole_head(handle, n, where):
+    """One row of one operand decides the loop: the first or the last row of a head, of Q or of K, or large rows of Q against
+    small ones of K that stay inside the bound.  The decision shows in L only by rounding, so the bound is the existing
+    tests': the rows of 64-bit softmax, L to 2e-3 where scores reach 2^9."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(9)
+    heads = 3
+    q, k, v = (torch.randn(heads, n, 64, device="cuda", generator=g) for _ in range(3))
+    if where == "first":
+        q[1, 0] *= 60
+    elif where == "last":
+        k[1, n - 1] *= 60
+    elif where == "apart":
+        q[0, 3] *= 10
+        k[0, n - 2] *= 10
+    else:
+        q *= 64
+        k /= 64
+    q, k, v = q.bfloat16(), k.bfloat16(), v.bfloat16()
+    o, l = torch.empty(heads, n, 64, device="cuda"), torch.empty(heads, n, device="cuda")
+    fa.run_flash_bf16(handle, q, k, v, o, l, n, False)
+    handle.check_status()
+    for h in range(heads):
+        s = q[h].double() @ k[h].double().T * 0.125
+        assert (o[h].double() - torch.softmax(s, -1) @ v[h].double()).abs().max() <= 2.2e-2
+        assert (l[h].double() - torch.logsumexp(s, -1)).abs().max() <= 2e-3
