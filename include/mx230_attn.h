@@ -292,7 +292,8 @@ int mx230_attn_decode_q8_batched(mx230_handle *h, void *stream, float *out, cons
  * kcache / vcache when kq == NULL, else int8 quantize-on-write; kb == vb == NULL: absmax) and attention over keys
  * 0..=pos -- what 03-llm-engine/src/gpu.rs:2570-2672 (and :2808-2918 with pos_ptr, the graph-captured form) does in
  * three launches per layer.  Host position: the row written is write_row (the caller's phys_row); device position:
- * through bt / bs, or pos itself without a table.  The table names a block once: no earlier position may share the new
+ * through bt / bs, or pos itself without a table (a caller that means the device form passes pos = -1: a null pos_ptr is then
+ * refused).  The table names a block once: no earlier position may share the new
  * token's row.  The rotated row and the cache have the same bits as from the separate entry points, the attention row
  * agrees with theirs to fp32 rounding (the new key is added last); those also run when a group has more than 8 query
  * heads per K/V head or the int8 cache is scored on CUDA cores.

@@ -1757,7 +1757,7 @@ extern "C" int mx230_decode_step(mx230_handle *h, void *stream, float *out, floa
                                  const int *pos_ptr, int write_row, int n_head, int n_kv_head, int head_dim, int use_rope,
                                  float theta, const int *bt, int bs) {
     MX_REQUIRE(h && qkv, MX230_ERR_INVALID_ARG, "decode_step: null argument");
-    MX_REQUIRE(pos_ptr || pos >= 0, MX230_ERR_INVALID_ARG, "decode_step: negative position %d", pos);
+    MX_REQUIRE(pos_ptr || pos >= 0, MX230_ERR_INVALID_ARG, "decode_step: null pos_ptr and no host position (%d)", pos);
     if (step_is_fused(h, kq, n_head, n_kv_head)) {
         DecodeParams P = base_params(out, n_head * 64, qkv, 0, n_head, n_kv_head);
         P.kcache = kcache, P.vcache = vcache;

@@ -273,7 +273,7 @@ def decode_step(h: Handle, out, qkv, c: KvCache, pos: int, n_head, n_kv_head, he
 def decode_step_dyn(h: Handle, out, qkv, c: KvCache, pos_ptr, n_head, n_kv_head, head_dim, theta,
                     pg: Paging | None = None, use_rope=True, stream=None):
     """The graph-capturable step of forward_body_dyn (gpu.rs:2808-2918)."""
-    check(lib().mx230_decode_step(h._h, stream_ptr(stream), ptr(out), ptr(qkv), *_cache_args(c), 0, ptr(pos_ptr), 0, n_head,
+    check(lib().mx230_decode_step(h._h, stream_ptr(stream), ptr(out), ptr(qkv), *_cache_args(c), -1, ptr(pos_ptr), 0, n_head,
                                   n_kv_head, head_dim, int(use_rope), theta, *_table_args(pg)))
 
 

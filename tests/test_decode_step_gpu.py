@@ -10,6 +10,7 @@ import torch
 
 import oracle
 from mx230_b200 import llm_attention as la
+from mx230_b200._lib import Mx230Error
 from tests.conftest import assert_close
 
 pytestmark = pytest.mark.gpu
@@ -158,3 +159,16 @@ def test_rows_of_one_sequence(handle, nh, nkv, quant, affine, rows, first):
         w = oracle_rows(cs, np.ascontiguousarray(sep[i].cpu().numpy()), int(pos[i]), nh, tables[i])
         assert_close(out[i].cpu().numpy(), w, f"row {i} at {pos[i]}", **TOL)
     handle.check_status()
+
+
+@pytest.mark.parametrize("quant", [False, True])
+@pytest.mark.parametrize("nh,nkv", [(14, 2), (18, 1)])
+def test_device_position_must_be_given(handle, nh, nkv, quant):
+    """A null device position is refused, and row and cache are left alone."""
+    c = filled_cache(handle, 64, nkv, quant)
+    before, qkv = copy_of(c), torch.randn((nh + 2 * nkv) * 64, device="cuda")
+    row, out = qkv.clone(), torch.zeros(nh * 64, device="cuda")
+    with pytest.raises(Mx230Error):
+        la.decode_step_dyn(handle, out, qkv, c, None, nh, nkv, 64, THETA)
+    assert torch.equal(qkv, row) and (out == 0).all()
+    same_cache(c, before, "refused step")
