@@ -283,7 +283,7 @@ __device__ void merge_and_store(const DecodeParams &P, int s, int head0, int gc,
 // instead of a fence, an atomic and a re-read of global memory (int8, one sequence of 2001 keys, 2 K/V heads: 16 splits
 // merged through the workspace 8.2 us, one cluster of 8 CTAs 5.3 us).
 // q_rot (fused step): rotated q, [G][64] in shared memory; it replaces the raw q in qkv once every CTA of the group
-// has read that.
+// has read that.  Null where out is the qkv row itself: the attention row then takes q's place.
 template <int G>
 __device__ void finish_group(const DecodeParams &P, float *mg, int n_warps, int s, int head0, int gc, int cl, int rank,
                              int active, const float *q_rot, int *is_last) {
@@ -1120,7 +1120,7 @@ decode_q8_mma_kernel(const DecodeParams P) {
         }
     }
     __syncthreads();
-    finish_group<MG>(P, mg, Q8_WARPS, s, head0, gc, cl, rank, active, FUSED ? qf : nullptr, &is_last);
+    finish_group<MG>(P, mg, Q8_WARPS, s, head0, gc, cl, rank, active, FUSED && P.out != P.qkv_rw ? qf : nullptr, &is_last);
 }
 
 // ---------------------------------------------------------------------------
@@ -1413,7 +1413,7 @@ decode_f32_ring_kernel(const DecodeParams P) {
         }
     }
     __syncthreads();
-    finish_group<G>(P, mg, F32_WARPS, s, head0, gc, cl, rank, active, FUSED ? qf : nullptr, &is_last);
+    finish_group<G>(P, mg, F32_WARPS, s, head0, gc, cl, rank, active, FUSED && P.out != P.qkv_rw ? qf : nullptr, &is_last);
 }
 
 // Log-sum-exp merge of gathered partial triples: one thread per (row, 4 dims).

@@ -172,3 +172,20 @@ def test_device_position_must_be_given(handle, nh, nkv, quant):
         la.decode_step_dyn(handle, out, qkv, c, None, nh, nkv, 64, THETA)
     assert torch.equal(qkv, row) and (out == 0).all()
     same_cache(c, before, "refused step")
+
+
+@pytest.mark.parametrize("quant", [False, True])
+@pytest.mark.parametrize("nh,nkv", [(14, 2), (12, 12), (32, 4)])
+@pytest.mark.parametrize("pos", [0, 40, 700, 4500])
+def test_step_in_place(handle, nh, nkv, quant, pos):
+    """out may be the qkv row itself, as with the separate calls: the attention row replaces q, K is left rotated."""
+    qd = nh * 64
+    c0 = filled_cache(handle, 4608, nkv, quant)
+    raw = torch.from_numpy(oracle.normal((qd + 2 * nkv * 64,), 79, pos)).cuda()
+    apart, inplace, ca, ci = raw.clone(), raw.clone(), copy_of(c0), copy_of(c0)
+    out = torch.empty(qd, device="cuda")
+    la.decode_step(handle, out, apart, ca, pos, nh, nkv, 64, THETA)
+    la.decode_step(handle, inplace, inplace, ci, pos, nh, nkv, 64, THETA)
+    assert torch.equal(inplace[:qd], out) and torch.equal(inplace[qd:], apart[qd:])
+    same_cache(ca, ci, "step in place")
+    handle.check_status()
