@@ -9,8 +9,10 @@ import pytest
 import torch
 
 import oracle
+from mx230_b200 import _lib
 from mx230_b200 import llm_attention as la
 from mx230_b200._lib import Mx230Error
+from mx230_b200.common import Handle
 from tests.conftest import assert_close
 
 pytestmark = pytest.mark.gpu
@@ -189,3 +191,32 @@ def test_step_in_place(handle, nh, nkv, quant, pos):
     assert torch.equal(inplace[:qd], out) and torch.equal(inplace[qd:], apart[qd:])
     same_cache(ca, ci, "step in place")
     handle.check_status()
+
+
+@pytest.mark.parametrize("mode,nh,nkv,n_seq,ctx", [
+    ("tensor", 14, 2, 64, 2048), ("exact", 14, 2, 64, 2048), ("exact", 14, 2, 60, 512), ("cores", 12, 12, 12, 4096),
+    ("fp32", 14, 2, 80, 800),   # groups for four fifths of the SMs and room for two splits
+])
+def test_short_contexts_need_no_workspace(handle, mode, nh, nkv, n_seq, ctx):
+    """A handle whose workspace holds no second split takes the call with one, and agrees with one that splits."""
+    quant, qd = mode != "fp32", nh * 64
+    n_log = ctx // BS
+    rng = np.random.default_rng(ctx)
+    c = filled_cache(handle, n_seq * n_log * BS, nkv, quant)
+    pg = la.Paging(torch.from_numpy(rng.permutation(n_seq * n_log).astype(np.int32).reshape(n_seq, n_log)).cuda(), BS)
+    pos = torch.from_numpy(np.concatenate([[ctx - 1, 0], rng.integers(0, ctx, n_seq - 2)]).astype(np.int32)).cuda()
+    qkv = torch.from_numpy(oracle.normal((n_seq, qd + 2 * nkv * 64), 80, n_seq)).cuda()
+    small = Handle(0, 4096)
+    rows = []
+    try:
+        for h in (small, handle):
+            h.set_option(_lib.OPT_Q8_SCORE_MODE, _lib.Q8_SCORE_EXACT if mode == "exact" else _lib.Q8_SCORE_REF)
+            h.set_option(_lib.OPT_DECODE_TENSOR, int(mode != "cores"))
+            rows.append(torch.empty(n_seq, qd, device="cuda"))
+            la.attn_decode_batched(h, rows[-1], qkv, c, pos, n_seq, nh, nkv, 64, pg, qkv.shape[1], qd)
+            h.check_status()
+    finally:
+        handle.set_option(_lib.OPT_Q8_SCORE_MODE, _lib.Q8_SCORE_REF)
+        handle.set_option(_lib.OPT_DECODE_TENSOR, 1)
+        small.close()
+    assert_close(rows[0].cpu().numpy(), rows[1].cpu().numpy(), mode, **TOL)
