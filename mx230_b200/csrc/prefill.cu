@@ -24,7 +24,7 @@ struct StageParams {
     // operands of the attention kernel
     __nv_bfloat16 *qout;             // [n_head][n_tok][64]
     __nv_bfloat16 *kout, *vout;      // [n_kv_head][n_keys][64]
-    float *q_norm2, *k_norm2;        // [heads][MX230_NORM_PARTS] largest squared norm of the (dequantised) rows of each part
+    float *q_norm2, *k_norm2;        // [heads][MX230_NORM_PARTS] largest squared norm of the (dequantised) rows of each part, or null
     float *row_a, *row_qsum, *kskb;  // int8 scores: per-row factor and code sum; per-key scale and offset by tiles of 128
     int i8_scores, n_k_tiles;
     // inputs
@@ -61,15 +61,17 @@ __device__ __forceinline__ float *stage_kskb(const StageParams &P, int h, int t)
 // each.  Row norms go through shared memory and, per cluster of four CTAs, into one of MX230_NORM_PARTS parts: with Q's
 // and K's the attention kernel bounds every score of a head and, where the bound is small, runs without a row max.
 __global__ void __launch_bounds__(ST_THREADS) prefill_stage_kernel(const StageParams P) {
-    extern __shared__ int smax[];    // [n_head + n_kv_head] squared norms as ordered integers (NaN largest)
+    extern __shared__ int smax[];    // [n_norms] squared norms of Q and K heads as ordered integers (NaN largest)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int n_max = P.n_head + P.n_kv_head;
+    const int n_max = P.n_head + P.n_kv_head, n_norms = P.q_norm2 ? n_max : 0;
     mx::pdl_trigger();
-    for (int i = tid; i < n_max; i += ST_THREADS) smax[i] = 0;
+    for (int i = tid; i < n_norms; i += ST_THREADS) smax[i] = 0;
     __syncthreads();
     mx::cluster_arrive_release();    // waited for before this CTA adds to the first one's maxima
     mx::pdl_wait();
-    auto raise = [&](int head, float norm2) { atomicMax(&smax[head], __float_as_int(norm2) & 0x7FFFFFFF); };
+    auto raise = [&](int head, float norm2) {
+        if (n_norms > 0) atomicMax(&smax[head], __float_as_int(norm2) & 0x7FFFFFFF);
+    };
     const size_t kvd = (size_t)P.n_kv_head * HD;
 
     // ---- new tokens ----
@@ -248,10 +250,10 @@ __global__ void __launch_bounds__(ST_THREADS) prefill_stage_kernel(const StagePa
     __syncthreads();
     mx::cluster_wait();
     if (rank != 0)
-        for (int i = tid; i < n_max; i += ST_THREADS) mx::cluster_red_max(mx::cluster_map(mx::smem_u32(&smax[i]), 0), smax[i]);
+        for (int i = tid; i < n_norms; i += ST_THREADS) mx::cluster_red_max(mx::cluster_map(mx::smem_u32(&smax[i]), 0), smax[i]);
     mx::cluster_sync();
     if (rank != 0) return;
-    for (int i = tid; i < n_max; i += ST_THREADS) {
+    for (int i = tid; i < n_norms; i += ST_THREADS) {
         float *dst = i < P.n_head ? P.q_norm2 + (size_t)i * MX230_NORM_PARTS : P.k_norm2 + (size_t)(i - P.n_head) * MX230_NORM_PARTS;
         dst[part] = __int_as_float(smax[i]);
     }
@@ -323,8 +325,11 @@ int prefill(mx230_handle *h, void *stream, float *out, const float *qkv, const f
     S.ks = const_cast<float *>(ks), S.vs = const_cast<float *>(vs), S.kb = const_cast<float *>(kb), S.vb = const_cast<float *>(vb);
     S.bt = bt, S.bs = bs;
     S.write_kv = step.write_kv, S.rope = step.rope, S.theta = step.theta;
-    const size_t sm = (size_t)(n_head + n_kv_head) * sizeof(int);
-    MX_REQUIRE(sm <= 48 * 1024, MX230_ERR_UNSUPPORTED, "%s: %d heads", who, n_head + n_kv_head);
+    size_t sm = (size_t)(n_head + n_kv_head) * sizeof(int);
+    if (sm > 48 * 1024) {   // more heads than a CTA keeps norms for: without them every head takes the general loop
+        sm = 0;
+        S.q_norm2 = S.k_norm2 = q_norm2 = k_norm2 = nullptr;
+    }
     MX_LAUNCH(h, st, MX230_K_PREFILL, mx_launch(prefill_stage_kernel, ST_GRID, ST_THREADS, sm, st, ST_CLUSTER, true, S));
     return mx230_launch_flash_fwd_ex(h, st, qb, kbuf, vbuf, out, nullptr, n_head, n_tok, n_keys, pos0, n_head / n_kv_head, HD,
                                      out_stride, 1, i8_scores ? 0 : 1, q_norm2, k_norm2, i8_scores ? row_a : nullptr,

@@ -153,3 +153,20 @@ def test_heads_inside_and_outside_the_bound_in_one_call(handle, nh, nkv, n_tok, 
                 la.attn_prefill(handle, one, q[:, h * 64:(h + 1) * 64].contiguous(), c1, pos0, n_tok, 1, 1, 64, 64)
                 assert torch.equal(one, got[:, h * 64:(h + 1) * 64]), f"head {g * rep + h}"
     handle.check_status()
+
+
+@pytest.mark.parametrize("quant", [False, True])
+@pytest.mark.parametrize("nh", [12284, 12286, 12288])   # with two K/V heads: the most whose norms a CTA keeps is 12286
+def test_very_many_heads(handle, quant, nh):
+    nkv, n_tok, pos0 = 2, 3, 5
+    n_keys, stride = pos0 + n_tok, (nh + 2 * nkv) * 64
+    c = filled_cache(handle, n_keys, nkv, quant, True, 732)
+    qkv = dev(oracle.normal((n_tok, stride), 731, 0))
+    out = torch.empty(n_tok, nh * 64, device="cuda")
+    handle.reserve(la.prefill_workspace_bytes(n_tok, n_keys, nh, nkv))
+    la.attn_prefill(handle, out, qkv, c, pos0, n_tok, nh, nkv, stride, nh * 64)
+    handle.check_status()
+    s, v = scores64(qkv, c, nh, nkv, n_keys, quant)
+    mask = torch.arange(n_keys, device="cuda")[None, :] > torch.arange(n_tok, device="cuda")[:, None] + pos0
+    want = torch.einsum("htk,khd->thd", torch.softmax(s.masked_fill(mask, -float("inf")), -1), v).reshape(n_tok, nh * 64)
+    assert (out.double() - want).abs().max() <= 4e-2 and (out.double() - want).abs().mean() / want.abs().mean() <= 6e-3   # as above
