@@ -767,10 +767,10 @@ decode_q8_kernel(const DecodeParams P) {
 //            codes become f16 exactly (byte permutes onto the mantissa of 1024, minus 1152); p vs
 //            goes in as a high and a low f16 part, so the product carries ~22 bits.  The low parts are
 //            rows 8..15 of the same A tile, which a group of at most 8 heads leaves empty: one MMA does
-//            both products and every accumulator tile is four registers of its own.  (Two MMAs whose
-//            unused rows shared a pair of zero registers cost 153 register moves among 576 instructions
-//            per 32-key tile: 8 x 131072 keys, 4 K/V heads, 118 -> 99 us = 6.1 TB/s; the loop is bound by
-//            issue slots whenever it is not bound by HBM.)
+//            both products and every accumulator tile is four registers of its own.  (Against two MMAs
+//            whose unused rows share a pair of zero registers: 8 x 131072 keys, 4 K/V heads, 118 -> 99 us
+//            in short runs; call after call the case is at 108 us = 5.6 TB/s, from 131.  The loop is
+//            bound by issue slots whenever it is not bound by HBM.)
 // ---------------------------------------------------------------------------
 constexpr int MG = 8;                               // heads per CTA (rows 8..15 of the tiles are padding)
 // Probabilities are taken against a running max that may lag by up to RAISE_MMA (natural-log units);
