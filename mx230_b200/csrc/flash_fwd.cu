@@ -93,7 +93,7 @@ constexpr int BAR_S_FREE = BAR_S_FULL + QT;          // [QT] softmax -> MMA: S_t
 constexpr int BAR_P_FULL = BAR_S_FREE + QT;          // [QT] softmax -> MMA: P_t written
 constexpr int BAR_O_DONE = BAR_P_FULL + QT;          // [QT] MMA -> softmax: O_t += P_t V complete
 constexpr int BAR_XCH = BAR_O_DONE + QT;             // [QT] row sums are published (key-split form: [0] only, by three groups)
-constexpr int BAR_XMAX = BAR_XCH + QT;               // [QT] general mode: both halves of tile t have published their part of the row max
+constexpr int BAR_XMAX = BAR_XCH + QT;               // [QT] both halves of tile t have published their part of the row max (general loop, first tile of REF sources)
 constexpr int BAR_O1_READ = BAR_XMAX + QT;           // key-split form: O_1 of the item has been read by the epilogue
 constexpr int N_BARS = BAR_O1_READ + 1;
 static_assert(8 * N_BARS + 16 <= 512, "barrier area");
@@ -268,10 +268,10 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                     mx::mbar_expect_tx(bar(BAR_K_FULL + s), TILE_BYTES + (SRC == SRC_I8 ? KSKB_BYTES : 0));
                     mx::tma_load_3d(smem_base + SMEM_K + s * TILE_BYTES, &tmK, bar(BAR_K_FULL + s), 0,
                                     j * BN, kvh);
-                    // The tile's scales and offsets land before its scores exist.  Slot g % 8 is free: the load of tile g
-                    // is issued after the Q K^T of tile g - 4, which waited for the softmax groups to have taken their
-                    // previous tile (g - 5; g - 6 in the key-split form) into registers, so every group is done with
-                    // tile g - 8.
+                    // The tile's scales and offsets land before its scores exist.  Slot g % 8 is free: this thread has
+                    // loaded V of tile g - 1 before, over V of tile g - 5, so P V of every tile up to g - 5 is complete, and
+                    // it waited for the probabilities of all warps that read the tile's scales (in both loops the last
+                    // read comes before the arrival on P_FULL).  That holds in either form, whichever groups a tile has.
                     if (SRC == SRC_I8)
                         mx::bulk_load(smem_base + SMEM_KSKB + (g % KSKB_SLOTS) * KSKB_BYTES,
                                       P.col_kskb + ((size_t)kvh * P.n_k_tiles + j) * 2 * BN, KSKB_BYTES, bar(BAR_K_FULL + s));
@@ -437,12 +437,14 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             return true;
         };
         const int last = P.causal ? min(N - 1, row + P.q_off) : N - 1;  // last visible key of this row
-        // Fixed-reference mode, chosen per head: when |q . k| * scale * log2(e) <= 80 for every row pair of the head --
-        // by Cauchy-Schwarz from the largest row norms of Q and K that the staging pass left -- the probabilities are
-        // taken as 2^s against the reference 0: no row max, no subtraction, no rescale of O.  bf16 probabilities and
-        // fp32 sums carry the same relative precision at 2^-80 .. 2^80 as around 1, every row sum stays inside
-        // [2^-80, N 2^80], and the result is that of the max-subtracted form.  Heads with larger scores (and calls
-        // without the norms) take the general path: running max, lazy rescale.
+        // Fixed-reference mode, chosen per head: when |q . k| * scale * log2(e) is bounded for every row pair of the head --
+        // by Cauchy-Schwarz from the largest row norms of Q and K -- the probabilities are taken against a reference that
+        // stays: no running max, no rescale of O.  Q staged in log2 units (SRC_PRE): bound 80, reference 0, not even a
+        // subtraction.  int8 scores and bounded bf16 operands (REF): bound 40, reference the row's max over its first key
+        // tile.  Either way a probability is at most 2^80; bf16 probabilities and fp32 sums carry the same relative
+        // precision at 2^-80 .. 2^80 as around 1, every row sum stays inside [2^-80, N 2^80], and the result is that of the
+        // max-subtracted form.  Heads with larger scores (and calls without a bound) take the general path: running max,
+        // lazy rescale.
         const bool fast = SRC == SRC_RAW ? false
                           : SRC == SRC_RAW_BOUND ? fwd_fast_raw(P, bh, row0)
                                                  : fwd_fast_head(P, bh, lane, REF ? FAST_BOUND_REF : FAST_BOUND);
