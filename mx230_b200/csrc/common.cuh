@@ -207,9 +207,10 @@ inline size_t mx230_flash_norm_bytes(int batch_heads) {
 // O + h*o_head_stride + r*o_row_stride.  q_prescaled: Qb holds Q * MX230_QK_LOG2_SCALE.  q_norm2 / k_norm2 (both or
 // neither): largest squared row norm per head of the unscaled Q [heads][MX230_NORM_PARTS] and of K
 // [heads / kv_group][MX230_NORM_PARTS] (int8 score mode: of the dequantised rows); with them a head whose scores are
-// provably small takes the kernel's max-free softmax loop.  row_a / row_qsum / col_kskb (all or none; with them q_prescaled must be 0 and Qb, Kb
-// hold int8 codes as bf16): the int8 score mode -- score = row_a[h][i] * (dot * ks[j] + row_qsum[h][i] * kb[j]), with
-// col_kskb [heads / kv_group][tiles of 128 keys][ks of the 128 keys, then their kb], 16-byte aligned.
+// provably small takes the kernel's max-free softmax loop.  row_a / row_qsum / col_kskb (all or none; with them q_prescaled
+// must be 0 and Qb, Kb hold int8 codes as bf16): the int8 score mode -- score = row_a[h][i] * (dot * ks[j] +
+// row_qsum[h][i] * kb[j]), with col_kskb [heads / kv_group][tiles of 128 keys][ks of the 128 keys, then their kb], 16-byte
+// aligned.
 int mx230_launch_flash_fwd_ex(mx230_handle *h, cudaStream_t st, const void *Qb, const void *Kb,
                               const void *Vb, float *O, float *L, int heads, int n_q, int n_k, int q_off,
                               int kv_group, long long o_head_stride, long long o_row_stride, int causal,

@@ -52,8 +52,9 @@ struct DecodeParams {
     int max_keys;        // capacity of one sequence (slab rows, or table entries x block) when positions come from the device; 0 = unknown
     int n_head, n_kv_head, group, head_groups;
     int score_mode;
-    // key splits of one (sequence, K/V head) group: grid.x = max_clusters clusters of cl_size CTAs (up to 8); a sequence of `len` keys uses the first ceil(len / cluster_keys) clusters (all of them when cluster_keys == 0),
-    // so that the split follows the length of each sequence and not only the largest one
+    // key splits of one (sequence, K/V head) group: grid.x = max_clusters clusters of cl_size CTAs (up to 8); a sequence of
+    // `len` keys uses the first ceil(len / cluster_keys) clusters (all of them when cluster_keys == 0), so that the split
+    // follows the length of each sequence and not only the largest one
     int cl_size, max_clusters, cluster_keys;
     // Let the next kernel of the stream in once this one's loops are done: only a grid that leaves SMs free.  After a larger
     // one the next grid's CTAs would fill the slots that fall free first and sit unevenly on the SMs (8 x 131072 int8 keys

@@ -817,10 +817,12 @@ int launch_dq(mx230_handle *h, cudaStream_t st, const Maps &m, const float *L, c
     dim3 grid((unsigned)set_items(P, batch_heads, n));   // one item per CTA
     if (pre)
         MX_LAUNCH(h, st, MX230_K_BWD_DQ,
-                  mx_launch(bwd_kernel<0, true>, grid, BWD_THREADS, SM_ALLOC, st, 1, true, m.box128[0], m.box128[3], m.box128[1], m.box128[2], m.box128[0], m.box128[0], m.box128[0], P));
+                  mx_launch(bwd_kernel<0, true>, grid, BWD_THREADS, SM_ALLOC, st, 1, true,
+                            m.box128[0], m.box128[3], m.box128[1], m.box128[2], m.box128[0], m.box128[0], m.box128[0], P));
     else
         MX_LAUNCH(h, st, MX230_K_BWD_DQ,
-                  mx_launch(bwd_kernel<0, false>, grid, BWD_THREADS, SM_ALLOC, st, 1, true, m.box128[0], m.box128[3], m.box128[1], m.box128[2], m.box128[0], m.box128[0], m.box128[0], P));
+                  mx_launch(bwd_kernel<0, false>, grid, BWD_THREADS, SM_ALLOC, st, 1, true,
+                            m.box128[0], m.box128[3], m.box128[1], m.box128[2], m.box128[0], m.box128[0], m.box128[0], P));
     return MX230_OK;
 }
 
@@ -830,10 +832,12 @@ int launch_dkv(mx230_handle *h, cudaStream_t st, const Maps &m, const float *L, 
     dim3 grid((unsigned)set_items(P, batch_heads, n));   // one item per CTA
     if (pre)
         MX_LAUNCH(h, st, MX230_K_BWD_DKV,
-                  mx_launch(bwd_kernel<1, true>, grid, BWD_THREADS, SM_ALLOC, st, 1, true, m.box128[1], m.box128[2], m.box128[0], m.box128[3], m.box128[0], m.box128[0], m.box128[0], P));
+                  mx_launch(bwd_kernel<1, true>, grid, BWD_THREADS, SM_ALLOC, st, 1, true,
+                            m.box128[1], m.box128[2], m.box128[0], m.box128[3], m.box128[0], m.box128[0], m.box128[0], P));
     else
         MX_LAUNCH(h, st, MX230_K_BWD_DKV,
-                  mx_launch(bwd_kernel<1, false>, grid, BWD_THREADS, SM_ALLOC, st, 1, true, m.box128[1], m.box128[2], m.box128[0], m.box128[3], m.box128[0], m.box128[0], m.box128[0], P));
+                  mx_launch(bwd_kernel<1, false>, grid, BWD_THREADS, SM_ALLOC, st, 1, true,
+                            m.box128[1], m.box128[2], m.box128[0], m.box128[3], m.box128[0], m.box128[0], m.box128[0], P));
     return MX230_OK;
 }
 
@@ -856,10 +860,12 @@ int launch_fused(mx230_handle *h, cudaStream_t st, const Maps &m, const float *L
     dim3 grid((unsigned)(n_items < h->sm_count ? n_items : h->sm_count));
     if (pre)
         MX_LAUNCH(h, st, MX230_K_BWD_FUSED,
-                  mx_launch(bwd_kernel<2, true>, grid, BWD_THREADS, SM_ALLOC, st, 1, true, m.box128[1], m.box128[2], m.box128[0], m.box128[3], tm_dq, tm_dk, tm_dv, P));
+                  mx_launch(bwd_kernel<2, true>, grid, BWD_THREADS, SM_ALLOC, st, 1, true,
+                            m.box128[1], m.box128[2], m.box128[0], m.box128[3], tm_dq, tm_dk, tm_dv, P));
     else
         MX_LAUNCH(h, st, MX230_K_BWD_FUSED,
-                  mx_launch(bwd_kernel<2, false>, grid, BWD_THREADS, SM_ALLOC, st, 1, true, m.box128[1], m.box128[2], m.box128[0], m.box128[3], tm_dq, tm_dk, tm_dv, P));
+                  mx_launch(bwd_kernel<2, false>, grid, BWD_THREADS, SM_ALLOC, st, 1, true,
+                            m.box128[1], m.box128[2], m.box128[0], m.box128[3], tm_dq, tm_dk, tm_dv, P));
     return MX230_OK;
 }
 

@@ -342,9 +342,11 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 #pragma unroll
                 for (int t = 0; t < QT; ++t) n_it[t] = fwd_tile_iters(P, q0, KEY_SPLIT ? 0 : t);
                 const int n_max = max(n_it[0], n_it[1]);
+                // each pair of groups sums into an O of its own
                 const bool own_o = !KEY_SPLIT || SRC == SRC_RAW ||
-                                   !(SRC == SRC_RAW_BOUND ? fwd_fast_raw(P, bh, q0)
-                                                          : fwd_fast_head(P, bh, lane, SRC == SRC_I8 ? FAST_BOUND_REF : FAST_BOUND));   // each pair of groups sums into an O of its own
+                                   !(SRC == SRC_RAW_BOUND
+                                         ? fwd_fast_raw(P, bh, q0)
+                                         : fwd_fast_head(P, bh, lane, SRC == SRC_I8 ? FAST_BOUND_REF : FAST_BOUND));
                 for (int j = 0; j < n_max && ok; ++j, ++g) {
                     const int s = g % KV_STAGES;
                     ok = ISSUER_WAIT(mx::mbar_wait(bar(BAR_V_FULL + s), (g / KV_STAGES) & 1, abort_flag, P.status));

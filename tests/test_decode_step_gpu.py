@@ -1,5 +1,6 @@
-"""The one-launch decode step (RoPE, KV write and attention in the attention kernel) against the separate entry points:
-the rotated row and the cache must be the same bits, and the attention row must meet the oracle on that very cache.
+"""The decode step (one sequence: RoPE, KV write and attention in the attention kernel; a batch: all rows written, then
+attention) against the separate entry points: the rotated row and the cache must be the same bits, and the attention row must
+meet the oracle on that very cache (a batch: have the same bits as well).
 
 Positions sit at the edges of the kernels' splits: tiles of 16 (fp32) and 32 (int8) keys, one pass of a CTA (64 / 256
 keys), a cluster of eight CTAs, the point from which a second cluster joins in.  The tolerance of the row is that of the
