@@ -17,7 +17,7 @@
 // of the other axis, streamed through a TMA ring.  The two-pass kernels run one item per CTA; the fused pass is
 // persistent: one CTA per SM walks its share of the items (heaviest first, dealt out in snake order), ring
 // positions and barrier parities run on from item to item, and the next item's owned and first streamed tiles
-// are requested as soon as the current item's last MMAs have completed, while its dK / dV are still being stored.
+// arrive while the current item's last tiles are still worked on.
 // Per streamed tile:
 //
 //   X = A_own A_str^T, Y = B_own B_str^T      (S, dP   |  S^T, dP^T)   128 x 128, N = 128 MMAs
@@ -62,6 +62,10 @@ constexpr int BWD_THREADS = 512;
 #ifndef BWD_SPLIT_LOAD
 #define BWD_SPLIT_LOAD 1   // X, Y of a tile are pulled in two 32-column pieces, the second under the first one's arithmetic (fused pass: 290 -> 281 us)
 #endif
+#ifndef BWD_SECOND_AT
+#define BWD_SECOND_AT 24   // columns of the first piece that are done when the second one is taken as landed and X, Y are handed back
+                           // (step of 48 x 4096 rows causal 527, 525, 520, 522 us at 8, 16, 24, 32; 24 x 2048 bf16 148, 150, 145, 148)
+#endif
 #ifndef BWD_POLY
 #define BWD_POLY 0         // fused pass: of every four column pairs, how many take 2^x from the FMA-pipe polynomial
 #endif
@@ -104,7 +108,8 @@ constexpr int BAR_DS_READY = BAR_SDP_FREE + 1;           // compute -> MMA: E, P
 constexpr int BAR_ACC_DONE = BAR_DS_READY + 1;
 constexpr int BAR_DQ_FULL = BAR_ACC_DONE + 1;            // fused pass: MMA -> drain warps
 constexpr int BAR_DQ_FREE = BAR_DQ_FULL + 1;             // drain warps -> MMA
-constexpr int N_BARS = BAR_DQ_FREE + 1;
+constexpr int BAR_OWN_B_FREE = BAR_DQ_FREE + 1;          // fused pass: the item's last Y is complete, V's tile may be replaced
+constexpr int N_BARS = BAR_OWN_B_FREE + 1;
 
 // tensor memory columns
 constexpr int TM_X = 0, TM_Y = 128, TM_E = 256, TM_P = 320;   // E, P: bf16 pairs, 64 columns each
@@ -132,6 +137,20 @@ struct BwdParams {
     int n_items;         // heads * n_tiles work items (owned tile, head), heads fastest, heaviest tiles first
     int test_drop_tile;  // test hook (fused pass): streamed tile (counted over the CTA's items) that CTA 0's producer never requests; -1 = off
 };
+
+// Fused pass: the 16 KB places of the owned K tile and of the three stages' Q tiles change roles from item to item.  The next
+// item's K goes into the place of its second streamed tile's stage, which falls free a tile before the current item ends, and
+// that stage takes over the place of the current K.  A nibble per stage, the fourth one for K: place in units of 16 KB.
+struct QPlaces {
+    uint32_t nib = 0x0432u;   // stages 0, 1, 2 at 2, 3, 4 (SM_STR_A); K at 0 (SM_OWN_A)
+    __device__ __forceinline__ uint32_t at(int i) const { return ((nib >> (4 * i)) & 15u) * STR_BYTES; }
+    __device__ __forceinline__ void next_item(uint32_t g) {   // g: the item's first streamed tile
+        const int sh = 4 * (int)((g + 1) % (STAGES - 1));
+        const uint32_t x = ((nib >> sh) ^ (nib >> 12)) & 15u;
+        nib ^= (x << sh) | (x << 12);
+    }
+};
+static_assert(SM_OWN_A == 0 && SM_STR_A == 2 * STR_BYTES && OWN_BYTES == STR_BYTES, "QPlaces");
 
 // One CTA's `round`-th work item: an owned 128-row tile of one head and the range of streamed tiles it sees.
 // Items are listed heaviest first (dQ: late query tiles see the most keys; dK/dV: early key tiles see the most
@@ -197,6 +216,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmOwnA, const __grid_constant__ C
         mx::mbar_init(bar(BAR_SDP_FULL), FUSED ? 1 : 2);  // the X and the Y issuer (one thread in the fused pass)
         mx::mbar_init(bar(BAR_DQ_FULL), 1);
         mx::mbar_init(bar(BAR_DQ_FREE), 4);
+        mx::mbar_init(bar(BAR_OWN_B_FREE), 1);
         mx::mbar_init(bar(BAR_SDP_FREE), 2 * BT / 32);    // one elected lane per compute warp arrives
         mx::mbar_init(bar(BAR_DS_READY), 2 * BT / 32);
         mx::mbar_init(bar(BAR_ACC_DONE), N_ACC);
@@ -233,13 +253,15 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmOwnA, const __grid_constant__ C
             }
             bool ok = true;
             uint32_t g = 0;   // streamed tiles so far, over all items: ring slot g % NST, use g / NST
+            QPlaces pl;
             BwdItem I;
             for (int it = 0; ok && bwd_item<MODE>(P, it, I); ++it) {
                 const int bh = I.bh;
-                if (MODE >= 1) {
-                    // the owned tiles are single-buffered: every MMA of the previous item must have completed
-                    if (it > 0) ok = __all_sync(0xFFFFFFFFu, mx::mbar_wait(bar(BAR_ACC_DONE), (it - 1) & 1, abort_flag, P.status));
-                    if (!ok) break;
+                auto wait_acc_done = [&]() {   // every MMA of the previous item has completed
+                    return (bool)__all_sync(0xFFFFFFFFu, mx::mbar_wait(bar(BAR_ACC_DONE), (it - 1) & 1, abort_flag, P.status));
+                };
+                if (FUSED && it > 0) pl.next_item(g);
+                if (MODE == 1 || (FUSED && it == 0)) {   // (a two-pass CTA has one item)
                     if (lane == 0) {
                         mx::mbar_expect_tx(bar(BAR_OWN_FULL), 2 * OWN_BYTES);
                         mx::tma_load_3d(smem_base + SM_OWN_A, &tmOwnA, bar(BAR_OWN_FULL), 0, I.own0, bh);
@@ -250,6 +272,9 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmOwnA, const __grid_constant__ C
                     const int s = g % NST;
                     const uint32_t r = g / NST;
                     const int row0 = (I.it_beg + y) * BS;
+                    // the previous item's K lies where this tile's Q goes
+                    if (FUSED && it > 0 && y == 1) ok = wait_acc_done();
+                    if (!ok) break;
                     // -L*log2(e) and -Delta of the streamed queries: fetched before the wait, stored after it
                     float lv[4], dv[4];
                     if (MODE >= 1) {
@@ -269,7 +294,8 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmOwnA, const __grid_constant__ C
                     if (FUSED && P.test_drop_tile == (int)g && blockIdx.x == 0) continue;   // test hook: this tile never arrives
                     if (lane == 0) {
                         mx::mbar_expect_tx(bar(BAR_STR_FULL + s), 2 * STR_BYTES);
-                        mx::tma_load_3d(smem_base + SM_STR_A + s * STR_BYTES, &tmStrA, bar(BAR_STR_FULL + s), 0, row0, bh);
+                        mx::tma_load_3d(smem_base + (FUSED ? pl.at(s) : SM_STR_A + s * STR_BYTES), &tmStrA, bar(BAR_STR_FULL + s), 0,
+                                        row0, bh);
                         mx::tma_load_3d(smem_base + SM_STR_B + s * STR_BYTES, &tmStrB, bar(BAR_STR_FULL + s), 0, row0, bh);
                     }
                     if (FUSED) {
@@ -290,6 +316,28 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmOwnA, const __grid_constant__ C
                         }
                         mx::fence_proxy_async_smem();   // read by the MMAs
                         mx::mbar_arrive(bar(BAR_STR_FULL + s));
+                        if (it > 0 && y == 0) {
+                            // The item's owned tiles, behind its first streamed one: V once the previous item's last Y is
+                            // complete, K once the tile before the previous item's last is consumed -- both while that item
+                            // still runs, so that this one's first X, Y are ready when its exponentials are.  (Loaded after
+                            // ACC_DONE, the streamed tiles queued behind them: step of 48 x 4096 rows causal 530 us against
+                            // 520, 24 x 2048 bf16 150 against 145.)
+                            ok = __all_sync(0xFFFFFFFFu, mx::mbar_wait(bar(BAR_OWN_B_FREE), (it - 1) & 1, abort_flag, P.status));
+                            if (!ok) break;
+                            if (lane == 0) {
+                                mx::mbar_expect_tx(bar(BAR_OWN_FULL), 2 * OWN_BYTES);
+                                mx::tma_load_3d(smem_base + SM_OWN_B, &tmOwnB, bar(BAR_OWN_FULL), 0, I.own0, bh);
+                            }
+                            const int s1 = (g + 1) % NST;
+                            const uint32_t r1 = (g + 1) / NST;
+                            if (r1 > 0)
+                                ok = __all_sync(0xFFFFFFFFu, mx::mbar_wait(bar(BAR_STR_EMPTY + s1), (r1 - 1) & 1, abort_flag, P.status));
+                            // an item of one tile: asked here, before the item can complete (a parity wait tells a phase only
+                            // from its neighbour)
+                            if (ok && I.n == 1) ok = wait_acc_done();
+                            if (!ok) break;
+                            if (lane == 0) mx::tma_load_3d(smem_base + pl.at(3), &tmOwnA, bar(BAR_OWN_FULL), 0, I.own0, bh);
+                        }
                     } else if (MODE >= 1) {
                         float *ld = (float *)(smem + SM_LD + s * (2 * BS * 4));
 #pragma unroll
@@ -376,14 +424,16 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmOwnA, const __grid_constant__ C
             // (the compute warps are busy with the previous tile for far longer than both take)
             {
                 constexpr uint32_t IDESC_S = mx::mma_idesc_bf16(BT, BS, false, false);
-                const uint64_t own_k = mx::smem_desc_sw128(smem_base + SM_OWN_A);
                 const uint64_t own_v = mx::smem_desc_sw128(smem_base + SM_OWN_B);
                 const uint64_t aug_x = mx::smem_desc_kmajor_plain(smem_base + SM_AUG_AX, SM_AUG_Z - SM_AUG_AX);
                 const uint64_t aug_y = mx::smem_desc_kmajor_plain(smem_base + SM_AUG_AY, SM_AUG_Z - SM_AUG_AY);
                 bool ok = true;
                 uint32_t g = 0;
+                QPlaces pl;
                 BwdItem I;
                 for (int it = 0; ok && bwd_item<MODE>(P, it, I); ++it) {
+                    if (it > 0) pl.next_item(g);
+                    const uint64_t own_k = mx::smem_desc_sw128(smem_base + pl.at(3));
                     ok = __all_sync(0xFFFFFFFFu, mx::mbar_wait(bar(BAR_OWN_FULL), it & 1, abort_flag, P.status));
                     for (int y = 0; y < I.n && ok; ++y, ++g) {
                         const int s = g % NST;
@@ -391,7 +441,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmOwnA, const __grid_constant__ C
                         if (ok && g > 0) ok = __all_sync(0xFFFFFFFFu, mx::mbar_wait(bar(BAR_SDP_FREE), (g - 1) & 1, abort_flag, P.status));
                         if (!ok) break;
                         mx::tc_fence_after();
-                        const uint64_t sq = mx::smem_desc_sw128(smem_base + SM_STR_A + s * STR_BYTES);
+                        const uint64_t sq = mx::smem_desc_sw128(smem_base + pl.at(s));
                         const uint64_t so = mx::smem_desc_sw128(smem_base + SM_STR_B + s * STR_BYTES);
                         const uint64_t bq = mx::smem_desc_kmajor_plain(smem_base + SM_AUG_B + s * AUG_BYTES,
                                                                        SM_AUG_Z - SM_AUG_B - s * AUG_BYTES);
@@ -403,6 +453,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmOwnA, const __grid_constant__ C
                             for (int k = 0; k < HD / 16; ++k) mx::mma_ss(tmem + TM_Y, own_v + 2 * k, so + 2 * k, IDESC_S, k > 0);
                             mx::mma_ss(tmem + TM_Y, aug_y, bq, IDESC_S, 1);   // Y -= Delta of the query column
                             mx::mma_commit(bar(BAR_SDP_FULL));
+                            if (y == I.n - 1) mx::mma_commit(bar(BAR_OWN_B_FREE));
                         }
                     }
                 }
@@ -415,15 +466,17 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmOwnA, const __grid_constant__ C
                 const uint64_t ds0 = mx::smem_desc_sw128(smem_base + SM_DS), ds1 = mx::smem_desc_sw128(smem_base + SM_DS1_A);
                 bool ok = true;
                 uint32_t g = 0;
+                QPlaces pl;
                 BwdItem I;
                 for (int it = 0; ok && bwd_item<MODE>(P, it, I); ++it) {
+                    if (it > 0) pl.next_item(g);
                     for (int y = 0; y < I.n && ok; ++y, ++g) {
                         const int s = g % NST;
                         ok = __all_sync(0xFFFFFFFFu, mx::mbar_wait(bar(BAR_STR_FULL + s), (g / NST) & 1, abort_flag, P.status));
                         if (ok) ok = __all_sync(0xFFFFFFFFu, mx::mbar_wait(bar(BAR_DS_READY), g & 1, abort_flag, P.status));
                         if (!ok) break;
                         mx::tc_fence_after();
-                        const uint64_t sd = mx::smem_desc_sw128(smem_base + SM_STR_A + s * STR_BYTES);
+                        const uint64_t sd = mx::smem_desc_sw128(smem_base + pl.at(s));
                         // 16 queries of contraction = 32 B inside a row; queries 64.. are the second half tile
                         const uint64_t lo = (g & 1) ? ds1 : ds0;
                         const uint64_t hi = lo + (uint64_t)(((g & 1) ? SM_DS1_B - SM_DS1_A : DS_HALF_BYTES) >> 4);
@@ -449,11 +502,13 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmOwnA, const __grid_constant__ C
                 constexpr uint32_t IDESC_Q = mx::mma_idesc_bf16(BS, HD, true, true);
                 const uint64_t ad0 = mx::smem_desc_sw128_mn(smem_base + SM_DS, DS_HALF_BYTES);
                 const uint64_t ad1 = mx::smem_desc_sw128_mn(smem_base + SM_DS1_A, SM_DS1_B - SM_DS1_A);
-                const uint64_t bd = mx::smem_desc_sw128(smem_base + SM_OWN_A);
                 bool ok = true;
                 uint32_t g = 0;
+                QPlaces pl;
                 BwdItem I;
                 for (int it = 0; ok && bwd_item<MODE>(P, it, I); ++it) {
+                    if (it > 0) pl.next_item(g);
+                    const uint64_t bd = mx::smem_desc_sw128(smem_base + pl.at(3));
                     for (int y = 0; y < I.n && ok; ++y, ++g) {
                         const int s = g % NST;
                         ok = __all_sync(0xFFFFFFFFu, mx::mbar_wait(bar(BAR_STR_FULL + s), (g / NST) & 1, abort_flag, P.status));
@@ -608,6 +663,10 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmOwnA, const __grid_constant__ C
                 }
             };
             if (need_mask) mask_cols(0, BWD_SPLIT_LOAD ? 32 : HS);
+            if (FUSED && it > 0 && y == 0) {   // this warp's rows of the E buffers were the staging tiles of the previous item's dK, dV
+                if (lane == 0) mx::bulk_wait_group_read<0>();
+                __syncwarp();
+            }
             uint32_t pe[HS / 2], pp[MODE >= 1 ? HS / 2 : 1];
             // fused pass: E goes to shared memory as bf16, this thread's key row = one 128-byte swizzled line of
             // 64 queries.  Two buffers: the MMAs of tile y-1 may still read the other one (those of y-2 are
@@ -617,7 +676,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmOwnA, const __grid_constant__ C
 #pragma unroll
             for (int i = 0; i < HS; i += 2) {
 #if BWD_SPLIT_LOAD
-                if (i == 32) {   // the second half of this thread's X, Y is in registers: the MMAs may overwrite them
+                if (i == BWD_SECOND_AT) {   // the second half of this thread's X, Y is in registers: the MMAs may overwrite them
                     mx::tmem_wait_ld();
                     mx::tc_fence_before();
                     __syncwarp();
@@ -711,10 +770,8 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmOwnA, const __grid_constant__ C
                 if (lane == 0 && wrow0 < N) {
                     mx::tma_store_3d(tm, smem_base + st_off[0], 0, wrow0, bh);
                     mx::tma_store_3d(tm, smem_base + st_off[1], 32, wrow0, bh);
-                    mx::bulk_commit_group();
-                    mx::bulk_wait_group_read<0>();   // the staging tiles must outlive the reads
+                    mx::bulk_commit_group();   // (waited for before this warp writes E again, and before the kernel ends)
                 }
-                __syncwarp();
             } else {
                 // the left warpgroup stores dK (scaled), the right one dV
                 const float sc = h == 0 ? DK_SCALE : 1.0f;
@@ -735,6 +792,10 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmOwnA, const __grid_constant__ C
             }
         }
         }  // items
+        if (FUSED) {
+            if (lane == 0) mx::bulk_wait_group_read<0>();
+            __syncwarp();
+        }
     }
     mx::tc_fence_before();
     __syncthreads();
