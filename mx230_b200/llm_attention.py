@@ -9,7 +9,7 @@ from __future__ import annotations
 
 import torch
 
-from ._lib import check, lib, ptr
+from ._lib import addr, check, lib, ptr
 from .common import Handle, stream_ptr
 
 KV_BLOCK = 16  # 03-llm-engine/src/gpu.rs:209
@@ -36,7 +36,10 @@ class KvCache:
             self.v = torch.zeros(slots, kvd, dtype=torch.float32, device=device)
 
     def q8_args(self):
-        return (ptr(self.k), ptr(self.v), ptr(self.ks), ptr(self.vs), ptr(self.kb), ptr(self.vb))
+        return tuple(ptr(x) for x in (self.k, self.v, self.ks, self.vs, self.kb, self.vb))
+
+    def _q8_addrs(self):
+        return (addr(self.k), addr(self.v), addr(self.ks), addr(self.vs), addr(self.kb), addr(self.vb))
 
     def nbytes(self) -> int:
         n = self.k.numel() * self.k.element_size() * 2
@@ -60,91 +63,91 @@ class Paging:
 
 # ---------------------------------------------------------------- rope
 def rope(h: Handle, qkv, pos: int, n_head, n_kv_head, head_dim, theta, stream=None):
-    check(lib().mx230_rope(h._h, stream_ptr(stream), ptr(qkv), pos, n_head, n_kv_head, head_dim, theta))
+    check(lib().mx230_rope(h._h, stream_ptr(stream), addr(qkv), pos, n_head, n_kv_head, head_dim, theta))
 
 
 def rope_dyn(h: Handle, qkv, pos_ptr, n_head, n_kv_head, head_dim, theta, stream=None):
-    check(lib().mx230_rope_dyn(h._h, stream_ptr(stream), ptr(qkv), ptr(pos_ptr), n_head, n_kv_head,
+    check(lib().mx230_rope_dyn(h._h, stream_ptr(stream), addr(qkv), addr(pos_ptr), n_head, n_kv_head,
                                head_dim, theta))
 
 
 def rope_batch(h: Handle, qkv, pos0, n_tok, n_head, n_kv_head, head_dim, stride, theta, stream=None):
-    check(lib().mx230_rope_batch(h._h, stream_ptr(stream), ptr(qkv), pos0, n_tok, n_head, n_kv_head,
+    check(lib().mx230_rope_batch(h._h, stream_ptr(stream), addr(qkv), pos0, n_tok, n_head, n_kv_head,
                                  head_dim, stride, theta))
 
 
 def rope_seqpos(h: Handle, qkv, pos, n_seq, n_head, n_kv_head, head_dim, stride, theta, stream=None):
-    check(lib().mx230_rope_seqpos(h._h, stream_ptr(stream), ptr(qkv), ptr(pos), n_seq, n_head,
+    check(lib().mx230_rope_seqpos(h._h, stream_ptr(stream), addr(qkv), addr(pos), n_seq, n_head,
                                   n_kv_head, head_dim, stride, theta))
 
 
 # ---------------------------------------------------------------- fp32 KV write
 def copy_kv(h: Handle, c: KvCache, qkv, pos: int, q_dim, kv_dim, stream=None):
-    check(lib().mx230_copy_kv(h._h, stream_ptr(stream), ptr(c.k), ptr(c.v), ptr(qkv), pos, q_dim, kv_dim))
+    check(lib().mx230_copy_kv(h._h, stream_ptr(stream), addr(c.k), addr(c.v), addr(qkv), pos, q_dim, kv_dim))
 
 
 def copy_kv_dyn(h: Handle, c: KvCache, qkv, pos_ptr, q_dim, kv_dim, stream=None):
-    check(lib().mx230_copy_kv_dyn(h._h, stream_ptr(stream), ptr(c.k), ptr(c.v), ptr(qkv),
-                                  ptr(pos_ptr), q_dim, kv_dim))
+    check(lib().mx230_copy_kv_dyn(h._h, stream_ptr(stream), addr(c.k), addr(c.v), addr(qkv),
+                                  addr(pos_ptr), q_dim, kv_dim))
 
 
 def copy_kv_paged_dyn(h: Handle, c: KvCache, qkv, pos_ptr, q_dim, kv_dim, pg: Paging, stream=None):
-    check(lib().mx230_copy_kv_paged_dyn(h._h, stream_ptr(stream), ptr(c.k), ptr(c.v), ptr(qkv),
-                                        ptr(pos_ptr), q_dim, kv_dim, ptr(pg.table_dev), pg.block_size))
+    check(lib().mx230_copy_kv_paged_dyn(h._h, stream_ptr(stream), addr(c.k), addr(c.v), addr(qkv),
+                                        addr(pos_ptr), q_dim, kv_dim, addr(pg.table_dev), pg.block_size))
 
 
 def copy_kv_batch(h: Handle, c: KvCache, qkv, pos0, n_tok, q_dim, kv_dim, stride, pg: Paging | None = None,
                   stream=None):
     if pg is None:
-        check(lib().mx230_copy_kv_batch(h._h, stream_ptr(stream), ptr(c.k), ptr(c.v), ptr(qkv), pos0,
+        check(lib().mx230_copy_kv_batch(h._h, stream_ptr(stream), addr(c.k), addr(c.v), addr(qkv), pos0,
                                         n_tok, q_dim, kv_dim, stride))
     else:
-        check(lib().mx230_copy_kv_batch_paged(h._h, stream_ptr(stream), ptr(c.k), ptr(c.v), ptr(qkv),
-                                              pos0, n_tok, q_dim, kv_dim, stride, ptr(pg.table_dev),
+        check(lib().mx230_copy_kv_batch_paged(h._h, stream_ptr(stream), addr(c.k), addr(c.v), addr(qkv),
+                                              pos0, n_tok, q_dim, kv_dim, stride, addr(pg.table_dev),
                                               pg.block_size))
 
 
 def copy_kv_seqpos(h: Handle, c: KvCache, qkv, pos, n_seq, q_dim, kv_dim, qkv_stride, pg: Paging,
                    stream=None):
-    check(lib().mx230_copy_kv_seqpos(h._h, stream_ptr(stream), ptr(c.k), ptr(c.v), ptr(qkv), ptr(pos),
-                                     n_seq, q_dim, kv_dim, qkv_stride, ptr(pg.table_dev),
+    check(lib().mx230_copy_kv_seqpos(h._h, stream_ptr(stream), addr(c.k), addr(c.v), addr(qkv), addr(pos),
+                                     n_seq, q_dim, kv_dim, qkv_stride, addr(pg.table_dev),
                                      pg.block_size, pg.n_log))
 
 
 # ---------------------------------------------------------------- int8 quantize-on-write
 def quantize_kv(h: Handle, c: KvCache, qkv, pos: int, q_dim, n_kv_head, head_dim, stream=None):
-    check(lib().mx230_quantize_kv(h._h, stream_ptr(stream), *c.q8_args(), ptr(qkv), pos, q_dim,
+    check(lib().mx230_quantize_kv(h._h, stream_ptr(stream), *c._q8_addrs(), addr(qkv), pos, q_dim,
                                   n_kv_head, head_dim))
 
 
 def quantize_kv_dyn(h: Handle, c: KvCache, qkv, pos_ptr, q_dim, n_kv_head, head_dim, stream=None):
-    check(lib().mx230_quantize_kv_dyn(h._h, stream_ptr(stream), *c.q8_args(), ptr(qkv), ptr(pos_ptr),
+    check(lib().mx230_quantize_kv_dyn(h._h, stream_ptr(stream), *c._q8_addrs(), addr(qkv), addr(pos_ptr),
                                       q_dim, n_kv_head, head_dim))
 
 
 def quantize_kv_paged_dyn(h: Handle, c: KvCache, qkv, pos_ptr, q_dim, n_kv_head, head_dim, pg: Paging,
                           stream=None):
-    check(lib().mx230_quantize_kv_paged_dyn(h._h, stream_ptr(stream), *c.q8_args(), ptr(qkv),
-                                            ptr(pos_ptr), q_dim, n_kv_head, head_dim,
-                                            ptr(pg.table_dev), pg.block_size))
+    check(lib().mx230_quantize_kv_paged_dyn(h._h, stream_ptr(stream), *c._q8_addrs(), addr(qkv),
+                                            addr(pos_ptr), q_dim, n_kv_head, head_dim,
+                                            addr(pg.table_dev), pg.block_size))
 
 
 def quantize_kv_batch(h: Handle, c: KvCache, qkv, pos0, n_tok, q_dim, n_kv_head, head_dim, stride,
                       pg: Paging | None = None, stream=None):
     if pg is None:
-        check(lib().mx230_quantize_kv_batch(h._h, stream_ptr(stream), *c.q8_args(), ptr(qkv), pos0,
+        check(lib().mx230_quantize_kv_batch(h._h, stream_ptr(stream), *c._q8_addrs(), addr(qkv), pos0,
                                             n_tok, q_dim, n_kv_head, head_dim, stride))
     else:
-        check(lib().mx230_quantize_kv_batch_paged(h._h, stream_ptr(stream), *c.q8_args(), ptr(qkv),
+        check(lib().mx230_quantize_kv_batch_paged(h._h, stream_ptr(stream), *c._q8_addrs(), addr(qkv),
                                                   pos0, n_tok, q_dim, n_kv_head, head_dim, stride,
-                                                  ptr(pg.table_dev), pg.block_size))
+                                                  addr(pg.table_dev), pg.block_size))
 
 
 def quantize_kv_seqpos(h: Handle, c: KvCache, qkv, pos, n_seq, q_dim, n_kv_head, head_dim, qkv_stride,
                        pg: Paging, stream=None):
-    check(lib().mx230_quantize_kv_seqpos(h._h, stream_ptr(stream), *c.q8_args(), ptr(qkv), ptr(pos),
+    check(lib().mx230_quantize_kv_seqpos(h._h, stream_ptr(stream), *c._q8_addrs(), addr(qkv), addr(pos),
                                          n_seq, q_dim, n_kv_head, head_dim, qkv_stride,
-                                         ptr(pg.table_dev), pg.block_size, pg.n_log))
+                                         addr(pg.table_dev), pg.block_size, pg.n_log))
 
 
 # ---------------------------------------------------------------- decode attention
@@ -156,18 +159,18 @@ def attn_decode(h: Handle, out, qkv, c: KvCache, t_cur: int, n_head, n_kv_head, 
     L = lib()
     if c.quant:
         if pg is None:
-            check(L.mx230_attn_decode_q8(h._h, s, ptr(out), ptr(qkv), *c.q8_args(), t_cur, n_head,
+            check(L.mx230_attn_decode_q8(h._h, s, addr(out), addr(qkv), *c._q8_addrs(), t_cur, n_head,
                                          n_kv_head, head_dim))
         else:
-            check(L.mx230_attn_decode_q8_paged(h._h, s, ptr(out), ptr(qkv), *c.q8_args(), t_cur, n_head,
-                                               n_kv_head, head_dim, ptr(pg.table_dev), pg.block_size))
+            check(L.mx230_attn_decode_q8_paged(h._h, s, addr(out), addr(qkv), *c._q8_addrs(), t_cur, n_head,
+                                               n_kv_head, head_dim, addr(pg.table_dev), pg.block_size))
     else:
         if pg is None:
-            check(L.mx230_attn_decode(h._h, s, ptr(out), ptr(qkv), ptr(c.k), ptr(c.v), t_cur, n_head,
+            check(L.mx230_attn_decode(h._h, s, addr(out), addr(qkv), addr(c.k), addr(c.v), t_cur, n_head,
                                       n_kv_head, head_dim))
         else:
-            check(L.mx230_attn_decode_paged(h._h, s, ptr(out), ptr(qkv), ptr(c.k), ptr(c.v), t_cur,
-                                            n_head, n_kv_head, head_dim, ptr(pg.table_dev),
+            check(L.mx230_attn_decode_paged(h._h, s, addr(out), addr(qkv), addr(c.k), addr(c.v), t_cur,
+                                            n_head, n_kv_head, head_dim, addr(pg.table_dev),
                                             pg.block_size))
 
 
@@ -178,20 +181,20 @@ def attn_decode_dyn(h: Handle, out, qkv, c: KvCache, pos_ptr, n_head, n_kv_head,
     L = lib()
     if c.quant:
         if pg is None:
-            check(L.mx230_attn_decode_q8_dyn(h._h, s, ptr(out), ptr(qkv), *c.q8_args(), ptr(pos_ptr),
+            check(L.mx230_attn_decode_q8_dyn(h._h, s, addr(out), addr(qkv), *c._q8_addrs(), addr(pos_ptr),
                                              n_head, n_kv_head, head_dim))
         else:
-            check(L.mx230_attn_decode_q8_paged_dyn(h._h, s, ptr(out), ptr(qkv), *c.q8_args(),
-                                                   ptr(pos_ptr), n_head, n_kv_head, head_dim,
-                                                   ptr(pg.table_dev), pg.block_size))
+            check(L.mx230_attn_decode_q8_paged_dyn(h._h, s, addr(out), addr(qkv), *c._q8_addrs(),
+                                                   addr(pos_ptr), n_head, n_kv_head, head_dim,
+                                                   addr(pg.table_dev), pg.block_size))
     else:
         if pg is None:
-            check(L.mx230_attn_decode_dyn(h._h, s, ptr(out), ptr(qkv), ptr(c.k), ptr(c.v), ptr(pos_ptr),
+            check(L.mx230_attn_decode_dyn(h._h, s, addr(out), addr(qkv), addr(c.k), addr(c.v), addr(pos_ptr),
                                           n_head, n_kv_head, head_dim))
         else:
-            check(L.mx230_attn_decode_paged_dyn(h._h, s, ptr(out), ptr(qkv), ptr(c.k), ptr(c.v),
-                                                ptr(pos_ptr), n_head, n_kv_head, head_dim,
-                                                ptr(pg.table_dev), pg.block_size))
+            check(L.mx230_attn_decode_paged_dyn(h._h, s, addr(out), addr(qkv), addr(c.k), addr(c.v),
+                                                addr(pos_ptr), n_head, n_kv_head, head_dim,
+                                                addr(pg.table_dev), pg.block_size))
 
 
 def attn_decode_batched(h: Handle, out, qkv, c: KvCache, pos, n_seq, n_head, n_kv_head, head_dim,
@@ -199,38 +202,38 @@ def attn_decode_batched(h: Handle, out, qkv, c: KvCache, pos, n_seq, n_head, n_k
     """attn_decode_batched / attn_decode_q8_batched, gpu.rs:3530-3628."""
     s = stream_ptr(stream)
     if c.quant:
-        check(lib().mx230_attn_decode_q8_batched(h._h, s, ptr(out), ptr(qkv), *c.q8_args(), ptr(pos),
-                                                 n_seq, n_head, n_kv_head, head_dim, ptr(pg.table_dev),
+        check(lib().mx230_attn_decode_q8_batched(h._h, s, addr(out), addr(qkv), *c._q8_addrs(), addr(pos),
+                                                 n_seq, n_head, n_kv_head, head_dim, addr(pg.table_dev),
                                                  pg.block_size, pg.n_log, qkv_stride, out_stride))
     else:
-        check(lib().mx230_attn_decode_batched(h._h, s, ptr(out), ptr(qkv), ptr(c.k), ptr(c.v), ptr(pos),
-                                              n_seq, n_head, n_kv_head, head_dim, ptr(pg.table_dev),
+        check(lib().mx230_attn_decode_batched(h._h, s, addr(out), addr(qkv), addr(c.k), addr(c.v), addr(pos),
+                                              n_seq, n_head, n_kv_head, head_dim, addr(pg.table_dev),
                                               pg.block_size, pg.n_log, qkv_stride, out_stride))
 
 
 def _cache_args(c: KvCache):
     if c.quant:
-        return (None, None) + c.q8_args()
-    return (ptr(c.k), ptr(c.v), None, None, None, None, None, None)
+        return (None, None) + c._q8_addrs()
+    return (addr(c.k), addr(c.v), None, None, None, None, None, None)
 
 
 def _table_args(pg: Paging | None):
-    return (None, 0) if pg is None else (ptr(pg.table_dev), pg.block_size)
+    return (None, 0) if pg is None else (addr(pg.table_dev), pg.block_size)
 
 
 def attn_decode_slab(h: Handle, out, qkv, c: KvCache, pos, n_seq, n_head, n_kv_head, head_dim,
                      seq_rows, qkv_stride, out_stride, stream=None):
     """Batched decode over contiguous per-sequence cache slabs of `seq_rows` rows."""
-    check(lib().mx230_attn_decode_slab(h._h, stream_ptr(stream), ptr(out), ptr(qkv), *_cache_args(c),
-                                       ptr(pos), n_seq, n_head, n_kv_head, head_dim, seq_rows,
+    check(lib().mx230_attn_decode_slab(h._h, stream_ptr(stream), addr(out), addr(qkv), *_cache_args(c),
+                                       addr(pos), n_seq, n_head, n_kv_head, head_dim, seq_rows,
                                        qkv_stride, out_stride))
 
 
 def attn_decode_partial(h: Handle, part_m, part_l, part_acc, qkv, c: KvCache, t0, t1, n_seq, n_head,
                         n_kv_head, head_dim, seq_rows, qkv_stride, stream=None):
     """Unnormalised (m, l, acc) of keys [t0, t1) per (sequence, query head)."""
-    check(lib().mx230_attn_decode_partial(h._h, stream_ptr(stream), ptr(part_m), ptr(part_l),
-                                          ptr(part_acc), ptr(qkv), *_cache_args(c), t0, t1, n_seq,
+    check(lib().mx230_attn_decode_partial(h._h, stream_ptr(stream), addr(part_m), addr(part_l),
+                                          addr(part_acc), addr(qkv), *_cache_args(c), t0, t1, n_seq,
                                           n_head, n_kv_head, head_dim, seq_rows, qkv_stride))
 
 
@@ -238,7 +241,7 @@ def attn_decode_partial_push(h: Handle, comm, qkv, c: KvCache, t0, t1, n_seq, n_
                              qkv_stride, stream=None):
     """attn_decode_partial whose finishing CTAs store the triples into every rank's split-KV exchange region
     (`comm`: the mx230_splitkv_comm of `multi_gpu.PeerExchange`)."""
-    check(lib().mx230_attn_decode_partial_push(h._h, stream_ptr(stream), comm, ptr(qkv), *_cache_args(c), t0, t1,
+    check(lib().mx230_attn_decode_partial_push(h._h, stream_ptr(stream), comm, addr(qkv), *_cache_args(c), t0, t1,
                                                n_seq, n_head, n_kv_head, head_dim, seq_rows, qkv_stride))
 
 
@@ -246,18 +249,18 @@ def attn_decode_splitkv(h: Handle, comm, out, qkv, c: KvCache, t0, t1, n_seq, n_
                         qkv_stride, stream=None):
     """A whole split-KV step in one kernel: partial attention over keys [t0, t1), stores to every other rank's
     exchange region, wait for their triples, merged rows to out[n_seq * n_head][64]."""
-    check(lib().mx230_attn_decode_splitkv(h._h, stream_ptr(stream), comm, ptr(out), ptr(qkv), *_cache_args(c), t0, t1,
+    check(lib().mx230_attn_decode_splitkv(h._h, stream_ptr(stream), comm, addr(out), addr(qkv), *_cache_args(c), t0, t1,
                                           n_seq, n_head, n_kv_head, head_dim, seq_rows, qkv_stride))
 
 
 def merge_partials(h: Handle, out, m, l, acc, parts, rows, head_dim=64, stream=None):
-    check(lib().mx230_merge_partials(h._h, stream_ptr(stream), ptr(out), ptr(m), ptr(l), ptr(acc),
+    check(lib().mx230_merge_partials(h._h, stream_ptr(stream), addr(out), addr(m), addr(l), addr(acc),
                                      parts, rows, head_dim))
 
 
 def merge_partials_packed(h: Handle, out, gathered, parts, rows, head_dim=64, stream=None):
     """Merge straight from the all-gathered buffer [parts][m | l | acc] (rows even)."""
-    check(lib().mx230_merge_partials_packed(h._h, stream_ptr(stream), ptr(out), ptr(gathered), parts, rows, head_dim))
+    check(lib().mx230_merge_partials_packed(h._h, stream_ptr(stream), addr(out), addr(gathered), parts, rows, head_dim))
 
 
 # ---------------------------------------------------------------- the step
@@ -266,14 +269,14 @@ def decode_step(h: Handle, out, qkv, c: KvCache, pos: int, n_head, n_kv_head, he
     """One token of one sequence, as forward_layers does per layer (gpu.rs:2570-2672):
     RoPE, KV write at the host-resolved physical row, then attention over 0..=pos -- one launch."""
     phys = pos if pg is None else pg.phys_row(host_table, pos)
-    check(lib().mx230_decode_step(h._h, stream_ptr(stream), ptr(out), ptr(qkv), *_cache_args(c), pos, None, phys, n_head,
+    check(lib().mx230_decode_step(h._h, stream_ptr(stream), addr(out), addr(qkv), *_cache_args(c), pos, None, phys, n_head,
                                   n_kv_head, head_dim, int(use_rope), theta, *_table_args(pg)))
 
 
 def decode_step_dyn(h: Handle, out, qkv, c: KvCache, pos_ptr, n_head, n_kv_head, head_dim, theta,
                     pg: Paging | None = None, use_rope=True, stream=None):
     """The graph-capturable step of forward_body_dyn (gpu.rs:2808-2918)."""
-    check(lib().mx230_decode_step(h._h, stream_ptr(stream), ptr(out), ptr(qkv), *_cache_args(c), -1, ptr(pos_ptr), 0, n_head,
+    check(lib().mx230_decode_step(h._h, stream_ptr(stream), addr(out), addr(qkv), *_cache_args(c), -1, addr(pos_ptr), 0, n_head,
                                   n_kv_head, head_dim, int(use_rope), theta, *_table_args(pg)))
 
 
@@ -281,8 +284,8 @@ def batched_step(h: Handle, out, qkv, c: KvCache, pos, n_seq, n_head, n_kv_head,
                  pg: Paging, qkv_stride, out_stride, use_rope=True, stream=None):
     """One token for each of n_seq sequences, as forward_batched (gpu.rs:3530-3628) -- two launches, so that rows of the same
     sequence see one another."""
-    check(lib().mx230_batched_step(h._h, stream_ptr(stream), ptr(out), ptr(qkv), *_cache_args(c), ptr(pos), n_seq, n_head,
-                                   n_kv_head, head_dim, int(use_rope), theta, ptr(pg.table_dev), pg.block_size, pg.n_log,
+    check(lib().mx230_batched_step(h._h, stream_ptr(stream), addr(out), addr(qkv), *_cache_args(c), addr(pos), n_seq, n_head,
+                                   n_kv_head, head_dim, int(use_rope), theta, addr(pg.table_dev), pg.block_size, pg.n_log,
                                    qkv_stride, out_stride))
 
 
@@ -299,19 +302,19 @@ def attn_prefill(h: Handle, out, qkv, c: KvCache, pos0, n_tok, n_head, n_kv_head
     L = lib()
     if c.quant:
         if pg is None:
-            check(L.mx230_attn_prefill_q8(h._h, s, ptr(out), ptr(qkv), *c.q8_args(), pos0, n_tok, n_head,
+            check(L.mx230_attn_prefill_q8(h._h, s, addr(out), addr(qkv), *c._q8_addrs(), pos0, n_tok, n_head,
                                           n_kv_head, qkv_stride, out_stride))
         else:
-            check(L.mx230_attn_prefill_q8_paged(h._h, s, ptr(out), ptr(qkv), *c.q8_args(), pos0, n_tok, n_head,
-                                                n_kv_head, qkv_stride, out_stride, ptr(pg.table_dev),
+            check(L.mx230_attn_prefill_q8_paged(h._h, s, addr(out), addr(qkv), *c._q8_addrs(), pos0, n_tok, n_head,
+                                                n_kv_head, qkv_stride, out_stride, addr(pg.table_dev),
                                                 pg.block_size))
     else:
         if pg is None:
-            check(L.mx230_attn_prefill(h._h, s, ptr(out), ptr(qkv), ptr(c.k), ptr(c.v), pos0, n_tok, n_head,
+            check(L.mx230_attn_prefill(h._h, s, addr(out), addr(qkv), addr(c.k), addr(c.v), pos0, n_tok, n_head,
                                        n_kv_head, qkv_stride, out_stride))
         else:
-            check(L.mx230_attn_prefill_paged(h._h, s, ptr(out), ptr(qkv), ptr(c.k), ptr(c.v), pos0, n_tok,
-                                             n_head, n_kv_head, qkv_stride, out_stride, ptr(pg.table_dev),
+            check(L.mx230_attn_prefill_paged(h._h, s, addr(out), addr(qkv), addr(c.k), addr(c.v), pos0, n_tok,
+                                             n_head, n_kv_head, qkv_stride, out_stride, addr(pg.table_dev),
                                              pg.block_size))
 
 
@@ -328,7 +331,7 @@ def prefill_step(h: Handle, out, qkv, c: KvCache, pos0, n_tok, n_head, n_kv_head
         else:
             copy_kv_batch(h, c, qkv, pos0, n_tok, q_dim, kv_dim, qkv_stride, pg, stream)
         return attn_prefill(h, out, qkv, c, pos0, n_tok, n_head, n_kv_head, qkv_stride, out_stride, pg, stream)
-    check(lib().mx230_prefill_step(h._h, stream_ptr(stream), ptr(out), ptr(qkv), *_cache_args(c), pos0, n_tok, n_head,
+    check(lib().mx230_prefill_step(h._h, stream_ptr(stream), addr(out), addr(qkv), *_cache_args(c), pos0, n_tok, n_head,
                                    n_kv_head, head_dim, int(use_rope), theta, qkv_stride, out_stride, *_table_args(pg)))
 
 
@@ -336,7 +339,7 @@ def attn_decode_q8_noalloc(out, qkv, c: KvCache, t_cur: int, n_head, n_kv_head, 
     """Handle-free int8-cache decode of one sequence whose split-KV scratch is a fixed array inside
     the library: for hosts that may not call cudaMalloc (all HBM already owned by their KV pool, or
     only allowed to enqueue on a given stream).  Current device; see include/mx230_attn.h."""
-    check(lib().mx230_attn_decode_q8_noalloc(stream_ptr(stream), ptr(out), ptr(qkv), *c.q8_args(), t_cur,
+    check(lib().mx230_attn_decode_q8_noalloc(stream_ptr(stream), addr(out), addr(qkv), *c._q8_addrs(), t_cur,
                                              n_head, n_kv_head, head_dim))
 
 
@@ -344,8 +347,8 @@ def attn_decode_q8_noalloc(out, qkv, c: KvCache, t_cur: int, n_head, n_kv_head, 
 def gemv(h: Handle, y, x, w, b=None, accum=False, stream=None):
     """gemv / gemv_half (llm.cu:144-177; gpu.rs:1158-1198): y (+)= x W + b, W [n_in][n_out] fp32 or fp16."""
     n_in, n_out = w.shape
-    check(lib().mx230_gemv(h._h, stream_ptr(stream), ptr(y), ptr(x), ptr(w), int(w.dtype == torch.float16),
-                           ptr(b), n_in, n_out, int(accum)))
+    check(lib().mx230_gemv(h._h, stream_ptr(stream), addr(y), addr(x), addr(w), int(w.dtype == torch.float16),
+                           addr(b), n_in, n_out, int(accum)))
 
 
 def gemm(h: Handle, c, a, w, b=None, stream=None):
@@ -355,7 +358,7 @@ def gemm(h: Handle, c, a, w, b=None, stream=None):
     n = w.shape[1]
     fp16 = 1 if w.dtype == torch.float16 else 0
     h.reserve(lib().mx230_gemm_workspace_bytes(m, n, k, fp16))
-    check(lib().mx230_gemm(h._h, stream_ptr(stream), ptr(c), ptr(a), ptr(w), fp16, ptr(b), m, n, k))
+    check(lib().mx230_gemm(h._h, stream_ptr(stream), addr(c), addr(a), addr(w), fp16, addr(b), m, n, k))
 
 
 def prefill_layer_attention(h: Handle, y, x, w_qkv, b_qkv, w_proj, b_proj, qkv, attn, c: KvCache, pos0, n_tok, n_head,
@@ -373,7 +376,7 @@ def prefill_layer_attention(h: Handle, y, x, w_qkv, b_qkv, w_proj, b_proj, qkv, 
 def gemv_int8(h: Handle, y, x, w_packed, scales, b=None, accum=False, act_group=8, stream=None):
     """gemv_int8 (llm.cu:226-316): `w_packed` int32 [n_in / 4][n_out], four consecutive input rows per word."""
     n_in, n_out = w_packed.shape[0] * 4, w_packed.shape[1]
-    check(lib().mx230_gemv_int8(h._h, stream_ptr(stream), ptr(y), ptr(x), ptr(w_packed), ptr(scales), ptr(b),
+    check(lib().mx230_gemv_int8(h._h, stream_ptr(stream), addr(y), addr(x), addr(w_packed), addr(scales), addr(b),
                                 n_in, n_out, int(accum), act_group))
 
 
@@ -385,8 +388,8 @@ def qkv_rope_kvwrite(h: Handle, qkv, x, w, b, pos, c: KvCache, n_head, n_kv_head
     n_in = w.shape[0] * (4 if int8 else 1)
     kind = 2 if int8 else int(w.dtype == torch.float16)
     dyn = not isinstance(pos, int)
-    caches = (None, None, *c.q8_args()) if c.quant else (ptr(c.k), ptr(c.v), None, None, None, None, None, None)
-    check(lib().mx230_qkv_rope_kvwrite(h._h, stream_ptr(stream), ptr(qkv), ptr(x), ptr(w),
-                                       kind, ptr(w_scales), act_group, ptr(b), n_in, 0 if dyn else pos,
-                                       ptr(pos) if dyn else None, n_head, n_kv_head, 64, theta, *caches,
-                                       ptr(pg.table_dev) if pg else None, pg.block_size if pg else 0))
+    caches = (None, None, *c._q8_addrs()) if c.quant else (addr(c.k), addr(c.v), None, None, None, None, None, None)
+    check(lib().mx230_qkv_rope_kvwrite(h._h, stream_ptr(stream), addr(qkv), addr(x), addr(w),
+                                       kind, addr(w_scales), act_group, addr(b), n_in, 0 if dyn else pos,
+                                       addr(pos) if dyn else None, n_head, n_kv_head, 64, theta, *caches,
+                                       addr(pg.table_dev) if pg else None, pg.block_size if pg else 0))
