@@ -320,6 +320,14 @@ int mx230_prefill_step(mx230_handle *h, void *stream, float *out, float *qkv, fl
                        int8_t *kq, int8_t *vq, float *ks, float *vs, float *kb, float *vb, int pos0, int n_tok,
                        int n_head, int n_kv_head, int head_dim, int use_rope, float theta, int qkv_stride,
                        int out_stride, const int *bt, int bs);
+/* The same step followed by the output projection over fp16 weights, y [n_tok][n_out] = out w + bias (gpu.rs:3354-3365; w
+ * [n_head * 64][n_out], n_out % 8 == 0, bias may be null; y, w, bias 16-byte aligned): every result equals that of
+ * mx230_prefill_step and mx230_gemm in turn.  The attention kernel leaves its rows in fp16 for the projection as well, so
+ * none is staged in between.  Workspace: mx230_prefill_workspace_bytes. */
+int mx230_prefill_step_proj(mx230_handle *h, void *stream, float *y, const void *w, const float *bias, int n_out,
+                            float *out, float *qkv, float *kcache, float *vcache, int8_t *kq, int8_t *vq, float *ks,
+                            float *vs, float *kb, float *vb, int pos0, int n_tok, int n_head, int n_kv_head, int head_dim,
+                            int use_rope, float theta, int qkv_stride, int out_stride, const int *bt, int bs);
 
 /* Decode over an int8 cache without a handle and without any allocation (no counterpart in
  * the reference, whose kernels use no scratch memory at all).  For hosts that cannot call

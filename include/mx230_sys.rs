@@ -199,6 +199,13 @@ extern "C" {
         n_head: c_int, n_kv_head: c_int, head_dim: c_int, use_rope: c_int, theta: f32, qkv_stride: c_int,
         out_stride: c_int, bt: *const c_int, bs: c_int,
     ) -> c_int;
+    pub fn mx230_prefill_step_proj(
+        h: *mut Mx230Handle, stream: *mut c_void, y: *mut f32, w: *const c_void, bias: *const f32, n_out: c_int,
+        out: *mut f32, qkv: *mut f32, kcache: *mut f32, vcache: *mut f32, kq: *mut i8, vq: *mut i8, ks: *mut f32,
+        vs: *mut f32, kb: *mut f32, vb: *mut f32, pos0: c_int, n_tok: c_int, n_head: c_int, n_kv_head: c_int,
+        head_dim: c_int, use_rope: c_int, theta: f32, qkv_stride: c_int, out_stride: c_int, bt: *const c_int,
+        bs: c_int,
+    ) -> c_int;
     pub fn mx230_attn_decode_q8_noalloc(
         stream: *mut c_void, out: *mut f32, qkv: *const f32, kq: *const i8, vq: *const i8, ks: *const f32,
         vs: *const f32, kb: *const f32, vb: *const f32, t_cur: c_int, n_head: c_int, n_kv_head: c_int,

@@ -210,12 +210,15 @@ inline size_t mx230_flash_norm_bytes(int batch_heads) {
 // provably small takes the kernel's max-free softmax loop.  row_a / row_qsum / col_kskb (all or none; with them q_prescaled
 // must be 0 and Qb, Kb hold int8 codes as bf16): the int8 score mode -- score = row_a[h][i] * (dot * ks[j] +
 // row_qsum[h][i] * kb[j]), with col_kskb [heads / kv_group][tiles of 128 keys][ks of the 128 keys, then their kb], 16-byte
-// aligned.
+// aligned.  O_half (may be null, may be Qb): [heads][n_q][64], receives the output rounded to fp16 as well.
 int mx230_launch_flash_fwd_ex(mx230_handle *h, cudaStream_t st, const void *Qb, const void *Kb,
                               const void *Vb, float *O, float *L, int heads, int n_q, int n_k, int q_off,
                               int kv_group, long long o_head_stride, long long o_row_stride, int causal,
                               int q_prescaled, const float *q_norm2, const float *k_norm2, const float *row_a,
-                              const float *row_qsum, const float *col_kskb);
+                              const float *row_qsum, const float *col_kskb, void *O_half);
+// C = A w + bias over A in fp16 as the forward's O_half leaves it, [k / 64 heads][m][64] (gemm.cu).  w fp16, n % 8 == 0.
+int mx230_launch_gemm_by_head(mx230_handle *h, cudaStream_t st, float *C, const void *A_half, const void *w, const float *bias,
+                              int m, int n, int k);
 
 // RoPE on the Q and K heads of one new row of each of n_seq sequences (use_rope != 0) and their K and V heads into the
 // paged cache (fp32 kcache / vcache when kq == NULL, else int8), in one launch (kvwrite.cu).

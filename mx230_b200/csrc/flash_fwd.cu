@@ -30,6 +30,7 @@
 //   scores and the other tile's P V while a tile's softmax runs on the CUDA cores.
 //
 // Operands are bf16 (rounded once by the cast pre-pass), accumulation is fp32.
+#include <cuda_fp16.h>
 #include <math_constants.h>
 
 #include <cstring>
@@ -111,6 +112,8 @@ constexpr float RESCALE_LOG2 = 8.0f;
 
 struct FwdParams {
     float *O;             // row r of head h at O + h*o_head_stride + r*o_row_stride (floats)
+    __half *O_half;       // [heads][n_q][64]: the same rows in fp16 for the projection that follows, or null.  May be where Q
+                          // is staged: an item's Q tile is read by that item alone, before the first row of its O exists
     float *L;             // [heads][n_q] or null
     long long o_head_stride, o_row_stride;
     int n_q;              // query rows per head
@@ -792,6 +795,18 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                         if (lane == 0) mx::mbar_arrive(bar(BAR_O1_READ));
                     }
                 };
+                auto store_half = [&](int cc) {   // this row's 32 columns of va: 64 bytes
+                    if (P.O_half == nullptr || row >= NQ) return;
+                    uint4 *dst = (uint4 *)(P.O_half + ((size_t)bh * NQ + row) * HD + cc * 32);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        __half2 h2[4];
+#pragma unroll
+                        for (int u = 0; u < 4; ++u)
+                            h2[u] = __floats2half2_rn(__uint_as_float(va[8 * i + 2 * u]) * inv, __uint_as_float(va[8 * i + 2 * u + 1]) * inv);
+                        dst[i] = *(const uint4 *)h2;
+                    }
+                };
                 float *orow = P.O + (size_t)bh * P.o_head_stride + (size_t)row * P.o_row_stride;
                 if (P.tma_out) {
                     // each warp stages its 32 rows, 32 columns at a time, in a swizzled 4 KB piece of this tile's Q
@@ -808,6 +823,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                             *(float4 *)(srow + ((cch ^ (lane & 7)) << 4)) =
                                 make_float4(__uint_as_float(va[4 * cch]) * inv, __uint_as_float(va[4 * cch + 1]) * inv,
                                             __uint_as_float(va[4 * cch + 2]) * inv, __uint_as_float(va[4 * cch + 3]) * inv);
+                        store_half(cc);
                         mx::fence_proxy_async_smem();
                         __syncwarp();
                         if (lane == 0 && wrow0 < NQ) {
@@ -828,6 +844,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                                                     __uint_as_float(va[i + 2]) * inv, __uint_as_float(va[i + 3]) * inv);
                             *(float4 *)(orow + cc * 32 + i) = o4;
                         }
+                        store_half(cc);
                     }
                 }
                 if (P.L != nullptr && row < NQ) P.L[(size_t)bh * NQ + row] = m * l_scale + __logf(l);
@@ -1072,7 +1089,7 @@ int mx230_launch_flash_fwd_ex(mx230_handle *h, cudaStream_t st, const void *Qb, 
                               const void *Vb, float *O, float *L, int heads, int n_q, int n_k, int q_off,
                               int kv_group, long long o_head_stride, long long o_row_stride, int causal,
                               int q_prescaled, const float *q_norm2, const float *k_norm2, const float *row_a,
-                              const float *row_qsum, const float *col_kskb) {
+                              const float *row_qsum, const float *col_kskb, void *O_half) {
     CUtensorMap tq, tk, tv, to;
     uint64_t rs = HD * 2;
     int rc;
@@ -1090,6 +1107,7 @@ int mx230_launch_flash_fwd_ex(mx230_handle *h, cudaStream_t st, const void *Qb, 
     if ((rc = mx230_make_tmap_bf16(h, &tv, Vb, n_k, heads / kv_group, rs, (uint64_t)n_k * HD * 2, BN))) return rc;
     FwdParams P;
     P.O = O;
+    P.O_half = (__half *)O_half;
     P.L = L;
     P.o_head_stride = o_head_stride;
     P.o_row_stride = o_row_stride;
@@ -1136,7 +1154,7 @@ int mx230_launch_flash_fwd(mx230_handle *h, cudaStream_t st, const void *Qb, con
                            const void *Vb, float *O, float *L, int batch_heads, int n, int causal,
                            int q_prescaled, const float *q_norm2, const float *k_norm2) {
     return mx230_launch_flash_fwd_ex(h, st, Qb, Kb, Vb, O, L, batch_heads, n, n, 0, 1, (long long)n * HD, HD,
-                                     causal, q_prescaled, q_norm2, k_norm2, nullptr, nullptr, nullptr);
+                                     causal, q_prescaled, q_norm2, k_norm2, nullptr, nullptr, nullptr, nullptr);
 }
 
 static int check_flash_args(const char *who, mx230_handle *h, int batch_heads, int n) {

@@ -41,6 +41,7 @@ struct GemmParams {
     float *C;
     const float *bias;
     int m, n, k;
+    int a_by_head; // A is [k / 64][m][64] instead of [m][k]
     int tma_out;   // C leaves through staged TMA stores (n a multiple of 64)
     int *status;
 };
@@ -97,7 +98,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CU
                 if (!ok) break;
                 const uint32_t base = smem_base + s * S::STAGE;
                 mx::mbar_expect_tx(bar(s), S::STAGE);
-                mx::tma_load_3d(base, &tmA0, bar(s), i * GK, m0, 0);
+                mx::tma_load_3d(base, &tmA0, bar(s), P.a_by_head ? 0 : i * GK, m0, P.a_by_head ? i : 0);
                 if (SPLIT) mx::tma_load_3d(base + A_TILE, &tmA1, bar(s), i * GK, m0, 0);
 #pragma unroll
                 for (int c = 0; c < GN / 64; ++c) {   // (a chunk past the last column is all zero fill)
@@ -220,6 +221,12 @@ __global__ void gemm_stage_kernel(StageParams P) {
     }
 }
 
+// Weights of one product: fp16 as the caller has them, or a staged (high, low) pair of bf16 matrices
+struct Weights {
+    const void *hi, *lo;
+    bool split;
+};
+
 size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 template <bool SPLIT, int GN>
@@ -229,6 +236,37 @@ int launch_tiles(mx230_handle *h, cudaStream_t st, const CUtensorMap &tA0, const
     MX_SMEM_ATTR_ONCE(h->device, (gemm_kernel<SPLIT, GN>), (Smem<SPLIT, GN>::ALLOC));
     MX_LAUNCH(h, st, MX230_K_GEMV, mx_launch(gemm_kernel<SPLIT, GN>, grid, THREADS, Smem<SPLIT, GN>::ALLOC, st, 1, true, tA0, tA1,
                                              tW0, tW1, tC, P));
+    return MX230_OK;
+}
+
+// The GEMM itself over a staged A
+int launch_gemm(mx230_handle *h, cudaStream_t st, float *C, const CUtensorMap &tA0, const CUtensorMap &tA1, bool a_by_head,
+                const Weights &w, const float *bias, int m, int n, int k) {
+    CUtensorMap tW0, tW1;
+    const bool split = w.split;
+    const int f16 = split ? 0 : 1;
+    int rc = mx230_make_tmap_2d_16bit(h, &tW0, w.hi, f16, (uint64_t)n, (uint64_t)k, (uint64_t)n * 2, 64, GK);
+    if (rc) return rc;
+    rc = mx230_make_tmap_2d_16bit(h, &tW1, w.lo, f16, (uint64_t)n, (uint64_t)k, (uint64_t)n * 2, 64, GK);
+    if (rc) return rc;
+
+    GemmParams P;
+    P.C = C, P.bias = bias, P.m = m, P.n = n, P.k = k, P.status = h->status_dev;
+    P.a_by_head = a_by_head ? 1 : 0;
+    // C [m][n] as [n / 64][m][64]: the store map of the attention kernels
+    CUtensorMap tC;
+    memset(&tC, 0, sizeof(tC));
+    P.tma_out = n % 64 == 0;
+    if (P.tma_out && (rc = mx230_make_tmap_f32_half_rows_strided(h, &tC, C, (uint64_t)m, (uint64_t)(n / 64), (uint64_t)n * 4, 256)))
+        return rc;
+    // 128-column tiles move two thirds of the bytes per CTA step that two 64-column ones do; they are taken when there are
+    // enough of them for two thirds of the SMs.  (Attention half of a layer, 1900 tokens, fp16 896 x 1152 and 896 x 896: these
+    // tiles, the TMA epilogue and programmatic launches of staging and GEMM 69.6 -> 55.2 us.)
+    const bool wide = (long long)((n + 127) / 128) * ((m + GM - 1) / GM) * 3 >= 2ll * h->sm_count;
+    if (split) rc = wide ? launch_tiles<true, 128>(h, st, tA0, tA1, tW0, tW1, tC, P) : launch_tiles<true, 64>(h, st, tA0, tA1, tW0, tW1, tC, P);
+    else rc = wide ? launch_tiles<false, 128>(h, st, tA0, tA1, tW0, tW1, tC, P) : launch_tiles<false, 64>(h, st, tA0, tA1, tW0, tW1, tC, P);
+    if (rc) return rc;
+    MX_CHECK_CUDA(cudaGetLastError());
     return MX230_OK;
 }
 
@@ -272,32 +310,19 @@ extern "C" int mx230_gemm(mx230_handle *h, void *stream, float *C, const float *
         MX_LAUNCH(h, st, MX230_K_CAST, mx_launch(gemm_stage_kernel<false>, dim3(blocks, 1), 256, 0, st, 1, true, SP));
     }
 
-    CUtensorMap tA0, tA1, tW0, tW1;
+    CUtensorMap tA0, tA1;
     const int f16 = split ? 0 : 1;
     int rc = mx230_make_tmap_2d_16bit(h, &tA0, a_hi, f16, (uint64_t)k, (uint64_t)m, (uint64_t)k * 2, GK, GM);
     if (rc) return rc;
     rc = mx230_make_tmap_2d_16bit(h, &tA1, split ? a_lo : a_hi, f16, (uint64_t)k, (uint64_t)m, (uint64_t)k * 2, GK, GM);
     if (rc) return rc;
-    rc = mx230_make_tmap_2d_16bit(h, &tW0, split ? w_hi : W_fp16, f16, (uint64_t)n, (uint64_t)k, (uint64_t)n * 2, 64, GK);
-    if (rc) return rc;
-    rc = mx230_make_tmap_2d_16bit(h, &tW1, split ? w_lo : W_fp16, f16, (uint64_t)n, (uint64_t)k, (uint64_t)n * 2, 64, GK);
-    if (rc) return rc;
+    return launch_gemm(h, st, C, tA0, tA1, false, split ? Weights{w_hi, w_lo, true} : Weights{W_fp16, W_fp16, false}, bias, m, n, k);
+}
 
-    GemmParams P;
-    P.C = C, P.bias = bias, P.m = m, P.n = n, P.k = k, P.status = h->status_dev;
-    // C [m][n] as [n / 64][m][64]: the store map of the attention kernels
-    CUtensorMap tC;
-    memset(&tC, 0, sizeof(tC));
-    P.tma_out = n % 64 == 0;
-    if (P.tma_out && (rc = mx230_make_tmap_f32_half_rows_strided(h, &tC, C, (uint64_t)m, (uint64_t)(n / 64), (uint64_t)n * 4, 256)))
-        return rc;
-    // 128-column tiles move two thirds of the bytes per CTA step that two 64-column ones do; they are taken when there are
-    // enough of them for two thirds of the SMs.  (Attention half of a layer, 1900 tokens, fp16 896 x 1152 and 896 x 896: these
-    // tiles, the TMA epilogue and programmatic launches of staging and GEMM 69.6 -> 55.2 us.)
-    const bool wide = (long long)((n + 127) / 128) * ((m + GM - 1) / GM) * 3 >= 2ll * h->sm_count;
-    if (split) rc = wide ? launch_tiles<true, 128>(h, st, tA0, tA1, tW0, tW1, tC, P) : launch_tiles<true, 64>(h, st, tA0, tA1, tW0, tW1, tC, P);
-    else rc = wide ? launch_tiles<false, 128>(h, st, tA0, tA1, tW0, tW1, tC, P) : launch_tiles<false, 64>(h, st, tA0, tA1, tW0, tW1, tC, P);
+int mx230_launch_gemm_by_head(mx230_handle *h, cudaStream_t st, float *C, const void *A_half, const void *w, const float *bias,
+                              int m, int n, int k) {
+    CUtensorMap tA;   // (16-bit values and zero fill: bf16 or fp16 is the same to a copy)
+    const int rc = mx230_make_tmap_bf16(h, &tA, A_half, (uint64_t)m, (uint64_t)(k / GK), GK * 2, (uint64_t)m * GK * 2, GM);
     if (rc) return rc;
-    MX_CHECK_CUDA(cudaGetLastError());
-    return MX230_OK;
+    return launch_gemm(h, st, C, tA, tA, true, Weights{w, w, false}, bias, m, n, k);
 }

@@ -268,11 +268,12 @@ struct StepArgs {
 
 size_t align1k(size_t x) { return (x + 1023) & ~(size_t)1023; }
 
-// With a step, qkv and the cache are written as well (the entry point that asks for one takes them non-const).
+// With a step, qkv and the cache are written as well (the entry point that asks for one takes them non-const).  o_half (may be
+// null) receives where the output lies in fp16, by heads: in the workspace, in Q's place.
 int prefill(mx230_handle *h, void *stream, float *out, const float *qkv, const float *kcache,
             const float *vcache, const int8_t *kq, const int8_t *vq, const float *ks, const float *vs,
             const float *kb, const float *vb, int pos0, int n_tok, int n_head, int n_kv_head, int qkv_stride,
-            int out_stride, const int *bt, int bs, const char *who, bool dp4a = false, StepArgs step = {}) {
+            int out_stride, const int *bt, int bs, const char *who, bool dp4a = false, StepArgs step = {}, void **o_half = nullptr) {
     MX_REQUIRE(h != nullptr, MX230_ERR_INVALID_ARG, "%s: null handle", who);
     MX_REQUIRE(pos0 >= 0 && n_tok >= 0, MX230_ERR_INVALID_ARG, "%s: negative pos0/n_tok", who);
     if (n_tok == 0) return MX230_OK;
@@ -303,6 +304,7 @@ int prefill(mx230_handle *h, void *stream, float *out, const float *qkv, const f
     cudaStream_t st = (cudaStream_t)stream;
     h->staged.valid = 0;   // the workspace is about to hold something else
     __nv_bfloat16 *qb = (__nv_bfloat16 *)h->ws;
+    if (o_half) *o_half = qb;
     __nv_bfloat16 *kbuf = (__nv_bfloat16 *)((char *)h->ws + qbytes);
     __nv_bfloat16 *vbuf = (__nv_bfloat16 *)((char *)h->ws + qbytes + kbytes);
     float *row_a = (float *)((char *)h->ws + qbytes + 2 * kbytes);
@@ -333,7 +335,7 @@ int prefill(mx230_handle *h, void *stream, float *out, const float *qkv, const f
     MX_LAUNCH(h, st, MX230_K_PREFILL, mx_launch(prefill_stage_kernel, ST_GRID, ST_THREADS, sm, st, ST_CLUSTER, true, S));
     return mx230_launch_flash_fwd_ex(h, st, qb, kbuf, vbuf, out, nullptr, n_head, n_tok, n_keys, pos0, n_head / n_kv_head, HD,
                                      out_stride, 1, i8_scores ? 0 : 1, q_norm2, k_norm2, i8_scores ? row_a : nullptr,
-                                     i8_scores ? row_qsum : nullptr, i8_scores ? kskb : nullptr);
+                                     i8_scores ? row_qsum : nullptr, i8_scores ? kskb : nullptr, o_half ? qb : nullptr);
 }
 
 }  // namespace
@@ -399,4 +401,22 @@ extern "C" int mx230_prefill_step(mx230_handle *h, void *stream, float *out, flo
     MX_REQUIRE(head_dim == HD, MX230_ERR_UNSUPPORTED, "prefill_step: head_dim %d unsupported (must be 64)", head_dim);
     return prefill(h, stream, out, qkv, kcache, vcache, kq, vq, ks, vs, kb, vb, pos0, n_tok, n_head, n_kv_head, qkv_stride,
                    out_stride, bt, bs, "prefill_step", false, StepArgs{true, use_rope, theta});
+}
+
+extern "C" int mx230_prefill_step_proj(mx230_handle *h, void *stream, float *y, const void *w, const float *bias, int n_out,
+                                       float *out, float *qkv, float *kcache, float *vcache, int8_t *kq, int8_t *vq, float *ks,
+                                       float *vs, float *kb, float *vb, int pos0, int n_tok, int n_head, int n_kv_head,
+                                       int head_dim, int use_rope, float theta, int qkv_stride, int out_stride, const int *bt,
+                                       int bs) {
+    MX_REQUIRE(head_dim == HD, MX230_ERR_UNSUPPORTED, "prefill_step_proj: head_dim %d unsupported (must be 64)", head_dim);
+    MX_REQUIRE(h && y && w, MX230_ERR_INVALID_ARG, "prefill_step_proj: null argument");
+    MX_REQUIRE(n_out > 0 && n_out % 8 == 0, MX230_ERR_UNSUPPORTED, "prefill_step_proj: n_out must be a multiple of 8 (got %d)", n_out);
+    MX_REQUIRE((((uintptr_t)y | (uintptr_t)w | (uintptr_t)bias) & 15) == 0, MX230_ERR_INVALID_ARG,
+               "prefill_step_proj: buffers must be 16-byte aligned");
+    void *o_half = nullptr;
+    const int rc = prefill(h, stream, out, qkv, kcache, vcache, kq, vq, ks, vs, kb, vb, pos0, n_tok, n_head, n_kv_head, qkv_stride,
+                           out_stride, bt, bs, "prefill_step_proj", false, StepArgs{true, use_rope, theta}, &o_half);
+    if (rc || n_tok == 0) return rc;
+    mx230_device_guard guard(h->device);
+    return mx230_launch_gemm_by_head(h, (cudaStream_t)stream, y, o_half, w, bias, n_tok, n_out, n_head * HD);
 }

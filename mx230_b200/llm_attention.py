@@ -369,6 +369,12 @@ def prefill_layer_attention(h: Handle, y, x, w_qkv, b_qkv, w_proj, b_proj, qkv, 
     and batch_attn); the residual add that follows stays with the caller, as in the reference."""
     q_dim = n_head * head_dim
     gemm(h, qkv, x, w_qkv, b_qkv, stream)
+    if w_proj.dtype == torch.float16 and head_dim == 64 and tuple(attn.shape) == (n_tok, q_dim):
+        # attention leaves its rows in fp16 for the projection: one staging launch less
+        check(lib().mx230_prefill_step_proj(h._h, stream_ptr(stream), addr(y), addr(w_proj), addr(b_proj), w_proj.shape[1],
+                                            addr(attn), addr(qkv), *_cache_args(c), pos0, n_tok, n_head, n_kv_head, head_dim,
+                                            int(use_rope), theta, qkv.shape[1], q_dim, *_table_args(pg)))
+        return
     prefill_step(h, attn, qkv, c, pos0, n_tok, n_head, n_kv_head, head_dim, theta, qkv.shape[1], q_dim, pg, use_rope, stream)
     gemm(h, y, attn, w_proj, b_proj, stream)
 
