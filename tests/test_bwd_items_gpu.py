@@ -29,19 +29,19 @@ def test_every_head_equals_itself_alone(handle, heads, n, causal, bf16):
     d_in = do.bfloat16() if bf16 else do
     handle.reserve(fa.workspace_bytes(heads, n, True))
 
-    def step(s):
-        o = torch.empty_like(do[s])
-        l, delta = (torch.empty(do[s].shape[:-1], device="cuda") for _ in range(2))
-        dq, dk, dv = (torch.full_like(do[s], float("nan")) for _ in range(3))
-        fwd(handle, q[s], k[s], v[s], o, l, n, causal)
-        fa.run_preprocess(handle, do[s], o, delta, n)
-        bwd(handle, q[s], k[s], v[s], d_in[s], l, delta, dq, dk, dv, n, causal)
-        handle.check_status()
-        return dq, dk, dv
+    o, (l, delta) = torch.empty_like(do), (torch.empty(heads, n, device="cuda") for _ in range(2))
+    fwd(handle, q, k, v, o, l, n, causal)
+    fa.run_preprocess(handle, do, o, delta, n)
 
-    dq, dk, dv = step(slice(0, heads))
+    def grads(s):   # of these heads, from the same L and Delta
+        out = [torch.full_like(do[s], float("nan")) for _ in range(3)]
+        bwd(handle, q[s], k[s], v[s], d_in[s], l[s], delta[s], *out, n, causal)
+        handle.check_status()
+        return out
+
+    dq, dk, dv = grads(slice(0, heads))
     for h in sorted({0, 1, heads // 3, 147, 148, heads - 2, heads - 1} & set(range(heads))):
-        aq, ak, av = step(slice(h, h + 1))
+        aq, ak, av = grads(slice(h, h + 1))
         assert torch.equal(dk[h], ak[0]) and torch.equal(dv[h], av[0]), f"head {h}"
         assert (dq[h] - aq[0]).abs().max() <= 2 * 9 * 2 ** -24 * 16 * aq.abs().max(), f"head {h}"
     for h in (0, heads - 1):   # against 64-bit gradients: operands rounded to bf16, as in the backward's other tests
