@@ -61,6 +61,7 @@ struct DecodeParams {
     // step after step: 116 us with the trigger at the top, 105 here, 100 without; 16 fp32 sequences of 1500 keys 23.1 / 22.8 /
     // 19.9; one int8 sequence in a 24-layer token, 64 CTAs: 259 / 245 / 272).
     int trigger;
+    int wide;            // fp32 cache: CTAs of F32_WARPS_WIDE warps
     int bs_shift;        // log2(bs) when bs is a power of two, else -1
     // fused step (RoPE and KV write of the new token inside the attention kernel): keys [0, pos) come from the cache,
     // key `pos` from the qkv row, whose K and V heads are written to cache row `write_row` (< 0: through the table)
@@ -278,19 +279,20 @@ __device__ void merge_and_store(const DecodeParams &P, int s, int head0, int gc,
 }
 
 // Merge of a CTA's warps, then of its cluster's CTAs, then (several clusters) of the clusters through the workspace.
-// mg: shared memory, [n_warps][G][68] = m (log2 domain), l, sum of p * V offset, pad, acc[64] per warp and head; the
-// CTA's own totals go behind it, [G][68], where the cluster's other CTAs read them: rank r finishes the heads
-// g = r (mod cl_size), so that the merge of up to eight CTAs costs one cluster barrier and one round of remote loads
-// instead of a fence, an atomic and a re-read of global memory (int8, one sequence of 2001 keys, 2 K/V heads: 16 splits
-// merged through the workspace 8.2 us, one cluster of 8 CTAs 5.3 us).
+// mg: shared memory, [n_warps][G][68] = m (log2 domain), l, sum of p * V offset, pad, acc[64] per warp and head.
+// xb: shared memory of its own, MERGE_ROWS rows of 68, for the cluster: rank r finishes the heads g = r (mod cl_size), and
+// every CTA pushes its totals of such a head into rank r's xb, so that the merge of up to eight CTAs costs one cluster
+// barrier behind stores that nobody waits for, instead of a fence, an atomic and a re-read of global memory (int8, one
+// sequence of 2001 keys, 2 K/V heads: 16 splits merged through the workspace 8.2 us, one cluster of 8 CTAs 5.3 us with the
+// totals pulled between two barriers).  The caller has arrived on the cluster barrier once (cl_size > 1).
 // q_rot (fused step): rotated q, [G][64] in shared memory; it replaces the raw q in qkv once every CTA of the group
 // has read that.  Null where out is the qkv row itself: the attention row then takes q's place.
+constexpr int MERGE_ROWS = 16;   // ceil(8 / C) heads from each of C CTAs, C <= 8: at most 14
 template <int G>
-__device__ void finish_group(const DecodeParams &P, float *mg, int n_warps, int s, int head0, int gc, int cl, int rank,
+__device__ void finish_group(const DecodeParams &P, float *mg, float *xb, int n_warps, int s, int head0, int gc, int cl, int rank,
                              int active, const float *q_rot, int *is_last) {
     const int tid = threadIdx.x, nt = blockDim.x, C = P.cl_size;
     const bool direct = active == 1 && P.fin_acc == nullptr;
-    float *cm = mg + n_warps * G * 68;
     auto emit = [&](int g, int d, float m2, float l, float a) {
         const int h = head0 + g;
         if (direct) {
@@ -305,6 +307,8 @@ __device__ void finish_group(const DecodeParams &P, float *mg, int n_warps, int 
         }
     };
     auto put_q = [&](int g, int d) { P.qkv_rw[(size_t)s * P.qkv_stride + (head0 + g) * 64 + d] = q_rot[g * 64 + d]; };
+    if (C > 1) mx::cluster_wait();   // every CTA of the cluster runs
+    const uint32_t xb_u32 = mx::smem_u32(xb);
     for (int i = tid; i < gc * 64; i += nt) {
         const int g = i >> 6, d = i & 63;
         float mm = -CUDART_INF_F;
@@ -320,13 +324,13 @@ __device__ void finish_group(const DecodeParams &P, float *mg, int n_warps, int 
             emit(g, d, mm, lt, a);
             if (q_rot && active == 1) put_q(g, d);
         } else {
-            cm[g * 68 + 4 + d] = a;
-            if (d == 0) cm[g * 68] = mm, cm[g * 68 + 1] = lt;
+            const uint32_t dst = mx::cluster_map(xb_u32 + (g / C * C + rank) * 68 * 4, g % C);
+            mx::cluster_st_f32(dst + 16 + d * 4, a);
+            if (d == 0) mx::cluster_st_f32(dst, mm), mx::cluster_st_f32(dst + 4, lt);
         }
     }
     if (C > 1) {
         mx::cluster_sync();
-        const uint32_t cm_u32 = mx::smem_u32(cm);
         for (int i = tid; (i >> 6) * C + rank < gc; i += nt) {
             const int g = (i >> 6) * C + rank, d = i & 63;
             float mp[8], lp[8], ap[8];
@@ -334,10 +338,8 @@ __device__ void finish_group(const DecodeParams &P, float *mg, int n_warps, int 
             for (int p = 0; p < 8; ++p) {
                 mp[p] = -CUDART_INF_F, lp[p] = ap[p] = 0.0f;
                 if (p < C) {
-                    const uint32_t src = mx::cluster_map(cm_u32 + g * 68 * 4, p);
-                    mp[p] = mx::cluster_ld_f32(src);
-                    lp[p] = mx::cluster_ld_f32(src + 4);
-                    ap[p] = mx::cluster_ld_f32(src + 16 + d * 4);
+                    const float *src = xb + ((i >> 6) * C + p) * 68;
+                    mp[p] = src[0], lp[p] = src[1], ap[p] = src[4 + d];
                 }
             }
             float mm = mp[0];
@@ -353,7 +355,6 @@ __device__ void finish_group(const DecodeParams &P, float *mg, int n_warps, int 
             emit(g, d, mm, lt, a);
             if (q_rot && active == 1) put_q(g, d);
         }
-        mx::cluster_sync();   // nobody leaves while its totals may still be read
     }
     if (direct) return;
 
@@ -813,8 +814,9 @@ __device__ __forceinline__ uint32_t hsub2(uint32_t a, uint32_t b) {
 struct Q8MmaSmem {
     static constexpr int Q_BYTES = MG * 64 * 4 + MG * 16 * 4 + 2 * MG * 4 + 64;
     static constexpr int PER_WARP = MMA_STAGES * WT_STAGE;
-    static constexpr int MERGE = (Q8_WARPS + 1) * MG * 68 * 4;
-    static constexpr int TOTAL = ((Q_BYTES + 127) & ~127) + WT_STAGE + (Q8_WARPS * PER_WARP > MERGE ? Q8_WARPS * PER_WARP : MERGE);
+    static constexpr int MERGE = Q8_WARPS * MG * 68 * 4;
+    static constexpr int XB = ((Q_BYTES + 127) & ~127) + WT_STAGE + (Q8_WARPS * PER_WARP > MERGE ? Q8_WARPS * PER_WARP : MERGE);
+    static constexpr int TOTAL = XB + MERGE_ROWS * 68 * 4;
 };
 
 template <bool PAGED, bool FUSED>
@@ -846,6 +848,7 @@ decode_q8_mma_kernel(const DecodeParams P) {
     if (FUSED) kend = pos;
     const int active = active_clusters(P, kend - kbeg);
     if (cl >= active) return;
+    if (P.cl_size > 1) mx::cluster_arrive_relaxed();      // waited for before the first store to another CTA's memory
     const int n_splits = active * P.cl_size;
     split_range(kbeg, kend, blockIdx.x, n_splits, ka, kb_);
     const int *table = PAGED ? P.tables + (P.pos_kind == 2 ? (size_t)s * P.n_log : 0) : nullptr;
@@ -1121,14 +1124,14 @@ decode_q8_mma_kernel(const DecodeParams P) {
         }
     }
     __syncthreads();
-    finish_group<MG>(P, mg, Q8_WARPS, s, head0, gc, cl, rank, active, FUSED && P.out != P.qkv_rw ? qf : nullptr, &is_last);
+    finish_group<MG>(P, mg, (float *)(smem_raw + SM::XB), Q8_WARPS, s, head0, gc, cl, rank, active, FUSED && P.out != P.qkv_rw ? qf : nullptr, &is_last);
 }
 
 // ---------------------------------------------------------------------------
 // fp32 cache: warp-autonomous streaming on CUDA cores (a key is 512 B per kv head here, so the
 // 2*G*64 multiply-adds per key fit the FMA pipes under the HBM stream)
 //
-// A CTA of F32_WARPS warps owns one (key split, kv head, sequence); each warp streams its own key
+// A CTA of four warps (eight in calls with few groups) owns one (key split, kv head, sequence); each warp streams its own key
 // sub-range in tiles of 16 keys (K and V rows, 8 KB) through a private two-stage cp.async ring.
 //   scores:  lane = (key, half of the 64 dims); the halves are added with one shuffle per head;
 //            running max per head raised lazily, as in the int8 kernel;
@@ -1137,25 +1140,26 @@ decode_q8_mma_kernel(const DecodeParams P) {
 // bank-conflict free.  Three CTAs are resident per SM.
 // ---------------------------------------------------------------------------
 constexpr int F32_WARPS = 4;
-constexpr int F32_THREADS = F32_WARPS * 32;
+constexpr int F32_WARPS_WIDE = 8;                    // calls that leave most of the SMs empty: see launch_decode
 constexpr int FT_KEYS = 16;                          // keys per warp tile
 constexpr int FT_STAGE = 2 * FT_KEYS * 256;          // K + V rows = 8192 B
 constexpr int FT_STAGES = 2;
 
-template <int G>
+template <int G, int WARPS>
 struct F32Smem {
     static constexpr int GP = (G + 3) & ~3;
     static constexpr int Q_BYTES = G * 64 * 4;
     static constexpr int WBUF = FT_KEYS * GP * 4;
     static constexpr int PER_WARP = FT_STAGES * FT_STAGE + WBUF;
-    static constexpr int MERGE = (F32_WARPS + 1) * G * 68 * 4;
-    static constexpr int TOTAL = ((Q_BYTES + 127) & ~127) + (F32_WARPS * PER_WARP > MERGE ? F32_WARPS * PER_WARP : MERGE);
+    static constexpr int MERGE = WARPS * G * 68 * 4;
+    static constexpr int XB = ((Q_BYTES + 127) & ~127) + (WARPS * PER_WARP > MERGE ? WARPS * PER_WARP : MERGE);
+    static constexpr int TOTAL = XB + MERGE_ROWS * 68 * 4;   // 3 CTAs per SM: 3 * (TOTAL + static + 1 KB) <= 228 KB
 };
 
-template <int G, bool PAGED, bool FUSED>
-__global__ void __launch_bounds__(F32_THREADS, 3)
+template <int G, bool PAGED, bool FUSED, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, WARPS == F32_WARPS_WIDE ? 1 : 3)
 decode_f32_ring_kernel(const DecodeParams P) {
-    using SM = F32Smem<G>;
+    using SM = F32Smem<G, WARPS>;
     constexpr int GP = SM::GP;
     constexpr float LOG2E = 1.4426950408889634f;
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -1180,6 +1184,7 @@ decode_f32_ring_kernel(const DecodeParams P) {
     if (FUSED) kend = pos;
     const int active = active_clusters(P, kend - kbeg);
     if (cl >= active) return;
+    if (P.cl_size > 1) mx::cluster_arrive_relaxed();      // waited for before the first store to another CTA's memory
     const int n_splits = active * P.cl_size;
     split_range(kbeg, kend, blockIdx.x, n_splits, ka, kb_);
     const int *table = PAGED ? P.tables + (P.pos_kind == 2 ? (size_t)s * P.n_log : 0) : nullptr;
@@ -1188,7 +1193,7 @@ decode_f32_ring_kernel(const DecodeParams P) {
 
     // ---- this warp's key sub-range ----
     const int n_keys = kb_ - ka;
-    int per_w = (n_keys + F32_WARPS - 1) / F32_WARPS;
+    int per_w = (n_keys + WARPS - 1) / WARPS;
     per_w = (per_w + FT_KEYS - 1) & ~(FT_KEYS - 1);
     const int wa = min(kb_, ka + warp * per_w), wb = min(kb_, wa + per_w);
     const int n_tiles = (wb - wa + FT_KEYS - 1) / FT_KEYS;
@@ -1260,7 +1265,7 @@ decode_f32_ring_kernel(const DecodeParams P) {
     {
         float cs = 1.0f, sn = 0.0f;
         if (FUSED && P.use_rope) mx::rope_angle(pos, lane, 64, P.theta, cs, sn);
-        for (int g = warp; g < G; g += F32_WARPS) {
+        for (int g = warp; g < G; g += WARPS) {
             const float *qrow = P.qkv + (size_t)s * P.qkv_stride + (head0 + g) * 64;
             float a = 0.0f, b = 0.0f;
             if (g < gc) a = qrow[lane], b = qrow[32 + lane];
@@ -1372,7 +1377,7 @@ decode_f32_ring_kernel(const DecodeParams P) {
     if (P.trigger) mx::pdl_trigger();
 
     // ---- fused step: the new token's own key, by the owning CTA's last warp (the one with the fewest keys) ----
-    if (FUSED && owner && warp == F32_WARPS - 1) {
+    if (FUSED && owner && warp == WARPS - 1) {
 #pragma unroll
         for (int g = 0; g < G; ++g) {
             const float sg = warp_sum_f(fmaf(qf[g * 64 + lane], new_k[lane], qf[g * 64 + 32 + lane] * new_k[lane + 32])) * scale;
@@ -1414,7 +1419,7 @@ decode_f32_ring_kernel(const DecodeParams P) {
         }
     }
     __syncthreads();
-    finish_group<G>(P, mg, F32_WARPS, s, head0, gc, cl, rank, active, FUSED && P.out != P.qkv_rw ? qf : nullptr, &is_last);
+    finish_group<G>(P, mg, (float *)(smem_raw + SM::XB), WARPS, s, head0, gc, cl, rank, active, FUSED && P.out != P.qkv_rw ? qf : nullptr, &is_last);
 }
 
 // Log-sum-exp merge of gathered partial triples: one thread per (row, 4 dims).
@@ -1454,13 +1459,18 @@ int launch_q8_mma(mx230_handle *h, cudaStream_t st, const DecodeParams &P, dim3 
               mx_launch(decode_q8_mma_kernel<PAGED, FUSED>, grid, Q8_THREADS, sm, st, P.cl_size, P.push_regions == nullptr, P));
     return MX230_OK;
 }
+template <int G, bool PAGED, bool FUSED, int WARPS>
+int launch_f32_warps(mx230_handle *h, cudaStream_t st, const DecodeParams &P, dim3 grid) {
+    const size_t sm = (size_t)F32Smem<G, WARPS>::TOTAL;
+    MX_SMEM_ATTR_ONCE(h->device, (decode_f32_ring_kernel<G, PAGED, FUSED, WARPS>), sm);
+    MX_LAUNCH(h, st, MX230_K_DECODE_F32,
+              mx_launch(decode_f32_ring_kernel<G, PAGED, FUSED, WARPS>, grid, WARPS * 32, sm, st, P.cl_size, P.push_regions == nullptr, P));
+    return MX230_OK;
+}
 template <int G, bool PAGED, bool FUSED>
 int launch_f32(mx230_handle *h, cudaStream_t st, const DecodeParams &P, dim3 grid) {
-    const size_t sm = (size_t)F32Smem<G>::TOTAL;
-    MX_SMEM_ATTR_ONCE(h->device, (decode_f32_ring_kernel<G, PAGED, FUSED>), sm);
-    MX_LAUNCH(h, st, MX230_K_DECODE_F32,
-              mx_launch(decode_f32_ring_kernel<G, PAGED, FUSED>, grid, F32_THREADS, sm, st, P.cl_size, P.push_regions == nullptr, P));
-    return MX230_OK;
+    return P.wide ? launch_f32_warps<G, PAGED, FUSED, F32_WARPS_WIDE>(h, st, P, grid)
+                  : launch_f32_warps<G, PAGED, FUSED, F32_WARPS>(h, st, P, grid);
 }
 
 // int8 cache in the reference score mode: the tensor-core kernel serves any group size up to 8 per CTA
@@ -1587,7 +1597,12 @@ int launch_decode(mx230_handle *h, void *stream, DecodeParams P, int n_seq, int 
         P.cl_size = 1, P.cluster_keys = 0;
         P.max_clusters = (int)(n < 1 ? 1 : n > 256 ? 256 : n);
     } else {
-        plan_splits(P, slots, base_ctas, known_keys, mma ? Q8_WARPS * WT_KEYS : F32_WARPS * FT_KEYS);
+        // fp32 cache, a cluster of eight CTAs per group leaves every CTA an SM of its own: eight warps in it take half as many
+        // key tiles in turn (one sequence: 778 keys, 14/2 heads 8.2 -> 7.2 us, 4001 keys, 32/4 heads 15.4 -> 13.6; token of 24
+        // layers at 1000 341 -> 313).  Known sequences beyond one cluster's keys keep three CTAs of four warps per SM.
+        P.wide = !q8 && base_ctas * 8 <= h->sm_count && known_keys <= 4 * 8 * F32_WARPS_WIDE * FT_KEYS;
+        plan_splits(P, P.wide ? h->sm_count : slots, base_ctas, known_keys,
+                    mma ? Q8_WARPS * WT_KEYS : (P.wide ? F32_WARPS_WIDE : F32_WARPS) * FT_KEYS);
     }
     const size_t split_bytes = (size_t)n_seq * P.n_head * 66 * sizeof(float);   // a split's triples
     // Where one CTA per group covers four fifths of the SMs and sequences hold up to 4096 keys, a second split only makes the
