@@ -260,15 +260,26 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
 // hint runs out) instead of re-issuing the poll: a spinning single-lane issuer warp otherwise takes
 // issue slots from the compute warp that shares its scheduler.
 constexpr uint32_t TRY_WAIT_SUSPEND_HINT = 0x989680u;
+// CLUSTER: the phase is completed by other CTAs of the cluster, whose stores are to be seen.
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
     uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity), "r"(TRY_WAIT_SUSPEND_HINT)
-        : "memory");
+    if (CLUSTER)
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity), "r"(TRY_WAIT_SUSPEND_HINT)
+            : "memory");
+    else
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity), "r"(TRY_WAIT_SUSPEND_HINT)
+            : "memory");
     return ok != 0;
 }
 
@@ -276,13 +287,14 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
 // up, everybody else leaves its waits at the next check.  Returns false on abort.
 // The bound is counted on the SM's own cycle counter (cheap to read; reading the global
 // nanosecond timer on every contended wait costs far more than the wait itself).
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag,
                                           int *status) {
-    if (mbar_try_wait(bar, parity)) return true;
+    if (mbar_try_wait<CLUSTER>(bar, parity)) return true;
     const long long t0 = clock64();
     unsigned polls = 0;
     while (true) {
-        if (mbar_try_wait(bar, parity)) return true;
+        if (mbar_try_wait<CLUSTER>(bar, parity)) return true;
         // A poll that finds the phase incomplete may have been parked by the hardware for up to the suspend hint,
         // so the abort flag and the clock are first looked at after 8 polls, then after 16, 32, ... (every 256 from
         // there on): early for a wait that is going to run out, rare for the short waits of the steady state, whose
@@ -620,9 +632,10 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 // ---- RoPE (HF rotate_half): the pair (d, d + 32) of a 64-value head at position `pos` ----
 // precise powf / sincosf: the reference's CPU path (03-llm-engine/src/cpu.rs:25-37); its GPU kernel uses the fast
 // intrinsics, which lose accuracy at large angles
+__device__ __forceinline__ float rope_freq(int d, int head_dim, float theta) { return powf(theta, -2.0f * (float)d / (float)head_dim); }
+__device__ __forceinline__ void rope_angle(int pos, float freq, float &cs, float &sn) { sincosf((float)pos * freq, &sn, &cs); }
 __device__ __forceinline__ void rope_angle(int pos, int d, int head_dim, float theta, float &cs, float &sn) {
-    const float freq = powf(theta, -2.0f * (float)d / (float)head_dim);
-    sincosf((float)pos * freq, &sn, &cs);
+    rope_angle(pos, rope_freq(d, head_dim, theta), cs, sn);
 }
 // one rounding order for every kernel that rotates, so that they all leave the same bits
 __device__ __forceinline__ void rope_pair(float &x1, float &x2, float cs, float sn) {
@@ -667,7 +680,6 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 __device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 // ---- thread-block clusters: barrier and loads from the shared memory of the cluster's other CTAs ----
-__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_arrive_release() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_sync() {
@@ -678,16 +690,15 @@ __device__ __forceinline__ uint32_t cluster_map(uint32_t saddr, int rank) {
     asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
     return r;
 }
-__device__ __forceinline__ void cluster_st_f32(uint32_t addr, float v) {
-    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+// Four floats into the shared memory of a CTA of the cluster, counted as 16 bytes of the current phase of an mbarrier of that
+// CTA (both addresses as cluster_map gives them): nobody waits for the stores but who reads them.
+__device__ __forceinline__ void cluster_st_async(uint32_t addr, uint32_t bar, float a, float b, float c, float d) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(addr),
+                 "f"(a), "f"(b), "f"(c), "f"(d), "r"(bar)
+                 : "memory");
 }
 __device__ __forceinline__ void cluster_red_max(uint32_t addr, int v) {
     asm volatile("red.relaxed.cluster.shared::cluster.max.s32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
-}
-__device__ __forceinline__ float cluster_ld_f32(uint32_t addr) {
-    float v;
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
-    return v;
 }
 
 // ---- {value, step} words of the split-KV exchange: 8-byte accesses are single-copy atomic, so a reader that

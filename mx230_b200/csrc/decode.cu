@@ -61,6 +61,7 @@ struct DecodeParams {
     // step after step: 116 us with the trigger at the top, 105 here, 100 without; 16 fp32 sequences of 1500 keys 23.1 / 22.8 /
     // 19.9; one int8 sequence in a 24-layer token, 64 CTAs: 259 / 245 / 272).
     int trigger;
+    int *status;         // where a wait within a cluster that ran out is recorded
     int wide;            // fp32 cache: CTAs of F32_WARPS_WIDE warps
     int bs_shift;        // log2(bs) when bs is a power of two, else -1
     // fused step (RoPE and KV write of the new token inside the attention kernel): keys [0, pos) come from the cache,
@@ -279,78 +280,107 @@ __device__ void merge_and_store(const DecodeParams &P, int s, int head0, int gc,
 }
 
 // Merge of a CTA's warps, then of its cluster's CTAs, then (several clusters) of the clusters through the workspace.
-// mg: shared memory, [n_warps][G][68] = m (log2 domain), l, sum of p * V offset, pad, acc[64] per warp and head.
-// xb: shared memory of its own, MERGE_ROWS rows of 68, for the cluster: rank r finishes the heads g = r (mod cl_size), and
-// every CTA pushes its totals of such a head into rank r's xb, so that the merge of up to eight CTAs costs one cluster
-// barrier behind stores that nobody waits for, instead of a fence, an atomic and a re-read of global memory (int8, one
-// sequence of 2001 keys, 2 K/V heads: 16 splits merged through the workspace 8.2 us, one cluster of 8 CTAs 5.3 us with the
-// totals pulled between two barriers).  The caller has arrived on the cluster barrier once (cl_size > 1).
+// mg: shared memory, [NW][G][68] = m (log2 domain), l, sum of p * V offset, pad, acc[64] per warp and head.
+// X: shared memory of its own for the cluster: rank r finishes the heads g = r (mod cl_size), and every CTA pushes its totals of
+// such a head into rank r's rows with asynchronous stores, which complete the one phase of rank r's barrier.  What bounds it is
+// latency: token of 24 layers over 2001 int8 keys (two clusters of eight CTAs per layer), us: splits merged through the
+// workspace 340, totals pulled between two cluster barriers 272, pushed in front of one 263, this and the same in the
+// projections 254.
 // q_rot (fused step): rotated q, [G][64] in shared memory; it replaces the raw q in qkv once every CTA of the group
 // has read that.  Null where out is the qkv row itself: the attention row then takes q's place.
 constexpr int MERGE_ROWS = 16;   // ceil(8 / C) heads from each of C CTAs, C <= 8: at most 14
-template <int G>
-__device__ void finish_group(const DecodeParams &P, float *mg, float *xb, int n_warps, int s, int head0, int gc, int cl, int rank,
+struct ClusterMerge {
+    float rows[MERGE_ROWS * 68];
+    unsigned long long bar;
+    int aborted;
+};
+__device__ __forceinline__ int merge_heads(int gc, int rank, int C) { return gc > rank ? (gc - rank + C - 1) / C : 0; }
+// Before the first push: called by the whole CTA, of every CTA of the cluster
+__device__ __forceinline__ void merge_open(ClusterMerge &X, int gc, int rank, int C) {
+    if (C == 1) return;
+    if (threadIdx.x == 0) {
+        X.aborted = 0;
+        const uint32_t bar = mx::smem_u32(&X.bar);
+        mx::mbar_init(bar, 1);
+        mx::mbar_fence_init();
+        mx::mbar_expect_tx(bar, merge_heads(gc, rank, C) * C * 68 * 4);
+    }
+    mx::cluster_arrive_release();   // waited for before the first push
+}
+template <int G, int NW>
+__device__ void finish_group(const DecodeParams &P, const float *mg, ClusterMerge &X, int s, int head0, int gc, int cl, int rank,
                              int active, const float *q_rot, int *is_last) {
     const int tid = threadIdx.x, nt = blockDim.x, C = P.cl_size;
     const bool direct = active == 1 && P.fin_acc == nullptr;
-    auto emit = [&](int g, int d, float m2, float l, float a) {
+    auto emit = [&](int g, int d, float m2, float l, const float4 &a) {
         const int h = head0 + g;
         if (direct) {
-            P.out[(size_t)s * P.out_stride + h * 64 + d] = a / l;
+            *(float4 *)(P.out + (size_t)s * P.out_stride + h * 64 + d) = make_float4(a.x / l, a.y / l, a.z / l, a.w / l);
         } else {   // partial triples carry the max in natural-log units, as the split-KV interface states
             const size_t pi = ((size_t)s * P.n_head + h) * active + cl;
-            P.ws_acc[pi * 64 + d] = a;
+            *(float4 *)(P.ws_acc + pi * 64 + d) = a;
             if (d == 0) {
                 P.ws_m[pi] = m2 * 0.6931471805599453f;
                 P.ws_l[pi] = l;
             }
         }
     };
-    auto put_q = [&](int g, int d) { P.qkv_rw[(size_t)s * P.qkv_stride + (head0 + g) * 64 + d] = q_rot[g * 64 + d]; };
-    if (C > 1) mx::cluster_wait();   // every CTA of the cluster runs
-    const uint32_t xb_u32 = mx::smem_u32(xb);
-    for (int i = tid; i < gc * 64; i += nt) {
-        const int g = i >> 6, d = i & 63;
-        float mm = -CUDART_INF_F;
-        for (int w = 0; w < n_warps; ++w) mm = fmaxf(mm, mg[(w * G + g) * 68]);
-        float lt = 0.0f, a = 0.0f;
-        for (int w = 0; w < n_warps; ++w) {
-            const float *src = mg + (w * G + g) * 68;
-            const float wgt = (src[0] == -CUDART_INF_F) ? 0.0f : mx::ex2(src[0] - mm);
-            lt += src[1] * wgt;
-            a += (src[4 + d] + src[2]) * wgt;  // V's affine offset sum_j p_j vb_j folds into every dim
+    auto put_q = [&](int g, int d) {
+        *(float4 *)(P.qkv_rw + (size_t)s * P.qkv_stride + (head0 + g) * 64 + d) = *(const float4 *)(q_rot + g * 64 + d);
+    };
+    if (C > 1) mx::cluster_wait();   // every CTA of the cluster runs and has its barrier set up
+    for (int i = tid; i < gc * 16; i += nt) {   // thread: four dims of a head
+        const int g = i >> 4, d = (i & 15) * 4;
+        float4 hd[NW];   // m, l, sum of p * V offset
+#pragma unroll
+        for (int w = 0; w < NW; ++w) hd[w] = *(const float4 *)(mg + (w * G + g) * 68);
+        float mm = hd[0].x;
+#pragma unroll
+        for (int w = 1; w < NW; ++w) mm = fmaxf(mm, hd[w].x);
+        float lt = 0.0f;
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int w = 0; w < NW; ++w) {
+            const float4 v = *(const float4 *)(mg + (w * G + g) * 68 + 4 + d);
+            const float wgt = (hd[w].x == -CUDART_INF_F) ? 0.0f : mx::ex2(hd[w].x - mm);
+            lt += hd[w].y * wgt;
+            // V's affine offset sum_j p_j vb_j folds into every dim
+            a.x += (v.x + hd[w].z) * wgt, a.y += (v.y + hd[w].z) * wgt, a.z += (v.z + hd[w].z) * wgt, a.w += (v.w + hd[w].z) * wgt;
         }
         if (C == 1) {
             emit(g, d, mm, lt, a);
             if (q_rot && active == 1) put_q(g, d);
         } else {
-            const uint32_t dst = mx::cluster_map(xb_u32 + (g / C * C + rank) * 68 * 4, g % C);
-            mx::cluster_st_f32(dst + 16 + d * 4, a);
-            if (d == 0) mx::cluster_st_f32(dst, mm), mx::cluster_st_f32(dst + 4, lt);
+            const int r = g % C;
+            const uint32_t dst = mx::cluster_map(mx::smem_u32(X.rows + (g / C * C + rank) * 68), r);
+            const uint32_t bar = mx::cluster_map(mx::smem_u32(&X.bar), r);
+            mx::cluster_st_async(dst + 16 + d * 4, bar, a.x, a.y, a.z, a.w);
+            if (d == 0) mx::cluster_st_async(dst, bar, mm, lt, 0.0f, 0.0f);
         }
     }
-    if (C > 1) {
-        mx::cluster_sync();
-        for (int i = tid; (i >> 6) * C + rank < gc; i += nt) {
-            const int g = (i >> 6) * C + rank, d = i & 63;
-            float mp[8], lp[8], ap[8];
+    if (C > 1 && merge_heads(gc, rank, C) * 16 > tid) {
+        const bool ok = mx::mbar_wait<true>(mx::smem_u32(&X.bar), 0, &X.aborted, P.status);
+        for (int i = tid; ok && (i >> 4) * C + rank < gc; i += nt) {   // (nothing is written after a wait that ran out)
+            const int g = (i >> 4) * C + rank, d = (i & 15) * 4;
+            float4 hd[8], ap[8];
 #pragma unroll
             for (int p = 0; p < 8; ++p) {
-                mp[p] = -CUDART_INF_F, lp[p] = ap[p] = 0.0f;
+                hd[p] = make_float4(-CUDART_INF_F, 0.f, 0.f, 0.f), ap[p] = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (p < C) {
-                    const float *src = xb + ((i >> 6) * C + p) * 68;
-                    mp[p] = src[0], lp[p] = src[1], ap[p] = src[4 + d];
+                    const float *src = X.rows + ((i >> 4) * C + p) * 68;
+                    hd[p] = *(const float4 *)src, ap[p] = *(const float4 *)(src + 4 + d);
                 }
             }
-            float mm = mp[0];
+            float mm = hd[0].x;
 #pragma unroll
-            for (int p = 1; p < 8; ++p) mm = fmaxf(mm, mp[p]);
-            float lt = 0.0f, a = 0.0f;
+            for (int p = 1; p < 8; ++p) mm = fmaxf(mm, hd[p].x);
+            float lt = 0.0f;
+            float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
             for (int p = 0; p < 8; ++p) {
-                const float wgt = (mp[p] == -CUDART_INF_F) ? 0.0f : mx::ex2(mp[p] - mm);
-                lt += lp[p] * wgt;
-                a += ap[p] * wgt;
+                const float wgt = (hd[p].x == -CUDART_INF_F) ? 0.0f : mx::ex2(hd[p].x - mm);
+                lt += hd[p].y * wgt;
+                a.x += ap[p].x * wgt, a.y += ap[p].y * wgt, a.z += ap[p].z * wgt, a.w += ap[p].w * wgt;
             }
             emit(g, d, mm, lt, a);
             if (q_rot && active == 1) put_q(g, d);
@@ -369,7 +399,7 @@ __device__ void finish_group(const DecodeParams &P, float *mg, float *xb, int n_
     if (!*is_last) return;
     __threadfence();
     if (q_rot && active > 1)
-        for (int i = tid; i < gc * 64; i += nt) put_q(i >> 6, i & 63);
+        for (int i = tid; i < gc * 16; i += nt) put_q(i >> 4, (i & 15) * 4);
     merge_and_store<G>(P, s, head0, gc, active, nt);
 }
 
@@ -815,8 +845,7 @@ struct Q8MmaSmem {
     static constexpr int Q_BYTES = MG * 64 * 4 + MG * 16 * 4 + 2 * MG * 4 + 64;
     static constexpr int PER_WARP = MMA_STAGES * WT_STAGE;
     static constexpr int MERGE = Q8_WARPS * MG * 68 * 4;
-    static constexpr int XB = ((Q_BYTES + 127) & ~127) + WT_STAGE + (Q8_WARPS * PER_WARP > MERGE ? Q8_WARPS * PER_WARP : MERGE);
-    static constexpr int TOTAL = XB + MERGE_ROWS * 68 * 4;
+    static constexpr int TOTAL = ((Q_BYTES + 127) & ~127) + WT_STAGE + (Q8_WARPS * PER_WARP > MERGE ? Q8_WARPS * PER_WARP : MERGE);
 };
 
 template <bool PAGED, bool FUSED>
@@ -830,6 +859,7 @@ decode_q8_mma_kernel(const DecodeParams P) {
     float *hq = (float *)(qq + MG * 16);                  // [2][8]: score scale (log2 domain), sum of q codes
     unsigned char *extra = smem_raw + ((SM::Q_BYTES + 127) & ~127);   // fused step: the new token as a one-key tile
     unsigned char *warp_base = extra + WT_STAGE;
+    __shared__ __align__(16) ClusterMerge X;
     __shared__ int is_last;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -841,14 +871,21 @@ decode_q8_mma_kernel(const DecodeParams P) {
     const int nkv = P.n_kv_head, kvd = nkv * 64;
     const int cl = blockIdx.x / P.cl_size, rank = blockIdx.x - cl * P.cl_size;
 
+    const float freq = FUSED ? mx::rope_freq(lane, 64, P.theta) : 0.0f;
     if (P.push_regions == nullptr) mx::pdl_wait();   // (a split-KV step, whose CTAs wait for other ranks, is launched plainly)
+    // q: requested before the position, whose chain of dependent loads (position, table, first tile) it then runs beside
+    float qa_raw = 0.0f, qb_raw = 0.0f;   // warp = head (Q8_WARPS == MG)
+    if (warp < gc) {
+        const float *qrow = P.qkv + (size_t)s * P.qkv_stride + (head0 + warp) * 64;
+        qa_raw = qrow[lane], qb_raw = qrow[32 + lane];
+    }
     int kbeg, kend, ka, kb_;
     key_range(P, s, kbeg, kend);
     const int pos = kend - 1;                             // fused step: the new token's position
     if (FUSED) kend = pos;
     const int active = active_clusters(P, kend - kbeg);
     if (cl >= active) return;
-    if (P.cl_size > 1) mx::cluster_arrive_relaxed();      // waited for before the first store to another CTA's memory
+    merge_open(X, gc, rank, P.cl_size);
     const int n_splits = active * P.cl_size;
     split_range(kbeg, kend, blockIdx.x, n_splits, ka, kb_);
     const int *table = PAGED ? P.tables + (P.pos_kind == 2 ? (size_t)s * P.n_log : 0) : nullptr;
@@ -956,13 +993,11 @@ decode_q8_mma_kernel(const DecodeParams P) {
     const bool owner = FUSED && (int)blockIdx.x == n_splits - 1;   // the CTA that takes the new token's own key
     {
         const int g = warp;  // Q8_WARPS == MG
-        const float *qrow = P.qkv + (size_t)s * P.qkv_stride + (head0 + g) * 64;
-        float a = 0.0f, b = 0.0f;
-        if (g < gc) a = qrow[lane], b = qrow[32 + lane];
+        float a = qa_raw, b = qb_raw;
         if (FUSED) {
             float cs = 1.0f, sn = 0.0f;
             if (P.use_rope) {
-                mx::rope_angle(pos, lane, 64, P.theta, cs, sn);
+                mx::rope_angle(pos, freq, cs, sn);
                 mx::rope_pair(a, b, cs, sn);
             }
             qf[g * 64 + lane] = a, qf[g * 64 + 32 + lane] = b;
@@ -1111,20 +1146,17 @@ decode_q8_mma_kernel(const DecodeParams P) {
     float *mg = (float *)warp_base;  // [warp][g][68]: m (log2 domain), l, beta sum, pad, acc[64]
     {
         float *dst = mg + (warp * MG + g) * 68;
-        if (j == 0) {
-            dst[0] = m_run;
-            dst[1] = l_thr;
-            dst[2] = b_thr;
-        }
+        if (j == 0) *(float4 *)dst = make_float4(m_run, l_thr, b_thr, 0.0f);
         // tile t, columns 2j, 2j+1 <-> dims 16j + t, 16j + 8 + t
 #pragma unroll
-        for (int t = 0; t < 8; ++t) {
-            dst[4 + 16 * j + t] = oacc[t][0] + oacc[t][2];
-            dst[4 + 16 * j + 8 + t] = oacc[t][1] + oacc[t][3];
+        for (int u = 0; u < 4; ++u) {
+            const int t = (u & 1) * 4, c = u >> 1;
+            *(float4 *)(dst + 4 + 16 * j + 4 * u) = make_float4(oacc[t][c] + oacc[t][c + 2], oacc[t + 1][c] + oacc[t + 1][c + 2],
+                                                                oacc[t + 2][c] + oacc[t + 2][c + 2], oacc[t + 3][c] + oacc[t + 3][c + 2]);
         }
     }
     __syncthreads();
-    finish_group<MG>(P, mg, (float *)(smem_raw + SM::XB), Q8_WARPS, s, head0, gc, cl, rank, active, FUSED && P.out != P.qkv_rw ? qf : nullptr, &is_last);
+    finish_group<MG, Q8_WARPS>(P, mg, X, s, head0, gc, cl, rank, active, FUSED && P.out != P.qkv_rw ? qf : nullptr, &is_last);
 }
 
 // ---------------------------------------------------------------------------
@@ -1152,8 +1184,8 @@ struct F32Smem {
     static constexpr int WBUF = FT_KEYS * GP * 4;
     static constexpr int PER_WARP = FT_STAGES * FT_STAGE + WBUF;
     static constexpr int MERGE = WARPS * G * 68 * 4;
-    static constexpr int XB = ((Q_BYTES + 127) & ~127) + (WARPS * PER_WARP > MERGE ? WARPS * PER_WARP : MERGE);
-    static constexpr int TOTAL = XB + MERGE_ROWS * 68 * 4;   // 3 CTAs per SM: 3 * (TOTAL + static + 1 KB) <= 228 KB
+    // 3 CTAs of four warps per SM: 3 * (TOTAL + 5 KB static + 1 KB) <= 228 KB
+    static constexpr int TOTAL = ((Q_BYTES + 127) & ~127) + (WARPS * PER_WARP > MERGE ? WARPS * PER_WARP : MERGE);
 };
 
 template <int G, bool PAGED, bool FUSED, int WARPS>
@@ -1166,6 +1198,7 @@ decode_f32_ring_kernel(const DecodeParams P) {
     float *qf = (float *)smem_raw;                        // [G][64]
     unsigned char *warp_base = smem_raw + ((SM::Q_BYTES + 127) & ~127);
     __shared__ float new_k[64], new_v[64];                // fused step: the new token's rows (owning CTA)
+    __shared__ __align__(16) ClusterMerge X;
     __shared__ int is_last;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1177,14 +1210,27 @@ decode_f32_ring_kernel(const DecodeParams P) {
     const int nkv = P.n_kv_head, kvd = nkv * 64;
     const int cl = blockIdx.x / P.cl_size, rank = blockIdx.x - cl * P.cl_size;
 
+    const float freq = FUSED && P.use_rope ? mx::rope_freq(lane, 64, P.theta) : 0.0f;
     if (P.push_regions == nullptr) mx::pdl_wait();   // (a split-KV step, whose CTAs wait for other ranks, is launched plainly)
+    // q: requested before the position, whose chain of dependent loads (position, table, first tile) it then runs beside
+    constexpr int QH = (G + WARPS - 1) / WARPS;   // heads of a warp: warp, warp + WARPS, ...
+    float qa_raw[QH], qb_raw[QH];
+#pragma unroll
+    for (int i = 0; i < QH; ++i) {
+        const int g = warp + i * WARPS;
+        qa_raw[i] = qb_raw[i] = 0.0f;
+        if (g < gc) {
+            const float *qrow = P.qkv + (size_t)s * P.qkv_stride + (head0 + g) * 64;
+            qa_raw[i] = qrow[lane], qb_raw[i] = qrow[32 + lane];
+        }
+    }
     int kbeg, kend, ka, kb_;
     key_range(P, s, kbeg, kend);
     const int pos = kend - 1;                             // fused step: the new token's position
     if (FUSED) kend = pos;
     const int active = active_clusters(P, kend - kbeg);
     if (cl >= active) return;
-    if (P.cl_size > 1) mx::cluster_arrive_relaxed();      // waited for before the first store to another CTA's memory
+    merge_open(X, gc, rank, P.cl_size);
     const int n_splits = active * P.cl_size;
     split_range(kbeg, kend, blockIdx.x, n_splits, ka, kb_);
     const int *table = PAGED ? P.tables + (P.pos_kind == 2 ? (size_t)s * P.n_log : 0) : nullptr;
@@ -1264,11 +1310,12 @@ decode_f32_ring_kernel(const DecodeParams P) {
     const bool owner = FUSED && (int)blockIdx.x == n_splits - 1;   // the CTA that takes the new token's own key
     {
         float cs = 1.0f, sn = 0.0f;
-        if (FUSED && P.use_rope) mx::rope_angle(pos, lane, 64, P.theta, cs, sn);
-        for (int g = warp; g < G; g += WARPS) {
-            const float *qrow = P.qkv + (size_t)s * P.qkv_stride + (head0 + g) * 64;
-            float a = 0.0f, b = 0.0f;
-            if (g < gc) a = qrow[lane], b = qrow[32 + lane];
+        if (FUSED && P.use_rope) mx::rope_angle(pos, freq, cs, sn);
+#pragma unroll
+        for (int i = 0; i < QH; ++i) {
+            const int g = warp + i * WARPS;
+            if (g >= G) break;
+            float a = qa_raw[i], b = qb_raw[i];
             if (FUSED && P.use_rope) mx::rope_pair(a, b, cs, sn);
             qf[g * 64 + lane] = a, qf[g * 64 + 32 + lane] = b;
         }
@@ -1408,18 +1455,14 @@ decode_f32_ring_kernel(const DecodeParams P) {
 #pragma unroll
     for (int g = 0; g < G; ++g) {
         float *dst = mg + (warp * G + g) * 68;
-        if (lane == 0) {
-            dst[0] = m_run[g];
-            dst[1] = l_thr[g];
-            dst[2] = 0.0f;
-        }
+        if (lane == 0) *(float4 *)dst = make_float4(m_run[g], l_thr[g], 0.0f, 0.0f);
         if (lane < 8) {
             *(float4 *)(dst + 4 + lane * 8) = make_float4(acc[g][0], acc[g][1], acc[g][2], acc[g][3]);
             *(float4 *)(dst + 8 + lane * 8) = make_float4(acc[g][4], acc[g][5], acc[g][6], acc[g][7]);
         }
     }
     __syncthreads();
-    finish_group<G>(P, mg, (float *)(smem_raw + SM::XB), WARPS, s, head0, gc, cl, rank, active, FUSED && P.out != P.qkv_rw ? qf : nullptr, &is_last);
+    finish_group<G, WARPS>(P, mg, X, s, head0, gc, cl, rank, active, FUSED && P.out != P.qkv_rw ? qf : nullptr, &is_last);
 }
 
 // Log-sum-exp merge of gathered partial triples: one thread per (row, 4 dims).
@@ -1624,6 +1667,7 @@ int launch_decode(mx230_handle *h, void *stream, DecodeParams P, int n_seq, int 
         P.ws_l = P.ws_m + rows;
     }
     P.counters = h->counters;
+    P.status = h->status_dev;
 
     mx230_device_guard guard(h->device);
     dim3 grid(P.cl_size * P.max_clusters, gy, n_seq);

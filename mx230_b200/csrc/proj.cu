@@ -57,6 +57,7 @@ struct GemvParams {
     int slots, ctas, cl_size;       // slices per CTA, CTAs per column block; cl_size = ctas, or 1: merge through the workspace
     float *partials;                // [n_slices][n_out]
     unsigned *counters;      // one per column block, self-resetting
+    int *status;             // where a wait within a cluster that ran out is recorded
     QkvEpilogue e;
 };
 
@@ -116,10 +117,10 @@ gemv_heads_kernel(const GemvParams P) {
     constexpr int BATCH = 4;                        // passes whose loads are issued together
     constexpr int ELT = I8 ? 4 : (int)sizeof(WT);   // bytes of a stored weight word
     constexpr int IN_PER_ROW = I8 ? 4 : 1;          // input rows in one stored row
-    __shared__ float red[PJ_SLOTS][PJ_ROWLANES][PJ_COLS];
-    __shared__ float parts[PJ_CLUSTER * PJ_SLOTS][PJ_COLS];   // first CTA of the cluster: the sums of every slice
-    __shared__ float val[PJ_COLS];
-    __shared__ int is_last;
+    __shared__ __align__(16) float red[PJ_SLOTS][PJ_ROWLANES][PJ_COLS];
+    __shared__ __align__(16) float parts[PJ_CLUSTER * PJ_SLOTS][PJ_COLS];   // first CTA of the cluster: the sums of every slice
+    __shared__ __align__(8) unsigned long long parts_bar;                   // completed by their bytes
+    __shared__ int is_last, aborted;
     extern __shared__ float xs[];                   // int8: the CTA's part of x as packed codes, then group scales
     const int tid = threadIdx.x, nt = blockDim.x, C = P.cl_size;
     const int blk = blockIdx.x / P.ctas, rank = blockIdx.x - blk * P.ctas;
@@ -132,13 +133,25 @@ gemv_heads_kernel(const GemvParams P) {
     const int r1 = min(P.n_in, (slice + 1) * P.rows_per_slice) / IN_PER_ROW;
 
     mx::pdl_trigger();
-    if (C > 1) mx::cluster_arrive_relaxed();        // waited for before the first access to another CTA's memory
+    const uint32_t bar = mx::smem_u32(&parts_bar);
+    if (C > 1) {
+        if (tid == 0) {
+            aborted = 0;
+            mx::mbar_init(bar, 1);
+            mx::mbar_fence_init();
+            if (rank == 0) mx::mbar_expect_tx(bar, P.n_slices * PJ_COLS * 4);
+        }
+        mx::cluster_arrive_release();               // waited for before the first store to another CTA's memory
+    }
     // start of the CTA's rows into L2 under the previous kernel's tail
     for (int r = c0 / IN_PER_ROW + tid, n = 0; r < c1 / IN_PER_ROW && n < 2; r += nt, ++n) {
         const char *line = (const char *)P.w + ((size_t)r * P.n_out + col0) * ELT;
         mx::prefetch_l2(line);
         if (ELT == 4 && col0 + 32 < P.n_out) mx::prefetch_l2(line + 128);
     }
+    const QkvEpilogue &E = P.e;
+    const bool finishes = (rank == 0 || C == 1) && tid < 32;   // the warp that finishes the block: lane l has columns l and l + 32
+    const float freq = finishes && E.enabled ? mx::rope_freq(tid, 64, E.theta) : 0.0f;
     mx::pdl_wait();
 
     const int cq = tl % TPR, rl = tl / TPR;
@@ -161,20 +174,22 @@ gemv_heads_kernel(const GemvParams P) {
     };
     load(r0 + rl);
     // what the epilogue needs, under the weight loads
-    const QkvEpilogue &E = P.e;
     const bool is_v = blk >= E.n_head + E.n_kv_head;
-    float bias = 0.0f, scale_o = 1.0f, y_old = 0.0f, cs = 1.0f, sn = 0.0f;
+    float bias[2] = {0.0f, 0.0f}, scale_o[2] = {1.0f, 1.0f}, y_old[2] = {0.0f, 0.0f};
     int pos = 0;
     size_t row = 0;
-    if ((rank == 0 || C == 1) && tid < PJ_COLS && col0 + tid < P.n_out) {
-        const int o = col0 + tid;
-        if (P.b) bias = P.b[o];
-        if (I8) scale_o = P.scales[o];
-        if (P.accum) y_old = P.y[o];
-        if (E.enabled && tid < 32) {
+    if (finishes) {
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int o = col0 + tid + 32 * k;
+            if (o >= P.n_out) break;
+            if (P.b) bias[k] = P.b[o];
+            if (I8) scale_o[k] = P.scales[o];
+            if (P.accum) y_old[k] = P.y[o];
+        }
+        if (E.enabled) {
             pos = E.pos_dev ? *E.pos_dev : E.pos;
             row = E.bt && blk >= E.n_head ? (size_t)(E.bt[pos / E.bs] * E.bs + pos % E.bs) : (size_t)pos;
-            if (!is_v) mx::rope_angle(pos, tid, 64, E.theta, cs, sn);
         }
     }
     if constexpr (I8) {
@@ -219,76 +234,83 @@ gemv_heads_kernel(const GemvParams P) {
     for (int c = 0; c < CPT; c += 4) *(float4 *)&red[slot][rl][CPT * cq + c] = make_float4(acc[c], acc[c + 1], acc[c + 2], acc[c + 3]);
     __syncthreads();
     // ---- lanes -> slices -> block, each in index order ----
-    if (C > 1) mx::cluster_wait();   // every CTA of the cluster runs
-    for (int i = tid; i < P.slots * PJ_COLS; i += nt) {
-        const int sl = i / PJ_COLS, c = i - sl * PJ_COLS, g = rank * P.slots + sl;
+    if (C > 1) mx::cluster_wait();   // every CTA of the cluster runs and has its barrier set up
+    for (int i = tid; i < P.slots * (PJ_COLS / 4); i += nt) {
+        const int sl = i / (PJ_COLS / 4), c = (i - sl * (PJ_COLS / 4)) * 4, g = rank * P.slots + sl;
         if (g >= P.n_slices) break;
-        float sum = 0.0f;
+        float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int r = 0; r < PJ_ROWLANES; ++r) sum += red[sl][r][c];
-        if (C > 1) mx::cluster_st_f32(mx::cluster_map(mx::smem_u32(&parts[g][c]), 0), sum);
-        else if (P.ctas == 1) parts[g][c] = sum;
-        else if (col0 + c < P.n_out) P.partials[(size_t)g * P.n_out + col0 + c] = sum;
+        for (int r = 0; r < PJ_ROWLANES; ++r) {
+            const float4 v = *(const float4 *)&red[sl][r][c];
+            sum.x += v.x, sum.y += v.y, sum.z += v.z, sum.w += v.w;
+        }
+        // (asynchronous stores that complete the first CTA's barrier: the cluster barrier behind plain ones took 1500 cycles of
+        // the 5000 of a launch)
+        if (C > 1) mx::cluster_st_async(mx::cluster_map(mx::smem_u32(&parts[g][c]), 0), mx::cluster_map(bar, 0), sum.x, sum.y, sum.z, sum.w);
+        else if (P.ctas == 1) *(float4 *)&parts[g][c] = sum;
+        else if (col0 + c < P.n_out) *(float4 *)(P.partials + (size_t)g * P.n_out + col0 + c) = sum;   // (n_out % 4 == 0)
     }
     if (C > 1) {
-        mx::cluster_sync();
-        if (rank != 0) return;
+        if (!finishes) return;
     } else if (P.ctas > 1) {
         __threadfence();
         __syncthreads();
         if (tid == 0) is_last = atomicInc(&P.counters[blk], P.ctas - 1) == (unsigned)(P.ctas - 1);
         __syncthreads();
-        if (!is_last) return;
+        if (!is_last || !finishes) return;
         __threadfence();
     } else {
         __syncthreads();
+        if (!finishes) return;
     }
-    // ---- epilogue on the 64 finished sums of this column block ----
-    if (tid < PJ_COLS) {
+    // ---- epilogue on the 64 finished sums of this column block: one warp ----
+    float cs = 1.0f, sn = 0.0f;
+    if (E.enabled && !is_v) mx::rope_angle(pos, freq, cs, sn);   // (while the other CTAs' sums are on their way)
+    if (C > 1 && !__all_sync(0xFFFFFFFFu, mx::mbar_wait<true>(bar, 0, &aborted, P.status))) return;
+    float v[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const int c = tid + 32 * k;
         float sum = 0.0f;
         if (P.n_slices == 1) {
-            sum = parts[0][tid];
+            sum = parts[0][c];
         } else if (C == 1 && P.ctas > 1) {
-            if (col0 + tid < P.n_out)
-                for (int g = 0; g < P.n_slices; ++g) sum += __ldcg(P.partials + (size_t)g * P.n_out + col0 + tid);
+            if (col0 + c < P.n_out)
+                for (int g = 0; g < P.n_slices; ++g) sum += __ldcg(P.partials + (size_t)g * P.n_out + col0 + c);
         } else {
 #pragma unroll 8
-            for (int g = 0; g < P.n_slices; ++g) sum += parts[g][tid];
+            for (int g = 0; g < P.n_slices; ++g) sum += parts[g][c];
         }
-        val[tid] = (I8 ? sum * scale_o : sum) + bias;
+        v[k] = (I8 ? sum * scale_o[k] : sum) + bias[k];
     }
-    __syncthreads();
     if (!E.enabled) {
-        if (tid < PJ_COLS && col0 + tid < P.n_out) P.y[col0 + tid] = P.accum ? y_old + val[tid] : val[tid];
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+            if (col0 + tid + 32 * k < P.n_out) P.y[col0 + tid + 32 * k] = P.accum ? y_old[k] + v[k] : v[k];
         return;
     }
-    // qkv step: this block is head `hb` of the row [Q heads | K heads | V heads]
-    const int hb = blk;
-    if (tid < 32) {   // one warp: lane l owns the rotation pair (l, l + 32), then elements 2l, 2l+1
-        if (!is_v) mx::rope_pair(val[tid], val[tid + 32], cs, sn);
-        __syncwarp();
-        const float2 x2 = make_float2(val[2 * tid], val[2 * tid + 1]);
-        *(float2 *)(P.y + (size_t)hb * 64 + 2 * tid) = x2;
-        if (hb >= E.n_head) {   // K or V head: the cache row of this position
-            const int kvh = is_v ? hb - E.n_head - E.n_kv_head : hb - E.n_head;
-            const int kvd = E.n_kv_head * 64;
-            if (E.kq == nullptr) {
-                float *dst = (is_v ? E.vcache : E.kcache) + row * kvd + kvh * 64;
-                *(float2 *)(dst + 2 * tid) = x2;
-            } else {
-                int8_t *dst = (is_v ? E.vq : E.kq) + row * kvd + kvh * 64;
-                float *sc = is_v ? E.vs : E.ks, *be = is_v ? E.vb : E.kb;
-                const size_t sd = row * E.n_kv_head + kvh;
-                int c0, c1;
-                float scale, beta;
-                mx::quant_head_row(x2.x, x2.y, be != nullptr, c0, c1, scale, beta);
-                if (tid == 0) {
-                    sc[sd] = scale;
-                    if (be != nullptr) be[sd] = beta;
-                }
-                *(unsigned short *)(dst + 2 * tid) = (unsigned short)((c0 & 0xFF) | ((c1 & 0xFF) << 8));
-            }
+    // qkv step: this block is head `blk` of the row [Q heads | K heads | V heads]; lane l owns the rotation pair (l, l + 32)
+    if (!is_v) mx::rope_pair(v[0], v[1], cs, sn);
+    P.y[(size_t)blk * 64 + tid] = v[0], P.y[(size_t)blk * 64 + 32 + tid] = v[1];
+    if (blk < E.n_head) return;
+    // K or V head: the cache row of this position
+    const int kvh = is_v ? blk - E.n_head - E.n_kv_head : blk - E.n_head;
+    const int kvd = E.n_kv_head * 64;
+    if (E.kq == nullptr) {
+        float *dst = (is_v ? E.vcache : E.kcache) + row * kvd + kvh * 64;
+        dst[tid] = v[0], dst[tid + 32] = v[1];
+    } else {
+        int8_t *dst = (is_v ? E.vq : E.kq) + row * kvd + kvh * 64;
+        float *sc = is_v ? E.vs : E.ks, *be = is_v ? E.vb : E.kb;
+        const size_t sd = row * E.n_kv_head + kvh;
+        int c0, c1;
+        float scale, beta;
+        mx::quant_head_row(v[0], v[1], be != nullptr, c0, c1, scale, beta);
+        if (tid == 0) {
+            sc[sd] = scale;
+            if (be != nullptr) be[sd] = beta;
         }
+        dst[tid] = (int8_t)c0, dst[tid + 32] = (int8_t)c1;
     }
 }
 
@@ -333,6 +355,7 @@ int launch_gemv(mx230_handle *h, void *stream, GemvParams P, int w_kind, const c
         P.partials = (float *)h->ws;
         P.counters = h->counters;
     }
+    P.status = h->status_dev;
     mx230_device_guard guard(h->device);
     cudaStream_t st = (cudaStream_t)stream;
     const dim3 grid((unsigned)(n_blocks * P.ctas));
