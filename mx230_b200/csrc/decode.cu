@@ -285,7 +285,7 @@ __device__ void merge_and_store(const DecodeParams &P, int s, int head0, int gc,
 // such a head into rank r's rows with asynchronous stores, which complete the one phase of rank r's barrier.  What bounds it is
 // latency: token of 24 layers over 2001 int8 keys (two clusters of eight CTAs per layer), us: splits merged through the
 // workspace 340, totals pulled between two cluster barriers 272, pushed in front of one 263, this and the same in the
-// projections 254.
+// projections 254, its one-warp epilogue and relaxed barrier arrivals 229.
 // q_rot (fused step): rotated q, [G][64] in shared memory; it replaces the raw q in qkv once every CTA of the group
 // has read that.  Null where out is the qkv row itself: the attention row then takes q's place.
 constexpr int MERGE_ROWS = 16;   // ceil(8 / C) heads from each of C CTAs, C <= 8: at most 14
@@ -295,7 +295,8 @@ struct ClusterMerge {
     int aborted;
 };
 __device__ __forceinline__ int merge_heads(int gc, int rank, int C) { return gc > rank ? (gc - rank + C - 1) / C : 0; }
-// Before the first push: called by the whole CTA, of every CTA of the cluster
+// Before the first push, by every thread of every CTA of the cluster.  (A push may reach a barrier before its owner has stated
+// the bytes to expect: the phase stays open until it has.)
 __device__ __forceinline__ void merge_open(ClusterMerge &X, int gc, int rank, int C) {
     if (C == 1) return;
     if (threadIdx.x == 0) {
@@ -305,7 +306,7 @@ __device__ __forceinline__ void merge_open(ClusterMerge &X, int gc, int rank, in
         mx::mbar_fence_init();
         mx::mbar_expect_tx(bar, merge_heads(gc, rank, C) * C * 68 * 4);
     }
-    mx::cluster_arrive_release();   // waited for before the first push
+    mx::cluster_arrive_relaxed();   // waited for before the first push
 }
 template <int G, int NW>
 __device__ void finish_group(const DecodeParams &P, const float *mg, ClusterMerge &X, int s, int head0, int gc, int cl, int rank,
@@ -872,6 +873,7 @@ decode_q8_mma_kernel(const DecodeParams P) {
     const int cl = blockIdx.x / P.cl_size, rank = blockIdx.x - cl * P.cl_size;
 
     const float freq = FUSED ? mx::rope_freq(lane, 64, P.theta) : 0.0f;
+    merge_open(X, gc, rank, P.cl_size);
     if (P.push_regions == nullptr) mx::pdl_wait();   // (a split-KV step, whose CTAs wait for other ranks, is launched plainly)
     // q: requested before the position, whose chain of dependent loads (position, table, first tile) it then runs beside
     float qa_raw = 0.0f, qb_raw = 0.0f;   // warp = head (Q8_WARPS == MG)
@@ -884,8 +886,10 @@ decode_q8_mma_kernel(const DecodeParams P) {
     const int pos = kend - 1;                             // fused step: the new token's position
     if (FUSED) kend = pos;
     const int active = active_clusters(P, kend - kbeg);
-    if (cl >= active) return;
-    merge_open(X, gc, rank, P.cl_size);
+    if (cl >= active) {
+        if (P.cl_size > 1) mx::cluster_wait();
+        return;
+    }
     const int n_splits = active * P.cl_size;
     split_range(kbeg, kend, blockIdx.x, n_splits, ka, kb_);
     const int *table = PAGED ? P.tables + (P.pos_kind == 2 ? (size_t)s * P.n_log : 0) : nullptr;
@@ -1211,6 +1215,7 @@ decode_f32_ring_kernel(const DecodeParams P) {
     const int cl = blockIdx.x / P.cl_size, rank = blockIdx.x - cl * P.cl_size;
 
     const float freq = FUSED && P.use_rope ? mx::rope_freq(lane, 64, P.theta) : 0.0f;
+    merge_open(X, gc, rank, P.cl_size);
     if (P.push_regions == nullptr) mx::pdl_wait();   // (a split-KV step, whose CTAs wait for other ranks, is launched plainly)
     // q: requested before the position, whose chain of dependent loads (position, table, first tile) it then runs beside
     constexpr int QH = (G + WARPS - 1) / WARPS;   // heads of a warp: warp, warp + WARPS, ...
@@ -1229,8 +1234,10 @@ decode_f32_ring_kernel(const DecodeParams P) {
     const int pos = kend - 1;                             // fused step: the new token's position
     if (FUSED) kend = pos;
     const int active = active_clusters(P, kend - kbeg);
-    if (cl >= active) return;
-    merge_open(X, gc, rank, P.cl_size);
+    if (cl >= active) {
+        if (P.cl_size > 1) mx::cluster_wait();
+        return;
+    }
     const int n_splits = active * P.cl_size;
     split_range(kbeg, kend, blockIdx.x, n_splits, ka, kb_);
     const int *table = PAGED ? P.tables + (P.pos_kind == 2 ? (size_t)s * P.n_log : 0) : nullptr;

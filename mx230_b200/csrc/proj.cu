@@ -141,7 +141,7 @@ gemv_heads_kernel(const GemvParams P) {
             mx::mbar_fence_init();
             if (rank == 0) mx::mbar_expect_tx(bar, P.n_slices * PJ_COLS * 4);
         }
-        mx::cluster_arrive_release();               // waited for before the first store to another CTA's memory
+        mx::cluster_arrive_relaxed();               // waited for before the first store to another CTA's memory
     }
     // start of the CTA's rows into L2 under the previous kernel's tail
     for (int r = c0 / IN_PER_ROW + tid, n = 0; r < c1 / IN_PER_ROW && n < 2; r += nt, ++n) {
@@ -150,7 +150,7 @@ gemv_heads_kernel(const GemvParams P) {
         if (ELT == 4 && col0 + 32 < P.n_out) mx::prefetch_l2(line + 128);
     }
     const QkvEpilogue &E = P.e;
-    const bool finishes = (rank == 0 || C == 1) && tid < 32;   // the warp that finishes the block: lane l has columns l and l + 32
+    const bool finishes = (rank == 0 || C == 1) && tid < 32;   // the warp that finishes the block: lane l has columns 2l and 2l + 1
     const float freq = finishes && E.enabled ? mx::rope_freq(tid, 64, E.theta) : 0.0f;
     mx::pdl_wait();
 
@@ -181,7 +181,7 @@ gemv_heads_kernel(const GemvParams P) {
     if (finishes) {
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
-            const int o = col0 + tid + 32 * k;
+            const int o = col0 + 2 * tid + k;   // (n_out % 4 == 0)
             if (o >= P.n_out) break;
             if (P.b) bias[k] = P.b[o];
             if (I8) scale_o[k] = P.scales[o];
@@ -267,45 +267,53 @@ gemv_heads_kernel(const GemvParams P) {
     float cs = 1.0f, sn = 0.0f;
     if (E.enabled && !is_v) mx::rope_angle(pos, freq, cs, sn);   // (while the other CTAs' sums are on their way)
     if (C > 1 && !__all_sync(0xFFFFFFFFu, mx::mbar_wait<true>(bar, 0, &aborted, P.status))) return;
-    float v[2];
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-        const int c = tid + 32 * k;
-        float sum = 0.0f;
-        if (P.n_slices == 1) {
-            sum = parts[0][c];
-        } else if (C == 1 && P.ctas > 1) {
-            if (col0 + c < P.n_out)
-                for (int g = 0; g < P.n_slices; ++g) sum += __ldcg(P.partials + (size_t)g * P.n_out + col0 + c);
-        } else {
+    // (a loop that is short in code as well: what runs once per launch is fetched once per launch)
+    const bool in = col0 + 2 * tid < P.n_out;
+    float2 sum = make_float2(0.f, 0.f);
+    if (P.n_slices == 1) {
+        sum = *(const float2 *)&parts[0][2 * tid];
+    } else if (C == 1 && P.ctas > 1) {
+        if (in)
+            for (int g = 0; g < P.n_slices; ++g) {
+                const float2 p = __ldcg((const float2 *)(P.partials + (size_t)g * P.n_out + col0 + 2 * tid));
+                sum.x += p.x, sum.y += p.y;
+            }
+    } else {
 #pragma unroll 8
-            for (int g = 0; g < P.n_slices; ++g) sum += parts[g][c];
+        for (int g = 0; g < P.n_slices; ++g) {
+            const float2 p = *(const float2 *)&parts[g][2 * tid];
+            sum.x += p.x, sum.y += p.y;
         }
-        v[k] = (I8 ? sum * scale_o[k] : sum) + bias[k];
     }
+    float2 v = make_float2((I8 ? sum.x * scale_o[0] : sum.x) + bias[0], (I8 ? sum.y * scale_o[1] : sum.y) + bias[1]);
     if (!E.enabled) {
-#pragma unroll
-        for (int k = 0; k < 2; ++k)
-            if (col0 + tid + 32 * k < P.n_out) P.y[col0 + tid + 32 * k] = P.accum ? y_old[k] + v[k] : v[k];
+        if (P.accum) v.x = y_old[0] + v.x, v.y = y_old[1] + v.y;
+        if (in) *(float2 *)(P.y + col0 + 2 * tid) = v;
         return;
     }
     // qkv step: this block is head `blk` of the row [Q heads | K heads | V heads]; lane l owns the rotation pair (l, l + 32)
-    if (!is_v) mx::rope_pair(v[0], v[1], cs, sn);
-    P.y[(size_t)blk * 64 + tid] = v[0], P.y[(size_t)blk * 64 + 32 + tid] = v[1];
+    float x1, x2;
+    {
+        const float e1 = __shfl_sync(0xFFFFFFFFu, v.x, tid >> 1), o1 = __shfl_sync(0xFFFFFFFFu, v.y, tid >> 1);
+        const float e2 = __shfl_sync(0xFFFFFFFFu, v.x, 16 + (tid >> 1)), o2 = __shfl_sync(0xFFFFFFFFu, v.y, 16 + (tid >> 1));
+        x1 = (tid & 1) ? o1 : e1, x2 = (tid & 1) ? o2 : e2;
+    }
+    if (!is_v) mx::rope_pair(x1, x2, cs, sn);
+    P.y[(size_t)blk * 64 + tid] = x1, P.y[(size_t)blk * 64 + 32 + tid] = x2;
     if (blk < E.n_head) return;
     // K or V head: the cache row of this position
     const int kvh = is_v ? blk - E.n_head - E.n_kv_head : blk - E.n_head;
     const int kvd = E.n_kv_head * 64;
     if (E.kq == nullptr) {
         float *dst = (is_v ? E.vcache : E.kcache) + row * kvd + kvh * 64;
-        dst[tid] = v[0], dst[tid + 32] = v[1];
+        dst[tid] = x1, dst[tid + 32] = x2;
     } else {
         int8_t *dst = (is_v ? E.vq : E.kq) + row * kvd + kvh * 64;
         float *sc = is_v ? E.vs : E.ks, *be = is_v ? E.vb : E.kb;
         const size_t sd = row * E.n_kv_head + kvh;
         int c0, c1;
         float scale, beta;
-        mx::quant_head_row(v[0], v[1], be != nullptr, c0, c1, scale, beta);
+        mx::quant_head_row(x1, x2, be != nullptr, c0, c1, scale, beta);
         if (tid == 0) {
             sc[sd] = scale;
             if (be != nullptr) be[sd] = beta;
