@@ -193,7 +193,9 @@ enum { SRC_PRE = 0, SRC_RAW = 1, SRC_RAW_BOUND = 2, SRC_I8 = 3 };
 // large (fwd_key_split says when).  Without a row max P V of all key tiles is summed into one O in key order, and both
 // forms sum a row's probabilities over even and odd key tiles apart: a head's result has the same bits in either form.
 // With a row max each pair of groups has its own max and its own O, which the first group joins at the end.
-template <int SRC, bool KEY_SPLIT>
+// HALF: the output goes to O_half as well (an instantiation of its own: as a run-time choice it made the int8 key-split loop 3 to
+// 5 % slower, 512 tokens over 2048 keys 28.4 -> 29.2 us).
+template <int SRC, bool KEY_SPLIT, bool HALF>
 __global__ void __launch_bounds__(FWD_THREADS, 1)
 flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                  const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO,
@@ -796,7 +798,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                     }
                 };
                 auto store_half = [&](int cc) {   // this row's 32 columns of va: 64 bytes
-                    if (P.O_half == nullptr || row >= NQ) return;
+                    if (!HALF || row >= NQ) return;
                     uint4 *dst = (uint4 *)(P.O_half + ((size_t)bh * NQ + row) * HD + cc * 32);
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
@@ -1073,12 +1075,14 @@ bool fwd_key_split(int heads, int n_q, int n_k, int q_off, int causal, int sms) 
     return fullest(true) < fullest(false);
 }
 
-template <int SRC, bool KEY_SPLIT>
+template <int SRC, bool KEY_SPLIT, bool HALF = false>
 int launch_variant(mx230_handle *h, cudaStream_t st, dim3 grid, const CUtensorMap &tq, const CUtensorMap &tk,
                    const CUtensorMap &tv, const CUtensorMap &to, const FwdParams &P) {
-    MX_SMEM_ATTR_ONCE(h->device, (flash_fwd_kernel<SRC, KEY_SPLIT>), SMEM_ALLOC);
+    if constexpr (!HALF && (SRC == SRC_PRE || SRC == SRC_I8))   // (what prefill stages)
+        if (P.O_half) return launch_variant<SRC, KEY_SPLIT, true>(h, st, grid, tq, tk, tv, to, P);
+    MX_SMEM_ATTR_ONCE(h->device, (flash_fwd_kernel<SRC, KEY_SPLIT, HALF>), SMEM_ALLOC);
     MX_LAUNCH(h, st, MX230_K_FLASH_FWD,
-              mx_launch(flash_fwd_kernel<SRC, KEY_SPLIT>, grid, FWD_THREADS, SMEM_ALLOC, st, 1, true, tq, tk, tv, to, P));
+              mx_launch(flash_fwd_kernel<SRC, KEY_SPLIT, HALF>, grid, FWD_THREADS, SMEM_ALLOC, st, 1, true, tq, tk, tv, to, P));
     return MX230_OK;
 }
 
