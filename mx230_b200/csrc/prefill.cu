@@ -36,15 +36,16 @@ struct StageParams {
     const int *bt;
     int bs;
     // the step's work in front of attention
+    int old_warps;                   // warps of a CTA that take cached keys, from the last one on
     int write_kv;                    // the new rows' K and V come from qkv and go to the cache (else they are in it)
     int rope;
     float theta;
 };
 
 constexpr int ST_THREADS = 512;
-constexpr int ST_CLUSTER = 4;        // CTAs that share one norm part
-constexpr int ST_GRID = MX230_NORM_PARTS * ST_CLUSTER;
+constexpr int ST_WARPS = ST_THREADS / 32;
 constexpr int ST_SUBS = 4;           // warps that share a token (they take its heads in turn)
+constexpr int ST_HEADS = 5;          // heads of a warp whose loads are issued together (14 + 2 * 2 heads: one round)
 
 __device__ __forceinline__ size_t stage_row(const StageParams &P, int t) {
     return P.bt ? (size_t)(P.bt[t / P.bs] * P.bs + t % P.bs) : (size_t)t;
@@ -53,16 +54,20 @@ __device__ __forceinline__ float *stage_kskb(const StageParams &P, int h, int t)
     return P.kskb + ((size_t)h * P.n_k_tiles + (t >> 7)) * 256 + (t & 127);
 }
 
-// 128 CTAs whatever the size: the kernel is a few microseconds of latency (launch, one or two memory round trips), so what
-// counts is that it is ONE launch and that every thread's loads are issued together.  In its place stood rope 5.4 us,
+// 128 or 256 CTAs whatever the size: the kernel is a few microseconds of latency (launch, one or two memory round trips), so
+// what counts is that it is ONE launch and that every thread's loads are issued together.  In its place stood rope 5.4 us,
 // quantise 4, two staging kernels 3.8 + 4 (512 tokens over 1536 cached keys, int8), and 11.7 + 5 + 4.7 + 5 (1900 tokens,
 // fp32).  New tokens: four warps per token, lane l holds dims l and l + 32 of a head, so RoPE's angle is computed once
 // per token and warp and a head's quantiser is a warp reduction.  Cached keys: eight threads per key and head, eight dims
-// each.  Row norms go through shared memory and, per cluster of four CTAs, into one of MX230_NORM_PARTS parts: with Q's
+// each.  Row norms go through shared memory and, per cluster of CTAs, into one of MX230_NORM_PARTS parts: with Q's
 // and K's the attention kernel bounds every score of a head and, where the bound is small, runs without a row max.
-__global__ void __launch_bounds__(ST_THREADS) prefill_stage_kernel(const StageParams P) {
+// CLUSTER: CTAs that share one norm part, 4 or 8.  (Sizes are constants or come from the host: a division costs more here than
+// the work of a thread.)
+template <int CLUSTER>
+__global__ void __launch_bounds__(ST_THREADS, 2) prefill_stage_kernel(const StageParams P) {
     extern __shared__ int smax[];    // [n_norms] squared norms of Q and K heads as ordered integers (NaN largest)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int n_ctas = MX230_NORM_PARTS * CLUSTER;
     const int n_max = P.n_head + P.n_kv_head, n_norms = P.q_norm2 ? n_max : 0;
     mx::pdl_trigger();
     for (int i = tid; i < n_norms; i += ST_THREADS) smax[i] = 0;
@@ -77,16 +82,16 @@ __global__ void __launch_bounds__(ST_THREADS) prefill_stage_kernel(const StagePa
     // ---- new tokens ----
     const int n_units = P.n_head + (P.write_kv ? 2 * P.n_kv_head : 0);
     const int sub = warp & (ST_SUBS - 1);
-    for (int tok = blockIdx.x + ST_GRID * (warp / ST_SUBS); tok < P.n_tok; tok += ST_GRID * (ST_THREADS / 32 / ST_SUBS)) {
+    for (int tok = blockIdx.x + n_ctas * (warp / ST_SUBS); tok < P.n_tok; tok += n_ctas * (ST_WARPS / ST_SUBS)) {
         const int pos = P.pos0 + tok;
         float *row = P.qkv + (size_t)tok * P.stride;
         const size_t crow = P.write_kv ? stage_row(P, pos) : 0;
         float cs = 1.0f, sn = 0.0f;
         bool have_angle = false;
-        for (int u0 = sub; u0 < n_units; u0 += 4 * ST_SUBS) {
-            float va[4], vb[4];
+        for (int u0 = sub; u0 < n_units; u0 += ST_HEADS * ST_SUBS) {
+            float va[ST_HEADS], vb[ST_HEADS];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
+            for (int i = 0; i < ST_HEADS; ++i) {
                 const int u = u0 + i * ST_SUBS;
                 if (u < n_units) va[i] = row[u * HD + lane], vb[i] = row[u * HD + 32 + lane];
             }
@@ -95,7 +100,7 @@ __global__ void __launch_bounds__(ST_THREADS) prefill_stage_kernel(const StagePa
                 have_angle = true;
             }
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
+            for (int i = 0; i < ST_HEADS; ++i) {
                 const int u = u0 + i * ST_SUBS;
                 if (u >= n_units) break;
                 float a = va[i], b = vb[i];
@@ -174,15 +179,18 @@ __global__ void __launch_bounds__(ST_THREADS) prefill_stage_kernel(const StagePa
         }
     }
 
-    // ---- cached keys [0, n_old) ----
+    // ---- cached keys [0, n_old): from the last warp of every CTA on, the first ones have the new tokens ----
     const int n_old = P.write_kv ? P.pos0 : P.n_keys;
     const size_t total = (size_t)n_old * P.n_kv_head * 8;
-    for (size_t base = (size_t)blockIdx.x * ST_THREADS; base < total; base += (size_t)ST_GRID * ST_THREADS) {
-        const bool live = base + tid < total;
-        const size_t idx = live ? base + tid : total - 1;   // keep the row's lanes together for the shuffles below
+    const int W = P.old_warps;
+    for (size_t base = (blockIdx.x * (size_t)W + (ST_WARPS - 1 - warp)) * 32; ST_WARPS - 1 - warp < W && base < total;
+         base += (size_t)n_ctas * W * 32) {
+        const bool live = base + lane < total;
+        const size_t idx = live ? base + lane : total - 1;   // keep the row's lanes together for the shuffles below
         const int c = (int)(idx & 7);
         const size_t th = idx >> 3;
-        const int t = (int)(th / P.n_kv_head), h = (int)(th - (size_t)t * P.n_kv_head);
+        const int t = total >> 32 ? (int)(th / P.n_kv_head) : (int)((uint32_t)th / (uint32_t)P.n_kv_head);
+        const int h = (int)(th - (size_t)t * P.n_kv_head);
         const size_t row = stage_row(P, t);
         const size_t dst = ((size_t)h * P.n_keys + t) * HD + c * 8;
         float k[8], v[8], ksc = 0.0f, kbe = 0.0f, ss = 0.0f;
@@ -246,7 +254,7 @@ __global__ void __launch_bounds__(ST_THREADS) prefill_stage_kernel(const StagePa
     }
 
     // ---- the cluster's maxima -> its part ----
-    const int part = blockIdx.x / ST_CLUSTER, rank = blockIdx.x % ST_CLUSTER;
+    const int part = blockIdx.x / CLUSTER, rank = blockIdx.x % CLUSTER;
     __syncthreads();
     mx::cluster_wait();
     if (rank != 0)
@@ -332,7 +340,15 @@ int prefill(mx230_handle *h, void *stream, float *out, const float *qkv, const f
         sm = 0;
         S.q_norm2 = S.k_norm2 = q_norm2 = k_norm2 = nullptr;
     }
-    MX_LAUNCH(h, st, MX230_K_PREFILL, mx_launch(prefill_stage_kernel, ST_GRID, ST_THREADS, sm, st, ST_CLUSTER, true, S));
+    // 256 CTAs, two per SM, where 128 would take tokens or cached keys in more than one round (2048 tokens over 6144 int8 keys,
+    // 32/4 heads, us a call: 128 176.6, 256 168.7); below that 128, the smaller launch
+    const size_t old = (size_t)(step.write_kv ? pos0 : n_keys) * n_kv_head * 8;   // threads
+    const int cluster = n_tok > 4 * MX230_NORM_PARTS * (ST_WARPS / ST_SUBS) || old > (size_t)4 * MX230_NORM_PARTS * ST_THREADS ? 8 : 4;
+    const size_t per_cta = (old + 32 * MX230_NORM_PARTS * cluster - 1) / (32 * MX230_NORM_PARTS * cluster);
+    S.old_warps = per_cta < ST_WARPS ? (int)per_cta : ST_WARPS;
+    MX_LAUNCH(h, st, MX230_K_PREFILL,
+              mx_launch(cluster == 8 ? prefill_stage_kernel<8> : prefill_stage_kernel<4>, MX230_NORM_PARTS * cluster, ST_THREADS, sm, st,
+                        cluster, true, S));
     return mx230_launch_flash_fwd_ex(h, st, qb, kbuf, vbuf, out, nullptr, n_head, n_tok, n_keys, pos0, n_head / n_kv_head, HD,
                                      out_stride, 1, i8_scores ? 0 : 1, q_norm2, k_norm2, i8_scores ? row_a : nullptr,
                                      i8_scores ? row_qsum : nullptr, i8_scores ? kskb : nullptr, o_half ? qb : nullptr);
