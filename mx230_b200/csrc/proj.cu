@@ -108,8 +108,11 @@ struct WeightRow<int8_t, 4> {
 };
 
 // Grid: column blocks x CTAs, the CTAs of a block next to each other.  A slice takes 64 / CPT * 8 threads.
+// Registers: two CTAs of five slices (640 threads at four columns a thread, 320 at eight) have to fit an SM, so that the next
+// launch's are there, with their weights on the way into L2, while this one's still run: 896 -> 1152 fp32, launch after launch
+// over fresh weights, 4.6 us at 50 registers (one CTA), 3.2 at 48.
 template <typename WT, int CPT>
-__global__ void __launch_bounds__(PJ_SLOTS * PJ_COLS / CPT * PJ_ROWLANES)
+__global__ void __maxnreg__(CPT == 8 ? 56 : 48)
 gemv_heads_kernel(const GemvParams P) {
     constexpr bool I8 = sizeof(WT) == 1;
     constexpr int TPR = PJ_COLS / CPT;              // threads across a weight row
