@@ -933,7 +933,7 @@ int launch_fused(mx230_handle *h, cudaStream_t st, const Maps &m, const float *L
     if (!dq_is_zero && (rc = launch_zero(st, dQ, (size_t)batch_heads * n * HD))) return rc;
     BwdParams P{L, Delta, dK, dV, dQ, nullptr, nullptr, n, causal ? 1 : 0, h->status_dev};
     // persistent: one CTA per SM (the kernel holds all of an SM's tensor memory) walks its share of the items, the
-    // next item's owned and first streamed tiles loading while the compute warps store the current item's dK, dV
+    // next item's owned and first streamed tiles loading under the current item's last ones
     const int n_items = set_items(P, batch_heads, n);
     P.test_drop_tile = h->test_drop_tile;
     dim3 grid((unsigned)(n_items < h->sm_count ? n_items : h->sm_count));
