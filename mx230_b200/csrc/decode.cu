@@ -359,8 +359,12 @@ __device__ void finish_group(const DecodeParams &P, const float *mg, ClusterMerg
             if (d == 0) mx::cluster_st_async(dst, bar, mm, lt, 0.0f, 0.0f);
         }
     }
+    if (C > 1) {
+        __syncwarp();
+        mx::cluster_arrive_relaxed();   // this thread's stores are issued
+    }
     if (C > 1 && merge_heads(gc, rank, C) * 16 > tid) {
-        const bool ok = mx::mbar_wait<true>(mx::smem_u32(&X.bar), 0, &X.aborted, P.status);
+        const bool ok = mx::cluster_sums_wait(mx::smem_u32(&X.bar), &X.aborted, P.status);
         for (int i = tid; ok && (i >> 4) * C + rank < gc; i += nt) {   // (nothing is written after a wait that ran out)
             const int g = (i >> 4) * C + rank, d = (i & 15) * 4;
             float4 hd[8], ap[8];

@@ -254,6 +254,8 @@ gemv_heads_kernel(const GemvParams P) {
         else if (col0 + c < P.n_out) *(float4 *)(P.partials + (size_t)g * P.n_out + col0 + c) = sum;   // (n_out % 4 == 0)
     }
     if (C > 1) {
+        __syncwarp();
+        mx::cluster_arrive_relaxed();   // this thread's stores are issued
         if (!finishes) return;
     } else if (P.ctas > 1) {
         __threadfence();
@@ -269,7 +271,7 @@ gemv_heads_kernel(const GemvParams P) {
     // ---- epilogue on the 64 finished sums of this column block: one warp ----
     float cs = 1.0f, sn = 0.0f;
     if (E.enabled && !is_v) mx::rope_angle(pos, freq, cs, sn);   // (while the other CTAs' sums are on their way)
-    if (C > 1 && !__all_sync(0xFFFFFFFFu, mx::mbar_wait<true>(bar, 0, &aborted, P.status))) return;
+    if (C > 1 && !__all_sync(0xFFFFFFFFu, mx::cluster_sums_wait(bar, &aborted, P.status))) return;
     // (a loop that is short in code as well: what runs once per launch is fetched once per launch)
     const bool in = col0 + 2 * tid < P.n_out;
     float2 sum = make_float2(0.f, 0.f);
