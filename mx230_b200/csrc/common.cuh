@@ -314,19 +314,21 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     }
 }
 
-// Wait for the stores of the other CTAs of a cluster that complete the first phase of this CTA's barrier.  Every thread of the
-// cluster calls cluster_arrive_relaxed() behind its last such store.  Where they are late, the thread first waits until all are
+// Wait for the stores of the other CTAs of a cluster that complete the first phase of this CTA's barrier; by whole warps (a thread
+// in a cluster barrier waits for the rest of its warp, which may be on its way to a barrier of the CTA).  Every thread of the
+// cluster calls cluster_arrive_relaxed() behind its last such store.  Where they are late, the warp first waits until all are
 // issued: a CTA that left before them would be stored into after its end.  (That barrier is the hardware's and ends, since no
 // CTA waits for another in front of its own stores.)  Only then, bounded, until they have landed: a microsecond or two, so they
-// are given LANDING_CYCLES whatever smaller bound the caller has set.  The arrivals cost a launch 0.05 us, this wait in place of
-// a plain bounded one 0.03 (host-launched step at 777 fp32 keys 6.67 -> 6.74 us, token of 24 layers 228.9 -> 230.4).
+// are given LANDING_CYCLES whatever smaller bound the caller has set.  Costs a launch 0.1 us against a plain bounded wait
+// (host-launched step over 777 fp32 keys 6.5 -> 6.6 us, token of 24 layers over 2000 int8 keys 229.0 -> 231.1).
 constexpr int CLUSTER_POLLS = 64;
 __device__ __forceinline__ bool cluster_sums_wait(uint32_t bar, volatile int *abort_flag, int *status) {
+    bool ok = false;
 #pragma unroll 1
-    for (int poll = 0; poll < CLUSTER_POLLS; ++poll)
-        if (mbar_try_wait<true>(bar, 0)) return true;
-    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");   // (not .aligned: some threads of a warp may be through)
-    return mbar_wait<true>(bar, 0, abort_flag, status);
+    for (int poll = 0; poll < CLUSTER_POLLS && !ok; ++poll) ok = mbar_try_wait<true>(bar, 0);
+    if (__all_sync(0xFFFFFFFFu, ok)) return true;
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    return __all_sync(0xFFFFFFFFu, mbar_wait<true>(bar, 0, abort_flag, status));
 }
 
 // One lane of the (converged) warp: the branch it guards leaves the rest of the warp's code warp-uniform, so

@@ -363,7 +363,7 @@ __device__ void finish_group(const DecodeParams &P, const float *mg, ClusterMerg
         __syncwarp();
         mx::cluster_arrive_relaxed();   // this thread's stores are issued
     }
-    if (C > 1 && merge_heads(gc, rank, C) * 16 > tid) {
+    if (C > 1 && merge_heads(gc, rank, C) * 16 > (tid & ~31)) {
         const bool ok = mx::cluster_sums_wait(mx::smem_u32(&X.bar), &X.aborted, P.status);
         for (int i = tid; ok && (i >> 4) * C + rank < gc; i += nt) {   // (nothing is written after a wait that ran out)
             const int g = (i >> 4) * C + rank, d = (i & 15) * 4;

@@ -271,7 +271,7 @@ gemv_heads_kernel(const GemvParams P) {
     // ---- epilogue on the 64 finished sums of this column block: one warp ----
     float cs = 1.0f, sn = 0.0f;
     if (E.enabled && !is_v) mx::rope_angle(pos, freq, cs, sn);   // (while the other CTAs' sums are on their way)
-    if (C > 1 && !__all_sync(0xFFFFFFFFu, mx::cluster_sums_wait(bar, &aborted, P.status))) return;
+    if (C > 1 && !mx::cluster_sums_wait(bar, &aborted, P.status)) return;
     // (a loop that is short in code as well: what runs once per launch is fetched once per launch)
     const bool in = col0 + 2 * tid < P.n_out;
     float2 sum = make_float2(0.f, 0.f);
