@@ -32,7 +32,7 @@ struct mx230_handle {
     void *ws;              // workspace: bf16 operand staging / split-KV partials
     size_t ws_bytes;
     int *status_dev;       // [8] device words: [0..3] status (0 = ok), [4..5] the wait limit in SM cycles (64-bit)
-    int test_drop_tile;    // test hook: streamed tile that CTA 0's producer never requests (-1 = off)
+    int test_drop_tile;    // test hook: streamed tile that CTA 0's producer never requests, CTA that sends nothing to its cluster (-1 = off)
     unsigned *counters;    // split-KV arrival counters (self-resetting)
     size_t n_counters;
     int q8_score_mode;     // MX230_Q8_SCORE_*

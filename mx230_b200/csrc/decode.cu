@@ -62,6 +62,7 @@ struct DecodeParams {
     // 19.9; one int8 sequence in a 24-layer token, 64 CTAs: 259 / 245 / 272).
     int trigger;
     int *status;         // where a wait within a cluster that ran out is recorded
+    int test_drop;       // test hook: CTA (x) of the first group that never sends its totals to its cluster; -1 = off
     int wide;            // fp32 cache: CTAs of F32_WARPS_WIDE warps
     int bs_shift;        // log2(bs) when bs is a power of two, else -1
     // fused step (RoPE and KV write of the new token inside the attention kernel): keys [0, pos) come from the cache,
@@ -351,7 +352,7 @@ __device__ void finish_group(const DecodeParams &P, const float *mg, ClusterMerg
         if (C == 1) {
             emit(g, d, mm, lt, a);
             if (q_rot && active == 1) put_q(g, d);
-        } else {
+        } else if (P.test_drop != (int)blockIdx.x || blockIdx.y + blockIdx.z > 0) {
             const int r = g % C;
             const uint32_t dst = mx::cluster_map(mx::smem_u32(X.rows + (g / C * C + rank) * 68), r);
             const uint32_t bar = mx::cluster_map(mx::smem_u32(&X.bar), r);
@@ -365,7 +366,7 @@ __device__ void finish_group(const DecodeParams &P, const float *mg, ClusterMerg
     }
     if (C > 1 && merge_heads(gc, rank, C) * 16 > (tid & ~31)) {
         const bool ok = mx::cluster_sums_wait(mx::smem_u32(&X.bar), &X.aborted, P.status);
-        for (int i = tid; ok && (i >> 4) * C + rank < gc; i += nt) {   // (nothing is written after a wait that ran out)
+        for (int i = tid; (i >> 4) * C + rank < gc; i += nt) {
             const int g = (i >> 4) * C + rank, d = (i & 15) * 4;
             float4 hd[8], ap[8];
 #pragma unroll
@@ -387,6 +388,8 @@ __device__ void finish_group(const DecodeParams &P, const float *mg, ClusterMerg
                 lt += hd[p].y * wgt;
                 a.x += ap[p].x * wgt, a.y += ap[p].y * wgt, a.z += ap[p].z * wgt, a.w += ap[p].w * wgt;
             }
+            // totals that never came: NaN, also in the workspace, where rows of an earlier call would pass for this one's
+            if (!ok) mm = 0.0f, lt = CUDART_NAN_F, a = make_float4(CUDART_NAN_F, CUDART_NAN_F, CUDART_NAN_F, CUDART_NAN_F);
             emit(g, d, mm, lt, a);
             if (q_rot && active == 1) put_q(g, d);
         }
@@ -1679,6 +1682,7 @@ int launch_decode(mx230_handle *h, void *stream, DecodeParams P, int n_seq, int 
     }
     P.counters = h->counters;
     P.status = h->status_dev;
+    P.test_drop = h->test_drop_tile;
 
     mx230_device_guard guard(h->device);
     dim3 grid(P.cl_size * P.max_clusters, gy, n_seq);

@@ -58,6 +58,7 @@ struct GemvParams {
     float *partials;                // [n_slices][n_out]
     unsigned *counters;      // one per column block, self-resetting
     int *status;             // where a wait within a cluster that ran out is recorded
+    int test_drop;           // test hook: CTA of the first column block that never sends its sums to its cluster; -1 = off
     QkvEpilogue e;
 };
 
@@ -249,8 +250,10 @@ gemv_heads_kernel(const GemvParams P) {
         }
         // (asynchronous stores that complete the first CTA's barrier: the cluster barrier behind plain ones took 1500 cycles of
         // the 5000 of a launch)
-        if (C > 1) mx::cluster_st_async(mx::cluster_map(mx::smem_u32(&parts[g][c]), 0), mx::cluster_map(bar, 0), sum.x, sum.y, sum.z, sum.w);
-        else if (P.ctas == 1) *(float4 *)&parts[g][c] = sum;
+        if (C > 1) {
+            if (P.test_drop != (int)blockIdx.x || blk > 0)
+                mx::cluster_st_async(mx::cluster_map(mx::smem_u32(&parts[g][c]), 0), mx::cluster_map(bar, 0), sum.x, sum.y, sum.z, sum.w);
+        } else if (P.ctas == 1) *(float4 *)&parts[g][c] = sum;
         else if (col0 + c < P.n_out) *(float4 *)(P.partials + (size_t)g * P.n_out + col0 + c) = sum;   // (n_out % 4 == 0)
     }
     if (C > 1) {
@@ -271,7 +274,7 @@ gemv_heads_kernel(const GemvParams P) {
     // ---- epilogue on the 64 finished sums of this column block: one warp ----
     float cs = 1.0f, sn = 0.0f;
     if (E.enabled && !is_v) mx::rope_angle(pos, freq, cs, sn);   // (while the other CTAs' sums are on their way)
-    if (C > 1 && !mx::cluster_sums_wait(bar, &aborted, P.status)) return;
+    if (C > 1 && !mx::cluster_sums_wait(bar, &aborted, P.status)) return;   // (nothing is written)
     // (a loop that is short in code as well: what runs once per launch is fetched once per launch)
     const bool in = col0 + 2 * tid < P.n_out;
     float2 sum = make_float2(0.f, 0.f);
@@ -369,6 +372,7 @@ int launch_gemv(mx230_handle *h, void *stream, GemvParams P, int w_kind, const c
         P.counters = h->counters;
     }
     P.status = h->status_dev;
+    P.test_drop = h->test_drop_tile;
     mx230_device_guard guard(h->device);
     cudaStream_t st = (cudaStream_t)stream;
     const dim3 grid((unsigned)(n_blocks * P.ctas));

@@ -1,6 +1,6 @@
 """The cluster merge of decode attention and of the projections when CTAs wait for one another longer than they may: with the
 smallest bound that a handle takes an ordinary call is still right and leaves no status, for only stores that are issued are
-waited for against the bound."""
+waited for against the bound.  Where sums never come (a test hook) the launch ends with a status and the handle keeps working."""
 import numpy as np
 import pytest
 import torch
@@ -11,6 +11,7 @@ from mx230_b200 import llm_attention as la
 from mx230_b200.common import Handle
 from tests.conftest import assert_close
 from tests.test_decode_gpu import TOL, build_caches, dev, to_dev_f32, to_dev_q8
+from tests.test_decode_step_gpu import filled_cache
 
 pytestmark = pytest.mark.gpu
 
@@ -54,3 +55,56 @@ def test_projection_with_the_smallest_bound(own_handle):
             la.gemv(h, y, dev(x), dev(w), dev(b))
             h.check_status()
             assert_close(y.cpu().numpy(), oracle.gemv(x, w, b), "gemv", max_abs=2e-4, mean_rel=2e-5)
+
+
+def _run_out(h, call):
+    """The call with CTA 1 of its first cluster sending nothing, and a bound of about a millisecond."""
+    try:
+        h.set_option(_lib.OPT_WAIT_LIMIT, 2000)
+        h.set_option(_lib.OPT_TEST_DROP_TILE, 1)
+        call()
+        with pytest.raises(_lib.Mx230Error) as e:
+            h.check_status()
+        assert e.value.code == _lib.ERR_DEVICE_STATUS
+    finally:
+        h.set_option(_lib.OPT_TEST_DROP_TILE, -1)
+        h.set_option(_lib.OPT_WAIT_LIMIT, 4000000)
+
+
+@pytest.mark.parametrize("quant", [False, True])
+@pytest.mark.parametrize("keys", [600, 9000])   # one cluster, two: their partial rows go through the workspace
+def test_decode_merge_that_runs_out(own_handle, quant, keys):
+    """No row of an earlier call, which the workspace still holds, passes for one of the call that failed."""
+    h, (nh, nkv) = own_handle, (14, 2)
+    c = filled_cache(h, keys, nkv, quant)
+    qkv = torch.randn(2, (nh + 2 * nkv) * 64, device="cuda")
+    pos = torch.tensor([keys - 1], dtype=torch.int32, device="cuda")
+    out = torch.zeros(nh * 64, device="cuda")
+
+    def call(i):
+        la.attn_decode_dyn(h, out, qkv[i], c, pos, nh, nkv, 64)
+    call(0)
+    h.check_status()
+    want = out.clone()
+    call(1)   # leaves its partial rows in the workspace
+    _run_out(h, lambda: call(0))
+    first = nh // nkv * 64
+    assert torch.isnan(out[:first]).all() and torch.equal(out[first:], want[first:])
+    call(0)
+    h.check_status()
+    assert torch.equal(out, want)
+
+
+def test_projection_merge_that_runs_out(own_handle):
+    h = own_handle
+    x, w, b = torch.randn(896, device="cuda"), torch.randn(896, 1152, device="cuda").half(), torch.randn(1152, device="cuda")
+    y = torch.zeros(1152, device="cuda")
+    la.gemv(h, y, x, w, b)
+    h.check_status()
+    want = y.clone()
+    y.fill_(7.0)
+    _run_out(h, lambda: la.gemv(h, y, x, w, b))
+    assert (y[:64] == 7.0).all() and torch.equal(y[64:], want[64:])
+    la.gemv(h, y, x, w, b)
+    h.check_status()
+    assert torch.equal(y, want)
