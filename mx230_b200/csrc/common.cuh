@@ -33,6 +33,7 @@ struct mx230_handle {
     size_t ws_bytes;
     int *status_dev;       // [8] device words: [0..3] status (0 = ok), [4..5] the wait limit in SM cycles (64-bit)
     int test_drop_tile;    // test hook: streamed tile that CTA 0's producer never requests, CTA that sends nothing to its cluster (-1 = off)
+    int wide_fit[9];       // [c]: clusters of c eight-warp fp32 decode CTAs that the device holds at once
     unsigned *counters;    // split-KV arrival counters (self-resetting)
     size_t n_counters;
     int q8_score_mode;     // MX230_Q8_SCORE_*
@@ -72,6 +73,7 @@ void mx230_prof_end(mx230_handle *h, cudaStream_t st, int slot);
         MX_LAUNCHED(h);                                                                     \
     } while (0)
 
+void mx230_count_wide_clusters(mx230_handle *h);   // fills wide_fit (decode.cu)
 void mx230_set_error(const char *fmt, ...);
 int mx230_fail(int code, const char *fmt, ...);
 

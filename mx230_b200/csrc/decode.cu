@@ -25,6 +25,7 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "decode_plan.h"
 
 namespace {
 
@@ -1557,41 +1558,24 @@ int launch_g(mx230_handle *h, cudaStream_t st, const DecodeParams &P, dim3 grid)
     return fused ? launch_f32<G, false, true>(h, st, P, grid) : launch_f32<G, false, false>(h, st, P, grid);
 }
 
-// How a group's keys are split over CTAs.  slots: CTAs of the kernel that are resident at once; groups: (sequence, K/V
-// head group) pairs; keys: largest number of keys of a sequence, 0 = unknown (position on the device).
-//  * whole grid resident at once: cl_size * max_clusters * groups <= slots (a partial second wave would nearly double
-//    the time);
-//  * up to 8 CTAs of a group (any number, so that 6 per group fill 444 slots where 4 would leave a third of them empty) form
-//    a cluster, whose merge costs one cluster barrier; pass_keys = keys that a CTA's warps
-//    take in one tile each: a CTA is not given less than one such pass;
-//  * further clusters join in (merge through global memory, about 2 us) only for sequences with more than 4 passes per
-//    CTA of the first; the kernel decides that per sequence from its actual length;
-//  * clusters of five to eight CTAs share one GPC and leave an eighth of its slots empty, so they are counted against 7/8
-//    of them (3 fp32 sequences of 32540 keys as 54 clusters of 8 took a second wave: 43 us against 36.5 as 74 splits);
-//  * ranges of four and more tiles per warp use clusters of one: any number of splits then fits the machine (9 per group fill
-//    296 slots where 8 would leave a tenth of them empty), and the merge is small against the stream.
-void plan_splits(DecodeParams &P, long long slots, long long groups, long long keys, int pass_keys) {
-    long long want = slots / groups;
-    if (want < 1) want = 1;
-    if (want > 256) want = 256;
-    const bool known = keys > 0;
-    if (known && keys / want >= 4LL * pass_keys) {
-        P.cl_size = 1;
-        P.max_clusters = (int)want;
-        P.cluster_keys = pass_keys;
-        return;
+}  // namespace
+
+void mx230_count_wide_clusters(mx230_handle *h) {
+    const auto kernel = decode_f32_ring_kernel<8, false, false, F32_WARPS_WIDE>;   // (the instantiation with the most shared memory)
+    const size_t sm = (size_t)F32Smem<8, F32_WARPS_WIDE>::TOTAL;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    for (int c = 1; c <= 8; ++c) {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = c, at[0].val.clusterDim.y = 1, at[0].val.clusterDim.z = 1;
+        cfg.gridDim = dim3(c), cfg.blockDim = dim3(F32_WARPS_WIDE * 32), cfg.dynamicSmemBytes = sm, cfg.attrs = at, cfg.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&h->wide_fit[c], kernel, &cfg) != cudaSuccess) h->wide_fit[c] = 0;
     }
-    const long long fit = slots * 7 / 8;
-    int c = want < 8 ? (int)want : 8;
-    if (c > 4) c = fit / groups > 8 ? 8 : fit / groups < 4 ? 4 : (int)(fit / groups);
-    if (known && c > (keys + pass_keys - 1) / pass_keys) c = (int)((keys + pass_keys - 1) / pass_keys);
-    P.cl_size = c;
-    P.cluster_keys = 4 * c * pass_keys;
-    long long k = (c > 4 ? fit / groups : want) / c;
-    if (known && k > (keys + P.cluster_keys - 1) / P.cluster_keys) k = (keys + P.cluster_keys - 1) / P.cluster_keys;
-    if (!known && k > 4) k = 4;
-    P.max_clusters = (int)(k < 1 ? 1 : k);
+    cudaGetLastError();   // (no count: four-warp CTAs)
 }
+
+namespace {
 
 // `known_keys`: host-known upper bound of keys per sequence (<= 0 when the position
 // lives on the device); only steers how many key splits are launched.
@@ -1641,6 +1625,7 @@ int launch_decode(mx230_handle *h, void *stream, DecodeParams P, int n_seq, int 
     if (P.push_out && base_ctas >= h->sm_count) merge_after = P.push_out, P.push_out = nullptr;
     const bool mma = uses_q8_mma(h, P);
     const long long slots = (q8 ? 2LL : 3LL) * h->sm_count;
+    const size_t split_bytes = (size_t)n_seq * P.n_head * 66 * sizeof(float);   // a split's triples
     if (h->decode_chunk > 0 && known_keys > 0) {   // fixed chunks: the split depends on the capacity alone
         P.cl_size = 1, P.cluster_keys = 0;
         P.max_clusters = (int)((known_keys + h->decode_chunk - 1) / h->decode_chunk);
@@ -1654,14 +1639,19 @@ int launch_decode(mx230_handle *h, void *stream, DecodeParams P, int n_seq, int 
         P.cl_size = 1, P.cluster_keys = 0;
         P.max_clusters = (int)(n < 1 ? 1 : n > 256 ? 256 : n);
     } else {
-        // fp32 cache, a cluster of eight CTAs per group leaves every CTA an SM of its own: eight warps in it take half as many
-        // key tiles in turn (one sequence: 778 keys, 14/2 heads 8.2 -> 7.2 us, 4001 keys, 32/4 heads 15.4 -> 13.6; token of 24
-        // layers at 1000 341 -> 313).  Known sequences beyond one cluster's keys keep three CTAs of four warps per SM.
-        P.wide = !q8 && base_ctas * 8 <= h->sm_count && known_keys <= 4 * 8 * F32_WARPS_WIDE * FT_KEYS;
-        plan_splits(P, P.wide ? h->sm_count : slots, base_ctas, known_keys,
-                    mma ? Q8_WARPS * WT_KEYS : (P.wide ? F32_WARPS_WIDE : F32_WARPS) * FT_KEYS);
+        // fp32 cache, few groups: CTAs of eight warps with an SM to themselves take half as many key tiles in turn (one sequence: 778
+        // keys, 14/2 heads 8.2 -> 7.2 us, 4001 keys, 32/4 heads 15.4 -> 13.6; token of 24 layers at 1000 341 -> 313).  Known
+        // sequences beyond one cluster's keys keep three CTAs of four warps per SM.
+        DecodeSplit S;
+        const bool few = !q8 && base_ctas * 8 <= h->sm_count && known_keys <= 4 * 8 * F32_WARPS_WIDE * FT_KEYS;
+        P.wide = few && plan_wide(S, h->wide_fit, base_ctas, P.group, known_keys, F32_WARPS_WIDE * FT_KEYS);
+        if (!P.wide) {
+            S = plan_splits(slots, base_ctas, known_keys, mma ? Q8_WARPS * WT_KEYS : F32_WARPS * FT_KEYS);
+            // (one cluster, which needs no workspace, where the handle has none for more)
+            if (few && S.cl_size > 1 && (!h->ws || S.max_clusters * split_bytes > h->ws_bytes)) S.max_clusters = 1;
+        }
+        P.cl_size = S.cl_size, P.max_clusters = S.max_clusters, P.cluster_keys = S.cluster_keys;
     }
-    const size_t split_bytes = (size_t)n_seq * P.n_head * 66 * sizeof(float);   // a split's triples
     // Where one CTA per group covers four fifths of the SMs and sequences hold up to 4096 keys, a second split only makes the
     // call faster (64 x 2048 keys, 14/2 heads: CUDA-core kernels 37.2 -> 33.1 us in the exact score mode and 29.0 -> 26.9,
     // range mode 35.5 -> 32.0): a handle without the workspace for it gets one split.

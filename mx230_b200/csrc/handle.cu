@@ -71,6 +71,7 @@ extern "C" int mx230_create(mx230_handle **out, int device, size_t workspace_byt
     h->q8_score_mode = MX230_Q8_SCORE_REF;
     h->decode_tensor = 1;
     h->n_counters = N_COUNTERS;
+    mx230_count_wide_clusters(h);
 
     void *fn = nullptr;
     cudaDriverEntryPointQueryResult qres;

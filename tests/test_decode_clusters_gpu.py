@@ -5,6 +5,7 @@ import torch
 
 import oracle
 from mx230_b200 import llm_attention as la
+from mx230_b200.common import Handle
 from tests.conftest import assert_close
 from tests.test_decode_gpu import TOL, build_caches, dev, to_dev_f32, to_dev_q8
 
@@ -29,3 +30,22 @@ def test_every_cluster_size(handle, nh, nkv):
             la.attn_decode(handle, out, dev(row), c8, keys - 1, nh, nkv, 64)
             assert_close(out.cpu().numpy(), oracle.gqa_decode_q8(row, q8, keys - 1, nh, 1), f"int8 {keys} keys", **TOL)
     handle.check_status()
+
+
+@pytest.mark.parametrize("nkv", [16, 17, 18])
+def test_many_groups_with_little_workspace(lib_built, nkv):
+    """Groups of which eight eight-warp CTAs each are not resident at once: up to two clusters of four-warp CTAs where the host
+    knows the length, and one, without workspace, where the handle has none for more."""
+    keys = 4096
+    rows, kc, vc, _ = build_caches(nkv, nkv, keys, 44)
+    c, row = to_dev_f32(kc, vc, nkv), rows[keys - 1]
+    want = oracle.gqa_decode_f32(row, kc, vc, keys - 1, nkv, nkv)
+    pos = torch.tensor([keys - 1], dtype=torch.int32, device="cuda")
+    for splits in (2, 0):
+        h = Handle(0, nkv * 66 * 4 * splits)
+        for at, call in ((keys - 1, la.attn_decode), (pos, la.attn_decode_dyn)):
+            out = torch.full((nkv * 64,), float("nan"), device="cuda")
+            call(h, out, dev(row), c, at, nkv, nkv, 64)
+            h.check_status()
+            assert_close(out.cpu().numpy(), want, f"{splits} {call.__name__}", **TOL)
+        h.close()
