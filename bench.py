@@ -427,6 +427,7 @@ def run_ours(args):
     h.profile_enable(False)
     launches = h.launches - l0
     prof = h.profile_read()
+    launches += prof.get("zero_kernel", (0, 0.0))[0]   # (the handle's own count leaves out what stands for a memset)
     h.check_status()
 
     # the reference's atomic-free split (a dQ pass and a dK/dV pass, bit-reproducible) on the same step
@@ -522,7 +523,7 @@ def run_ours(args):
                 cnt, tot = prof[name]
                 kern[name] = {"launches": cnt, "ms_per_launch": tot / cnt,
                               "achieved_tflops": flop / (tot / cnt * 1e-3) / 1e12, "flop_per_launch": flop}
-        for name in ("cast_bf16_kernel", "bwd_preprocess_kernel"):
+        for name in ("cast_bf16_kernel", "bwd_preprocess_kernel", "zero_kernel"):
             if name in prof:
                 cnt, tot = prof[name]
                 kern[name] = {"launches": cnt, "ms_per_launch": tot / cnt}

@@ -97,7 +97,8 @@ enum {
     MX230_K_PREFILL = 11,
     MX230_K_GEMV = 12,
     MX230_K_BWD_FUSED = 13,
-    MX230_K_COUNT = 14
+    MX230_K_ZERO = 14, /* dQ cleared in front of the fused backward, where no staging launch does so on the way */
+    MX230_K_COUNT = 15
 };
 
 typedef struct mx230_handle mx230_handle;
@@ -120,7 +121,8 @@ size_t mx230_flash_workspace_bytes(int batch_heads, int n, int with_backward);
 size_t mx230_decode_workspace_bytes(int n_seq, int n_head, int max_splits);
 /* Synchronises `stream`, reads and clears the device status words. */
 int mx230_check_status(mx230_handle *h, void *stream);
-/* Number of kernels launched through this handle so far. */
+/* Number of kernels launched through this handle so far; the one that stands in for a memset (MX230_K_ZERO) is not among
+ * them, as a memset would not be.  The profile below has it. */
 long long mx230_launch_count(const mx230_handle *h);
 
 /* Seeded host-side input generators (no CUDA call; `out_host` is host memory).

@@ -841,10 +841,12 @@ __global__ void __launch_bounds__(ZERO_THREADS) zero_kernel(float4 *p, size_t n4
     for (int u = 0; u < ZERO_UNROLL; ++u, i += ZERO_THREADS)
         if (i < n4) p[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
-int launch_zero(cudaStream_t st, float *p, size_t n) {   // n a multiple of 4, p 16-byte aligned
+int launch_zero(mx230_handle *h, cudaStream_t st, float *p, size_t n) {   // n a multiple of 4, p 16-byte aligned
     const size_t n4 = n / 4, per = ZERO_THREADS * ZERO_UNROLL;
+    const int slot = h->prof_on ? mx230_prof_begin(h, st, MX230_K_ZERO) : -1;
     MX_CHECK_CUDA(mx_launch(zero_kernel, dim3((unsigned)((n4 + per - 1) / per)), ZERO_THREADS, 0, st, 1, true, (float4 *)p, n4));
-    return MX230_OK;   // (stands for a memset: not among the launches that the handle counts)
+    if (slot >= 0) mx230_prof_end(h, st, slot);
+    return MX230_OK;   // (in a memset's place: in the profile, not in the launch count)
 }
 
 // function attributes are per device: one handle per GPU may live in the same process
@@ -930,7 +932,7 @@ int launch_fused(mx230_handle *h, cudaStream_t st, const Maps &m, const float *L
     if (!rc) rc = mx230_make_tmap_f32_half_rows(h, &tm_dk, dK, n, batch_heads);
     if (!rc) rc = mx230_make_tmap_f32_half_rows(h, &tm_dv, dV, n, batch_heads);
     if (rc) return rc;
-    if (!dq_is_zero && (rc = launch_zero(st, dQ, (size_t)batch_heads * n * HD))) return rc;
+    if (!dq_is_zero && (rc = launch_zero(h, st, dQ, (size_t)batch_heads * n * HD))) return rc;
     BwdParams P{L, Delta, dK, dV, dQ, nullptr, nullptr, n, causal ? 1 : 0, h->status_dev};
     // persistent: one CTA per SM (the kernel holds all of an SM's tensor memory) walks its share of the items, the
     // next item's owned and first streamed tiles loading under the current item's last ones
@@ -1000,7 +1002,7 @@ int bwd_fp32(mx230_handle *h, void *stream, const float *Q, const float *K, cons
         // the forward's bf16 copies of these very tensors are still in the workspace: only dO is staged, and not even
         // that when the Delta pre-pass of this dO has left its bf16 copy in the fourth slot
         if (h->staged.d_o == dO) {
-            if (fused && (rc = launch_zero((cudaStream_t)stream, dQ, (size_t)batch_heads * n * HD))) return rc;
+            if (fused && (rc = launch_zero(h, (cudaStream_t)stream, dQ, (size_t)batch_heads * n * HD))) return rc;
         } else {
             h->staged.d_o = nullptr;   // the slot is about to hold another tensor's copy
             rc = mx230_launch_cast(h, (cudaStream_t)stream, src + 3, dst + 3, 1, batch_heads, (size_t)n * HD,

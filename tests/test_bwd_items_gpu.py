@@ -3,6 +3,7 @@ the place of a streamed tile.  Items of one, two and three streamed tiles in eve
 import pytest
 import torch
 
+from mx230_b200 import _lib
 from mx230_b200 import flash_attention as fa
 
 pytestmark = pytest.mark.gpu
@@ -52,3 +53,40 @@ def test_every_head_equals_itself_alone(handle, heads, n, causal, bf16):
         want = torch.autograd.grad(torch.softmax(s, -1) @ x[2], x, do[h].double())
         for got, w in zip((dq[h], dk[h], dv[h]), want):
             assert (got.double() - w).norm() / w.norm() <= 1e-2
+
+
+def test_profile_has_every_launch(handle):
+    """The kernel that clears dQ where no staging launch does is in the profile; the launch count leaves it out, as it would the
+    memset in whose place it stands."""
+    heads, n = 3, 200
+    x = [torch.randn(heads, n, 64, device="cuda") for _ in range(4)]
+    b = [t.bfloat16() for t in x]
+    o, dq, dk, dv = (torch.empty_like(x[0]) for _ in range(4))
+    l, delta = (torch.empty(heads, n, device="cuda") for _ in range(2))
+
+    def counted(f):
+        l0 = handle.launches
+        handle.profile_reset()
+        handle.profile_enable(True)
+        f()
+        handle.profile_enable(False)
+        prof = {k: v[0] for k, v in handle.profile_read().items()}
+        assert handle.launches - l0 == sum(prof.values()) - prof.get("zero_kernel", 0)
+        return prof
+
+    fa.run_flash_bf16(handle, *b[:3], o, l, n, True)
+    fa.run_preprocess(handle, x[3], o, delta, n)
+    got = counted(lambda: fa.run_bwd_flash_bf16(handle, *b, l, delta, dq, dk, dv, n, True))
+    assert got == {"zero_kernel": 1, "bwd_fused_kernel": 1}
+    handle.reserve(fa.workspace_bytes(heads, n, True))
+    handle.set_option(_lib.OPT_BWD_REUSE_STAGED, 1)
+    try:
+        fa.run_flash_lse(handle, *x[:3], o, l, n, True)
+        fa.run_preprocess(handle, x[3], o, delta, n)
+        got = counted(lambda: fa.run_bwd_flash(handle, *x, l, delta, dq, dk, dv, n, True))
+    finally:
+        handle.set_option(_lib.OPT_BWD_REUSE_STAGED, 0)
+    assert got == {"zero_kernel": 1, "bwd_fused_kernel": 1}
+    got = counted(lambda: fa.run_bwd_flash(handle, *x, l, delta, dq, dk, dv, n, True))
+    assert got == {"cast_bf16_kernel": 1, "bwd_fused_kernel": 1}
+    handle.check_status()
