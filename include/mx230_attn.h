@@ -74,11 +74,11 @@ enum {
                                     4000000 = 4e9 cycles, about 2 s); on expiry the kernel records a status and
                                     returns (mx230_check_status -> MX230_ERR_DEVICE_STATUS).  Synchronises the device */
     MX230_OPT_TEST_DROP_TILE = 7 /* test hook, default -1 = off: while set, the TMA producer of CTA 0 of a flash forward /
-                                    fused backward launch never requests its value-th streamed tile, and CTA `value`
-                                    of the first group of a decode launch (first 64 columns of a projection) that merges
-                                    by thread-block clusters never sends its sums, so that the bounded wait of their
-                                    consumer runs out and the abort path executes: the heads that lack sums become
-                                    NaN, the columns of a projection are not written */
+                                    fused backward launch never requests its value-th streamed tile, and in a launch that
+                                    merges by thread-block clusters CTA `value` of the first decode group (the first 64
+                                    columns of a projection) waits for sums that nobody sends, so that the bounded wait
+                                    of their consumer runs out and the abort path executes: the heads that lack sums
+                                    become NaN, the columns of a projection are not written */
 };
 
 /* kernel ids of the profiling interface */

@@ -32,7 +32,7 @@ struct mx230_handle {
     void *ws;              // workspace: bf16 operand staging / split-KV partials
     size_t ws_bytes;
     int *status_dev;       // [8] device words: [0..3] status (0 = ok), [4..5] the wait limit in SM cycles (64-bit)
-    int test_drop_tile;    // test hook: streamed tile that CTA 0's producer never requests, CTA that sends nothing to its cluster (-1 = off)
+    int test_drop_tile;    // test hook: streamed tile that CTA 0's producer never requests, CTA that waits for sums that its cluster never sends (-1 = off)
     int wide_fit[9];       // [c]: clusters of c eight-warp fp32 decode CTAs that the device holds at once
     unsigned *counters;    // split-KV arrival counters (self-resetting)
     size_t n_counters;
@@ -317,18 +317,21 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 }
 
 // Wait for the stores of the other CTAs of a cluster that complete the first phase of this CTA's barrier; by whole warps (a thread
-// in a cluster barrier waits for the rest of its warp, which may be on its way to a barrier of the CTA).  Every thread of the
-// cluster calls cluster_arrive_relaxed() behind its last such store.  Where they are late, the warp first waits until all are
-// issued: a CTA that left before them would be stored into after its end.  (That barrier is the hardware's and ends, since no
-// CTA waits for another in front of its own stores.)  Only then, bounded, until they have landed: a microsecond or two, so they
-// are given LANDING_CYCLES whatever smaller bound the caller has set.  Costs a launch 0.1 us against a plain bounded wait
-// (host-launched step over 777 fp32 keys 6.5 -> 6.6 us, token of 24 layers over 2000 int8 keys 229.0 -> 231.1).
+// in a cluster barrier waits for the rest of its warp).  Where they are late, the warp first waits until all are issued: a CTA that
+// left before them would be stored into after its end.  It does so in the cluster's barrier, which waits for every thread that has
+// not ended.  ARRIVED: every thread of the cluster has called cluster_arrive_relaxed() behind its last such store.  Else: those that
+// do not call this function end behind theirs.  Either way the barrier, the hardware's, completes, since no CTA waits for another
+// in front of its own stores.  Only then, bounded, until they have landed: a microsecond or two, so they are given LANDING_CYCLES
+// whatever smaller bound the caller has set.  Against a bounded wait alone, us: host-launched step over 777 fp32 keys 6.66 -> 6.73,
+// token of 24 layers over 2000 int8 keys 228.5 -> 229.3; arrivals in the projections as well would cost those 0.1 of 3 to 4.6.
 constexpr int CLUSTER_POLLS = 64;
+template <bool ARRIVED>
 __device__ __forceinline__ bool cluster_sums_wait(uint32_t bar, volatile int *abort_flag, int *status) {
     bool ok = false;
 #pragma unroll 1
     for (int poll = 0; poll < CLUSTER_POLLS && !ok; ++poll) ok = mbar_try_wait<true>(bar, 0);
     if (__all_sync(0xFFFFFFFFu, ok)) return true;
+    if (!ARRIVED) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     return __all_sync(0xFFFFFFFFu, mbar_wait<true>(bar, 0, abort_flag, status));
 }

@@ -63,7 +63,7 @@ struct DecodeParams {
     // 19.9; one int8 sequence in a 24-layer token, 64 CTAs: 259 / 245 / 272).
     int trigger;
     int *status;         // where a wait within a cluster that ran out is recorded
-    int test_drop;       // test hook: CTA (x) of the first group that never sends its totals to its cluster; -1 = off
+    int test_drop;       // test hook: CTA (x) of the first group that waits for totals that nobody sends; -1 = off
     int wide;            // fp32 cache: CTAs of F32_WARPS_WIDE warps
     int bs_shift;        // log2(bs) when bs is a power of two, else -1
     // fused step (RoPE and KV write of the new token inside the attention kernel): keys [0, pos) come from the cache,
@@ -299,14 +299,15 @@ struct ClusterMerge {
 __device__ __forceinline__ int merge_heads(int gc, int rank, int C) { return gc > rank ? (gc - rank + C - 1) / C : 0; }
 // Before the first push, by every thread of every CTA of the cluster.  (A push may reach a barrier before its owner has stated
 // the bytes to expect: the phase stays open until it has.)
-__device__ __forceinline__ void merge_open(ClusterMerge &X, int gc, int rank, int C) {
+__device__ __forceinline__ void merge_open(const DecodeParams &P, ClusterMerge &X, int gc, int rank, int C) {
     if (C == 1) return;
     if (threadIdx.x == 0) {
         X.aborted = 0;
         const uint32_t bar = mx::smem_u32(&X.bar);
         mx::mbar_init(bar, 1);
         mx::mbar_fence_init();
-        mx::mbar_expect_tx(bar, merge_heads(gc, rank, C) * C * 68 * 4);
+        const int never = P.test_drop == (int)blockIdx.x && blockIdx.y + blockIdx.z == 0 ? 16 : 0;
+        mx::mbar_expect_tx(bar, merge_heads(gc, rank, C) * C * 68 * 4 + never);
     }
     mx::cluster_arrive_relaxed();   // waited for before the first push
 }
@@ -353,7 +354,7 @@ __device__ void finish_group(const DecodeParams &P, const float *mg, ClusterMerg
         if (C == 1) {
             emit(g, d, mm, lt, a);
             if (q_rot && active == 1) put_q(g, d);
-        } else if (P.test_drop != (int)blockIdx.x || blockIdx.y + blockIdx.z > 0) {
+        } else {
             const int r = g % C;
             const uint32_t dst = mx::cluster_map(mx::smem_u32(X.rows + (g / C * C + rank) * 68), r);
             const uint32_t bar = mx::cluster_map(mx::smem_u32(&X.bar), r);
@@ -366,7 +367,12 @@ __device__ void finish_group(const DecodeParams &P, const float *mg, ClusterMerg
         mx::cluster_arrive_relaxed();   // this thread's stores are issued
     }
     if (C > 1 && merge_heads(gc, rank, C) * 16 > (tid & ~31)) {
-        const bool ok = mx::cluster_sums_wait(mx::smem_u32(&X.bar), &X.aborted, P.status);
+        if (!mx::cluster_sums_wait<true>(mx::smem_u32(&X.bar), &X.aborted, P.status)) {
+            // totals that never came: these heads become NaN, also in the workspace, where an earlier call's rows would pass for them
+            for (int i = tid; (i >> 4) * C + rank < gc; i += nt)
+                if ((i & 15) < C) *(float4 *)(X.rows + ((i >> 4) * C + (i & 15)) * 68) = make_float4(0.f, CUDART_NAN_F, 0.f, 0.f);
+            __syncwarp();
+        }
         for (int i = tid; (i >> 4) * C + rank < gc; i += nt) {
             const int g = (i >> 4) * C + rank, d = (i & 15) * 4;
             float4 hd[8], ap[8];
@@ -389,8 +395,6 @@ __device__ void finish_group(const DecodeParams &P, const float *mg, ClusterMerg
                 lt += hd[p].y * wgt;
                 a.x += ap[p].x * wgt, a.y += ap[p].y * wgt, a.z += ap[p].z * wgt, a.w += ap[p].w * wgt;
             }
-            // totals that never came: NaN, also in the workspace, where rows of an earlier call would pass for this one's
-            if (!ok) mm = 0.0f, lt = CUDART_NAN_F, a = make_float4(CUDART_NAN_F, CUDART_NAN_F, CUDART_NAN_F, CUDART_NAN_F);
             emit(g, d, mm, lt, a);
             if (q_rot && active == 1) put_q(g, d);
         }
@@ -881,7 +885,7 @@ decode_q8_mma_kernel(const DecodeParams P) {
     const int cl = blockIdx.x / P.cl_size, rank = blockIdx.x - cl * P.cl_size;
 
     const float freq = FUSED ? mx::rope_freq(lane, 64, P.theta) : 0.0f;
-    merge_open(X, gc, rank, P.cl_size);
+    merge_open(P, X, gc, rank, P.cl_size);
     if (P.push_regions == nullptr) mx::pdl_wait();   // (a split-KV step, whose CTAs wait for other ranks, is launched plainly)
     // q: requested before the position, whose chain of dependent loads (position, table, first tile) it then runs beside
     float qa_raw = 0.0f, qb_raw = 0.0f;   // warp = head (Q8_WARPS == MG)
@@ -1223,7 +1227,7 @@ decode_f32_ring_kernel(const DecodeParams P) {
     const int cl = blockIdx.x / P.cl_size, rank = blockIdx.x - cl * P.cl_size;
 
     const float freq = FUSED && P.use_rope ? mx::rope_freq(lane, 64, P.theta) : 0.0f;
-    merge_open(X, gc, rank, P.cl_size);
+    merge_open(P, X, gc, rank, P.cl_size);
     if (P.push_regions == nullptr) mx::pdl_wait();   // (a split-KV step, whose CTAs wait for other ranks, is launched plainly)
     // q: requested before the position, whose chain of dependent loads (position, table, first tile) it then runs beside
     constexpr int QH = (G + WARPS - 1) / WARPS;   // heads of a warp: warp, warp + WARPS, ...

@@ -58,7 +58,7 @@ struct GemvParams {
     float *partials;                // [n_slices][n_out]
     unsigned *counters;      // one per column block, self-resetting
     int *status;             // where a wait within a cluster that ran out is recorded
-    int test_drop;           // test hook: CTA of the first column block that never sends its sums to its cluster; -1 = off
+    int test_drop;           // test hook: >= 0: the first column block waits for sums that nobody sends
     QkvEpilogue e;
 };
 
@@ -143,7 +143,7 @@ gemv_heads_kernel(const GemvParams P) {
             aborted = 0;
             mx::mbar_init(bar, 1);
             mx::mbar_fence_init();
-            if (rank == 0) mx::mbar_expect_tx(bar, P.n_slices * PJ_COLS * 4);
+            if (rank == 0) mx::mbar_expect_tx(bar, P.n_slices * PJ_COLS * 4 + (P.test_drop >= 0 && blk == 0 ? 16 : 0));
         }
         mx::cluster_arrive_relaxed();               // waited for before the first store to another CTA's memory
     }
@@ -250,16 +250,12 @@ gemv_heads_kernel(const GemvParams P) {
         }
         // (asynchronous stores that complete the first CTA's barrier: the cluster barrier behind plain ones took 1500 cycles of
         // the 5000 of a launch)
-        if (C > 1) {
-            if (P.test_drop != (int)blockIdx.x || blk > 0)
-                mx::cluster_st_async(mx::cluster_map(mx::smem_u32(&parts[g][c]), 0), mx::cluster_map(bar, 0), sum.x, sum.y, sum.z, sum.w);
-        } else if (P.ctas == 1) *(float4 *)&parts[g][c] = sum;
+        if (C > 1) mx::cluster_st_async(mx::cluster_map(mx::smem_u32(&parts[g][c]), 0), mx::cluster_map(bar, 0), sum.x, sum.y, sum.z, sum.w);
+        else if (P.ctas == 1) *(float4 *)&parts[g][c] = sum;
         else if (col0 + c < P.n_out) *(float4 *)(P.partials + (size_t)g * P.n_out + col0 + c) = sum;   // (n_out % 4 == 0)
     }
     if (C > 1) {
-        __syncwarp();
-        mx::cluster_arrive_relaxed();   // this thread's stores are issued
-        if (!finishes) return;
+        if (!finishes) return;   // (see cluster_sums_wait)
     } else if (P.ctas > 1) {
         __threadfence();
         __syncthreads();
@@ -274,7 +270,7 @@ gemv_heads_kernel(const GemvParams P) {
     // ---- epilogue on the 64 finished sums of this column block: one warp ----
     float cs = 1.0f, sn = 0.0f;
     if (E.enabled && !is_v) mx::rope_angle(pos, freq, cs, sn);   // (while the other CTAs' sums are on their way)
-    if (C > 1 && !mx::cluster_sums_wait(bar, &aborted, P.status)) return;   // (nothing is written)
+    if (C > 1 && !mx::cluster_sums_wait<false>(bar, &aborted, P.status)) return;   // (nothing is written)
     // (a loop that is short in code as well: what runs once per launch is fetched once per launch)
     const bool in = col0 + 2 * tid < P.n_out;
     float2 sum = make_float2(0.f, 0.f);
