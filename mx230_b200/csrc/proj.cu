@@ -111,9 +111,12 @@ struct WeightRow<int8_t, 4> {
 // Grid: column blocks x CTAs, the CTAs of a block next to each other.  A slice takes 64 / CPT * 8 threads.
 // Registers: two CTAs of five slices (640 threads at four columns a thread, 320 at eight) have to fit an SM, so that the next
 // launch's are there, with their weights on the way into L2, while this one's still run: 896 -> 1152 fp32, launch after launch
-// over fresh weights, 4.6 us at 50 registers (one CTA), 3.2 at 48.
+// over fresh weights, 4.6 us at 50 registers (one CTA), 3.2 at 48.  fp16 rows of a multiple of 4 columns take six slices a CTA in
+// grids of more CTAs than SMs: two such CTAs of 768 threads at 40 registers (2048 -> 1220, launch after launch: 32 registers 4.0 us,
+// 48 5.6, 40 3.9).  int8 keeps its unpacked words in registers (1504 -> 1412: 58 registers 3.2, 48 3.6, 64 3.0; 896 -> 896 3.2, 3.2,
+// 3.0).
 template <typename WT, int CPT>
-__global__ void __maxnreg__(CPT == 8 ? 56 : 48)
+__global__ void __maxnreg__(CPT == 8 ? 56 : sizeof(WT) == 2 ? 40 : sizeof(WT) == 1 ? 64 : 48)
 gemv_heads_kernel(const GemvParams P) {
     constexpr bool I8 = sizeof(WT) == 1;
     constexpr int TPR = PJ_COLS / CPT;              // threads across a weight row
