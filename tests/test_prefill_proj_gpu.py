@@ -1,12 +1,15 @@
 """The prefill step followed by the output projection in one call: attention leaves its rows in fp16 for the projection, which
 gives the bits of the two calls in turn (the same rounding, the same products)."""
+import functools
+
 import numpy as np
 import pytest
 import torch
 
 import oracle
 from mx230_b200 import llm_attention as la
-from mx230_b200._lib import ERR_INVALID_ARG, ERR_UNSUPPORTED, Mx230Error, check, lib, ptr
+from mx230_b200._lib import (ERR_INVALID_ARG, ERR_UNSUPPORTED, OPT_Q8_SCORE_MODE, Q8_SCORE_EXACT, Q8_SCORE_REF, Mx230Error, check,
+                             lib, ptr)
 
 pytestmark = pytest.mark.gpu
 THETA = 1e6
@@ -16,38 +19,60 @@ def dev(a):
     return torch.from_numpy(np.ascontiguousarray(a)).cuda()
 
 
+@functools.lru_cache(maxsize=None)
+def normal(shape, seed):
+    return oracle.normal(shape, seed, 0)
+
+
 def caches(c):
     return [x for x in (c.k, c.v, c.ks, c.vs, c.kb, c.vb) if x is not None] if c.quant else [c.k, c.v]
 
 
 # query tiles of 128 rows: one row, either side of a tile, an odd number of tiles; both forms of the forward (40 heads: pair
-# form); output columns by whole and ragged 64-column chunks
-@pytest.mark.parametrize("quant", [False, True])
+# form); output columns by whole (stored by TMA) and ragged 64-column chunks; 1900 rows: 15 row tiles of the projection, the last
+# ragged.  Caches in order and paged; int8 in both score modes.
+@pytest.mark.parametrize("cache", ["fp32", "int8", "int8 exact"])
+@pytest.mark.parametrize("paged", [False, True])
 @pytest.mark.parametrize("nh,nkv,n_tok,pos0,n_out", [
-    (14, 2, 1, 0, 896), (14, 2, 127, 5, 72), (12, 12, 128, 0, 768), (14, 2, 129, 300, 896), (40, 8, 2050, 0, 200),
+    (14, 2, 1, 0, 896), (14, 2, 127, 5, 72), (12, 12, 128, 0, 768), (14, 2, 129, 300, 896), (14, 2, 1900, 44, 896),
+    (40, 8, 2050, 0, 200),
 ])
-def test_step_with_projection_equals_the_calls_in_turn(handle, quant, nh, nkv, n_tok, pos0, n_out):
+def test_step_with_projection_equals_the_calls_in_turn(handle, cache, paged, nh, nkv, n_tok, pos0, n_out):
+    quant = cache != "fp32"
+    handle.set_option(OPT_Q8_SCORE_MODE, Q8_SCORE_EXACT if cache == "int8 exact" else Q8_SCORE_REF)
+    try:
+        _equals_the_calls_in_turn(handle, quant, paged, nh, nkv, n_tok, pos0, n_out)
+    finally:
+        handle.set_option(OPT_Q8_SCORE_MODE, Q8_SCORE_REF)
+
+
+def _equals_the_calls_in_turn(handle, quant, paged, nh, nkv, n_tok, pos0, n_out):
     qd, row, e = nh * 64, (nh + 2 * nkv) * 64, 128
-    x = dev(oracle.normal((n_tok, e), 811, 0))
-    w_qkv = dev((oracle.normal((e, row), 812, 0) / np.sqrt(e)).astype(np.float16))
-    w_proj = dev((oracle.normal((qd, n_out), 813, 0) / np.sqrt(qd)).astype(np.float16))
-    b_proj = dev(oracle.normal((n_out,), 814, 0))
-    old = dev(oracle.normal((max(pos0, 1), 2 * nkv * 64), 815, 0))
+    x = dev(normal((n_tok, e), 811))
+    w_qkv = dev((normal((e, row), 812) / np.sqrt(e)).astype(np.float16))
+    w_proj = dev((normal((qd, n_out), 813) / np.sqrt(qd)).astype(np.float16))
+    b_proj = dev(normal((n_out,), 814))
+    old = dev(normal((max(pos0, 1), 2 * nkv * 64), 815))
     handle.reserve(la.prefill_workspace_bytes(n_tok, pos0 + n_tok, nh, nkv))
+    blocks = -(-(pos0 + n_tok) // la.KV_BLOCK)
+    table = np.random.default_rng(5).permutation(blocks).astype(np.int32)
+    pg = la.Paging(dev(table)) if paged else None
+    at = np.arange(pos0)   # the cache rows of the old positions
+    at = dev(table[at // la.KV_BLOCK] * la.KV_BLOCK + at % la.KV_BLOCK).long() if paged else slice(0, pos0)
     got = []
     for fused in (False, True):
-        c = la.KvCache(pos0 + n_tok, nkv, 64, quant)
+        c = la.KvCache(blocks * la.KV_BLOCK, nkv, 64, quant)
         if quant:
-            la.quantize_kv_batch(handle, c, old, 0, pos0, 0, nkv, 64, 2 * nkv * 64)
+            la.quantize_kv_batch(handle, c, old, 0, pos0, 0, nkv, 64, 2 * nkv * 64, pg)
         else:
-            c.k[:pos0], c.v[:pos0] = old[:pos0, :nkv * 64], old[:pos0, nkv * 64:]
+            c.k[at], c.v[at] = old[:pos0, :nkv * 64], old[:pos0, nkv * 64:]
         qkv, attn = torch.zeros(n_tok, row, device="cuda"), torch.full((n_tok, qd), float("nan"), device="cuda")
         y = torch.full((n_tok, n_out), float("nan"), device="cuda")
         if fused:
-            la.prefill_layer_attention(handle, y, x, w_qkv, None, w_proj, b_proj, qkv, attn, c, pos0, n_tok, nh, nkv, 64, THETA)
+            la.prefill_layer_attention(handle, y, x, w_qkv, None, w_proj, b_proj, qkv, attn, c, pos0, n_tok, nh, nkv, 64, THETA, pg)
         else:
             la.gemm(handle, qkv, x, w_qkv)
-            la.prefill_step(handle, attn, qkv, c, pos0, n_tok, nh, nkv, 64, THETA, row, qd)
+            la.prefill_step(handle, attn, qkv, c, pos0, n_tok, nh, nkv, 64, THETA, row, qd, pg)
             la.gemm(handle, y, attn, w_proj, b_proj)
         handle.check_status()
         got.append([y, attn, qkv] + caches(c))
