@@ -58,9 +58,9 @@ struct DecodeParams {
     // follows the length of each sequence and not only the largest one
     int cl_size, max_clusters, cluster_keys;
     // Let the next kernel of the stream in once this one's loops are done: only a grid that leaves SMs free.  After a larger
-    // one the next grid's CTAs would fill the slots that fall free first and sit unevenly on the SMs (8 x 131072 int8 keys
-    // step after step: 116 us with the trigger at the top, 105 here, 100 without; 16 fp32 sequences of 1500 keys 23.1 / 22.8 /
-    // 19.9; one int8 sequence in a 24-layer token, 64 CTAs: 259 / 245 / 272).
+    // one the next grid's CTAs would fill the slots that fall free first and sit unevenly on the SMs (when clusters still merged
+    // through the workspace, trigger at the top / here / none: 8 x 131072 int8 keys step after step 116 / 105 / 100 us, 16 fp32
+    // sequences of 1500 keys 23.1 / 22.8 / 19.9).  One int8 sequence in a 24-layer token, 64 CTAs: here 229, none 253.
     int trigger;
     int *status;         // where a wait within a cluster that ran out is recorded
     int test_drop;       // test hook: CTA (x) of the first group that waits for totals that nobody sends; -1 = off

@@ -12,7 +12,7 @@ struct DecodeSplit {
 //  * whole grid resident at once: cl_size * max_clusters * groups <= slots (a partial second wave would nearly double
 //    the time);
 //  * up to 8 CTAs of a group (any number, so that 6 per group fill 444 slots where 4 would leave a third of them empty) form
-//    a cluster, whose merge costs one cluster barrier; pass_keys = keys that a CTA's warps
+//    a cluster, merged by asynchronous stores into one another's shared memory; pass_keys = keys that a CTA's warps
 //    take in one tile each: a CTA is not given less than one such pass;
 //  * further clusters join in (merge through global memory, about 2 us) only for sequences with more than 4 passes per
 //    CTA of the first; the kernel decides that per sequence from its actual length;

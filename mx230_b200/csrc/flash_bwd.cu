@@ -64,7 +64,7 @@ constexpr int BWD_THREADS = 512;
 #endif
 #ifndef BWD_SECOND_AT
 #define BWD_SECOND_AT 24   // columns of the first piece that are done when the second one is taken as landed and X, Y are handed back
-                           // (step of 48 x 4096 rows causal 527, 525, 520, 522 us at 8, 16, 24, 32; 24 x 2048 bf16 148, 150, 145, 148)
+                           // (24 against 32, back to back: 48 x 4096 rows causal 539 / 537 us, 24 x 2048 bf16 142.4 / 142.3: level)
 #endif
 #ifndef BWD_POLY
 #define BWD_POLY 0         // fused pass: of every four column pairs, how many take 2^x from the FMA-pipe polynomial
@@ -320,8 +320,9 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmOwnA, const __grid_constant__ C
                             // The item's owned tiles, behind its first streamed one: V once the previous item's last Y is
                             // complete, K once the tile before the previous item's last is consumed -- both while that item
                             // still runs, so that this one's first X, Y are ready when its exponentials are.  (Loaded after
-                            // ACC_DONE, the streamed tiles queued behind them: step of 48 x 4096 rows causal 530 us against
-                            // 520, 24 x 2048 bf16 150 against 145.)
+                            // ACC_DONE, the streamed tiles queued behind them.  It is worth little: three seconds back to back,
+                            // 48 x 4096 rows causal 884 -> 871 thousand SM cycles a step, under the power limit 538 -> 535 us;
+                            // 24 x 2048 bf16 142.6 -> 144.1, both within what runs of one build differ.)
                             ok = __all_sync(0xFFFFFFFFu, mx::mbar_wait(bar(BAR_OWN_B_FREE), (it - 1) & 1, abort_flag, P.status));
                             if (!ok) break;
                             if (lane == 0) {
@@ -830,8 +831,9 @@ __global__ void bwd_preprocess_kernel(const float *dO, const float *O, float *De
 }
 
 // dQ = 0 in front of the fused pass where no staging launch clears it on the way.  A kernel and not a memset, so that it and the
-// fused pass are launched programmatically (us a step, memset / this: 12 x 1000 bf16 40.6 / 38.2, 12 x 1000 39.9 / 37.1, 48 x 4096
-// causal 485 / 480).
+// fused pass are launched programmatically.  That is where dO is not staged by this call: bf16 operands, or the forward's and the
+// pre-pass's copies reused (us a step back to back, memset / this: 12 x 1000 causal bf16 36.0 / 33.6, reusing 37.6 / 35.6; 48 x 4096
+// reusing 535 / 538, 24 x 2048 bf16 144 / 142: level).
 constexpr int ZERO_THREADS = 256, ZERO_UNROLL = 4;
 __global__ void __launch_bounds__(ZERO_THREADS) zero_kernel(float4 *p, size_t n4) {
     mx::pdl_trigger();

@@ -348,10 +348,10 @@ int launch_gemv(mx230_handle *h, void *stream, GemvParams P, int w_kind, const c
     const int gran = w_kind == 2 ? 4 * PJ_ROWLANES : PJ_ROWLANES;
     P.rows_per_slice = ((P.n_in + n_slices - 1) / n_slices + gran - 1) / gran * gran;
     P.n_slices = n_slices = (P.n_in + P.rows_per_slice - 1) / P.rows_per_slice;
-    // CTAs: up to 64 slices are one cluster per block, a few slices per CTA; the merge is then a cluster barrier.  Measured
+    // CTAs: up to 64 slices are one cluster per block, a few slices per CTA, merged by asynchronous stores.  Measured
     // on one token through 24 layers (fp16 896 x 1152 and 896 x 896, 38 and 56 slices, int8 cache of 2001 keys, one graph):
     // a CTA per slice and a merge through the workspace 10.5 and 9.4 us per launch, 536 us per token; this and programmatic
-    // launches of this kernel and the attention kernel, 268 us.  More slices (few columns, many rows) are merged
+    // launches of this kernel and the attention kernel, 229 us.  More slices (few columns, many rows) are merged
     // through the workspace.
     const bool wide = w_kind == 1 && P.n_out % 8 == 0;   // fp16 rows of whole 16-byte pieces
     if (n_slices <= PJ_CLUSTER * PJ_SLOTS) {
