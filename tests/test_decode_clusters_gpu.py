@@ -12,7 +12,7 @@ from tests.test_decode_gpu import TOL, build_caches, dev, to_dev_f32, to_dev_q8
 pytestmark = pytest.mark.gpu
 
 
-# groups of 7, 8, 3, 5, 1 heads; with 20 K/V heads the fp32 CTAs have four warps, below 19 eight
+# groups of 7, 8, 3, 5, 1 heads; with 20 K/V heads the fp32 CTAs have four warps, in the other calls eight
 @pytest.mark.parametrize("nh,nkv", [(7, 1), (8, 1), (3, 1), (10, 2), (5, 5), (20, 20)])
 def test_every_cluster_size(handle, nh, nkv):
     rows, kc, vc, q8 = build_caches(nh, nkv, 2049, 41)
