@@ -322,8 +322,8 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 // not ended.  ARRIVED: every thread of the cluster has called cluster_arrive_relaxed() behind its last such store.  Else: those that
 // do not call this function end behind theirs.  Either way the barrier, the hardware's, completes, since no CTA waits for another
 // in front of its own stores.  Only then, bounded, until they have landed: a microsecond or two, so they are given LANDING_CYCLES
-// whatever smaller bound the caller has set.  Against a bounded wait alone, us: host-launched step over 777 fp32 keys 6.66 -> 6.73,
-// token of 24 layers over 2000 int8 keys 228.5 -> 229.3; arrivals in the projections as well would cost those 0.1 of 3 to 4.6.
+// whatever smaller bound the caller has set.  Against a bounded wait alone, us: host-launched step over 777 fp32 keys 6.67 -> 6.77,
+// token of 24 layers over 2000 int8 keys 228.5 -> 228.7; arrivals in the projections as well would cost those 0.1 of 3 to 4.6.
 constexpr int CLUSTER_POLLS = 64;
 template <bool ARRIVED>
 __device__ __forceinline__ bool cluster_sums_wait(uint32_t bar, volatile int *abort_flag, int *status) {
