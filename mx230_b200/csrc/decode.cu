@@ -151,6 +151,13 @@ __device__ __forceinline__ void split_range(int kbeg, int kend, int c, int n, in
     if (b < a) b = a;
 }
 
+// Share c of n of `total` tiles, [a, b): the first ones get what does not divide.
+__device__ __forceinline__ void even_share(int total, int c, int n, int &a, int &b) {
+    const int per = total / n, more = total - per * n;
+    a = c * per + min(c, more);
+    b = a + per + (c < more);
+}
+
 // Final or partial write of one (sequence, kv head) group from merged values held
 // by the first threads of the CTA.
 template <int G>
@@ -1181,11 +1188,17 @@ decode_q8_mma_kernel(const DecodeParams P) {
 //
 // A CTA of four warps (eight in calls with few groups) owns one (key split, kv head, sequence); each warp streams its own key
 // sub-range in tiles of 16 keys (K and V rows, 8 KB) through a private two-stage cp.async ring.
-//   scores:  lane = (key, half of the 64 dims); the halves are added with one shuffle per head;
-//            running max per head raised lazily, as in the int8 kernel;
-//   values:  lane = (key lane of 4, 8-dim slice), weights through a per-warp shared buffer.
-// K rows are XOR-swizzled by key, V rows fold their upper half, so both read patterns are
-// bank-conflict free.  Three CTAs are resident per SM.
+//   lane = (key lane of 4, 8-dim slice) for scores and values alike: q of every head in registers, a K or V row's 256 bytes
+//            read once by eight lanes (no swizzle: a lane's two 16-byte pieces are 128 bytes apart);
+//   scores:  a lane's parts of q . k for all heads, summed over the eight lanes by handing on half of them at a time, which
+//            leaves one head in each; running max per head raised lazily, as in the int8 kernel;
+//   values:  weights through a per-warp shared buffer.
+// What bounds it: multiply-adds (2 * G * 64 per key, packed in pairs) beside a stream that a tile's worth of latency per warp
+// keeps going.  In its place lane = (key, half of the dims) read q from shared memory for every key: 88 16-byte reads a lane
+// and tile where 24 do, and 168 shuffles for a warp's totals where 52 do.  us a call, before / after: one sequence, host
+// position, 14/2 heads 1500 keys 8.1 / 6.1, 32/4 heads 4000 keys 13.0 / 9.0; 16 paged sequences of up to 1500 keys, 32/4 heads
+// 17.8 / 16.0; 1 x 32768 keys 14/2 heads 16.2 / 13.0; one K/V head per query head level.  Error against 64 bits 1.3e-7 to
+// 1.9e-7 where it was 1.5e-7 to 2.1e-7.  Three CTAs are resident per SM.
 // ---------------------------------------------------------------------------
 constexpr int F32_WARPS = 4;
 constexpr int F32_WARPS_WIDE = 8;                    // calls that leave most of the SMs empty: see launch_decode
@@ -1213,7 +1226,7 @@ decode_f32_ring_kernel(const DecodeParams P) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     float *qf = (float *)smem_raw;                        // [G][64]
     unsigned char *warp_base = smem_raw + ((SM::Q_BYTES + 127) & ~127);
-    __shared__ float new_k[64], new_v[64];                // fused step: the new token's rows (owning CTA)
+    __shared__ __align__(16) float new_k[64], new_v[64];             // fused step: the new token's rows (owning CTA)
     __shared__ __align__(16) ClusterMerge X;
     __shared__ int is_last;
 
@@ -1251,17 +1264,16 @@ decode_f32_ring_kernel(const DecodeParams P) {
         return;
     }
     const int n_splits = active * P.cl_size;
-    split_range(kbeg, kend, blockIdx.x, n_splits, ka, kb_);
+    even_share((kend - kbeg + FT_KEYS - 1) / FT_KEYS, blockIdx.x, n_splits, ka, kb_);   // in tiles
     const int *table = PAGED ? P.tables + (P.pos_kind == 2 ? (size_t)s * P.n_log : 0) : nullptr;
     const long long base = PAGED ? 0 : (long long)s * P.seq_rows;
     const float scale = 0.125f * LOG2E;  // scores are kept in the log2 domain
 
     // ---- this warp's key sub-range ----
-    const int n_keys = kb_ - ka;
-    int per_w = (n_keys + WARPS - 1) / WARPS;
-    per_w = (per_w + FT_KEYS - 1) & ~(FT_KEYS - 1);
-    const int wa = min(kb_, ka + warp * per_w), wb = min(kb_, wa + per_w);
-    const int n_tiles = (wb - wa + FT_KEYS - 1) / FT_KEYS;
+    int ta, tb;
+    even_share(kb_ - ka, warp, WARPS, ta, tb);
+    const int wa = kbeg + (ka + ta) * FT_KEYS, wb = min(kend, kbeg + (ka + tb) * FT_KEYS);
+    const int n_tiles = tb - ta;
     unsigned char *ring = warp_base + warp * SM::PER_WARP;
     float *wbuf = (float *)(ring + FT_STAGES * FT_STAGE);
     const uint32_t ring_u32 = mx::smem_u32(ring);
@@ -1269,62 +1281,53 @@ decode_f32_ring_kernel(const DecodeParams P) {
     // Lane l moves 16-byte pieces l, l+32, ... of the tile's K rows and V rows: piece p of a matrix is
     // (key = p / 16, chunk = p % 16) = (it*2 + l/16, l%16).
     const int pk = lane >> 4, pc = lane & 15;
-    auto k_off = [&](int key) { return (uint32_t)(key * 256 + (((pc & 8) | ((pc ^ key) & 7)) << 4)); };
-    const uint32_t v_chunk = (uint32_t)((pc ^ (pc >> 3)) << 4);
-    const float *ksrc = nullptr, *vsrc = nullptr;
-    if (!PAGED) {
-        size_t r0 = (size_t)(base + wa);
-        ksrc = P.kcache + (r0 + pk) * kvd + kvh * 64 + pc * 4;
-        vsrc = P.vcache + (r0 + pk) * kvd + kvh * 64 + pc * 4;
-    }
-    const size_t it_stride = (size_t)2 * kvd, tile_stride = (size_t)FT_KEYS * kvd;
-    // paged caches: lane l looks up the row of key l (mod 16) of the next tile one tile ahead, as in the int8 kernel
+    const uint32_t piece = (uint32_t)(pk * 256 + pc * 16);
+    const size_t it_stride = (size_t)2 * kvd;
+    // Paged caches: a tile that lies in one cache block has consecutive rows and takes one lookup, the same in all lanes; else lane
+    // l looks up the row of key l (mod 16).  Either way one tile ahead, off the chain of dependent loads.
+    const bool whole = !PAGED || (P.bs % FT_KEYS == 0 && kbeg % FT_KEYS == 0);
     auto row_ahead = [&](int tile) {
-        const int t = wa + tile * FT_KEYS + pc;
+        const int t0 = wa + tile * FT_KEYS, t = t0 + (whole ? 0 : pc);
         return paged_row(P, table, t < wb ? t : wa);
     };
     int row_l = 0;
     if (PAGED && n_tiles > 0) row_l = row_ahead(0);
 
-    auto issue = [&](int tile) {
-        const uint32_t dst = ring_u32 + (tile % FT_STAGES) * FT_STAGE;
-        const int key0 = wa + tile * FT_KEYS;
-        if (PAGED) {
+    // A tile's K rows and its V rows are requested, waited for and replaced apart: while one half of a slot is worked on three
+    // of the warp's four are in flight (both together: two)
+    auto issue = [&](int tile, bool is_v) {
+        if (tile < n_tiles) {
+            const uint32_t dst = ring_u32 + (tile % FT_STAGES) * FT_STAGE + (is_v ? FT_KEYS * 256 : 0) + piece;
+            const float *cache = (is_v ? P.vcache : P.kcache) + kvh * 64 + pc * 4;
+            const int key0 = wa + tile * FT_KEYS;
+            if (whole) {
+                const float *src = cache + ((PAGED ? (long long)row_l : base + key0) + pk) * kvd;
+                if (key0 + FT_KEYS <= wb) {
 #pragma unroll
-            for (int it = 0; it < 8; ++it) {
-                const int key = it * 2 + pk;
-                const size_t off = (size_t)__shfl_sync(0xFFFFFFFFu, row_l, key) * kvd + kvh * 64 + pc * 4;
-                const int n = key0 + key < wb ? 16 : 0;
-                cp_async16(dst + k_off(key), P.kcache + off, n);
-                cp_async16(dst + FT_KEYS * 256 + key * 256 + v_chunk, P.vcache + off, n);
+                    for (int it = 0; it < 8; ++it) cp_async16(dst + it * 512, src + it * it_stride, 16);
+                } else {
+#pragma unroll
+                    for (int it = 0; it < 8; ++it) {
+                        const bool ok = key0 + it * 2 + pk < wb;
+                        cp_async16(dst + it * 512, ok ? src + it * it_stride : cache, ok ? 16 : 0);
+                    }
+                }
+            } else {
+#pragma unroll
+                for (int it = 0; it < 8; ++it) {
+                    const int key = it * 2 + pk;
+                    const size_t off = (size_t)__shfl_sync(0xFFFFFFFFu, row_l, key) * kvd;
+                    cp_async16(dst + it * 512, cache + off, key0 + key < wb ? 16 : 0);
+                }
             }
-            if (tile + 1 < n_tiles) row_l = row_ahead(tile + 1);
-            return;
+            if (PAGED && is_v && tile + 1 < n_tiles) row_l = row_ahead(tile + 1);
         }
-        if (key0 + FT_KEYS <= wb) {  // full tile of a linear cache: no predicates
-#pragma unroll
-            for (int it = 0; it < 8; ++it) {
-                const int key = it * 2 + pk;
-                cp_async16(dst + k_off(key), ksrc + it * it_stride, 16);
-                cp_async16(dst + FT_KEYS * 256 + key * 256 + v_chunk, vsrc + it * it_stride, 16);
-            }
-        } else {
-#pragma unroll
-            for (int it = 0; it < 8; ++it) {
-                const int key = it * 2 + pk;
-                const int t = key0 + key;
-                const bool ok = t < wb;
-                const size_t off = (size_t)(base + (ok ? t : wa)) * kvd + kvh * 64 + pc * 4;
-                cp_async16(dst + k_off(key), P.kcache + off, ok ? 16 : 0);
-                cp_async16(dst + FT_KEYS * 256 + key * 256 + v_chunk, P.vcache + off, ok ? 16 : 0);
-            }
-        }
-        ksrc += tile_stride, vsrc += tile_stride;
+        cp_async_commit();
     };
 
-    // the first tile is requested before the q prologue, whose latency then runs under it
-    if (n_tiles > 0) issue(0);
-    cp_async_commit();
+    // the first tiles are requested before the q prologue, whose latency then runs under them
+#pragma unroll
+    for (int t = 0; t < FT_STAGES; ++t) issue(t, false), issue(t, true);
 
     const bool owner = FUSED && (int)blockIdx.x == n_splits - 1;   // the CTA that takes the new token's own key
     {
@@ -1350,75 +1353,111 @@ decode_f32_ring_kernel(const DecodeParams P) {
     }
     __syncthreads();
 
-    float m_run[G], l_thr[G];
-    float acc[G][8];
+    // ---- lane = (key lane kl of 4, dim slice dsl of 8): dims 4 dsl .. 4 dsl + 3 and 32 further on, as two float4s, of q (in
+    // registers for every head), of a key's K row and of its V row ----
+    const int kl = lane >> 3, dsl = lane & 7;
+    constexpr int GR = G > 4 ? 8 : G;                     // heads the score exchange works on: 1, 2, 4 or 8
+    // What a lane ends up with: the scores of one head, its own, for its key lane's key of every step; with one or two heads,
+    // which eight lanes share too often that way, for one key: that of step dsl / 2.
+    constexpr bool ONE_KEY = GR <= 2;
+    constexpr int NK = ONE_KEY ? 1 : FT_KEYS / 4;
+    constexpr int HS = GR == 8 ? 0 : 1;
+    const int own_head = ONE_KEY ? dsl & (GR - 1) : dsl >> HS;
+    const int key0_l = (ONE_KEY ? (dsl >> 1) * 4 : 0) + kl;   // its first key in a tile, the next ones 4 further on
+    constexpr int OWN_LANES = ONE_KEY ? 2 : 8;                // lanes that differ in this bit or a higher one share their head
+    uint64_t q2[G][4];
 #pragma unroll
     for (int g = 0; g < G; ++g) {
-        m_run[g] = -CUDART_INF_F;
-        l_thr[g] = 0.0f;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[g][j] = 0.0f;
+        const ulonglong2 lo = *(const ulonglong2 *)(qf + g * 64 + dsl * 4), hi = *(const ulonglong2 *)(qf + g * 64 + 32 + dsl * 4);
+        q2[g][0] = lo.x, q2[g][1] = lo.y, q2[g][2] = hi.x, q2[g][3] = hi.y;
     }
-
-    const int sk = lane & 15, sh = lane >> 4;          // scores: key, dim half
-    const int kl = lane >> 3, dsl = lane & 7;          // values: key lane, 8-dim slice
-    const uint32_t vo0 = (uint32_t)(((2 * dsl) ^ ((2 * dsl) >> 3)) << 4);
-    const uint32_t vo1 = (uint32_t)(((2 * dsl + 1) ^ ((2 * dsl + 1) >> 3)) << 4);
-    for (int tile = 0; tile < n_tiles; ++tile) {
-        if (tile + 1 < n_tiles) issue(tile + 1);
-        cp_async_commit();
-        cp_async_wait<1>();
-        __syncwarp();
-        const unsigned char *st = ring + (tile % FT_STAGES) * FT_STAGE;
-        const bool ok = wa + tile * FT_KEYS + sk < wb;
-
-        // ---- scores (log2 domain): this lane's half of its key's row against the G heads ----
-        float d0[G], d1[G];
+    // the part of q . k that this lane's dims make, for every head; `row`: the lane's first piece of the key's row
+    auto parts = [&](const unsigned char *row, float (&d)[GR]) {
+        const ulonglong2 lo = *(const ulonglong2 *)row, hi = *(const ulonglong2 *)(row + 128);
 #pragma unroll
-        for (int g = 0; g < G; ++g) d0[g] = d1[g] = 0.0f;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const float4 kv = *(const float4 *)(st + sk * 256 + (((sh << 3) | ((i ^ sk) & 7)) << 4));
-#pragma unroll
-            for (int g = 0; g < G; ++g) {
-                const float4 qv = *(const float4 *)(qf + g * 64 + sh * 32 + i * 4);
-                d0[g] = fmaf(qv.x, kv.x, fmaf(qv.z, kv.z, d0[g]));
-                d1[g] = fmaf(qv.y, kv.y, fmaf(qv.w, kv.w, d1[g]));
+        for (int g = 0; g < GR; ++g) {
+            d[g] = 0.0f;
+            if (g < G) {
+                float a, b;
+                mx::upk2(mx::fma2(q2[g][3], hi.y, mx::fma2(q2[g][2], hi.x, mx::fma2(q2[g][1], lo.y, mx::mul2(q2[g][0], lo.x)))), a, b);
+                d[g] = a + b;
             }
         }
-        float wv[GP];
+    };
+    // one step of a sum over eight lanes that leaves every lane its share of the values: it keeps one of two and hands the other on
+    auto halve = [&](float a, float b, int o) {
+        const bool up = lane & o;
+        return (up ? b : a) + __shfl_xor_sync(0xFFFFFFFFu, up ? a : b, o);
+    };
+
+    float m_run = -CUDART_INF_F, l_thr = 0.0f;   // of own_head: the max, the same in all lanes that hold it, and the sum over this lane's keys
+    uint64_t acc2[G][4];
 #pragma unroll
-        for (int g = 0; g < GP; ++g) wv[g] = 0.0f;
+    for (int g = 0; g < G; ++g) acc2[g][0] = acc2[g][1] = acc2[g][2] = acc2[g][3] = 0;
+    auto of_head = [&](float v, int g) { return __shfl_sync(0xFFFFFFFFu, v, ONE_KEY ? g : g << HS); };
+    auto raise_to = [&](float x) {   // x: the largest of this lane's scores
+#pragma unroll
+        for (int o = OWN_LANES; o < 32; o <<= 1) x = fmaxf(x, __shfl_xor_sync(0xFFFFFFFFu, x, o));
+        const float m_new = fmaxf(m_run, x);
+        const float alpha = (m_run == -CUDART_INF_F) ? 0.0f : mx::ex2(m_run - m_new);
+        l_thr *= alpha;
+        m_run = m_new;
 #pragma unroll
         for (int g = 0; g < G; ++g) {
-            float dot = d0[g] + d1[g];
-            dot += __shfl_xor_sync(0xFFFFFFFFu, dot, 16);
-            const float sg = ok ? dot * scale : -CUDART_INF_F;
-            // raise the running max only when a score exceeds it by RAISE (warp-uniform, rare)
-            if (__any_sync(0xFFFFFFFFu, sg > m_run[g] + RAISE * LOG2E)) {
-                const float m_new = warp_max_f(fmaxf(sg, m_run[g]));
-                const float alpha = (m_run[g] == -CUDART_INF_F) ? 0.0f : mx::ex2(m_run[g] - m_new);
-                l_thr[g] *= alpha;
+            const float al = of_head(alpha, g);
+            const uint64_t al2 = mx::pk2(al, al);
 #pragma unroll
-                for (int j = 0; j < 8; ++j) acc[g][j] *= alpha;
-                m_run[g] = m_new;
-            }
-            const float p = mx::ex2(sg - m_run[g]);
-            if (sh == 0) l_thr[g] += p;   // the two halves of a key hold the same score
-            wv[g] = p;
+            for (int j = 0; j < 4; ++j) acc2[g][j] = mx::mul2(acc2[g][j], al2);
         }
-        if (sh == 0) {
-#pragma unroll
-            for (int g4 = 0; g4 < GP / 4; ++g4)
-                *(float4 *)(wbuf + sk * GP + g4 * 4) = make_float4(wv[g4 * 4], wv[g4 * 4 + 1], wv[g4 * 4 + 2], wv[g4 * 4 + 3]);
-        }
+    };
+    constexpr int STEPS = FT_KEYS / 4;
+    for (int tile = 0; tile < n_tiles; ++tile) {
+        cp_async_wait<2 * FT_STAGES - 1>();
         __syncwarp();
-
-        // ---- values: lane = (key lane kl, 8-dim slice dsl), 4 steps of 4 keys ----
+        const unsigned char *st = ring + (tile % FT_STAGES) * FT_STAGE + kl * 256 + dsl * 16;
+        // ---- scores (log2 domain): 4 steps of 4 keys ----
+        float sc[NK], x = -CUDART_INF_F;
+        if constexpr (ONE_KEY) {
+            float d[STEPS][GR];
 #pragma unroll
-        for (int step = 0; step < FT_KEYS / 4; ++step) {
-            const unsigned char *vr = st + FT_KEYS * 256 + (step * 4 + kl) * 256;
-            const float4 va = *(const float4 *)(vr + vo0), vb4 = *(const float4 *)(vr + vo1);
+            for (int step = 0; step < STEPS; ++step) parts(st + step * 1024, d[step]);
+#pragma unroll
+            for (int g = 0; g < GR; ++g) d[0][g] = halve(halve(d[0][g], d[2][g], 4), halve(d[1][g], d[3][g], 4), 2);
+            sc[0] = GR > 1 ? halve(d[0][0], d[0][GR - 1], 1) : d[0][0] + __shfl_xor_sync(0xFFFFFFFFu, d[0][0], 1);
+        } else {
+#pragma unroll
+            for (int step = 0; step < STEPS; ++step) {
+                float d[GR];
+                parts(st + step * 1024, d);
+#pragma unroll
+                for (int i = 0; i < GR / 2; ++i) d[i] = halve(d[i], d[i + GR / 2], 4);
+#pragma unroll
+                for (int i = 0; i < GR / 4; ++i) d[i] = halve(d[i], d[i + GR / 4], 2);
+                sc[step] = GR > 4 ? halve(d[0], d[1], 1) : d[0] + __shfl_xor_sync(0xFFFFFFFFu, d[0], 1);
+            }
+        }
+        const int left = wb - (wa + tile * FT_KEYS) - key0_l;   // the lane's keys below it are the sequence's
+#pragma unroll
+        for (int i = 0; i < NK; ++i) {
+            sc[i] = i * 4 < left ? sc[i] * scale : -CUDART_INF_F;
+            x = fmaxf(x, sc[i]);
+        }
+        // raise the running maxima only when a score exceeds its own by RAISE (warp-uniform, rare)
+        if (__any_sync(0xFFFFFFFFu, x > m_run + RAISE * LOG2E)) raise_to(x);
+#pragma unroll
+        for (int i = 0; i < NK; ++i) {
+            const float p = mx::ex2(sc[i] - m_run);
+            l_thr += p;
+            if (ONE_KEY || HS == 0 || (dsl & 1) == 0) wbuf[(i * 4 + key0_l) * GP + own_head] = p;
+        }
+        __syncwarp();  // every lane is done with the K rows, and the weights are written
+        issue(tile + FT_STAGES, false);
+        cp_async_wait<2 * FT_STAGES - 1>();
+        __syncwarp();
+#pragma unroll
+        for (int step = 0; step < STEPS; ++step) {
+            const unsigned char *row = st + FT_KEYS * 256 + step * 1024;
+            const ulonglong2 lo = *(const ulonglong2 *)row, hi = *(const ulonglong2 *)(row + 128);
             float wk[GP];
 #pragma unroll
             for (int g4 = 0; g4 < GP / 4; ++g4) {
@@ -1427,58 +1466,61 @@ decode_f32_ring_kernel(const DecodeParams P) {
             }
 #pragma unroll
             for (int g = 0; g < G; ++g) {
-                acc[g][0] = fmaf(wk[g], va.x, acc[g][0]);
-                acc[g][1] = fmaf(wk[g], va.y, acc[g][1]);
-                acc[g][2] = fmaf(wk[g], va.z, acc[g][2]);
-                acc[g][3] = fmaf(wk[g], va.w, acc[g][3]);
-                acc[g][4] = fmaf(wk[g], vb4.x, acc[g][4]);
-                acc[g][5] = fmaf(wk[g], vb4.y, acc[g][5]);
-                acc[g][6] = fmaf(wk[g], vb4.z, acc[g][6]);
-                acc[g][7] = fmaf(wk[g], vb4.w, acc[g][7]);
+                const uint64_t w2 = mx::pk2(wk[g], wk[g]);
+                acc2[g][0] = mx::fma2(w2, lo.x, acc2[g][0]);
+                acc2[g][1] = mx::fma2(w2, lo.y, acc2[g][1]);
+                acc2[g][2] = mx::fma2(w2, hi.x, acc2[g][2]);
+                acc2[g][3] = mx::fma2(w2, hi.y, acc2[g][3]);
             }
         }
-        __syncwarp();  // the ring slot and the weight buffer are rewritten by the next iterations
+        __syncwarp();  // the V rows and the weight buffer are rewritten from here on
+        issue(tile + FT_STAGES, true);
     }
     cp_async_wait<0>();
     if (P.trigger) mx::pdl_trigger();
 
+    const bool first_key = key0_l == 0;   // lanes whose (first) key is a tile's first
     // ---- fused step: the new token's own key, by the owning CTA's last warp (the one with the fewest keys) ----
     if (FUSED && owner && warp == WARPS - 1) {
+        float d[GR], x = 0.0f;
+        parts((const unsigned char *)new_k + dsl * 16, d);
+#pragma unroll
+        for (int g = 0; g < GR; ++g) {
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) d[g] += __shfl_xor_sync(0xFFFFFFFFu, d[g], o);
+            if (g == own_head) x = d[g] * scale;
+        }
+        raise_to(x);
+        const float p = mx::ex2(x - m_run);
+        if (first_key) l_thr += p;
+        const ulonglong2 lo = *(const ulonglong2 *)(new_v + dsl * 4), hi = *(const ulonglong2 *)(new_v + 32 + dsl * 4);
 #pragma unroll
         for (int g = 0; g < G; ++g) {
-            const float sg = warp_sum_f(fmaf(qf[g * 64 + lane], new_k[lane], qf[g * 64 + 32 + lane] * new_k[lane + 32])) * scale;
-            const float m_new = fmaxf(m_run[g], sg);
-            const float alpha = (m_run[g] == -CUDART_INF_F) ? 0.0f : mx::ex2(m_run[g] - m_new);
-            const float p = mx::ex2(sg - m_new);
-            m_run[g] = m_new;
-            l_thr[g] = l_thr[g] * alpha + (lane == 0 ? p : 0.0f);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) acc[g][j] = acc[g][j] * alpha + (kl == 0 ? p * new_v[dsl * 8 + j] : 0.0f);
+            const float w = of_head(p, g);
+            const uint64_t w2 = mx::pk2(w, w);
+            if (kl == 0) {
+                acc2[g][0] = mx::fma2(w2, lo.x, acc2[g][0]), acc2[g][1] = mx::fma2(w2, lo.y, acc2[g][1]);
+                acc2[g][2] = mx::fma2(w2, hi.x, acc2[g][2]), acc2[g][3] = mx::fma2(w2, hi.y, acc2[g][3]);
+            }
         }
     }
 
     // ---- warp totals, then the CTA-level log-sum-exp merge of the warps ----
 #pragma unroll
-    for (int g = 0; g < G; ++g) {
-        l_thr[g] = warp_sum_f(l_thr[g]);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {  // key lanes differ in lane bits 3,4
-            float v = acc[g][j];
-            v += __shfl_xor_sync(0xFFFFFFFFu, v, 8);
-            v += __shfl_xor_sync(0xFFFFFFFFu, v, 16);
-            acc[g][j] = v;
-        }
-    }
+    for (int o = OWN_LANES; o < 32; o <<= 1) l_thr += __shfl_xor_sync(0xFFFFFFFFu, l_thr, o);
     __syncthreads();  // every warp is done with its ring: reuse the memory for the merge
     float *mg = (float *)warp_base;  // [warp][g][68]: m (log2 domain), l, 0, pad, acc[64]
+    if (first_key && own_head < G) *(float4 *)(mg + (warp * G + own_head) * 68) = make_float4(m_run, l_thr, 0.0f, 0.0f);
+    // over the key lanes as above: of a lane's eight dims half stay at lane bit 3, half of those at bit 4
 #pragma unroll
     for (int g = 0; g < G; ++g) {
-        float *dst = mg + (warp * G + g) * 68;
-        if (lane == 0) *(float4 *)dst = make_float4(m_run[g], l_thr[g], 0.0f, 0.0f);
-        if (lane < 8) {
-            *(float4 *)(dst + 4 + lane * 8) = make_float4(acc[g][0], acc[g][1], acc[g][2], acc[g][3]);
-            *(float4 *)(dst + 8 + lane * 8) = make_float4(acc[g][4], acc[g][5], acc[g][6], acc[g][7]);
-        }
+        float a[8], c[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) mx::upk2(acc2[g][j], a[2 * j], a[2 * j + 1]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) c[j] = halve(a[j], a[j + 4], 8);
+        *(float2 *)(mg + (warp * G + g) * 68 + 4 + (lane & 8) * 4 + dsl * 4 + (lane & 16) / 8) =
+            make_float2(halve(c[0], c[2], 16), halve(c[1], c[3], 16));
     }
     __syncthreads();
     finish_group<G, WARPS>(P, mg, X, s, head0, gc, cl, rank, active, FUSED && P.out != P.qkv_rw ? qf : nullptr, &is_last);
