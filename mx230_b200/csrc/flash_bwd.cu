@@ -228,20 +228,29 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmOwnA, const __grid_constant__ C
     __syncthreads();
     mx::tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    if (warp == 8 && lane == 0) {   // tensor maps and the first item's parameters on their way into the SM's caches
+        mx::tma_prefetch_desc(&tmStrA);
+        mx::tma_prefetch_desc(&tmStrB);
+        if (MODE >= 1) {
+            mx::tma_prefetch_desc(&tmOwnA);
+            mx::tma_prefetch_desc(&tmOwnB);
+        }
+        if (FUSED) {
+            mx::tma_prefetch_desc(&tmDQ);
+            mx::tma_prefetch_desc(&tmOut0);
+            mx::tma_prefetch_desc(&tmOut1);
+        }
+    }
+    {
+        BwdItem I;
+        if (bwd_item<MODE>(P, 0, I)) asm volatile("" ::"r"(I.bh), "r"(I.own0), "r"(I.n), "l"(P.L), "l"(P.Delta), "l"(P.status));
+    }
     mx::pdl_wait();   // (launched programmatically: the set-up above runs under the previous kernel's tail)
 
     if (warp >= 8) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS_SERVICE));
         if (warp == 8) {
             // ------------------------- producer -------------------------
-            if (lane == 0) {
-                mx::tma_prefetch_desc(&tmStrA);
-                mx::tma_prefetch_desc(&tmStrB);
-                if (MODE >= 1) {
-                    mx::tma_prefetch_desc(&tmOwnA);
-                    mx::tma_prefetch_desc(&tmOwnB);
-                }
-            }
             if (FUSED) {   // the constant operands: ones for X, ones for Y, zeros (ordered before the first arrive below)
                 uint4 *ax = (uint4 *)(smem + SM_AUG_AX), *ay = (uint4 *)(smem + SM_AUG_AY), *az = (uint4 *)(smem + SM_AUG_Z);
 #pragma unroll
@@ -548,7 +557,6 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmOwnA, const __grid_constant__ C
             const uint32_t ta = tmem + ((uint32_t)((warp & 3) * 32) << 16) + TMF_DQ;
             const uint32_t stage = smem_base + SM_DQ + (warp & 3) * DQ_STAGE_BYTES;
             unsigned char *stage_row = smem + SM_DQ + (warp & 3) * DQ_STAGE_BYTES + lane * 128;
-            if (lane == 0) mx::tma_prefetch_desc(&tmDQ);
             bool ok = true;
             uint32_t g = 0;
             BwdItem I;

@@ -165,6 +165,17 @@ __device__ __forceinline__ int fwd_tile_iters(const FwdParams &P, int q0, int t)
     return P.causal ? min(n_kv_total, (r0 + BM - 1 + P.q_off) / BN + 1) : n_kv_total;
 }
 
+// In front of the wait for the previous kernel: the tensor maps on their way into the SM's caches.
+__device__ __forceinline__ void fwd_prefetch_maps(const FwdParams &P, int warp, int lane, const CUtensorMap &tmQ, const CUtensorMap &tmK,
+                                                  const CUtensorMap &tmV, const CUtensorMap &tmO) {
+    if (warp == SOFT_WARPS && lane == 0) {
+        mx::tma_prefetch_desc(&tmQ);
+        mx::tma_prefetch_desc(&tmK);
+        mx::tma_prefetch_desc(&tmV);
+        if (P.tma_out) mx::tma_prefetch_desc(&tmO);
+    }
+}
+
 // Largest score, in log2 units, of a head that takes the max-free loop: against the reference 0, or (SRC_RAW_BOUND, SRC_I8) against
 // a row's max over the first key tile, from which a score may be twice as far (probabilities stay below 2^80 either way).
 constexpr float FAST_BOUND = 80.0f, FAST_BOUND_REF = 40.0f;
@@ -316,15 +327,16 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     __syncthreads();
     mx::tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    mx::pdl_wait();
+    if (KEY_SPLIT) fwd_prefetch_maps(P, warp, lane, tmQ, tmK, tmV, tmO);
+    // In the key-split form, which short calls take, every role waits for the previous kernel behind the arithmetic of its first
+    // item: it took 0.4 us behind the wait (code and parameters come into the caches with it; 12 x 1024 rows causal 15.2 -> 14.7).
+    if (!KEY_SPLIT) mx::pdl_wait();
 
     if (warp >= SOFT_WARPS) {
         if (warp == SOFT_WARPS) {
         // ------------------------- TMA producer -------------------------
         if (lane == 0) {
-            mx::tma_prefetch_desc(&tmQ);
-            mx::tma_prefetch_desc(&tmK);
-            mx::tma_prefetch_desc(&tmV);
+            if (!KEY_SPLIT) fwd_prefetch_maps(P, warp, lane, tmQ, tmK, tmV, tmO);
             bool ok = true;
             uint32_t g = 0;  // K/V tiles loaded so far, over all items: ring slot g % KV_STAGES, use g / KV_STAGES
             int bh, q0;
@@ -336,6 +348,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 if (it >= Q_BUFS) ok = mx::mbar_wait(bar(BAR_Q_EMPTY + qbuf), ((it >> 1) - 1) & 1, abort_flag, P.status);
                 if (!ok) break;
                 const int nq = (n_it1 > 0) ? 2 : 1;
+                if (KEY_SPLIT && it == 0) mx::pdl_wait();
                 mx::mbar_expect_tx(bar(BAR_Q_FULL + qbuf), nq * TILE_BYTES);
                 for (int t = 0; t < nq; ++t)
                     mx::tma_load_3d(smem_base + SMEM_Q + (qbuf * QT + t) * TILE_BYTES, &tmQ, bar(BAR_Q_FULL + qbuf), 0,
@@ -383,6 +396,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 for (int t = 0; t < QT; ++t) n_it[t] = fwd_tile_iters(P, q0, KEY_SPLIT ? 0 : t);
                 const int n_max = max(n_it[0], n_it[1]);
                 const int qbuf = it & 1;
+                if (KEY_SPLIT && it == 0) mx::pdl_wait();
                 ok = ISSUER_WAIT(mx::mbar_wait(bar(BAR_Q_FULL + qbuf), (it >> 1) & 1, abort_flag, P.status));
                 for (int j = 0; j < n_max && ok; ++j, ++g) {
                     const int s = g % KV_STAGES;
@@ -424,6 +438,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 #pragma unroll
                 for (int t = 0; t < QT; ++t) n_it[t] = fwd_tile_iters(P, q0, KEY_SPLIT ? 0 : t);
                 const int n_max = max(n_it[0], n_it[1]);
+                if (KEY_SPLIT && it == 0) mx::pdl_wait();
                 // each pair of groups sums into an O of its own
                 const bool own_o = !KEY_SPLIT || SRC == SRC_RAW ||
                                    !(SRC == SRC_RAW_BOUND
@@ -499,6 +514,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         // they would run ahead of the first tile from one such item to the next, and a barrier that counts one item's
         // arrivals cannot tell them from the next but one's.)
         const bool lone = !KEY_SPLIT && q0 + BM >= NQ;
+        if (KEY_SPLIT && it == 0) mx::pdl_wait();
         if (lone && t == 1) {
             g0 += fwd_tile_iters(P, q0, 0);
             continue;
@@ -746,6 +762,18 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         float l_norm = 0.0f;             // what O is divided by
         float w0 = 1.0f, w1 = 1.0f;      // key-split form, general mode: weights of O_0 and O_1
         if (half == 1 || (KEY_SPLIT && t == 1)) {
+            // The odd groups of the key-split form publish before their last P V is complete, so that the first group has their sums
+            // when it is.  None publishes twice before the first group has taken the first: O1_READ, which they wait for in every
+            // item, comes behind that.  (The others publish behind an item's last P V, which the first group's P precedes: with no
+            // such order a second arrival could pass for one that is missing.  The other sources' odd groups wait for an exchange
+            // first, below.)
+            const bool early = KEY_SPLIT && (SRC == SRC_PRE || SRC == SRC_RAW) && t == 1;
+            if (early && ok) {
+                xch(my_pub, 0) = l;
+                xch(my_pub, 1) = m;
+                __syncwarp();
+                if (lane == 0) mx::mbar_arrive(bar(BAR_XCH));
+            }
             // (the tile's last P V must have read this group's share of P_t before the next item's first tile overwrites it)
             if (ok && n_t > 0)
                 ok = __all_sync(0xFFFFFFFFu, mx::mbar_wait(bar(BAR_O_DONE + t), (cnt - 1) & 1, abort_flag, P.status));
@@ -758,7 +786,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 xmc0 += fast ? 1u : (uint32_t)((n_all + 1) >> 1);
                 if (ok) ok = __all_sync(0xFFFFFFFFu, mx::mbar_wait(bar(BAR_XMAX), (xmc0 - 1) & 1, abort_flag, P.status));
             }
-            if (ok) {
+            if (ok && !early) {
                 xch(my_pub, 0) = l;
                 xch(my_pub, 1) = KEY_SPLIT ? m : l_odd;
                 __syncwarp();
@@ -829,9 +857,11 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                     // buffer (its last Q K^T has completed) and hands it to the TMA unit, which clips rows past the
                     // end: 16-byte stores from lane = row registers each touch a sector of their own
                     const int wrow0 = row0 + (warp & 3) * 32;
-                    const int st_off = SMEM_Q + (qbuf * QT + t) * TILE_BYTES + (warp & 3) * 4096;
+                    // (key-split form: in two such pieces, the item's second Q tile having no rows)
+                    int st_off = SMEM_Q + (qbuf * QT + (KEY_SPLIT ? 0 : t)) * TILE_BYTES + (warp & 3) * 4096;
 #pragma unroll 1
                     for (int cc = 0; cc < HD / 32; ++cc) {
+                        if (KEY_SPLIT && cc > 0) st_off += TILE_BYTES;
                         load_o(cc);
                         unsigned char *srow = smem + st_off + lane * 128;
 #pragma unroll
@@ -845,7 +875,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                         if (lane == 0 && wrow0 < NQ) {
                             mx::tma_store_3d(&tmO, smem_base + st_off, cc * 32, wrow0, bh);
                             mx::bulk_commit_group();
-                            mx::bulk_wait_group_read<0>();   // the piece is reused for the second half and must outlive the read
+                            if (!KEY_SPLIT || cc > 0) mx::bulk_wait_group_read<0>();   // the piece is reused and must outlive the read
                         }
                         __syncwarp();
                     }
@@ -949,7 +979,7 @@ flash_fwd_rows64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     __syncthreads();
     mx::tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    mx::pdl_wait();
+    fwd_prefetch_maps(P, warp, lane, tmQ, tmK, tmV, tmO);   // (every role waits for the previous kernel at its first item)
 
     auto item_tiles = [&](int q0) {   // key tiles of the item's rows
         const int all = (N + BN - 1) / BN;
@@ -965,12 +995,10 @@ flash_fwd_rows64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     if (warp == SOFT_WARPS) {
         // ------------------------- TMA producer -------------------------
         if (lane == 0) {
-            mx::tma_prefetch_desc(&tmQ);
-            mx::tma_prefetch_desc(&tmK);
-            mx::tma_prefetch_desc(&tmV);
             uint32_t g = 0;
             for (int it = 0; ok && fwd_item(P, it, bh, q0); ++it) {
                 const int n = item_tiles(q0), qbuf = it & 1, kvh = bh / P.kv_group;
+                if (it == 0) mx::pdl_wait();
                 if (it >= Q_BUFS) ok = wait(RB_Q_EMPTY + qbuf, (it >> 1) - 1);
                 if (!ok) break;
                 mx::mbar_expect_tx(bar(RB_Q_FULL + qbuf), R_Q_BYTES);
@@ -1001,6 +1029,7 @@ flash_fwd_rows64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         for (int it = 0; ok && fwd_item(P, it, bh, q0); ++it) {
             const int n = item_tiles(q0), qbuf = it & 1;
             const uint64_t a = mx::smem_desc_sw128(smem_base + R_SMEM_Q + qbuf * R_Q_BYTES);
+            if (it == 0) mx::pdl_wait();
             ok = wait_warp(RB_Q_FULL + qbuf, it >> 1);
             for (int j0 = 0; j0 < n && ok; j0 += R_GROUPS) {
 #pragma unroll
@@ -1033,6 +1062,7 @@ flash_fwd_rows64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         uint32_t g = 0, cp[R_GROUPS] = {};
         for (int it = 0; ok && fwd_item(P, it, bh, q0); ++it) {
             const int n = item_tiles(q0);
+            if (it == 0) mx::pdl_wait();
             const bool own_o = !head_fast(bh, q0);   // each group sums into an O of its own
             for (int j0 = 0; j0 < n && ok; j0 += R_GROUPS) {
 #pragma unroll
@@ -1078,6 +1108,7 @@ flash_fwd_rows64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
             const int n = item_tiles(q0), n_w = (n + R_GROUPS - 1 - w) / R_GROUPS;
             const int row = q0 + row_in_tile;
             const int last = P.causal ? min(N - 1, row + P.q_off) : N - 1;   // last visible key of this row
+            if (it == 0) mx::pdl_wait();
             const bool fast = head_fast(bh, q0);
             float row_a = 0.0f, row_qsum = 0.0f;
             if (SRC == SRC_I8 && row < NQ) {

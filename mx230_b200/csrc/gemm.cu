@@ -84,13 +84,17 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CU
     __syncthreads();
     mx::tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    if (warp == 0 && lane == 0) {   // on their way into the SM's caches while the previous kernel ends
+        mx::tma_prefetch_desc(&tmA0);
+        mx::tma_prefetch_desc(&tmW0);
+        if (SPLIT) mx::tma_prefetch_desc(&tmA1), mx::tma_prefetch_desc(&tmW1);
+        if (P.tma_out) mx::tma_prefetch_desc(&tmC);
+    }
     mx::pdl_wait();
 
     if (warp == 0) {
         // ------------------------- TMA producer -------------------------
         if (lane == 0) {
-            mx::tma_prefetch_desc(&tmA0);
-            mx::tma_prefetch_desc(&tmW0);
             bool ok = true;
             for (int i = 0; i < n_steps && ok; ++i) {
                 const int s = i % STAGES;
