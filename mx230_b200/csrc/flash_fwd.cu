@@ -330,7 +330,9 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     if (KEY_SPLIT) fwd_prefetch_maps(P, warp, lane, tmQ, tmK, tmV, tmO);
     // In the key-split form, which short calls take, every role waits for the previous kernel behind the arithmetic of its first
     // item: it took 0.4 us behind the wait (code and parameters come into the caches with it; 12 x 1024 rows causal 15.2 -> 14.7).
-    if (!KEY_SPLIT) mx::pdl_wait();
+    // Not with int8 scores, whose loop comes out slower then (700 tokens over 4700 keys, 14/2 heads, 48.7 us against 46.2).
+    constexpr bool SHORT = KEY_SPLIT && SRC != SRC_I8;
+    if (!SHORT) mx::pdl_wait();
 
     if (warp >= SOFT_WARPS) {
         if (warp == SOFT_WARPS) {
@@ -348,7 +350,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 if (it >= Q_BUFS) ok = mx::mbar_wait(bar(BAR_Q_EMPTY + qbuf), ((it >> 1) - 1) & 1, abort_flag, P.status);
                 if (!ok) break;
                 const int nq = (n_it1 > 0) ? 2 : 1;
-                if (KEY_SPLIT && it == 0) mx::pdl_wait();
+                if (SHORT && it == 0) mx::pdl_wait();
                 mx::mbar_expect_tx(bar(BAR_Q_FULL + qbuf), nq * TILE_BYTES);
                 for (int t = 0; t < nq; ++t)
                     mx::tma_load_3d(smem_base + SMEM_Q + (qbuf * QT + t) * TILE_BYTES, &tmQ, bar(BAR_Q_FULL + qbuf), 0,
@@ -396,7 +398,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 for (int t = 0; t < QT; ++t) n_it[t] = fwd_tile_iters(P, q0, KEY_SPLIT ? 0 : t);
                 const int n_max = max(n_it[0], n_it[1]);
                 const int qbuf = it & 1;
-                if (KEY_SPLIT && it == 0) mx::pdl_wait();
+                if (SHORT && it == 0) mx::pdl_wait();
                 ok = ISSUER_WAIT(mx::mbar_wait(bar(BAR_Q_FULL + qbuf), (it >> 1) & 1, abort_flag, P.status));
                 for (int j = 0; j < n_max && ok; ++j, ++g) {
                     const int s = g % KV_STAGES;
@@ -410,7 +412,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                         if (cs[t] > 0) ok = ISSUER_WAIT(mx::mbar_wait(bar(BAR_S_FREE + t), (cs[t] - 1) & 1, abort_flag, P.status));
                         if (!ok) continue;
                         mx::tc_fence_after();
-                        const uint64_t a = mx::smem_desc_sw128(smem_base + SMEM_Q + (qbuf * QT + (KEY_SPLIT ? 0 : t)) * TILE_BYTES);
+                        const uint64_t a = mx::smem_desc_sw128(smem_base + SMEM_Q + (qbuf * QT + (SHORT ? 0 : t)) * TILE_BYTES);
                         if (ISSUER_LANE) {
 #pragma unroll
                             for (int k = 0; k < HD / 16; ++k)  // 32 bytes per 16-element step inside the swizzle span
@@ -438,7 +440,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 #pragma unroll
                 for (int t = 0; t < QT; ++t) n_it[t] = fwd_tile_iters(P, q0, KEY_SPLIT ? 0 : t);
                 const int n_max = max(n_it[0], n_it[1]);
-                if (KEY_SPLIT && it == 0) mx::pdl_wait();
+                if (SHORT && it == 0) mx::pdl_wait();
                 // each pair of groups sums into an O of its own
                 const bool own_o = !KEY_SPLIT || SRC == SRC_RAW ||
                                    !(SRC == SRC_RAW_BOUND
@@ -514,7 +516,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         // they would run ahead of the first tile from one such item to the next, and a barrier that counts one item's
         // arrivals cannot tell them from the next but one's.)
         const bool lone = !KEY_SPLIT && q0 + BM >= NQ;
-        if (KEY_SPLIT && it == 0) mx::pdl_wait();
+        if (SHORT && it == 0) mx::pdl_wait();
         if (lone && t == 1) {
             g0 += fwd_tile_iters(P, q0, 0);
             continue;
@@ -858,10 +860,10 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                     // end: 16-byte stores from lane = row registers each touch a sector of their own
                     const int wrow0 = row0 + (warp & 3) * 32;
                     // (key-split form: in two such pieces, the item's second Q tile having no rows)
-                    int st_off = SMEM_Q + (qbuf * QT + (KEY_SPLIT ? 0 : t)) * TILE_BYTES + (warp & 3) * 4096;
+                    int st_off = SMEM_Q + (qbuf * QT + (SHORT ? 0 : t)) * TILE_BYTES + (warp & 3) * 4096;
 #pragma unroll 1
                     for (int cc = 0; cc < HD / 32; ++cc) {
-                        if (KEY_SPLIT && cc > 0) st_off += TILE_BYTES;
+                        if (SHORT && cc > 0) st_off += TILE_BYTES;
                         load_o(cc);
                         unsigned char *srow = smem + st_off + lane * 128;
 #pragma unroll
@@ -875,7 +877,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                         if (lane == 0 && wrow0 < NQ) {
                             mx::tma_store_3d(&tmO, smem_base + st_off, cc * 32, wrow0, bh);
                             mx::bulk_commit_group();
-                            if (!KEY_SPLIT || cc > 0) mx::bulk_wait_group_read<0>();   // the piece is reused and must outlive the read
+                            if (!SHORT || cc > 0) mx::bulk_wait_group_read<0>();   // the piece is reused and must outlive the read
                         }
                         __syncwarp();
                     }
