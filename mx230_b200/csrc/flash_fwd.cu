@@ -412,7 +412,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                         if (cs[t] > 0) ok = ISSUER_WAIT(mx::mbar_wait(bar(BAR_S_FREE + t), (cs[t] - 1) & 1, abort_flag, P.status));
                         if (!ok) continue;
                         mx::tc_fence_after();
-                        const uint64_t a = mx::smem_desc_sw128(smem_base + SMEM_Q + (qbuf * QT + (SHORT ? 0 : t)) * TILE_BYTES);
+                        const uint64_t a = mx::smem_desc_sw128(smem_base + SMEM_Q + (qbuf * QT + (KEY_SPLIT ? 0 : t)) * TILE_BYTES);
                         if (ISSUER_LANE) {
 #pragma unroll
                             for (int k = 0; k < HD / 16; ++k)  // 32 bytes per 16-element step inside the swizzle span
@@ -860,7 +860,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                     // end: 16-byte stores from lane = row registers each touch a sector of their own
                     const int wrow0 = row0 + (warp & 3) * 32;
                     // (key-split form: in two such pieces, the item's second Q tile having no rows)
-                    int st_off = SMEM_Q + (qbuf * QT + (SHORT ? 0 : t)) * TILE_BYTES + (warp & 3) * 4096;
+                    int st_off = SMEM_Q + (qbuf * QT + (KEY_SPLIT ? 0 : t)) * TILE_BYTES + (warp & 3) * 4096;
 #pragma unroll 1
                     for (int cc = 0; cc < HD / 32; ++cc) {
                         if (SHORT && cc > 0) st_off += TILE_BYTES;
