@@ -678,30 +678,40 @@ __device__ __forceinline__ void rope_pair(float &x1, float &x2, float cs, float 
     x2 = __fmaf_rn(a, sn, __fmul_rn(b, cs));
 }
 
+// ---- maximum and minimum over the warp (NaN is passed over, as by fmaxf) ----
+__device__ __forceinline__ float warp_max(float v) {
+    float r;
+    asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+__device__ __forceinline__ float warp_min(float v) {
+    float r;
+    asm("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+
 // ---- int8 quantize-on-write of one head's 64 values by one warp, two values per lane (any assignment of values to
 // lanes): IEEE division and round-to-nearest-even exactly as quant_affine (03-llm-engine/kernels/llm.cu:1137-1149), or
 // symmetric absmax / 127 when !affine (beta 0) ----
-__device__ __forceinline__ void quant_head_row(float x0, float x1, bool affine, int &c0, int &c1, float &scale, float &beta) {
-    auto wmax = [](float v) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
-        return v;
-    };
+// (hi, lo: the largest and the smallest of the row's values)
+__device__ __forceinline__ void quant_head_row(float x0, float x1, float hi, float lo, bool affine, int &c0, int &c1, float &scale, float &beta) {
     if (affine) {
-        const float hi = wmax(fmaxf(x0, x1));
-        const float lo = -wmax(fmaxf(-x0, -x1));
         scale = (hi > lo) ? __fdiv_rn(hi - lo, 255.0f) : 1.0f;
         beta = __fmaf_rn(128.0f, scale, lo);   // exact: 128*scale is a power-of-two scaling
         c0 = max(-128, min(127, __float2int_rn(__fdiv_rn(x0 - beta, scale))));
         c1 = max(-128, min(127, __float2int_rn(__fdiv_rn(x1 - beta, scale))));
     } else {
-        const float amax = wmax(fmaxf(fabsf(x0), fabsf(x1)));
+        const float amax = fmaxf(fabsf(hi), fabsf(lo));
         const float id = amax > 0.0f ? __fdiv_rn(127.0f, amax) : 0.0f;
         c0 = max(-127, min(127, __float2int_rn(x0 * id)));
         c1 = max(-127, min(127, __float2int_rn(x1 * id)));
         scale = amax > 0.0f ? __fdiv_rn(amax, 127.0f) : 0.0f;
         beta = 0.0f;
     }
+}
+__device__ __forceinline__ void quant_head_row(float x0, float x1, bool affine, int &c0, int &c1, float &scale, float &beta) {
+    const float hi = warp_max(fmaxf(x0, x1)), lo = warp_min(fminf(x0, x1));
+    quant_head_row(x0, x1, hi, lo, affine, c0, c1, scale, beta);
 }
 
 // ---- programmatic dependent launch ----

@@ -87,8 +87,9 @@ struct SeqRows {
 // separate launches took 33.3 and 32.0.
 constexpr int SR_WARPS = 8, SR_UNITS = 2;
 __global__ void __launch_bounds__(SR_WARPS * 32) seq_rows_kernel(const SeqRows P) {
-    mx::pdl_wait();
     const int lane = threadIdx.x & 31, r = blockIdx.y;
+    const float freq = P.use_rope ? mx::rope_freq(lane, 64, P.theta) : 0.0f;
+    mx::pdl_wait();
     const int n_rot = P.n_head + P.n_kv_head, n_units = n_rot + P.n_kv_head;
     const int u0 = (P.use_rope ? 0 : P.n_head) + blockIdx.x * (SR_WARPS * SR_UNITS) + (threadIdx.x >> 5);
     float *row = P.qkv + (size_t)r * P.stride;
@@ -102,7 +103,7 @@ __global__ void __launch_bounds__(SR_WARPS * 32) seq_rows_kernel(const SeqRows P
     const int pos = min(max(row_position(P.rp, r), 0), P.max_pos);
     const size_t crow = phys_row(P.rp, r, pos), kvd = (size_t)P.n_kv_head * 64;
     float cs = 1.0f, sn = 0.0f;
-    if (P.use_rope && u0 < n_rot) mx::rope_angle(pos, lane, 64, P.theta, cs, sn);
+    if (P.use_rope && u0 < n_rot) mx::rope_angle(pos, freq, cs, sn);
 #pragma unroll
     for (int i = 0; i < SR_UNITS; ++i) {
         const int u = u0 + i * SR_WARPS;

@@ -26,7 +26,7 @@ struct StageParams {
     __nv_bfloat16 *kout, *vout;      // [n_kv_head][n_keys][64]
     float *q_norm2, *k_norm2;        // [heads][MX230_NORM_PARTS] largest squared norm of the (dequantised) rows of each part, or null
     float *row_a, *row_qsum, *kskb;  // int8 scores: per-row factor and code sum; per-key scale and offset by tiles of 128
-    int i8_scores, n_k_tiles;
+    int n_k_tiles;
     // inputs
     float *qkv;
     int stride, n_tok, pos0, n_keys, n_head, n_kv_head;
@@ -59,13 +59,17 @@ __device__ __forceinline__ float *stage_kskb(const StageParams &P, int h, int t)
 // quantise 4, two staging kernels 3.8 + 4 (512 tokens over 1536 cached keys, int8), and 11.7 + 5 + 4.7 + 5 (1900 tokens,
 // fp32).  New tokens: four warps per token, lane l holds dims l and l + 32 of a head, so RoPE's angle is computed once
 // per token and warp and a head's quantiser is a warp reduction.  Cached keys: eight threads per key and head, eight dims
-// each.  Row norms go through shared memory and, per cluster of CTAs, into one of MX230_NORM_PARTS parts: with Q's
+// each.  What a warp of new tokens costs is the code it fetches as much as its arithmetic: its heads are one rolled loop over
+// values in shared memory, an instantiation per cache and score mode, and the first angle is formed before the wait (512 tokens over
+// 1536 int8 keys, from the wait to the last token 4.4 -> 3.9 us, a call 26.9 -> 24.6; over fp32 keys 20.4 -> 19.0).  Row norms go through shared memory and, per cluster of CTAs, into one of MX230_NORM_PARTS parts: with Q's
 // and K's the attention kernel bounds every score of a head and, where the bound is small, runs without a row max.
-// CLUSTER: CTAs that share one norm part, 4 or 8.  (Sizes are constants or come from the host: a division costs more here than
+// CLUSTER: CTAs that share one norm part, 4 or 8.  I8: int8 scores; Q8: int8 cache (instantiations: code that a launch does not
+// run is not fetched either).  (Sizes are constants or come from the host: a division costs more here than
 // the work of a thread.)
-template <int CLUSTER>
+template <int CLUSTER, bool I8, bool Q8>
 __global__ void __launch_bounds__(ST_THREADS, 2) prefill_stage_kernel(const StageParams P) {
-    extern __shared__ int smax[];    // [n_norms] squared norms of Q and K heads as ordered integers (NaN largest)
+    extern __shared__ float2 heads[];   // [ST_WARPS][ST_HEADS][32] a warp's heads of its token: lane l's dims l and l + 32
+    int *smax = (int *)(heads + ST_WARPS * ST_HEADS * 32);   // [n_norms] squared norms of Q and K heads as ordered integers (NaN largest)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr int n_ctas = MX230_NORM_PARTS * CLUSTER;
     const int n_max = P.n_head + P.n_kv_head, n_norms = P.q_norm2 ? n_max : 0;
@@ -73,6 +77,9 @@ __global__ void __launch_bounds__(ST_THREADS, 2) prefill_stage_kernel(const Stag
     for (int i = tid; i < n_norms; i += ST_THREADS) smax[i] = 0;
     __syncthreads();
     mx::cluster_arrive_release();    // waited for before this CTA adds to the first one's maxima
+    const int sub = warp & (ST_SUBS - 1), tok0 = blockIdx.x + n_ctas * (warp / ST_SUBS);
+    float cs = 1.0f, sn = 0.0f;      // of the warp's next token; its first one's before the wait: the angle takes as long as a load
+    if (P.rope && tok0 < P.n_tok) mx::rope_angle(P.pos0 + tok0, lane, HD, P.theta, cs, sn);
     mx::pdl_wait();
     auto raise = [&](int head, float norm2) {
         if (n_norms > 0) atomicMax(&smax[head], __float_as_int(norm2) & 0x7FFFFFFF);
@@ -81,102 +88,107 @@ __global__ void __launch_bounds__(ST_THREADS, 2) prefill_stage_kernel(const Stag
 
     // ---- new tokens ----
     const int n_units = P.n_head + (P.write_kv ? 2 * P.n_kv_head : 0);
-    const int sub = warp & (ST_SUBS - 1);
-    for (int tok = blockIdx.x + n_ctas * (warp / ST_SUBS); tok < P.n_tok; tok += n_ctas * (ST_WARPS / ST_SUBS)) {
+    float va[ST_HEADS], vb[ST_HEADS];
+    auto load = [&](int tok, int u0) {
+        const float *row = P.qkv + (size_t)tok * P.stride;
+#pragma unroll
+        for (int i = 0; i < ST_HEADS; ++i) {
+            const int u = u0 + i * ST_SUBS;
+            if (u < n_units) va[i] = row[u * HD + lane], vb[i] = row[u * HD + 32 + lane];
+        }
+    };
+    if (tok0 < P.n_tok) load(tok0, sub);
+    for (int tok = tok0, u0 = sub; tok < P.n_tok;) {
         const int pos = P.pos0 + tok;
         float *row = P.qkv + (size_t)tok * P.stride;
         const size_t crow = P.write_kv ? stage_row(P, pos) : 0;
-        float cs = 1.0f, sn = 0.0f;
-        bool have_angle = false;
-        for (int u0 = sub; u0 < n_units; u0 += ST_HEADS * ST_SUBS) {
-            float va[ST_HEADS], vb[ST_HEADS];
 #pragma unroll
-            for (int i = 0; i < ST_HEADS; ++i) {
-                const int u = u0 + i * ST_SUBS;
-                if (u < n_units) va[i] = row[u * HD + lane], vb[i] = row[u * HD + 32 + lane];
+        for (int i = 0; i < ST_HEADS; ++i) heads[(warp * ST_HEADS + i) * 32 + lane] = make_float2(va[i], vb[i]);
+        // the warp's next heads, of this token or of its next, arrive under these
+        int next = tok, next_u0 = u0 + ST_HEADS * ST_SUBS;
+        if (next_u0 >= n_units) next += n_ctas * (ST_WARPS / ST_SUBS), next_u0 = sub;
+        if (next < P.n_tok) load(next, next_u0);
+        // (a lane reads what it wrote.  Not unrolled: with five copies of the loop, code for the instruction cache, 0.7 us slower)
+#pragma unroll 1
+        for (int i = 0; i < ST_HEADS; ++i) {
+            const int u = u0 + i * ST_SUBS;
+            if (u >= n_units) break;
+            const float2 ab = heads[(warp * ST_HEADS + i) * 32 + lane];
+            float a = ab.x, b = ab.y;
+            if (P.rope && u < n_max) {   // Q and K heads
+                mx::rope_pair(a, b, cs, sn);
+                row[u * HD + lane] = a, row[u * HD + 32 + lane] = b;
             }
-            if (P.rope && !have_angle) {
-                mx::rope_angle(pos, lane, HD, P.theta, cs, sn);
-                have_angle = true;
-            }
-#pragma unroll
-            for (int i = 0; i < ST_HEADS; ++i) {
-                const int u = u0 + i * ST_SUBS;
-                if (u >= n_units) break;
-                float a = va[i], b = vb[i];
-                if (P.rope && u < n_max) {   // Q and K heads
-                    mx::rope_pair(a, b, cs, sn);
-                    row[u * HD + lane] = a, row[u * HD + 32 + lane] = b;
-                }
-                if (u < P.n_head) {
-                    __nv_bfloat16 *dst = P.qout + ((size_t)u * P.n_tok + tok) * HD;
-                    if (P.i8_scores) {
-                        // q row -> int8 codes per (row, head): id = 127 / amax, code = clamp(rne(q * id), +-127); the
-                        // codes go out as bf16 (exact), with the row's score factor (amax / 127) * 1/sqrt(64) * log2(e)
-                        // and the sum of its codes (the reference's own arithmetic, llm.cu:3700-3716)
-                        float amax = fmaxf(fabsf(a), fabsf(b));
-#pragma unroll
-                        for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
-                        const float id = amax > 0.0f ? __fdiv_rn(127.0f, amax) : 0.0f;
-                        const int ca = max(-127, min(127, __float2int_rn(a * id))), cb = max(-127, min(127, __float2int_rn(b * id)));
-                        const int sum = __reduce_add_sync(0xFFFFFFFFu, ca + cb), sq = __reduce_add_sync(0xFFFFFFFFu, ca * ca + cb * cb);
-                        dst[lane] = __float2bfloat16((float)ca);
-                        dst[lane + 32] = __float2bfloat16((float)cb);
-                        if (lane == 0) {
-                            const float qs = amax > 0.0f ? __fdiv_rn(amax, 127.0f) : 0.0f;
-                            P.row_a[(size_t)u * P.n_tok + tok] = qs * 0.125f * 1.4426950408889634f;
-                            P.row_qsum[(size_t)u * P.n_tok + tok] = (float)sum;
-                            raise(u, qs * qs * (float)sq);
-                        }
-                    } else {
-                        // values times 1/sqrt(64) * log2(e), one rounding: the scores arrive in log2 units
-                        dst[lane] = __float2bfloat16_rn(a * MX230_QK_LOG2_SCALE);
-                        dst[lane + 32] = __float2bfloat16_rn(b * MX230_QK_LOG2_SCALE);
-                        float ss = a * a + b * b;
-#pragma unroll
-                        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, o);
-                        if (lane == 0) raise(u, ss);
-                    }
-                    continue;
-                }
-                const bool is_v = u >= n_max;
-                const int h = is_v ? u - n_max : u - P.n_head;
-                __nv_bfloat16 *dst = (is_v ? P.vout : P.kout) + ((size_t)h * P.n_keys + pos) * HD;
-                float x0 = a, x1 = b;   // what attention sees
-                if (P.kq) {
-                    int8_t *cdst = (is_v ? P.vq : P.kq) + crow * kvd + h * HD;
-                    float *sc = is_v ? P.vs : P.ks, *be = is_v ? P.vb : P.kb;
-                    int c0, c1;
-                    float scale, beta;
-                    mx::quant_head_row(a, b, be != nullptr, c0, c1, scale, beta);
-                    cdst[lane] = (int8_t)c0, cdst[lane + 32] = (int8_t)c1;
+            float hi = 0.0f, lo = 0.0f;   // range of the head's values, for the quantisers
+            if (I8 || Q8) hi = mx::warp_max(fmaxf(a, b)), lo = mx::warp_min(fminf(a, b));
+            if (u < P.n_head) {
+                __nv_bfloat16 *dst = P.qout + ((size_t)u * P.n_tok + tok) * HD;
+                if (I8) {
+                    // q row -> int8 codes per (row, head): id = 127 / amax, code = clamp(rne(q * id), +-127); the
+                    // codes go out as bf16 (exact), with the row's score factor (amax / 127) * 1/sqrt(64) * log2(e)
+                    // and the sum of its codes (the reference's own arithmetic, llm.cu:3700-3716)
+                    const float amax = fmaxf(fabsf(hi), fabsf(lo));
+                    const float id = amax > 0.0f ? __fdiv_rn(127.0f, amax) : 0.0f;
+                    const int ca = max(-127, min(127, __float2int_rn(a * id))), cb = max(-127, min(127, __float2int_rn(b * id)));
+                    const int sum = __reduce_add_sync(0xFFFFFFFFu, ca + cb), sq = __reduce_add_sync(0xFFFFFFFFu, ca * ca + cb * cb);
+                    dst[lane] = __float2bfloat16((float)ca);
+                    dst[lane + 32] = __float2bfloat16((float)cb);
                     if (lane == 0) {
-                        sc[crow * P.n_kv_head + h] = scale;
-                        if (be) be[crow * P.n_kv_head + h] = beta;
-                    }
-                    x0 = (float)c0 * scale + beta, x1 = (float)c1 * scale + beta;
-                    a = x0, b = x1;
-                    if (P.i8_scores && !is_v) {
-                        x0 = (float)c0, x1 = (float)c1;
-                        if (lane == 0) {
-                            float *kk = stage_kskb(P, h, pos);
-                            kk[0] = scale, kk[128] = beta;
-                        }
+                        const float qs = amax > 0.0f ? __fdiv_rn(amax, 127.0f) : 0.0f;
+                        P.row_a[(size_t)u * P.n_tok + tok] = qs * 0.125f * 1.4426950408889634f;
+                        P.row_qsum[(size_t)u * P.n_tok + tok] = (float)sum;
+                        raise(u, qs * qs * (float)sq);
                     }
                 } else {
-                    float *cdst = (is_v ? P.vcache : P.kcache) + crow * kvd + h * HD;
-                    cdst[lane] = a, cdst[lane + 32] = b;
-                }
-                dst[lane] = __float2bfloat16_rn(x0);
-                dst[lane + 32] = __float2bfloat16_rn(x1);
-                if (!is_v) {
+                    // values times 1/sqrt(64) * log2(e), one rounding: the scores arrive in log2 units
+                    dst[lane] = __float2bfloat16_rn(a * MX230_QK_LOG2_SCALE);
+                    dst[lane + 32] = __float2bfloat16_rn(b * MX230_QK_LOG2_SCALE);
                     float ss = a * a + b * b;
 #pragma unroll
                     for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, o);
-                    if (lane == 0) raise(P.n_head + h, ss);
+                    if (lane == 0) raise(u, ss);
                 }
+                continue;
+            }
+            const bool is_v = u >= n_max;
+            const int h = is_v ? u - n_max : u - P.n_head;
+            __nv_bfloat16 *dst = (is_v ? P.vout : P.kout) + ((size_t)h * P.n_keys + pos) * HD;
+            float x0 = a, x1 = b;   // what attention sees
+            if (Q8) {
+                int8_t *cdst = (is_v ? P.vq : P.kq) + crow * kvd + h * HD;
+                float *sc = is_v ? P.vs : P.ks, *be = is_v ? P.vb : P.kb;
+                int c0, c1;
+                float scale, beta;
+                mx::quant_head_row(a, b, hi, lo, be != nullptr, c0, c1, scale, beta);
+                cdst[lane] = (int8_t)c0, cdst[lane + 32] = (int8_t)c1;
+                if (lane == 0) {
+                    sc[crow * P.n_kv_head + h] = scale;
+                    if (be) be[crow * P.n_kv_head + h] = beta;
+                }
+                x0 = (float)c0 * scale + beta, x1 = (float)c1 * scale + beta;
+                a = x0, b = x1;
+                if (I8 && !is_v) {
+                    x0 = (float)c0, x1 = (float)c1;
+                    if (lane == 0) {
+                        float *kk = stage_kskb(P, h, pos);
+                        kk[0] = scale, kk[128] = beta;
+                    }
+                }
+            } else {
+                float *cdst = (is_v ? P.vcache : P.kcache) + crow * kvd + h * HD;
+                cdst[lane] = a, cdst[lane + 32] = b;
+            }
+            dst[lane] = __float2bfloat16_rn(x0);
+            dst[lane + 32] = __float2bfloat16_rn(x1);
+            if (!is_v) {
+                float ss = a * a + b * b;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, o);
+                if (lane == 0) raise(P.n_head + h, ss);
             }
         }
+        if (next != tok && next < P.n_tok && P.rope) mx::rope_angle(P.pos0 + next, lane, HD, P.theta, cs, sn);
+        tok = next, u0 = next_u0;
     }
 
     // ---- cached keys [0, n_old): from the last warp of every CTA on, the first ones have the new tokens ----
@@ -194,7 +206,7 @@ __global__ void __launch_bounds__(ST_THREADS, 2) prefill_stage_kernel(const Stag
         const size_t row = stage_row(P, t);
         const size_t dst = ((size_t)h * P.n_keys + t) * HD + c * 8;
         float k[8], v[8], ksc = 0.0f, kbe = 0.0f, ss = 0.0f;
-        if (P.kq) {
+        if (Q8) {
             const int2 kw = *(const int2 *)(P.kq + row * kvd + h * HD + c * 8);
             const int2 vw = *(const int2 *)(P.vq + row * kvd + h * HD + c * 8);
             ksc = P.ks[row * P.n_kv_head + h];
@@ -207,7 +219,7 @@ __global__ void __launch_bounds__(ST_THREADS, 2) prefill_stage_kernel(const Stag
                 const float code = (float)(int8_t)((kk[i >> 2] >> (8 * (i & 3))) & 0xFF);
                 const float val = code * ksc + kbe;
                 ss += val * val;
-                k[i] = P.i8_scores ? code : val;
+                k[i] = I8 ? code : val;
                 v[i] = (float)(int8_t)((vv[i >> 2] >> (8 * (i & 3))) & 0xFF) * vsc + vbe;
             }
         } else {
@@ -216,7 +228,7 @@ __global__ void __launch_bounds__(ST_THREADS, 2) prefill_stage_kernel(const Stag
             const float4 a = kp[0], b = kp[1], e = vp[0], f = vp[1];
             k[0] = a.x, k[1] = a.y, k[2] = a.z, k[3] = a.w, k[4] = b.x, k[5] = b.y, k[6] = b.z, k[7] = b.w;
             v[0] = e.x, v[1] = e.y, v[2] = e.z, v[3] = e.w, v[4] = f.x, v[5] = f.y, v[6] = f.z, v[7] = f.w;
-            if (P.i8_scores) {   // K quantised on the fly, symmetric absmax per row (the reference's attn_prefill_dp4a)
+            if (I8) {   // K quantised on the fly, symmetric absmax per row (the reference's attn_prefill_dp4a)
                 float amax = 0.0f;
 #pragma unroll
                 for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(k[i]));
@@ -245,7 +257,7 @@ __global__ void __launch_bounds__(ST_THREADS, 2) prefill_stage_kernel(const Stag
         *(uint4 *)(P.kout + dst) = ko;
         *(uint4 *)(P.vout + dst) = vo;
         if (c == 0) {
-            if (P.i8_scores) {
+            if (I8) {
                 float *kk = stage_kskb(P, h, t);
                 kk[0] = ksc, kk[128] = kbe;
             }
@@ -273,6 +285,18 @@ struct StepArgs {
     int rope;
     float theta;
 };
+
+// sm: bytes of the norms
+constexpr size_t ST_NORM_BYTES = 48 * 1024, ST_HEAD_BYTES = (size_t)ST_WARPS * ST_HEADS * 64 * sizeof(float);
+template <bool I8, bool Q8>
+int launch_stage(mx230_handle *h, cudaStream_t st, const StageParams &S, int cluster, size_t sm) {
+    MX_SMEM_ATTR_ONCE(h->device, (prefill_stage_kernel<4, I8, Q8>), ST_HEAD_BYTES + ST_NORM_BYTES);
+    MX_SMEM_ATTR_ONCE(h->device, (prefill_stage_kernel<8, I8, Q8>), ST_HEAD_BYTES + ST_NORM_BYTES);
+    MX_LAUNCH(h, st, MX230_K_PREFILL,
+              mx_launch(cluster == 8 ? prefill_stage_kernel<8, I8, Q8> : prefill_stage_kernel<4, I8, Q8>, MX230_NORM_PARTS * cluster, ST_THREADS,
+                        ST_HEAD_BYTES + sm, st, cluster, true, S));
+    return MX230_OK;
+}
 
 size_t align1k(size_t x) { return (x + 1023) & ~(size_t)1023; }
 
@@ -327,7 +351,7 @@ int prefill(mx230_handle *h, void *stream, float *out, const float *qkv, const f
     const bool i8_scores = dp4a || (kq && h->q8_score_mode == MX230_Q8_SCORE_REF);
     StageParams S;
     S.qout = qb, S.kout = kbuf, S.vout = vbuf, S.q_norm2 = q_norm2, S.k_norm2 = k_norm2;
-    S.row_a = row_a, S.row_qsum = row_qsum, S.kskb = kskb, S.i8_scores = i8_scores, S.n_k_tiles = n_k_pad / 128;
+    S.row_a = row_a, S.row_qsum = row_qsum, S.kskb = kskb, S.n_k_tiles = n_k_pad / 128;
     S.qkv = const_cast<float *>(qkv), S.stride = qkv_stride, S.n_tok = n_tok, S.pos0 = pos0, S.n_keys = n_keys;
     S.n_head = n_head, S.n_kv_head = n_kv_head;
     S.kcache = const_cast<float *>(kcache), S.vcache = const_cast<float *>(vcache);
@@ -336,19 +360,23 @@ int prefill(mx230_handle *h, void *stream, float *out, const float *qkv, const f
     S.bt = bt, S.bs = bs;
     S.write_kv = step.write_kv, S.rope = step.rope, S.theta = step.theta;
     size_t sm = (size_t)(n_head + n_kv_head) * sizeof(int);
-    if (sm > 48 * 1024) {   // more heads than a CTA keeps norms for: without them every head takes the general loop
+    if (sm > ST_NORM_BYTES) {   // more heads than a CTA keeps norms for: without them every head takes the general loop
         sm = 0;
         S.q_norm2 = S.k_norm2 = q_norm2 = k_norm2 = nullptr;
     }
-    // 256 CTAs, two per SM, where 128 would take tokens or cached keys in more than one round (2048 tokens over 6144 int8 keys,
-    // 32/4 heads, us a call: 128 176.6, 256 168.7); below that 128, the smaller launch
+    // 256 CTAs, two per SM, where the warps of 128 would take tokens and cached keys in more than one round (2048 tokens over 6144
+    // int8 keys, 32/4 heads, us a call: 128 176.6, 256 168.7; 512 over 1536, 14/2 heads, whose 128 CTAs have 16 warps of tokens
+    // and 6 of keys, 5.1 us from the wait to their end against 1.9); below that 128, the smaller launch
     const size_t old = (size_t)(step.write_kv ? pos0 : n_keys) * n_kv_head * 8;   // threads
-    const int cluster = n_tok > 4 * MX230_NORM_PARTS * (ST_WARPS / ST_SUBS) || old > (size_t)4 * MX230_NORM_PARTS * ST_THREADS ? 8 : 4;
-    const size_t per_cta = (old + 32 * MX230_NORM_PARTS * cluster - 1) / (32 * MX230_NORM_PARTS * cluster);
+    auto warps_of = [&](int ctas) { return (old + 32 * ctas - 1) / (32 * ctas); };   // of a CTA, for cached keys
+    const int c4 = 4 * MX230_NORM_PARTS;
+    const int cluster = (size_t)((n_tok + c4 - 1) / c4) * ST_SUBS + warps_of(c4) > ST_WARPS ? 8 : 4;
+    const size_t per_cta = warps_of(cluster * MX230_NORM_PARTS);
     S.old_warps = per_cta < ST_WARPS ? (int)per_cta : ST_WARPS;
-    MX_LAUNCH(h, st, MX230_K_PREFILL,
-              mx_launch(cluster == 8 ? prefill_stage_kernel<8> : prefill_stage_kernel<4>, MX230_NORM_PARTS * cluster, ST_THREADS, sm, st,
-                        cluster, true, S));
+    int rc;
+    if (kq) rc = i8_scores ? launch_stage<true, true>(h, st, S, cluster, sm) : launch_stage<false, true>(h, st, S, cluster, sm);
+    else rc = i8_scores ? launch_stage<true, false>(h, st, S, cluster, sm) : launch_stage<false, false>(h, st, S, cluster, sm);
+    if (rc) return rc;
     return mx230_launch_flash_fwd_ex(h, st, qb, kbuf, vbuf, out, nullptr, n_head, n_tok, n_keys, pos0, n_head / n_kv_head, HD,
                                      out_stride, 1, i8_scores ? 0 : 1, q_norm2, k_norm2, i8_scores ? row_a : nullptr,
                                      i8_scores ? row_qsum : nullptr, i8_scores ? kskb : nullptr, o_half ? qb : nullptr);
