@@ -1522,10 +1522,16 @@ __global__ void __launch_bounds__(256) cast_bf16_kernel(const CastParams P) {
             for (int u = 0; u < 4; ++u) row_norm(a[u]);
         }
     }
-    for (; i < n4; i += step) {
-        const float4 a = __ldcs(src + i);
-        dst[i] = make_uint2(mx::pack_bf16(a.x * sc, a.y * sc), mx::pack_bf16(a.z * sc, a.w * sc));
-        if (norm_out != nullptr) row_norm(a);
+    if (i < n4) {   // the last one to three of a ragged head, their loads together as well
+        float4 a[3];
+#pragma unroll
+        for (int u = 0; u < 3; ++u) a[u] = __ldcs(src + (i + u * step < n4 ? i + u * step : i));
+#pragma unroll
+        for (int u = 0; u < 3; ++u) {
+            if (u > 0 && i + u * step >= n4) break;
+            dst[i + u * step] = make_uint2(mx::pack_bf16(a[u].x * sc, a[u].y * sc), mx::pack_bf16(a[u].z * sc, a[u].w * sc));
+            if (norm_out != nullptr) row_norm(a[u]);
+        }
     }
     if (norm_out != nullptr) {   // block maximum -> this part's slot (parts the grid does not have are set to 0)
         __shared__ float red[8];
