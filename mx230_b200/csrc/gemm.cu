@@ -13,7 +13,9 @@
 // TMA ring (out-of-range rows and columns are zero-filled by the TMA unit, so m, n, k need no padding); one TMA warp, one
 // MMA-issuing warp, eight epilogue warps that add the bias and hand fp32 pieces to the TMA unit.
 // What bounds it at these sizes is the operands' way from L2 into shared memory (1900 x 896 x 1152: 90 MB with 64-column
-// tiles, 60 MB with 128-column ones) and the launches around it.
+// tiles, 60 MB with 128-column ones) and the launches around it.  Around the products: the bias is loaded under them, a warp's
+// pieces leave through 4 KB each, staging takes two loads a thread at a time (layer of 1900 tokens, 14/2 heads, two of these
+// each: 49.6 -> 47.6 us a call, 128 tokens 27.2 -> 24.6).
 #include <cstring>
 
 #include "common.cuh"
@@ -142,14 +144,20 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CU
         // ------------------------- epilogue: bias, fp32 rows out -------------------------
         // warp: 32 rows (its tensor-memory lanes), half of the tile's columns
         const int q = warp & 3, colh = ((warp - 4) >> 2) * (GN / 2);
+        float bias_l[GN / 64];   // lane l: the bias of column l of every piece, loaded under the products
+#pragma unroll
+        for (int part = 0; part < GN / 64; ++part) {
+            const int col = n0 + colh + part * 32 + lane;
+            bias_l[part] = P.bias && col < P.n ? P.bias[col] : 0.0f;
+        }
         bool ok = __all_sync(0xFFFFFFFFu, mx::mbar_wait(bar(2 * STAGES), 0, abort_flag, P.status));
         if (ok) {
             mx::tc_fence_after();
             const int row = m0 + q * 32 + lane;
             const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16);
-            // pieces of 32 x 32 go through 4 KB each of the ring's first stage or two (every MMA has read them) and the TMA
-            // unit, which clips rows past the end: 16-byte stores from lane = row registers each touch a sector of their own
-            const int st_off = (warp - 4) * 4096;
+            // pieces of 32 x 32 go through 4 KB each of the ring's first stages (every MMA has read them) and the TMA unit,
+            // which clips rows past the end: 16-byte stores from lane = row registers each touch a sector of their own
+            static_assert(EPI_WARPS * (GN / 64) * 4096 <= STAGES * S::STAGE, "pieces");
 #pragma unroll
             for (int part = 0; part < GN / 64; ++part) {
                 const int col0 = n0 + colh + part * 32;
@@ -157,15 +165,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CU
                 uint32_t v[32];
                 mx::tmem_ld32(ta + colh + part * 32, v);
                 mx::tmem_wait_ld();
-                if (part > 0 && P.tma_out) {
-                    if (lane == 0) mx::bulk_wait_group_read<0>();
-                    __syncwarp();
-                }
+                const int st_off = ((warp - 4) * (GN / 64) + part) * 4096;
                 float *crow = P.tma_out ? (float *)(smem + st_off + lane * 128) : P.C + (size_t)row * P.n + col0;
 #pragma unroll
                 for (int c = 0; c < 32; c += 4) {
+                    float4 b4;   // (a lane past the last column has 0)
+                    b4.x = __shfl_sync(0xFFFFFFFFu, bias_l[part], c), b4.y = __shfl_sync(0xFFFFFFFFu, bias_l[part], c + 1);
+                    b4.z = __shfl_sync(0xFFFFFFFFu, bias_l[part], c + 2), b4.w = __shfl_sync(0xFFFFFFFFu, bias_l[part], c + 3);
                     if (col0 + c >= P.n) break;   // n is a multiple of 4: a float4 is inside or outside as a whole
-                    const float4 b4 = P.bias ? *(const float4 *)(P.bias + col0 + c) : make_float4(0.f, 0.f, 0.f, 0.f);
                     const float4 o4 = make_float4(__uint_as_float(v[c]) + b4.x, __uint_as_float(v[c + 1]) + b4.y,
                                                   __uint_as_float(v[c + 2]) + b4.z, __uint_as_float(v[c + 3]) + b4.w);
                     if (P.tma_out) *(float4 *)((unsigned char *)crow + (((c >> 2) ^ (lane & 7)) << 4)) = o4;
@@ -205,8 +212,7 @@ __global__ void gemm_stage_kernel(StageParams P) {
     mx::pdl_wait();
     const int t = blockIdx.y;
     const float4 *src = (const float4 *)P.src[t];
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < P.n4[t]; i += (size_t)gridDim.x * blockDim.x) {
-        const float4 x = src[i];
+    auto convert = [&](size_t i, const float4 &x) {
         if (SPLIT) {
             const __nv_bfloat16 h0 = __float2bfloat16_rn(x.x), h1 = __float2bfloat16_rn(x.y), h2 = __float2bfloat16_rn(x.z),
                                 h3 = __float2bfloat16_rn(x.w);
@@ -222,6 +228,13 @@ __global__ void gemm_stage_kernel(StageParams P) {
             __half2 hv[2] = {__floats2half2_rn(x.x, x.y), __floats2half2_rn(x.z, x.w)};
             ((uint2 *)P.hi[t])[i] = *(const uint2 *)hv;
         }
+    };
+    const size_t n4 = P.n4[t], step = (size_t)gridDim.x * blockDim.x;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += 2 * step) {   // two loads in flight
+        const bool two = i + step < n4;
+        const float4 x = src[i], y = src[two ? i + step : i];
+        convert(i, x);
+        if (two) convert(i + step, y);
     }
 }
 
@@ -306,7 +319,7 @@ extern "C" int mx230_gemm(mx230_handle *h, void *stream, float *C, const float *
     SP.src[0] = A, SP.hi[0] = a_hi, SP.lo[0] = a_lo, SP.n4[0] = (size_t)m * k / 4;
     SP.src[1] = W, SP.hi[1] = w_hi, SP.lo[1] = w_lo, SP.n4[1] = split ? (size_t)k * n / 4 : 0;
     const size_t big = SP.n4[0] > SP.n4[1] ? SP.n4[0] : SP.n4[1];
-    unsigned blocks = (unsigned)((big + 255) / 256);
+    unsigned blocks = (unsigned)((big + 511) / 512);
     if (blocks > (unsigned)h->sm_count * 8) blocks = (unsigned)h->sm_count * 8;
     if (split) {
         MX_LAUNCH(h, st, MX230_K_CAST, mx_launch(gemm_stage_kernel<true>, dim3(blocks, 2), 256, 0, st, 1, true, SP));
