@@ -48,7 +48,8 @@ inline DecodeSplit plan_splits(long long slots, long long groups, long long keys
 // fp32 cache, CTAs of eight warps that have an SM to themselves.  fit[c]: clusters of c such CTAs that the device holds at once,
 // by its own count: how many GPCs have room for another cluster of seven or eight does not follow from the number of SMs (148 of
 // them hold 15; as 16, or as 17 and 18 of seven, they took a second wave).  False: the four-warp plan.
-// us a call, position on the device, at 500 / 4000 / 32000 keys; four-warp CTAs, clusters of eight counted as 7/8 of the SMs, this:
+// us a call, position on the device, at 500 / 4000 / 32000 keys (with the tile loop that read q from shared memory; with q in registers
+// groups of 7 and 8 heads are a fifth to a third faster in either plan); four-warp CTAs, clusters of eight counted as 7/8 of the SMs, this:
 //   16/16 heads  5.8 12.0 45.7 |  6.9 12.7 58.4 | 5.3 11.5 45.8        32/8  5.7 12.6 28.8 |  4.7  8.8 43.9 | 5.3 10.7 27.7
 //   32/4         8.1 16.1 41.1 |  6.7 12.6 40.7 | 6.8 12.7 27.0        72/9  8.3 18.2 50.2 |  6.8 13.2 58.3 | 7.2 13.6 43.7
 // Unknown length, more than two query heads a group (where the arithmetic of a key counts beside its loads): clusters of eight that

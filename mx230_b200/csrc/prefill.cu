@@ -61,7 +61,7 @@ __device__ __forceinline__ float *stage_kskb(const StageParams &P, int h, int t)
 // per token and warp and a head's quantiser is a warp reduction.  Cached keys: eight threads per key and head, eight dims
 // each.  What a warp of new tokens costs is the code it fetches as much as its arithmetic: its heads are one rolled loop over
 // values in shared memory, an instantiation per cache and score mode, and the first angle is formed before the wait (512 tokens over
-// 1536 int8 keys, from the wait to the last token 4.4 -> 3.9 us, a call 26.9 -> 24.6; over fp32 keys 20.4 -> 19.0).  Row norms go through shared memory and, per cluster of CTAs, into one of MX230_NORM_PARTS parts: with Q's
+// 1536 int8 keys, from the wait to the last token 4.3 -> 4.1 us and to the norms 5.9 -> 5.0, a call 26.9 -> 24.6; over fp32 keys 20.4 -> 19.0).  Row norms go through shared memory and, per cluster of CTAs, into one of MX230_NORM_PARTS parts: with Q's
 // and K's the attention kernel bounds every score of a head and, where the bound is small, runs without a row max.
 // CLUSTER: CTAs that share one norm part, 4 or 8.  I8: int8 scores; Q8: int8 cache (instantiations: code that a launch does not
 // run is not fetched either).  (Sizes are constants or come from the host: a division costs more here than
@@ -366,7 +366,7 @@ int prefill(mx230_handle *h, void *stream, float *out, const float *qkv, const f
     }
     // 256 CTAs, two per SM, where the warps of 128 would take tokens and cached keys in more than one round (2048 tokens over 6144
     // int8 keys, 32/4 heads, us a call: 128 176.6, 256 168.7; 512 over 1536, 14/2 heads, whose 128 CTAs have 16 warps of tokens
-    // and 6 of keys, 5.1 us from the wait to their end against 1.9); below that 128, the smaller launch
+    // and 6 of keys, 5.1 us from the wait to their end against 1.7); below that 128, the smaller launch
     const size_t old = (size_t)(step.write_kv ? pos0 : n_keys) * n_kv_head * 8;   // threads
     auto warps_of = [&](int ctas) { return (old + 32 * ctas - 1) / (32 * ctas); };   // of a CTA, for cached keys
     const int c4 = 4 * MX230_NORM_PARTS;
