@@ -1620,8 +1620,9 @@ bool fwd_key_split(int heads, int n_q, int n_k, int q_off, int causal, int sms) 
 }
 
 // Items of 64 rows wherever every one of them has an SM to itself: a key tile costs such an item less than a key-split item's
-// turn of two tiles (1050 cycles against 2 x 1275; both read every K and V tile from L2, and this one is bound by shared memory:
-// 104 KB a tile), but more per row, so a second round would lose.  us a call, key-split / 64 rows: 1 x 8192 rows causal 49.0 / 41.1, 4 x
+// turn of two tiles (1050 cycles against 2 x 1275), but more per row, so a second round would lose.  No unit is near its limit (1 x 8192
+// rows: 0.41 instructions a cycle and scheduler, exp pipe 37 %, tensor reads of shared memory 33 %): one warp per group and
+// scheduler waits for its tensor-memory loads, and P V of the four groups' tiles runs in key order.  us a call, key-split / 64 rows: 1 x 8192 rows causal 49.0 / 41.1, 4 x
 // 1024 13.2 / 11.6, 6 x 1400 16.6 / 15.3; prefill of 512 tokens over 2048 int8 keys, 14/2 heads, 28.7 / 26.7, 128 over 4128 41.5 /
 // 35.1, 512 over 512 17.5 / 17.8 (the worst of 60); beyond one round 12 x 1024 15.2 / 16.6, 8 x 2000 21.8 / 24.5, 4 x 4096 30.4 / 30.0.
 // Int8 scores, whose first tile costs more here, from eleven key tiles on (128 over 1128 keys, 32/4 heads, 24.1 / 25.1; 100 over 100
