@@ -1195,9 +1195,9 @@ decode_q8_mma_kernel(const DecodeParams P) {
 //   values:  weights through a per-warp shared buffer.
 // What bounds it: multiply-adds (2 * G * 64 per key, packed in pairs) beside a stream that a tile's worth of latency per warp
 // keeps going.  In its place lane = (key, half of the dims) read q from shared memory for every key: 88 16-byte reads a lane
-// and tile where 24 do, and 168 shuffles for a warp's totals where 52 do.  us a call, before / after: one sequence, host
+// and tile where 24 do, and 168 shuffles for a warp's totals where 50 do.  us a call, before / after: one sequence, host
 // position, 14/2 heads 1500 keys 8.1 / 6.1, 32/4 heads 4000 keys 13.0 / 9.0; 16 paged sequences of up to 1500 keys, 32/4 heads
-// 17.8 / 16.0; 1 x 32768 keys 14/2 heads 16.2 / 13.0; one K/V head per query head level.  Error against 64 bits 1.3e-7 to
+// 17.8 / 14.3; 1 x 32768 keys 14/2 heads 16.2 / 13.0; one K/V head per query head level.  Error against 64 bits 1.3e-7 to
 // 1.9e-7 where it was 1.5e-7 to 2.1e-7.  Three CTAs are resident per SM.
 // ---------------------------------------------------------------------------
 constexpr int F32_WARPS = 4;
@@ -1217,10 +1217,16 @@ struct F32Smem {
     static constexpr int TOTAL = ((Q_BYTES + 127) & ~127) + (WARPS * PER_WARP > MERGE ? WARPS * PER_WARP : MERGE);
 };
 
-template <int G, bool PAGED, bool FUSED, int WARPS>
+// The cache: rows by position, or through a table of blocks that hold whole tiles of a sequence, or of other blocks.  Instantiations:
+// with the three ways to request a tile behind one run-time choice the kernel with eight heads spilled 92 bytes and 16 paged
+// sequences of up to 1500 keys, 32/4 heads, took 13.0 us in blocks of 16 and 14.1 in blocks of 8 (12.0, 12.2 so).
+enum { F32_LINEAR = 0, F32_BLOCKS = 1, F32_ANY_BLOCKS = 2 };
+
+template <int G, int CACHE, bool FUSED, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, WARPS == F32_WARPS_WIDE ? 1 : 3)
 decode_f32_ring_kernel(const DecodeParams P) {
     using SM = F32Smem<G, WARPS>;
+    constexpr bool PAGED = CACHE != F32_LINEAR, ANY = CACHE == F32_ANY_BLOCKS;
     constexpr int GP = SM::GP;
     constexpr float LOG2E = 1.4426950408889634f;
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -1284,23 +1290,34 @@ decode_f32_ring_kernel(const DecodeParams P) {
     const uint32_t piece = (uint32_t)(pk * 256 + pc * 16);
     const size_t it_stride = (size_t)2 * kvd;
     // Paged caches: a tile that lies in one cache block has consecutive rows and takes one lookup, the same in all lanes; else lane
-    // l looks up the row of key l (mod 16).  Either way one tile ahead, off the chain of dependent loads.
-    const bool whole = !PAGED || (P.bs % FT_KEYS == 0 && kbeg % FT_KEYS == 0);
+    // l looks up the row of key l (mod 16).  Two tiles ahead: the row of the next tile to be requested is in row_l, that of the one
+    // after on its way (one ahead, the lookup was waited for under half a tile's work: 12/12 heads 17.8 us against 17.2).
     auto row_ahead = [&](int tile) {
-        const int t0 = wa + tile * FT_KEYS, t = t0 + (whole ? 0 : pc);
+        const int t0 = wa + tile * FT_KEYS, t = t0 + (ANY ? pc : 0);
         return paged_row(P, table, t < wb ? t : wa);
     };
-    int row_l = 0;
+    int row_l = 0, row_next = 0;
     if (PAGED && n_tiles > 0) row_l = row_ahead(0);
+    if (PAGED && n_tiles > 1) row_next = row_ahead(1);
 
     // A tile's K rows and its V rows are requested, waited for and replaced apart: while one half of a slot is worked on three
-    // of the warp's four are in flight (both together: two)
+    // of the warp's four are in flight (both together: two).  Where every key has a row of its own both are requested with V, so
+    // that a row's lookup is handed round and its address formed once (apart: 16 sequences of up to 1500 keys in blocks of 8,
+    // 16/8 heads, 13.4 us against 12.8).
     auto issue = [&](int tile, bool is_v) {
-        if (tile < n_tiles) {
-            const uint32_t dst = ring_u32 + (tile % FT_STAGES) * FT_STAGE + (is_v ? FT_KEYS * 256 : 0) + piece;
-            const float *cache = (is_v ? P.vcache : P.kcache) + kvh * 64 + pc * 4;
+        if (tile < n_tiles && (is_v || !ANY)) {
+            const uint32_t dst = ring_u32 + (tile % FT_STAGES) * FT_STAGE + (is_v && !ANY ? FT_KEYS * 256 : 0) + piece;
+            const float *cache = (is_v && !ANY ? P.vcache : P.kcache) + kvh * 64 + pc * 4;
             const int key0 = wa + tile * FT_KEYS;
-            if (whole) {
+            if (ANY) {
+#pragma unroll
+                for (int it = 0; it < 8; ++it) {
+                    const int key = it * 2 + pk, n = key0 + key < wb ? 16 : 0;
+                    const size_t off = (size_t)__shfl_sync(0xFFFFFFFFu, row_l, key) * kvd;
+                    cp_async16(dst + it * 512, cache + off, n);
+                    cp_async16(dst + FT_KEYS * 256 + it * 512, P.vcache + kvh * 64 + pc * 4 + off, n);
+                }
+            } else {
                 const float *src = cache + ((PAGED ? (long long)row_l : base + key0) + pk) * kvd;
                 if (key0 + FT_KEYS <= wb) {
 #pragma unroll
@@ -1312,15 +1329,11 @@ decode_f32_ring_kernel(const DecodeParams P) {
                         cp_async16(dst + it * 512, ok ? src + it * it_stride : cache, ok ? 16 : 0);
                     }
                 }
-            } else {
-#pragma unroll
-                for (int it = 0; it < 8; ++it) {
-                    const int key = it * 2 + pk;
-                    const size_t off = (size_t)__shfl_sync(0xFFFFFFFFu, row_l, key) * kvd;
-                    cp_async16(dst + it * 512, cache + off, key0 + key < wb ? 16 : 0);
-                }
             }
-            if (PAGED && is_v && tile + 1 < n_tiles) row_l = row_ahead(tile + 1);
+            if (PAGED && is_v) {
+                row_l = row_next;
+                if (tile + 2 < n_tiles) row_next = row_ahead(tile + 2);
+            }
         }
         cp_async_commit();
     };
@@ -1412,7 +1425,7 @@ decode_f32_ring_kernel(const DecodeParams P) {
     };
     constexpr int STEPS = FT_KEYS / 4;
     for (int tile = 0; tile < n_tiles; ++tile) {
-        cp_async_wait<2 * FT_STAGES - 1>();
+        cp_async_wait<2 * FT_STAGES - (ANY ? 2 : 1)>();   // the tile's K rows (ANY: with its V rows)
         __syncwarp();
         const unsigned char *st = ring + (tile % FT_STAGES) * FT_STAGE + kl * 256 + dsl * 16;
         // ---- scores (log2 domain): 4 steps of 4 keys ----
@@ -1563,18 +1576,18 @@ int launch_q8_mma(mx230_handle *h, cudaStream_t st, const DecodeParams &P, dim3 
               mx_launch(decode_q8_mma_kernel<PAGED, FUSED>, grid, Q8_THREADS, sm, st, P.cl_size, P.push_regions == nullptr, P));
     return MX230_OK;
 }
-template <int G, bool PAGED, bool FUSED, int WARPS>
+template <int G, int CACHE, bool FUSED, int WARPS>
 int launch_f32_warps(mx230_handle *h, cudaStream_t st, const DecodeParams &P, dim3 grid) {
     const size_t sm = (size_t)F32Smem<G, WARPS>::TOTAL;
-    MX_SMEM_ATTR_ONCE(h->device, (decode_f32_ring_kernel<G, PAGED, FUSED, WARPS>), sm);
+    MX_SMEM_ATTR_ONCE(h->device, (decode_f32_ring_kernel<G, CACHE, FUSED, WARPS>), sm);
     MX_LAUNCH(h, st, MX230_K_DECODE_F32,
-              mx_launch(decode_f32_ring_kernel<G, PAGED, FUSED, WARPS>, grid, WARPS * 32, sm, st, P.cl_size, P.push_regions == nullptr, P));
+              mx_launch(decode_f32_ring_kernel<G, CACHE, FUSED, WARPS>, grid, WARPS * 32, sm, st, P.cl_size, P.push_regions == nullptr, P));
     return MX230_OK;
 }
-template <int G, bool PAGED, bool FUSED>
+template <int G, int CACHE, bool FUSED>
 int launch_f32(mx230_handle *h, cudaStream_t st, const DecodeParams &P, dim3 grid) {
-    return P.wide ? launch_f32_warps<G, PAGED, FUSED, F32_WARPS_WIDE>(h, st, P, grid)
-                  : launch_f32_warps<G, PAGED, FUSED, F32_WARPS>(h, st, P, grid);
+    return P.wide ? launch_f32_warps<G, CACHE, FUSED, F32_WARPS_WIDE>(h, st, P, grid)
+                  : launch_f32_warps<G, CACHE, FUSED, F32_WARPS>(h, st, P, grid);
 }
 
 // int8 cache in the reference score mode: the tensor-core kernel serves any group size up to 8 per CTA
@@ -1600,14 +1613,16 @@ int launch_g(mx230_handle *h, cudaStream_t st, const DecodeParams &P, dim3 grid)
         }
         return MX230_OK;
     }
-    if (P.tables) return fused ? launch_f32<G, true, true>(h, st, P, grid) : launch_f32<G, true, false>(h, st, P, grid);
-    return fused ? launch_f32<G, false, true>(h, st, P, grid) : launch_f32<G, false, false>(h, st, P, grid);
+    if (P.tables && P.bs % FT_KEYS == 0)   // (paged sequences start at key 0: key ranges have linear caches)
+        return fused ? launch_f32<G, F32_BLOCKS, true>(h, st, P, grid) : launch_f32<G, F32_BLOCKS, false>(h, st, P, grid);
+    if (P.tables) return fused ? launch_f32<G, F32_ANY_BLOCKS, true>(h, st, P, grid) : launch_f32<G, F32_ANY_BLOCKS, false>(h, st, P, grid);
+    return fused ? launch_f32<G, F32_LINEAR, true>(h, st, P, grid) : launch_f32<G, F32_LINEAR, false>(h, st, P, grid);
 }
 
 }  // namespace
 
 void mx230_count_wide_clusters(mx230_handle *h) {
-    const auto kernel = decode_f32_ring_kernel<8, false, false, F32_WARPS_WIDE>;   // (the instantiation with the most shared memory)
+    const auto kernel = decode_f32_ring_kernel<8, F32_LINEAR, false, F32_WARPS_WIDE>;   // (the instantiation with the most shared memory)
     const size_t sm = (size_t)F32Smem<8, F32_WARPS_WIDE>::TOTAL;
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     for (int c = 1; c <= 8; ++c) {

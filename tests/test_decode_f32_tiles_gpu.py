@@ -61,3 +61,32 @@ def test_an_infinite_value_of_the_new_token_stays_in_its_dims(handle, nh, nkv, p
     hit = torch.zeros(nh, 64, dtype=torch.bool, device="cuda")
     hit[:nh // nkv, 5] = True
     assert torch.isinf(out[hit]).all() and torch.isfinite(out[~hit]).all()
+
+
+@pytest.mark.parametrize("bs", [8, 16, 24, 48])
+@pytest.mark.parametrize("nh,nkv,n_seq", [(12, 12, 20), (16, 8, 30), (24, 8, 30), (14, 2, 70), (16, 2, 70), (32, 4, 40)])
+def test_ranges_of_several_tiles(handle, nh, nkv, n_seq, bs):
+    """A warp's range of none to nine tiles, in a batch whose groups leave a sequence one CTA or two: a tile's rows are looked up two
+    tiles ahead.  Rows beyond a sequence's keys are NaN.  Bound as above."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(23)
+    n_log = -(-560 // bs)
+    keys = torch.tensor([(1 + 37 * i) % 560 + 1 for i in range(n_seq)], device="cuda")
+    keys[0] = 560
+    table = torch.randperm(n_seq * n_log, device="cuda", generator=g).to(torch.int32).reshape(n_seq, n_log)
+    c = la.KvCache(n_seq * n_log * bs, nkv)
+    c.k.fill_(float("nan")), c.v.fill_(float("nan"))
+    rows = torch.randn(n_seq, (nh + 2 * nkv) * 64, device="cuda", generator=g)
+    out = torch.full((n_seq, nh * 64), float("nan"), device="cuda")
+    want = []
+    for s in range(n_seq):
+        n = int(keys[s])
+        at = torch.arange(n, device="cuda")
+        phys = table[s][at // bs].long() * bs + at % bs
+        k, v = (torch.randn(n, nkv * 64, device="cuda", generator=g) for _ in range(2))
+        c.k[phys], c.v[phys] = k, v
+        want.append(attention64(rows[s], k, v, nh, nkv, n))
+    la.attn_decode_batched(handle, out, rows, c, (keys - 1).to(torch.int32), n_seq, nh, nkv, 64, la.Paging(table, bs), rows.shape[1], nh * 64)
+    handle.check_status()
+    want = torch.stack(want)
+    assert ((out.double() - want).norm(dim=1) <= 2e-6 * want.norm(dim=1)).all()
