@@ -921,32 +921,35 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 }
 
 // ---- few items: 64 query rows each, the key tiles dealt to the four softmax groups in turn ----
-// The same computation for calls whose 128-row items would leave SMs idle: an item is 64 query rows, half the work of a
+// The same computation for calls whose 128-row items would leave SMs idle: a CTA has one item, 64 query rows, half the work of a
 // key-split item, and its score tiles j, j + 1, j + 2, j + 3 are worked on at a time, one by each softmax group.  The tensor core
 // computes 64 x 128 tiles (tcgen05.mma.ws), whose accumulators use all 128 lanes: lane l holds row l % 64, key columns
 // 64 (l / 64) .., so that a thread has, as in the other forms, one row and 64 key columns, and everything a row sums up it sums
 // up in the same order: P V of the key tiles into one O in key order, probabilities over even and odd key tiles apart.  A
 // head's bits are those of the other forms (heads beyond the bound, whose groups each have a max and an O of their own, aside).
 // P goes through shared memory (its lanes are not those that the tensor core would read it from).
+// One item is the kernel's premise, not a loop's first turn: Q, the reference and the sums have one buffer, and a group's tile counts
+// are its barriers' phases.  (With a loop over items, which no call ever took a second time, int8 scores spilled 252 bytes,
+// staged fp32 92; 136 and 40 so.)
 constexpr int R_ROWS = 64, R_GROUPS = 4, R_KS = 3, R_VS = 4;
 constexpr int R_Q_BYTES = R_ROWS * HD * 2, R_P_BYTES = R_ROWS * BN * 2;   // P: two [64 rows][64 keys] swizzled tiles
 constexpr int R_SLOTS = 4;
 constexpr int R_SMEM_Q = 0;
-constexpr int R_SMEM_K = R_SMEM_Q + Q_BUFS * R_Q_BYTES;
+constexpr int R_SMEM_K = R_SMEM_Q + R_Q_BYTES;
 constexpr int R_SMEM_V = R_SMEM_K + R_KS * TILE_BYTES;
 constexpr int R_SMEM_P = R_SMEM_V + R_VS * TILE_BYTES;
 constexpr int R_SMEM_BAR = R_SMEM_P + R_GROUPS * R_P_BYTES;
 constexpr int R_SMEM_KSKB = R_SMEM_BAR + 512;
 constexpr int R_SMEM_SUM = R_SMEM_KSKB + KSKB_SLOTS * KSKB_BYTES;   // [groups 1..3][R_SLOTS][2][128] floats: what a group hands on with a tile
 constexpr int R_SMEM_XMAX = R_SMEM_SUM + (R_GROUPS - 1) * R_SLOTS * 2 * 128 * 4;   // [groups][2][128] floats: row maxima of the halves
-constexpr int R_SMEM_REF = R_SMEM_XMAX + R_GROUPS * 2 * 128 * 4;    // [2 item parities][64] floats: reference of the max-free loop
-constexpr int R_SMEM_END = R_SMEM_REF + 2 * R_ROWS * 4;             // [2 item parities][3][128] floats: sums of the halves
-constexpr int R_ALLOC = R_SMEM_END + 2 * 3 * 128 * 4 + 1024;
+constexpr int R_SMEM_REF = R_SMEM_XMAX + R_GROUPS * 2 * 128 * 4;    // [64] floats: reference of the max-free loop
+constexpr int R_SMEM_END = R_SMEM_REF + R_ROWS * 4;                 // [3][128] floats: sums of the halves
+constexpr int R_ALLOC = R_SMEM_END + 3 * 128 * 4 + 1024;
 static_assert(R_ALLOC <= 227 * 1024, "shared memory per CTA");
-constexpr int RB_Q_FULL = 0, RB_Q_EMPTY = RB_Q_FULL + Q_BUFS, RB_K_FULL = RB_Q_EMPTY + Q_BUFS, RB_K_EMPTY = RB_K_FULL + R_KS,
-              RB_V_FULL = RB_K_EMPTY + R_KS, RB_V_EMPTY = RB_V_FULL + R_VS, RB_S_FULL = RB_V_EMPTY + R_VS,
-              RB_S_FREE = RB_S_FULL + R_GROUPS, RB_P_FULL = RB_S_FREE + R_GROUPS, RB_P_DONE = RB_P_FULL + R_GROUPS,
-              RB_XMAX = RB_P_DONE + R_GROUPS, RB_REF = RB_XMAX + R_GROUPS, RB_PASS = RB_REF + 1, RB_END = RB_PASS + 1, R_BARS = RB_END + 1;
+constexpr int RB_Q_FULL = 0, RB_K_FULL = RB_Q_FULL + 1, RB_K_EMPTY = RB_K_FULL + R_KS, RB_V_FULL = RB_K_EMPTY + R_KS,
+              RB_V_EMPTY = RB_V_FULL + R_VS, RB_S_FULL = RB_V_EMPTY + R_VS, RB_S_FREE = RB_S_FULL + R_GROUPS,
+              RB_P_FULL = RB_S_FREE + R_GROUPS, RB_P_DONE = RB_P_FULL + R_GROUPS, RB_XMAX = RB_P_DONE + R_GROUPS,
+              RB_REF = RB_XMAX + R_GROUPS, RB_END = RB_REF + 1, R_BARS = RB_END + 1;
 static_assert(8 * R_BARS + 16 <= 512, "barrier area");
 constexpr int R_TM_S = 0, R_TM_O = R_GROUPS * (BN / 2);   // S of group w at w * 64, O of group w (max-free: one O, the first) at 256 + w * 32
 
@@ -971,7 +974,7 @@ flash_fwd_rows64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     if (tid == 0) {
         for (int i = 0; i < R_BARS; ++i) {
             const bool by_warps = (i >= RB_S_FREE && i < RB_P_DONE) || i >= RB_XMAX;   // one elected lane of each of a group's warps
-            mx::mbar_init(bar(i), i == RB_PASS ? (R_GROUPS - 1) * 4 : by_warps ? 4 : 1);
+            mx::mbar_init(bar(i), by_warps ? 4 : 1);
         }
         *abort_flag = 0;
         mx::mbar_fence_init();
@@ -981,111 +984,91 @@ flash_fwd_rows64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     __syncthreads();
     mx::tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    fwd_prefetch_maps(P, warp, lane, tmQ, tmK, tmV, tmO);   // (every role waits for the previous kernel at its first item)
+    fwd_prefetch_maps(P, warp, lane, tmQ, tmK, tmV, tmO);
 
-    auto item_tiles = [&](int q0) {   // key tiles of the item's rows
-        const int all = (N + BN - 1) / BN;
-        return P.causal ? min(all, (q0 + R_ROWS - 1 + P.q_off) / BN + 1) : all;
-    };
+    // the item, heaviest first; n: key tiles that its rows see
+    const int rank = blockIdx.x / P.heads, bh = blockIdx.x - rank * P.heads;
+    const int q0 = (P.causal ? P.n_qblocks - 1 - rank : rank) * R_ROWS;
+    const int n = P.causal ? min((N + BN - 1) / BN, (q0 + R_ROWS - 1 + P.q_off) / BN + 1) : (N + BN - 1) / BN;
     auto wait = [&](int b, uint32_t phase) { return mx::mbar_wait(bar(b), phase & 1, abort_flag, P.status); };
     auto wait_warp = [&](int b, uint32_t phase) { return (bool)__all_sync(0xFFFFFFFFu, wait(b, phase)); };
-    auto head_fast = [&](int bh, int q0) {
+    auto head_fast = [&]() {
         return SRC == SRC_RAW ? false : SRC == SRC_RAW_BOUND ? fwd_fast_raw(P, bh, q0) : fwd_fast_head(P, bh, lane, REF ? FAST_BOUND_REF : FAST_BOUND);
     };
-    int bh, q0;
-    bool ok = true;
+    bool ok = true;   // (every role waits for the previous kernel behind its own arithmetic, as in flash_fwd_kernel)
     if (warp == SOFT_WARPS) {
         // ------------------------- TMA producer -------------------------
         if (lane == 0) {
-            uint32_t g = 0;
-            for (int it = 0; ok && fwd_item(P, it, bh, q0); ++it) {
-                const int n = item_tiles(q0), qbuf = it & 1, kvh = bh / P.kv_group;
-                if (it == 0) mx::pdl_wait();
-                if (it >= Q_BUFS) ok = wait(RB_Q_EMPTY + qbuf, (it >> 1) - 1);
+            const int kvh = bh / P.kv_group;
+            mx::pdl_wait();
+            mx::mbar_expect_tx(bar(RB_Q_FULL), R_Q_BYTES);
+            mx::tma_load_3d(smem_base + R_SMEM_Q, &tmQ, bar(RB_Q_FULL), 0, q0, bh);
+            for (int j = 0; j < n; ++j) {
+                const int sk = j % R_KS, sv = j % R_VS;
+                if (j >= R_KS) ok = wait(RB_K_EMPTY + sk, j / R_KS - 1);
                 if (!ok) break;
-                mx::mbar_expect_tx(bar(RB_Q_FULL + qbuf), R_Q_BYTES);
-                mx::tma_load_3d(smem_base + R_SMEM_Q + qbuf * R_Q_BYTES, &tmQ, bar(RB_Q_FULL + qbuf), 0, q0, bh);
-                for (int j = 0; j < n; ++j, ++g) {
-                    const int sk = g % R_KS, sv = g % R_VS;
-                    if (g >= R_KS) ok = wait(RB_K_EMPTY + sk, g / R_KS - 1);
-                    if (!ok) break;
-                    if (P.test_drop_tile == (int)g && blockIdx.x == 0) continue;   // test hook: this tile never arrives
-                    mx::mbar_expect_tx(bar(RB_K_FULL + sk), TILE_BYTES + (SRC == SRC_I8 ? KSKB_BYTES : 0));
-                    mx::tma_load_3d(smem_base + R_SMEM_K + sk * TILE_BYTES, &tmK, bar(RB_K_FULL + sk), 0, j * BN, kvh);
-                    // (the slot of the scales of tile g - 8 is free: P V of every tile up to g - 5 is complete, see flash_fwd_kernel)
-                    if (SRC == SRC_I8)
-                        mx::bulk_load(smem_base + R_SMEM_KSKB + (g % KSKB_SLOTS) * KSKB_BYTES,
-                                      P.col_kskb + ((size_t)kvh * P.n_k_tiles + j) * 2 * BN, KSKB_BYTES, bar(RB_K_FULL + sk));
-                    if (g >= R_VS) ok = wait(RB_V_EMPTY + sv, g / R_VS - 1);
-                    if (!ok) break;
-                    mx::mbar_expect_tx(bar(RB_V_FULL + sv), TILE_BYTES);
-                    mx::tma_load_3d(smem_base + R_SMEM_V + sv * TILE_BYTES, &tmV, bar(RB_V_FULL + sv), 0, j * BN, kvh);
-                }
+                if (P.test_drop_tile == j && blockIdx.x == 0) continue;   // test hook: this tile never arrives
+                mx::mbar_expect_tx(bar(RB_K_FULL + sk), TILE_BYTES + (SRC == SRC_I8 ? KSKB_BYTES : 0));
+                mx::tma_load_3d(smem_base + R_SMEM_K + sk * TILE_BYTES, &tmK, bar(RB_K_FULL + sk), 0, j * BN, kvh);
+                // (the slot of the scales of tile j - 8 is free: P V of every tile up to j - 5 is complete, see flash_fwd_kernel)
+                if (SRC == SRC_I8)
+                    mx::bulk_load(smem_base + R_SMEM_KSKB + (j % KSKB_SLOTS) * KSKB_BYTES,
+                                  P.col_kskb + ((size_t)kvh * P.n_k_tiles + j) * 2 * BN, KSKB_BYTES, bar(RB_K_FULL + sk));
+                if (j >= R_VS) ok = wait(RB_V_EMPTY + sv, j / R_VS - 1);
+                if (!ok) break;
+                mx::mbar_expect_tx(bar(RB_V_FULL + sv), TILE_BYTES);
+                mx::tma_load_3d(smem_base + R_SMEM_V + sv * TILE_BYTES, &tmV, bar(RB_V_FULL + sv), 0, j * BN, kvh);
             }
         }
         __syncwarp();
     } else if (warp == SOFT_WARPS + 1) {
         // ------------------------- MMA issuer 1: S = Q K^T --------------
         constexpr uint32_t IDESC_S = mx::mma_idesc_bf16(R_ROWS, BN, false, false);
-        uint32_t g = 0, cs[R_GROUPS] = {};
-        for (int it = 0; ok && fwd_item(P, it, bh, q0); ++it) {
-            const int n = item_tiles(q0), qbuf = it & 1;
-            const uint64_t a = mx::smem_desc_sw128(smem_base + R_SMEM_Q + qbuf * R_Q_BYTES);
-            if (it == 0) mx::pdl_wait();
-            ok = wait_warp(RB_Q_FULL + qbuf, it >> 1);
-            for (int j0 = 0; j0 < n && ok; j0 += R_GROUPS) {
+        const uint64_t a = mx::smem_desc_sw128(smem_base + R_SMEM_Q);
+        mx::pdl_wait();
+        ok = wait_warp(RB_Q_FULL, 0);
+        for (int i = 0, j = 0; j < n && ok; ++i) {
 #pragma unroll
-                for (int w = 0; w < R_GROUPS; ++w) {
-                    if (!ok || j0 + w >= n) continue;
-                    const int s = g % R_KS;
-                    ok = wait_warp(RB_K_FULL + s, g / R_KS);
-                    // (the group's previous scores may be of the item before: this is where the items overlap)
-                    if (ok && cs[w] > 0) ok = wait_warp(RB_S_FREE + w, cs[w] - 1);
-                    if (!ok) continue;
-                    mx::tc_fence_after();
-                    const uint64_t b = mx::smem_desc_sw128(smem_base + R_SMEM_K + s * TILE_BYTES);
-                    if (ISSUER_LANE) {
+            for (int w = 0; w < R_GROUPS; ++w, ++j) {
+                if (!ok || j >= n) continue;
+                const int s = j % R_KS;
+                ok = wait_warp(RB_K_FULL + s, j / R_KS);
+                if (ok && i > 0) ok = wait_warp(RB_S_FREE + w, i - 1);
+                if (!ok) continue;
+                mx::tc_fence_after();
+                const uint64_t b = mx::smem_desc_sw128(smem_base + R_SMEM_K + s * TILE_BYTES);
+                if (ISSUER_LANE) {
 #pragma unroll
-                        for (int k = 0; k < HD / 16; ++k) mx::mma_ws_ss(tmem + R_TM_S + w * (BN / 2), a + 2 * k, b + 2 * k, IDESC_S, k > 0);
-                        mx::mma_commit(bar(RB_S_FULL + w));
-                        mx::mma_commit(bar(RB_K_EMPTY + s));
-                        if (j0 + w == n - 1) mx::mma_commit(bar(RB_Q_EMPTY + qbuf));
-                    }
-                    ++cs[w], ++g;
+                    for (int k = 0; k < HD / 16; ++k) mx::mma_ws_ss(tmem + R_TM_S + w * (BN / 2), a + 2 * k, b + 2 * k, IDESC_S, k > 0);
+                    mx::mma_commit(bar(RB_S_FULL + w));
+                    mx::mma_commit(bar(RB_K_EMPTY + s));
                 }
             }
         }
         __syncwarp();
     } else if (warp == SOFT_WARPS + 2) {
         // ------------------------- MMA issuer 2: O += P V, in key order --
-        // An item's first P V overwrites O: that of tile 0, whose P the first group writes after it has taken the previous
-        // item's O, of every group, out of tensor memory; the other groups' come behind it in this warp's order.
         constexpr uint32_t IDESC_O = mx::mma_idesc_bf16(R_ROWS, HD, false, true);
-        uint32_t g = 0, cp[R_GROUPS] = {};
-        for (int it = 0; ok && fwd_item(P, it, bh, q0); ++it) {
-            const int n = item_tiles(q0);
-            if (it == 0) mx::pdl_wait();
-            const bool own_o = !head_fast(bh, q0);   // each group sums into an O of its own
-            for (int j0 = 0; j0 < n && ok; j0 += R_GROUPS) {
+        mx::pdl_wait();
+        const bool own_o = !head_fast();   // each group sums into an O of its own
+        for (int i = 0, j = 0; j < n && ok; ++i) {
 #pragma unroll
-                for (int w = 0; w < R_GROUPS; ++w) {
-                    if (!ok || j0 + w >= n) continue;
-                    const int s = g % R_VS;
-                    ok = wait_warp(RB_V_FULL + s, g / R_VS);
-                    if (ok) ok = wait_warp(RB_P_FULL + w, cp[w]);
-                    if (!ok) continue;
-                    mx::tc_fence_after();
-                    const uint64_t b = mx::smem_desc_sw128(smem_base + R_SMEM_V + s * TILE_BYTES);
-                    const uint64_t a = mx::smem_desc_sw128(smem_base + R_SMEM_P + w * R_P_BYTES);
-                    if (ISSUER_LANE) {
+            for (int w = 0; w < R_GROUPS; ++w, ++j) {
+                if (!ok || j >= n) continue;
+                const int s = j % R_VS;
+                ok = wait_warp(RB_V_FULL + s, j / R_VS);
+                if (ok) ok = wait_warp(RB_P_FULL + w, i);
+                if (!ok) continue;
+                mx::tc_fence_after();
+                const uint64_t b = mx::smem_desc_sw128(smem_base + R_SMEM_V + s * TILE_BYTES);
+                const uint64_t a = mx::smem_desc_sw128(smem_base + R_SMEM_P + w * R_P_BYTES);
+                if (ISSUER_LANE) {
 #pragma unroll
-                        for (int k = 0; k < BN / 16; ++k)   // 16 keys: 32 bytes of P's rows, the second 64 keys in its second tile
-                            mx::mma_ws_ss(tmem + R_TM_O + (own_o ? w * (HD / 2) : 0), a + (k >> 2) * (R_P_BYTES / 2 / 16) + 2 * (k & 3),
-                                          b + 128 * k, IDESC_O, (own_o ? j0 > 0 : j0 + w > 0) || k > 0);
-                        mx::mma_commit(bar(RB_P_DONE + w));
-                        mx::mma_commit(bar(RB_V_EMPTY + s));
-                    }
-                    ++cp[w], ++g;
+                    for (int k = 0; k < BN / 16; ++k)   // 16 keys: 32 bytes of P's rows, the second 64 keys in its second tile
+                        mx::mma_ws_ss(tmem + R_TM_O + (own_o ? w * (HD / 2) : 0), a + (k >> 2) * (R_P_BYTES / 2 / 16) + 2 * (k & 3),
+                                      b + 128 * k, IDESC_O, (own_o ? i > 0 : j > 0) || k > 0);
+                    mx::mma_commit(bar(RB_P_DONE + w));
+                    mx::mma_commit(bar(RB_V_EMPTY + s));
                 }
             }
         }
@@ -1097,308 +1080,279 @@ flash_fwd_rows64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         const uint32_t tm_s = tmem + lane_off + R_TM_S + w * (BN / 2);
         const uint32_t tm_o = tmem + lane_off + R_TM_O;
         const int p_off = R_SMEM_P + w * R_P_BYTES + half * (R_P_BYTES / 2) + row_in_tile * 128;   // this thread's row of P
-        uint32_t cnt = 0;            // score tiles this group has taken so far, over all items
-        uint32_t at[R_GROUPS] = {};  // those of every group in the items before
-        uint32_t g0 = 0;             // key tiles in the items before
+        const int n_w = (n + R_GROUPS - 1 - w) / R_GROUPS;   // the group's tiles: w, w + 4, ...
+        const int row = q0 + row_in_tile;
+        const int last = P.causal ? min(N - 1, row + P.q_off) : N - 1;   // last visible key of this row
         uint32_t xmc = 0;            // row-max exchanges of this group so far
-        // what group `of` (1..3) handed on with its tile `idx` of this item: group 1 and 3 | 2: [sum over the chain before, the tile's sum];
-        // with a row max [sum, max].  A slot is written again three tiles of its group later, when it has been read.
-        auto slot = [&](int of, uint32_t count, int what) -> float & {
-            return ((float *)(smem + R_SMEM_SUM))[(((of - 1) * R_SLOTS + (count & (R_SLOTS - 1))) * 2 + what) * 128 + thr];
+        // what group `of` (1..3) handed on with its tile `i`: group 1 and 3 | 2: [sum over the chain before, the tile's sum]; with a
+        // row max [sum, max].  A slot is written again four tiles of its group later, when it has been read.
+        auto slot = [&](int of, int i, int what) -> float & {
+            return ((float *)(smem + R_SMEM_SUM))[(((of - 1) * R_SLOTS + (i & (R_SLOTS - 1))) * 2 + what) * 128 + thr];
         };
-        for (int it = 0; ok && fwd_item(P, it, bh, q0); ++it) {
-            const int n = item_tiles(q0), n_w = (n + R_GROUPS - 1 - w) / R_GROUPS;
-            const int row = q0 + row_in_tile;
-            const int last = P.causal ? min(N - 1, row + P.q_off) : N - 1;   // last visible key of this row
-            if (it == 0) mx::pdl_wait();
-            const bool fast = head_fast(bh, q0);
-            float row_a = 0.0f, row_qsum = 0.0f;
-            if (SRC == SRC_I8 && row < NQ) {
-                row_a = P.row_a[(size_t)bh * NQ + row];
-                row_qsum = P.row_qsum[(size_t)bh * NQ + row];
-            }
-            auto kskb_of = [&](int j) {
-                return (const float *)(smem + R_SMEM_KSKB + ((g0 + (uint32_t)j) % KSKB_SLOTS) * KSKB_BYTES) + half * (BN / 2);
+        mx::pdl_wait();
+        const bool fast = head_fast();
+        float row_a = 0.0f, row_qsum = 0.0f;
+        if (SRC == SRC_I8 && row < NQ) {
+            row_a = P.row_a[(size_t)bh * NQ + row];
+            row_qsum = P.row_qsum[(size_t)bh * NQ + row];
+        }
+        auto kskb_of = [&](int j) {
+            return (const float *)(smem + R_SMEM_KSKB + (j % KSKB_SLOTS) * KSKB_BYTES) + half * (BN / 2);
+        };
+        auto row_max = [&](float own) -> float {   // over the halves of the row
+            float *xm = (float *)(smem + R_SMEM_XMAX) + (w * 2 + (xmc & 1)) * 128;
+            xm[thr] = own;
+            __syncwarp();
+            if (lane == 0) mx::mbar_arrive(bar(RB_XMAX + w));
+            ok = wait_warp(RB_XMAX + w, xmc);
+            ++xmc;
+            return fmaxf(own, xm[thr ^ 64]);
+        };
+        float m = fast ? 0.0f : -CUDART_INF_F, l = 0.0f, corr = 0.0f;
+        // The reference of the max-free loop (sources that have one) is the row's max over key tile 0, which the first group
+        // publishes.
+        float *ref = (float *)(smem + R_SMEM_REF);
+        if (REF && SRC != SRC_RAW && fast && w > 0 && n_w > 0) {
+            ok = wait_warp(RB_REF, 0);
+            if (ok) m = ref[row_in_tile];
+        }
+        // the group's P buffer is free: P V of its previous tile is complete
+        auto p_free = [&](int i) { return i == 0 || wait_warp(RB_P_DONE + w, i - 1); };
+        auto put = [&](const uint32_t *pk, int at0) {   // 32 probabilities: four 16-byte pieces of the row, from piece at0 on
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                *(uint4 *)(smem + p_off + (((at0 + i) ^ (lane & 7)) << 4)) = make_uint4(pk[4 * i], pk[4 * i + 1], pk[4 * i + 2], pk[4 * i + 3]);
+        };
+        auto hand_p = [&]() {
+            mx::fence_proxy_async_smem();   // read by the MMAs
+            __syncwarp();
+            if (lane == 0) mx::mbar_arrive(bar(RB_P_FULL + w));
+        };
+        uint32_t va[32], vb[32];
+        float s_prev = 0.0f;   // sum of the group's previous tile, not yet in l
+        if (fast) {
+            // Sums: l of group 0 (1) is that over even (odd) key tiles in key order.  With its tile i the group takes in
+            // tile i - 2 of its partner, group 2 (3), and tile i - 1 of its own: P V of those, and so their sums, precede
+            // P V of its tile i - 1, which p_free has waited for.
+            float nmc = REF ? -m * c : 0.0f;
+            auto sum_of = [](uint64_t v) {
+                float a0, a1;
+                mx::upk2(v, a0, a1);
+                return a0 + a1;
             };
-            float *xmax = (float *)(smem + R_SMEM_XMAX) + w * 2 * 128;
-            auto row_max = [&](float own) -> float {   // over the halves of the row
-                float *xm = xmax + (xmc & 1) * 128;
-                xm[thr] = own;
-                __syncwarp();
-                if (lane == 0) mx::mbar_arrive(bar(RB_XMAX + w));
-                ok = wait_warp(RB_XMAX + w, xmc);
-                ++xmc;
-                return fmaxf(own, xm[thr ^ 64]);
-            };
-            // The reference of the max-free loop (sources that have one) is the row's max over key tile 0, which the first group
-            // publishes.  Once per item, whether used or not, and not before every other warp has seen the previous item's: a
-            // parity wait tells a phase only from its neighbour.
-            float *ref = (float *)(smem + R_SMEM_REF) + (it & 1) * R_ROWS;
-            auto publish_ref = [&](float m) {
-                if (half == 0) ref[row_in_tile] = m;
-                __syncwarp();
-                if (lane == 0) mx::mbar_arrive(bar(RB_REF));
-            };
-            float m = fast ? 0.0f : -CUDART_INF_F, l = 0.0f, corr = 0.0f;
-            if (REF && SRC != SRC_RAW) {
-                if (w == 0) {
-                    if (it > 0) ok = wait_warp(RB_PASS, it - 1);
-                    if (ok && !fast) publish_ref(0.0f);
-                } else {
-                    ok = wait_warp(RB_REF, it);
-                    if (ok && fast) m = ref[row_in_tile];
+            auto tile = [&](auto first_c, int i) -> bool {
+                constexpr bool FIRST = decltype(first_c)::value;   // of the item: key tile 0
+                const int j = R_GROUPS * i + w;
+                if (!wait_warp(RB_S_FULL + w, i)) return false;
+                mx::tc_fence_after();
+                mx::tmem_ld32(tm_s, va);
+                mx::tmem_wait_ld();
+                mx::tmem_ld32(tm_s + 32, vb);   // lands under the first exponentials
+                const int key0 = j * BN, col0 = key0 + half * (BN / 2);
+                const bool need_mask = (key0 + BN > N) || (P.causal && key0 + BN - 1 > q0 + P.q_off);
+                const float *kskb = SRC == SRC_I8 ? kskb_of(j) : nullptr;
+                uint64_t rs2;
+                uint32_t pk[16];
+                constexpr bool LEAD = REF && FIRST;
+                if (LEAD) {
+                    mx::tmem_wait_ld();
+                    if (SRC == SRC_I8) fwd_rebuild32(va, kskb, 0.0f, row_a, row_qsum), fwd_rebuild32(vb, kskb + 32, 0.0f, row_a, row_qsum);
+                    if (need_mask) fwd_mask64(va, vb, col0, last);
+                    m = row_max(fwd_max64(va, vb));
+                    if (!ok) return false;
+                    if (half == 0) ref[row_in_tile] = m;
                     __syncwarp();
-                    if (ok && lane == 0) mx::mbar_arrive(bar(RB_PASS));
+                    if (lane == 0) mx::mbar_arrive(bar(RB_REF));
+                    nmc = -m * c;
                 }
-            }
-            // the group's P buffer is free: P V of its previous tile is complete (first group: and its rows, where the previous item's
-            // O was staged, have been stored)
-            auto p_free = [&](bool first) -> bool {
-                if (cnt > 0 && !wait_warp(RB_P_DONE + w, cnt - 1)) return false;
-                if (first && w == 0 && it > 0) {
-                    if (lane == 0) mx::bulk_wait_group_read<0>();
-                    __syncwarp();
+                fwd_exp32<SRC>(va, pk, col0, last, need_mask, kskb, true, LEAD, nmc, row_a, row_qsum, rs2);
+                mx::tmem_wait_ld();
+                mx::tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mx::mbar_arrive(bar(RB_S_FREE + w));   // this group's columns have left S
+                if (!p_free(i)) return false;
+                if (w < 2) {
+                    if (i >= 2) l += slot(w + 2, i - 2, 1);
+                    if (i >= 1) l += s_prev;
                 }
+                put(pk, 0);
+                float rb[4] = {0.0f, 0.0f, 0.0f, 0.0f};   // the first key tile's ROUNDED probabilities (see flash_fwd_kernel)
+                auto sum_rounded16 = [&]() {
+#pragma unroll
+                    for (int u = 0; u < 16; ++u) mx::add_bf16x2(pk[u], rb[(u & 1) * 2], rb[(u & 1) * 2 + 1]);
+                };
+                if (FIRST) sum_rounded16();
+                fwd_exp32<SRC>(vb, pk, col0 + 32, last, need_mask, kskb + 32, false, LEAD, nmc, row_a, row_qsum, rs2);
+                put(pk, 4);
+                s_prev = sum_of(rs2);
+                if (FIRST) {
+                    sum_rounded16();
+                    corr = ((rb[0] + rb[1]) + (rb[2] + rb[3])) - s_prev;
+                }
+                if (w > 0) {
+                    if (w == 1) slot(1, i, 0) = l;
+                    slot(w, i, 1) = s_prev;
+                }
+                hand_p();
                 return true;
             };
-            auto put = [&](const uint32_t *pk, int at0) {   // 32 probabilities: four 16-byte pieces of the row, from piece at0 on
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    *(uint4 *)(smem + p_off + (((at0 + i) ^ (lane & 7)) << 4)) = make_uint4(pk[4 * i], pk[4 * i + 1], pk[4 * i + 2], pk[4 * i + 3]);
-            };
-            auto hand_p = [&]() {
-                mx::fence_proxy_async_smem();   // read by the MMAs
-                __syncwarp();
-                if (lane == 0) mx::mbar_arrive(bar(RB_P_FULL + w));
-            };
-            uint32_t va[32], vb[32];
-            float s_prev = 0.0f;   // sum of the group's previous tile, not yet in l
-            if (fast) {
-                // Sums: l of group 0 (1) is that over even (odd) key tiles in key order.  With its tile i the group takes in
-                // tile i - 2 of its partner, group 2 (3), and tile i - 1 of its own: P V of those, and so their sums, precede
-                // P V of its tile i - 1, which p_free has waited for.
-                float nmc = REF ? -m * c : 0.0f;
-                auto sum_of = [](uint64_t v) {
-                    float a0, a1;
-                    mx::upk2(v, a0, a1);
-                    return a0 + a1;
-                };
-                auto tile = [&](auto first_c, int i) -> bool {
-                    constexpr bool FIRST = decltype(first_c)::value;   // of the item: key tile 0
-                    const int j = R_GROUPS * i + w;
-                    if (!wait_warp(RB_S_FULL + w, cnt)) return false;
-                    mx::tc_fence_after();
-                    mx::tmem_ld32(tm_s, va);
-                    mx::tmem_wait_ld();
-                    mx::tmem_ld32(tm_s + 32, vb);   // lands under the first exponentials
-                    const int key0 = j * BN, col0 = key0 + half * (BN / 2);
-                    const bool need_mask = (key0 + BN > N) || (P.causal && key0 + BN - 1 > q0 + P.q_off);
-                    const float *kskb = SRC == SRC_I8 ? kskb_of(j) : nullptr;
-                    uint64_t rs2;
-                    uint32_t pk[16];
-                    constexpr bool LEAD = REF && FIRST;
-                    if (LEAD) {
-                        mx::tmem_wait_ld();
-                        if (SRC == SRC_I8) fwd_rebuild32(va, kskb, 0.0f, row_a, row_qsum), fwd_rebuild32(vb, kskb + 32, 0.0f, row_a, row_qsum);
-                        if (need_mask) fwd_mask64(va, vb, col0, last);
-                        m = row_max(fwd_max64(va, vb));
-                        if (!ok) return false;
-                        publish_ref(m);
-                        nmc = -m * c;
-                    }
-                    fwd_exp32<SRC>(va, pk, col0, last, need_mask, kskb, true, LEAD, nmc, row_a, row_qsum, rs2);
-                    mx::tmem_wait_ld();
-                    mx::tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mx::mbar_arrive(bar(RB_S_FREE + w));   // this group's columns have left S
-                    if (!p_free(i == 0)) return false;
-                    if (w < 2) {
-                        if (i >= 2) l += slot(w + 2, at[w + 2] + i - 2, 1);
-                        if (i >= 1) l += s_prev;
-                    }
-                    put(pk, 0);
-                    float rb[4] = {0.0f, 0.0f, 0.0f, 0.0f};   // the first key tile's ROUNDED probabilities (see flash_fwd_kernel)
-                    auto sum_rounded16 = [&]() {
-#pragma unroll
-                        for (int u = 0; u < 16; ++u) mx::add_bf16x2(pk[u], rb[(u & 1) * 2], rb[(u & 1) * 2 + 1]);
-                    };
-                    if (FIRST) sum_rounded16();
-                    fwd_exp32<SRC>(vb, pk, col0 + 32, last, need_mask, kskb + 32, false, LEAD, nmc, row_a, row_qsum, rs2);
-                    put(pk, 4);
-                    s_prev = sum_of(rs2);
-                    if (FIRST) {
-                        sum_rounded16();
-                        corr = ((rb[0] + rb[1]) + (rb[2] + rb[3])) - s_prev;
-                    }
-                    if (w > 0) {
-                        if (w == 1) slot(1, cnt, 0) = l;
-                        slot(w, cnt, 1) = s_prev;
-                    }
-                    hand_p();
-                    ++cnt;
-                    return true;
-                };
-                int i = 0;
-                if (w == 0) ok = ok && tile(std::true_type{}, i++);
-                for (; ok && i < n_w; ++i) ok = tile(std::false_type{}, i);
-            } else {
-                // ---- running row max, raised lazily: every group has its own, over its key tiles, and its own O ----
-                for (int i = 0; ok && i < n_w; ++i, ++cnt) {
-                    const int j = R_GROUPS * i + w;
-                    ok = wait_warp(RB_S_FULL + w, cnt);
-                    if (!ok) break;
-                    mx::tc_fence_after();
-                    mx::tmem_ld32(tm_s, va);
-                    mx::tmem_ld32(tm_s + 32, vb);
-                    mx::tmem_wait_ld();
-                    mx::tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mx::mbar_arrive(bar(RB_S_FREE + w));
-                    const int key0 = j * BN, col0 = key0 + half * (BN / 2);
-                    if (SRC == SRC_I8) {
-                        const float *kskb = kskb_of(j);
-                        fwd_rebuild32(va, kskb, 0.0f, row_a, row_qsum);
-                        fwd_rebuild32(vb, kskb + 32, 0.0f, row_a, row_qsum);
-                    }
-                    if ((key0 + BN > N) || (P.causal && key0 + BN - 1 > q0 + P.q_off)) fwd_mask64(va, vb, col0, last);
-                    const float mx_ = row_max(fwd_max64(va, vb));
-                    if (!ok) break;
-                    const bool raise = (i == 0) || ((mx_ - m) * c > RESCALE_LOG2);
-                    const float m_new = raise ? mx_ : m;
-                    const float alpha = (raise && i > 0) ? mx::ex2((m - m_new) * c) : 1.0f;
-                    const float nmc = m_new == -CUDART_INF_F ? 0.0f : -m_new * c;   // (a row may see none of the group's first keys)
-                    ok = p_free(i == 0);
-                    if (!ok) break;
-                    if (i > 0 && __any_sync(0xFFFFFFFFu, raise)) {   // this thread's 32 columns of the group's O
-                        mx::tc_fence_after();
-#pragma unroll 1
-                        for (int cc = 0; cc < 2; ++cc) {
-                            uint32_t o[16];
-                            mx::tmem_ld16(tm_o + w * (HD / 2) + cc * 16, o);
-                            mx::tmem_wait_ld();
-#pragma unroll
-                            for (int u = 0; u < 16; ++u) o[u] = __float_as_uint(__uint_as_float(o[u]) * alpha);
-                            mx::tmem_st16(tm_o + w * (HD / 2) + cc * 16, o);
-                        }
-                        mx::tmem_wait_st();
-                    }
-                    float rs[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-                    uint32_t pk[16];
-                    auto exp_general = [&](const uint32_t *v, int piece) {
-#pragma unroll
-                        for (int u = 0; u < 32; u += 2) {
-                            const float p0 = mx::ex2(fmaf(__uint_as_float(v[u]), c, nmc));
-                            const float p1 = mx::ex2(fmaf(__uint_as_float(v[u + 1]), c, nmc));
-                            rs[u & 2] += p0;
-                            rs[(u & 2) + 1] += p1;
-                            pk[u >> 1] = mx::pack_bf16(p0, p1);
-                        }
-                        put(pk, piece);
-                    };
-                    exp_general(va, 0);
-                    exp_general(vb, 4);
-                    l = l * alpha + ((rs[0] + rs[1]) + (rs[2] + rs[3]));
-                    m = m_new;
-                    if (w > 0) slot(w, cnt, 0) = l, slot(w, cnt, 1) = m;
-                    mx::tc_fence_before();
-                    hand_p();
-                }
-            }
-            // ---- the first group joins the sums and takes O out: thread = row, 32 of its columns ----
-            if (ok && w == 0) {
-                uint32_t n_of[R_GROUPS];
-#pragma unroll
-                for (int u = 0; u < R_GROUPS; ++u) n_of[u] = (uint32_t)(n + R_GROUPS - 1 - u) / R_GROUPS;
-                const int e = (n - 1) & (R_GROUPS - 1);   // group of the last key tile
-                ok = wait_warp(RB_P_DONE, cnt - 1);       // (first its own last tile: P V of the last group's tile before precedes it)
-                if (ok && e > 0) ok = wait_warp(RB_P_DONE + e, (e == 1 ? at[1] + n_of[1] : e == 2 ? at[2] + n_of[2] : at[3] + n_of[3]) - 1);
+            int i = 0;
+            if (w == 0) ok = ok && tile(std::true_type{}, i++);
+            for (; ok && i < n_w; ++i) ok = tile(std::false_type{}, i);
+        } else {
+            // ---- running row max, raised lazily: every group has its own, over its key tiles, and its own O ----
+            for (int i = 0; ok && i < n_w; ++i) {
+                const int j = R_GROUPS * i + w;
+                ok = wait_warp(RB_S_FULL + w, i);
+                if (!ok) break;
                 mx::tc_fence_after();
-                float wt[R_GROUPS] = {1.0f, 0.0f, 0.0f, 0.0f}, l_odd = 0.0f;
-                if (ok && fast) {
-                    if (n_of[0] >= 2) l += slot(2, at[2] + n_of[0] - 2, 1);
-                    l += s_prev;
-                    if (n_of[2] == n_of[0]) l += slot(2, at[2] + n_of[0] - 1, 1);
-                    if (n_of[1] > 0) {
-                        l_odd = slot(1, at[1] + n_of[1] - 1, 0);
-                        if (n_of[1] >= 2) l_odd += slot(3, at[3] + n_of[1] - 2, 1);
-                        l_odd += slot(1, at[1] + n_of[1] - 1, 1);
-                        if (n_of[3] == n_of[1]) l_odd += slot(3, at[3] + n_of[1] - 1, 1);
-                    }
-                } else if (ok) {
-                    float mm = m;
-#pragma unroll
-                    for (int u = 1; u < R_GROUPS; ++u)
-                        if (n_of[u] > 0) mm = fmaxf(mm, slot(u, at[u] + n_of[u] - 1, 1));
-                    wt[0] = mx::ex2((m - mm) * c);   // m is finite: key tile 0 has a key that every row sees
-                    l *= wt[0];
-#pragma unroll
-                    for (int u = 1; u < R_GROUPS; ++u)
-                        if (n_of[u] > 0) {
-                            wt[u] = mx::ex2((slot(u, at[u] + n_of[u] - 1, 1) - mm) * c);
-                            l += slot(u, at[u] + n_of[u] - 1, 0) * wt[u];
-                        }
-                    m = mm;
-                }
-                // the halves of a row
-                float *xe = (float *)(smem + R_SMEM_END) + (it & 1) * 3 * 128;
-                xe[thr] = l, xe[128 + thr] = l_odd, xe[256 + thr] = corr;
+                mx::tmem_ld32(tm_s, va);
+                mx::tmem_ld32(tm_s + 32, vb);
+                mx::tmem_wait_ld();
+                mx::tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mx::mbar_arrive(bar(RB_END));
-                if (ok) ok = wait_warp(RB_END, it);
-                if (ok) {
-                    l = (l + xe[thr ^ 64]) + (l_odd + xe[128 + (thr ^ 64)]);
-                    const float inv = 1.0f / (l + (corr + xe[256 + (thr ^ 64)]));
-                    mx::tmem_ld32(tm_o, va);
-                    mx::tmem_wait_ld();
-                    if (!fast) {
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) va[i] = __float_as_uint(__uint_as_float(va[i]) * wt[0]);
-#pragma unroll
-                        for (int u = 1; u < R_GROUPS; ++u) {
-                            if (n_of[u] == 0) continue;
-                            mx::tmem_ld32(tm_o + u * (HD / 2), vb);
-                            mx::tmem_wait_ld();
-#pragma unroll
-                            for (int i = 0; i < 32; ++i) va[i] = __float_as_uint(fmaf(__uint_as_float(vb[i]), wt[u], __uint_as_float(va[i])));
-                        }
-                    }
-                    mx::tc_fence_before();   // (the next item's first P is handed over behind this)
-                    float4 o4[8];
-#pragma unroll
-                    for (int i = 0; i < 8; ++i)
-                        o4[i] = make_float4(__uint_as_float(va[4 * i]) * inv, __uint_as_float(va[4 * i + 1]) * inv,
-                                            __uint_as_float(va[4 * i + 2]) * inv, __uint_as_float(va[4 * i + 3]) * inv);
-                    if (HALF && row < NQ) {
-                        uint4 *dst = (uint4 *)(P.O_half + ((size_t)bh * NQ + row) * HD + half * 32);
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            const __half2 h2[4] = {__floats2half2_rn(o4[2 * i].x, o4[2 * i].y), __floats2half2_rn(o4[2 * i].z, o4[2 * i].w),
-                                                   __floats2half2_rn(o4[2 * i + 1].x, o4[2 * i + 1].y), __floats2half2_rn(o4[2 * i + 1].z, o4[2 * i + 1].w)};
-                            dst[i] = *(const uint4 *)h2;
-                        }
-                    }
-                    if (P.tma_out) {
-                        // every warp stages its 32 rows and 32 columns in its own rows of the group's P buffer
-                        const int wrow0 = q0 + (warp & 1) * 32, st_off = p_off - lane * 128;
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) *(float4 *)(smem + st_off + lane * 128 + ((i ^ (lane & 7)) << 4)) = o4[i];
-                        mx::fence_proxy_async_smem();
-                        __syncwarp();
-                        if (lane == 0 && wrow0 < NQ) {
-                            mx::tma_store_3d(&tmO, smem_base + st_off, half * 32, wrow0, bh);
-                            mx::bulk_commit_group();   // (waited for before this warp writes P again, and before the kernel ends)
-                        }
-                    } else if (row < NQ) {
-                        float *orow = P.O + (size_t)bh * P.o_head_stride + (size_t)row * P.o_row_stride + half * 32;
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) *(float4 *)(orow + 4 * i) = o4[i];
-                    }
-                    if (half == 0 && P.L != nullptr && row < NQ) P.L[(size_t)bh * NQ + row] = m * l_scale + __logf(l);
+                if (lane == 0) mx::mbar_arrive(bar(RB_S_FREE + w));
+                const int key0 = j * BN, col0 = key0 + half * (BN / 2);
+                if (SRC == SRC_I8) {
+                    const float *kskb = kskb_of(j);
+                    fwd_rebuild32(va, kskb, 0.0f, row_a, row_qsum);
+                    fwd_rebuild32(vb, kskb + 32, 0.0f, row_a, row_qsum);
                 }
-            }
+                if ((key0 + BN > N) || (P.causal && key0 + BN - 1 > q0 + P.q_off)) fwd_mask64(va, vb, col0, last);
+                const float mx_ = row_max(fwd_max64(va, vb));
+                if (!ok) break;
+                const bool raise = (i == 0) || ((mx_ - m) * c > RESCALE_LOG2);
+                const float m_new = raise ? mx_ : m;
+                const float alpha = (raise && i > 0) ? mx::ex2((m - m_new) * c) : 1.0f;
+                const float nmc = m_new == -CUDART_INF_F ? 0.0f : -m_new * c;   // (a row may see none of the group's first keys)
+                ok = p_free(i);
+                if (!ok) break;
+                if (i > 0 && __any_sync(0xFFFFFFFFu, raise)) {   // this thread's 32 columns of the group's O
+                    mx::tc_fence_after();
+#pragma unroll 1
+                    for (int cc = 0; cc < 2; ++cc) {
+                        uint32_t o[16];
+                        mx::tmem_ld16(tm_o + w * (HD / 2) + cc * 16, o);
+                        mx::tmem_wait_ld();
 #pragma unroll
-            for (int u = 0; u < R_GROUPS; ++u) at[u] += (uint32_t)(n + R_GROUPS - 1 - u) / R_GROUPS;
-            g0 += n;
+                        for (int u = 0; u < 16; ++u) o[u] = __float_as_uint(__uint_as_float(o[u]) * alpha);
+                        mx::tmem_st16(tm_o + w * (HD / 2) + cc * 16, o);
+                    }
+                    mx::tmem_wait_st();
+                }
+                float rs[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                uint32_t pk[16];
+                auto exp_general = [&](const uint32_t *v, int piece) {
+#pragma unroll
+                    for (int u = 0; u < 32; u += 2) {
+                        const float p0 = mx::ex2(fmaf(__uint_as_float(v[u]), c, nmc));
+                        const float p1 = mx::ex2(fmaf(__uint_as_float(v[u + 1]), c, nmc));
+                        rs[u & 2] += p0;
+                        rs[(u & 2) + 1] += p1;
+                        pk[u >> 1] = mx::pack_bf16(p0, p1);
+                    }
+                    put(pk, piece);
+                };
+                exp_general(va, 0);
+                exp_general(vb, 4);
+                l = l * alpha + ((rs[0] + rs[1]) + (rs[2] + rs[3]));
+                m = m_new;
+                if (w > 0) slot(w, i, 0) = l, slot(w, i, 1) = m;
+                mx::tc_fence_before();
+                hand_p();
+            }
+        }
+        // ---- the first group joins the sums and takes O out: thread = row, 32 of its columns ----
+        if (ok && w == 0) {
+            int n_of[R_GROUPS];
+#pragma unroll
+            for (int u = 0; u < R_GROUPS; ++u) n_of[u] = (n + R_GROUPS - 1 - u) / R_GROUPS;
+            const int e = (n - 1) & (R_GROUPS - 1);   // group of the last key tile
+            ok = wait_warp(RB_P_DONE, n_w - 1);       // (first its own last tile: P V of the last group's tile before precedes it)
+            if (ok && e > 0) ok = wait_warp(RB_P_DONE + e, (e == 1 ? n_of[1] : e == 2 ? n_of[2] : n_of[3]) - 1);
+            mx::tc_fence_after();
+            float wt[R_GROUPS] = {1.0f, 0.0f, 0.0f, 0.0f}, l_odd = 0.0f;
+            if (ok && fast) {
+                if (n_of[0] >= 2) l += slot(2, n_of[0] - 2, 1);
+                l += s_prev;
+                if (n_of[2] == n_of[0]) l += slot(2, n_of[0] - 1, 1);
+                if (n_of[1] > 0) {
+                    l_odd = slot(1, n_of[1] - 1, 0);
+                    if (n_of[1] >= 2) l_odd += slot(3, n_of[1] - 2, 1);
+                    l_odd += slot(1, n_of[1] - 1, 1);
+                    if (n_of[3] == n_of[1]) l_odd += slot(3, n_of[1] - 1, 1);
+                }
+            } else if (ok) {
+                float mm = m;
+#pragma unroll
+                for (int u = 1; u < R_GROUPS; ++u)
+                    if (n_of[u] > 0) mm = fmaxf(mm, slot(u, n_of[u] - 1, 1));
+                wt[0] = mx::ex2((m - mm) * c);   // m is finite: key tile 0 has a key that every row sees
+                l *= wt[0];
+#pragma unroll
+                for (int u = 1; u < R_GROUPS; ++u)
+                    if (n_of[u] > 0) {
+                        wt[u] = mx::ex2((slot(u, n_of[u] - 1, 1) - mm) * c);
+                        l += slot(u, n_of[u] - 1, 0) * wt[u];
+                    }
+                m = mm;
+            }
+            // the halves of a row
+            float *xe = (float *)(smem + R_SMEM_END);
+            xe[thr] = l, xe[128 + thr] = l_odd, xe[256 + thr] = corr;
+            __syncwarp();
+            if (lane == 0) mx::mbar_arrive(bar(RB_END));
+            if (ok) ok = wait_warp(RB_END, 0);
+            if (ok) {
+                l = (l + xe[thr ^ 64]) + (l_odd + xe[128 + (thr ^ 64)]);
+                const float inv = 1.0f / (l + (corr + xe[256 + (thr ^ 64)]));
+                mx::tmem_ld32(tm_o, va);
+                mx::tmem_wait_ld();
+                if (!fast) {
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) va[i] = __float_as_uint(__uint_as_float(va[i]) * wt[0]);
+#pragma unroll
+                    for (int u = 1; u < R_GROUPS; ++u) {
+                        if (n_of[u] == 0) continue;
+                        mx::tmem_ld32(tm_o + u * (HD / 2), vb);
+                        mx::tmem_wait_ld();
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) va[i] = __float_as_uint(fmaf(__uint_as_float(vb[i]), wt[u], __uint_as_float(va[i])));
+                    }
+                }
+                mx::tc_fence_before();
+                float4 o4[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    o4[i] = make_float4(__uint_as_float(va[4 * i]) * inv, __uint_as_float(va[4 * i + 1]) * inv,
+                                        __uint_as_float(va[4 * i + 2]) * inv, __uint_as_float(va[4 * i + 3]) * inv);
+                if (HALF && row < NQ) {
+                    uint4 *dst = (uint4 *)(P.O_half + ((size_t)bh * NQ + row) * HD + half * 32);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const __half2 h2[4] = {__floats2half2_rn(o4[2 * i].x, o4[2 * i].y), __floats2half2_rn(o4[2 * i].z, o4[2 * i].w),
+                                               __floats2half2_rn(o4[2 * i + 1].x, o4[2 * i + 1].y), __floats2half2_rn(o4[2 * i + 1].z, o4[2 * i + 1].w)};
+                        dst[i] = *(const uint4 *)h2;
+                    }
+                }
+                if (P.tma_out) {
+                    // every warp stages its 32 rows and 32 columns in its own rows of the group's P buffer
+                    const int wrow0 = q0 + (warp & 1) * 32, st_off = p_off - lane * 128;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) *(float4 *)(smem + st_off + lane * 128 + ((i ^ (lane & 7)) << 4)) = o4[i];
+                    mx::fence_proxy_async_smem();
+                    __syncwarp();
+                    if (lane == 0 && wrow0 < NQ) {
+                        mx::tma_store_3d(&tmO, smem_base + st_off, half * 32, wrow0, bh);
+                        mx::bulk_commit_group();   // (waited for before the kernel ends)
+                    }
+                } else if (row < NQ) {
+                    float *orow = P.O + (size_t)bh * P.o_head_stride + (size_t)row * P.o_row_stride + half * 32;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) *(float4 *)(orow + 4 * i) = o4[i];
+                }
+                if (half == 0 && P.L != nullptr && row < NQ) P.L[(size_t)bh * NQ + row] = m * l_scale + __logf(l);
+            }
         }
         if (w == 0 && lane == 0) mx::bulk_wait_group_read<0>();
         __syncwarp();
@@ -1710,8 +1664,9 @@ int mx230_launch_flash_fwd_ex(mx230_handle *h, cudaStream_t st, const void *Qb, 
     P.col_kskb = col_kskb;
     P.n_k_tiles = (n_k + BN - 1) / BN;
     P.status = h->status_dev;
-    // persistent: one CTA per SM (the kernel holds all of an SM's tensor memory), each walking its share of the items
-    dim3 grid((unsigned)(P.n_items < h->sm_count ? P.n_items : h->sm_count));
+    // persistent: one CTA per SM (the kernel holds all of an SM's tensor memory), each walking its share of the items; 64-row items
+    // have a CTA each
+    dim3 grid((unsigned)(rows64 || P.n_items < h->sm_count ? P.n_items : h->sm_count));
     if (rows64) {
         if (row_a) return launch_rows64<SRC_I8>(h, st, grid, tq, tk, tv, to, P);
         if (q_prescaled) return launch_rows64<SRC_PRE>(h, st, grid, tq, tk, tv, to, P);
