@@ -1574,16 +1574,14 @@ bool fwd_key_split(int heads, int n_q, int n_k, int q_off, int causal, int sms) 
 }
 
 // Items of 64 rows wherever every one of them has an SM to itself: a key tile costs such an item less than a key-split item's
-// turn of two tiles (1050 cycles against 2 x 1275), but more per row, so a second round would lose.  No unit is near its limit (1 x 8192
-// rows: 0.41 instructions a cycle and scheduler, exp pipe 37 %, tensor reads of shared memory 33 %): one warp per group and
-// scheduler waits for its tensor-memory loads, and P V of the four groups' tiles runs in key order.  us a call, key-split / 64 rows: 1 x 8192 rows causal 49.0 / 41.1, 4 x
-// 1024 13.2 / 11.6, 6 x 1400 16.6 / 15.3; prefill of 512 tokens over 2048 int8 keys, 14/2 heads, 28.7 / 26.7, 128 over 4128 41.5 /
-// 35.1, 512 over 512 17.5 / 17.8 (the worst of 60); beyond one round 12 x 1024 15.2 / 16.6, 8 x 2000 21.8 / 24.5, 4 x 4096 30.4 / 30.0.
-// Int8 scores, whose first tile costs more here, from eleven key tiles on (128 over 1128 keys, 32/4 heads, 24.1 / 25.1; 100 over 100
-// 14.9 / 16.5; 512 over 2048 as above; 700 over 4700, 12/12 heads, 54.7 / 48.1).
-bool fwd_rows64(int heads, int n_q, int n_k, bool i8, int sms) {
-    return (long long)((n_q + R_ROWS - 1) / R_ROWS) * heads <= sms && (!i8 || n_k > 10 * BN);
-}
+// turn of two tiles (1060 cycles against 2 x 1275), but more per row, so a second round would lose (with a loop over items 12 x 1024 15.2 / 16.6,
+// 8 x 2000 21.8 / 24.5, 4 x 4096 30.4 / 30.0).  us a call, key-split / 64 rows.  Heads inside the bound: 1 x 8192 rows causal 48.9 /
+// 39.4, 4 x 1024 11.9 / 10.1, 6 x 1400 15.2 / 13.6, 12 x 768 no mask 11.8 / 11.8, prefill of 512 tokens over fp32 keys, 14/2 heads,
+// none before them 11.0 / 11.0 (the worst), 512 13.9 / 13.2.  Heads beyond it: 1 x 8192 71.5 / 42.4, 12 x 768 13.5 / 11.9.  bf16
+// without a bound: 4 x 1900 19.4 / 12.9, 12 x 768 10.3 / 8.4, 24 x 384 8.0 / 6.9.  Int8 scores, inside the bound and beyond: 512
+// over 2048 keys 25.7 / 20.5 and 34.1 / 22.2, 128 over 1128 18.1 / 14.6 and 21.8 / 14.9, 512 alone 15.0 / 12.7 and 16.1 / 12.2, 1
+// alone 9.4 / 7.7 and 9.6 / 8.3 (36 sizes below 1280 keys: 0.72 to 0.86 of the key-split form's time, beyond the bound 0.60 to 0.89).
+bool fwd_rows64(int heads, int n_q, int sms) { return (long long)((n_q + R_ROWS - 1) / R_ROWS) * heads <= sms; }
 
 template <int SRC, bool KEY_SPLIT, bool HALF = false>
 int launch_variant(mx230_handle *h, cudaStream_t st, dim3 grid, const CUtensorMap &tq, const CUtensorMap &tk,
@@ -1627,7 +1625,7 @@ int mx230_launch_flash_fwd_ex(mx230_handle *h, cudaStream_t st, const void *Qb, 
     } else {
         memset(&to, 0, sizeof(to));
     }
-    const bool rows64 = fwd_rows64(heads, n_q, n_k, row_a != nullptr, h->sm_count);
+    const bool rows64 = fwd_rows64(heads, n_q, h->sm_count);
     const bool key_split = !rows64 && fwd_key_split(heads, n_q, n_k, q_off, causal, h->sm_count);
     if ((rc = mx230_make_tmap_bf16(h, &tq, Qb, n_q, heads, rs, (uint64_t)n_q * HD * 2, rows64 ? R_ROWS : BM))) return rc;
     if ((rc = mx230_make_tmap_bf16(h, &tk, Kb, n_k, heads / kv_group, rs, (uint64_t)n_k * HD * 2, BN))) return rc;

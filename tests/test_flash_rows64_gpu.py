@@ -1,4 +1,4 @@
-"""Forward with 64-row items (calls whose 64-row items fit the SMs at once; int8 scores beyond 1280 keys) against the other forms, which calls with more heads
+"""Forward with 64-row items (calls whose 64-row items fit the SMs at once) against the other forms, which calls with more heads
 take: a head inside the bound has the same bits in either, a head beyond it (its own max per softmax group) the same rows up to
 the rounding of P.  Sizes are the edges of 64-row tiles, of 128-key tiles and of rounds of four key tiles."""
 import pytest
