@@ -55,6 +55,42 @@ def test_forward_wait_runs_out_and_handle_recovers():
     h.close()
 
 
+@pytest.mark.parametrize("heads,n,tile", [
+    (2, 640, 4),      # 64-row form
+    (12, 1024, 1),    # key-split form, one item per CTA
+    (19, 2177, 19),   # key-split form, in the second item of CTA 0 (its first one has 18 tiles)
+    (48, 1024, 1),    # pair form
+    (96, 1024, 9),    # pair form, in the second item (8 tiles in the first)
+])
+def test_forward_wait_runs_out_in_every_form(heads, n, tile):
+    """A K/V tile that never arrives, in each form of the forward: the launch ends with a status, and the next one has the bits of
+    the one before."""
+    torch.cuda.set_device(0)
+    h = Handle(0, 64 << 20)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(57)
+    q, k, v = (torch.randn(heads, n, 64, device="cuda", generator=g) for _ in range(3))
+    q[1] *= 40   # beyond the bound: its items take the general loop
+    o, l = torch.empty_like(q), torch.empty(heads, n, device="cuda")
+    o2, l2 = torch.empty_like(q), torch.empty(heads, n, device="cuda")
+    fa.run_flash_lse(h, q, k, v, o, l, n, True)
+    h.check_status()
+    try:
+        h.set_option(_lib.OPT_WAIT_LIMIT, 2000)
+        h.set_option(_lib.OPT_TEST_DROP_TILE, tile)
+        fa.run_flash_lse(h, q, k, v, o2, l2, n, True)
+        with pytest.raises(_lib.Mx230Error) as e:
+            h.check_status()
+        assert e.value.code == _lib.ERR_DEVICE_STATUS
+    finally:
+        h.set_option(_lib.OPT_TEST_DROP_TILE, -1)
+        h.set_option(_lib.OPT_WAIT_LIMIT, 4000000)
+    fa.run_flash_lse(h, q, k, v, o2, l2, n, True)
+    h.check_status()
+    assert torch.equal(o, o2) and torch.equal(l, l2)
+    h.close()
+
+
 def test_fused_backward_wait_runs_out_and_handle_recovers():
     torch.cuda.set_device(0)
     h = Handle(0, 64 << 20)

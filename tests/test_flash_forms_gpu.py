@@ -9,7 +9,9 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("causal", [False, True])
-@pytest.mark.parametrize("heads,n", [(3, 1920), (3, 1921), (3, 2177), (1, 4096), (40, 2050)])   # 40: pair form
+@pytest.mark.parametrize("heads,n", [(3, 1920), (3, 1921), (3, 2177), (1, 4096),     # 64-row form
+                                     (17, 1024), (8, 1921), (10, 1920), (9, 2177),   # key-split (the last two: causal, over 148 items)
+                                     (40, 2050)])                                    # pair form
 def test_bf16_forward_modes(handle, heads, n, causal):
     """bf16 operands are exact, so scores differ from 64 bits by fp32 rounding only (2^-24 * 64 * |q||k|/8 < 2e-3 at the
     largest scale here, below 1e-5 at scale 1): what remains is P in bf16, 2^-9 relative per probability, which moves a row by
@@ -38,9 +40,10 @@ def test_bf16_forward_modes(handle, heads, n, causal):
                 assert torch.equal(one, o[h]) and torch.equal(l_one, l[h])
 
 
-def test_bf16_forward_non_finite_operand(handle):
+@pytest.mark.parametrize("heads", [2, 8, 40])   # 64-row, key-split, pair form
+def test_bf16_forward_non_finite_operand(handle, heads):
     """A NaN in one head leaves the other heads alone and reaches every row of its own head that sees it."""
-    heads, n = 2, 2048
+    n = 2048
     g = torch.Generator(device="cuda")
     g.manual_seed(6)
     q, k, v = (torch.randn(heads, n, 64, device="cuda", generator=g).bfloat16() for _ in range(3))
@@ -50,7 +53,8 @@ def test_bf16_forward_non_finite_operand(handle):
     o2, l2 = torch.empty_like(o), torch.empty_like(l)
     fa.run_flash_bf16(handle, q, k, v, o2, l2, n, False)
     handle.check_status()
-    assert torch.equal(o[0], o2[0]) and torch.equal(l[0], l2[0])
+    others = [h for h in range(heads) if h != 1]
+    assert torch.equal(o[others], o2[others]) and torch.equal(l[others], l2[others])
     assert torch.isnan(l2[1]).all()
 
 
@@ -115,14 +119,14 @@ def test_bf16_heads_inside_and_outside_the_bound_key_split(handle, heads, n, cau
 
 
 @pytest.mark.parametrize("n", [1921, 4096, 5000])
+@pytest.mark.parametrize("heads", [3, 8])   # 1921 rows: 64-row and key-split form
 @pytest.mark.parametrize("where", ["first", "last", "apart", "swapped"])
-def test_bf16_bound_is_of_the_whole_head(handle, n, where):
+def test_bf16_bound_is_of_the_whole_head(handle, n, heads, where):
     """One row of one operand decides the loop: the first or the last row of a head, of Q or of K, or large rows of Q against
     small ones of K that stay inside the bound.  The decision shows in L only by rounding, so the bound is the existing
     tests': the rows of 64-bit softmax, L to 2e-3 where scores reach 2^9."""
     g = torch.Generator(device="cuda")
     g.manual_seed(9)
-    heads = 3
     q, k, v = (torch.randn(heads, n, 64, device="cuda", generator=g) for _ in range(3))
     if where == "first":
         q[1, 0] *= 60
@@ -142,3 +146,35 @@ def test_bf16_bound_is_of_the_whole_head(handle, n, where):
         s = q[h].double() @ k[h].double().T * 0.125
         assert (o[h].double() - torch.softmax(s, -1) @ v[h].double()).abs().max() <= 2.2e-2
         assert (l[h].double() - torch.logsumexp(s, -1)).abs().max() <= 2e-3
+
+
+@pytest.mark.parametrize("bf16,heads,n", [(False, 12, 2048), (False, 20, 1900), (True, 12, 1900), (True, 20, 1810)])
+@pytest.mark.parametrize("every,first", [(3, 1), (2, 0), (5, 2)])
+def test_odd_groups_publish_early_over_several_items(handle, bf16, heads, n, every, first):
+    """Causal, key-split, 180 to 300 items: the odd groups hand on an item's sums before its last P V, item after item, over fp32
+    operands (heads inside and beyond the bound) and bf16 ones without a bound.  The bits of every repetition and, in the max-free
+    loop, of the head in a call of its own; else that call's rows to 2 * 2^-9 * max|v| (each takes P, rounded to bf16, against
+    other maxima; max|v| < 5.5)."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(10)
+    q, k, v = (torch.randn(heads, n, 64, device="cuda", generator=g) for _ in range(3))
+    beyond = [h for h in range(heads) if h % every == first]
+    q[beyond] *= 30
+    if bf16:
+        q, k, v = q.bfloat16(), k.bfloat16(), v.bfloat16()
+    run = fa.run_flash_bf16 if bf16 else fa.run_flash_lse
+    handle.reserve(fa.workspace_bytes(heads, n, False))
+    o, l = torch.empty(heads, n, 64, device="cuda"), torch.empty(heads, n, device="cuda")
+    o2, l2 = torch.empty_like(o), torch.empty_like(l)
+    run(handle, q, k, v, o, l, n, True)
+    for _ in range(10):
+        run(handle, q, k, v, o2, l2, n, True)
+        assert torch.equal(o, o2) and torch.equal(l, l2)
+    one, l_one = torch.empty(n, 64, device="cuda"), torch.empty(n, device="cuda")
+    for h in range(heads):
+        run(handle, q[h], k[h], v[h], one, l_one, n, True)
+        if not bf16 and h not in beyond:
+            assert torch.equal(one, o[h]) and torch.equal(l_one, l[h]), f"head {h}"
+        else:
+            assert (one - o[h]).abs().max() <= 2.2e-2 and (l_one - l[h]).abs().max() <= 1e-3, f"head {h}"
+    handle.check_status()

@@ -82,9 +82,9 @@ def scores64(qkv, c, nh, nkv, n_keys, quant):
 @pytest.mark.parametrize("quant", [False, True])
 @pytest.mark.parametrize("scale", [1.0, 40.0])   # 40: scores beyond the bound of the max-free loop
 @pytest.mark.parametrize("nh,nkv,n_tok,pos0", [
-    (2, 1, 1, 0), (2, 1, 128, 0), (3, 3, 129, 1), (2, 2, 100, 200), (14, 2, 257, 130),       # few items: key-split form
-    (3, 1, 640, 129), (14, 2, 1410, 77),                                                     # several items per CTA
-    (40, 8, 1024, 0),                                                                        # pair form
+    (2, 1, 1, 0), (2, 1, 128, 0), (3, 3, 129, 1), (2, 2, 100, 200), (14, 2, 257, 130), (3, 1, 640, 129),   # few items: 64-row form
+    (14, 2, 700, 300), (14, 2, 1200, 0), (14, 2, 1410, 77),          # key-split form, the last one with several items per CTA
+    (40, 8, 1024, 0),                                                # pair form
 ])
 def test_forms_and_edges(handle, quant, scale, nh, nkv, n_tok, pos0):
     """Every form against 64-bit softmax.  The probabilities and V are rounded to bf16 (2^-9 each, relative): a row is an
