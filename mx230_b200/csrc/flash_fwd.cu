@@ -1116,8 +1116,11 @@ flash_fwd_rows64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
             ok = wait_warp(RB_REF, 0);
             if (ok) m = ref[row_in_tile];
         }
-        // the group's P buffer is free: P V of its previous tile is complete
-        auto p_free = [&](int i) { return i == 0 || wait_warp(RB_P_DONE + w, i - 1); };
+        // the group's P buffer is free: P V of its previous tile is complete (usually for long: one cheap look first, 1.5 to 3 % of a
+        // long range, 1024 tokens over 30000 fp32 keys 131.1 -> 126.7 us)
+        auto p_free = [&](int i) {
+            return i == 0 || (bool)__all_sync(0xFFFFFFFFu, mx::mbar_wait_fast(bar(RB_P_DONE + w), (i - 1) & 1, abort_flag, P.status));
+        };
         auto put = [&](const uint32_t *pk, int at0) {   // 32 probabilities: four 16-byte pieces of the row, from piece at0 on
 #pragma unroll
             for (int i = 0; i < 4; ++i)
@@ -1574,7 +1577,7 @@ bool fwd_key_split(int heads, int n_q, int n_k, int q_off, int causal, int sms) 
 }
 
 // Items of 64 rows wherever every one of them has an SM to itself: a key tile costs such an item less than a key-split item's
-// turn of two tiles (1060 cycles against 2 x 1275), but more per row, so a second round would lose (with a loop over items 12 x 1024 15.2 / 16.6,
+// turn of two tiles (980 to 1100 cycles against 2 x 1275), but more per row, so a second round would lose (with a loop over items 12 x 1024 15.2 / 16.6,
 // 8 x 2000 21.8 / 24.5, 4 x 4096 30.4 / 30.0).  us a call, key-split / 64 rows.  Heads inside the bound: 1 x 8192 rows causal 48.9 /
 // 39.4, 4 x 1024 11.9 / 10.1, 6 x 1400 15.2 / 13.6, 12 x 768 no mask 11.8 / 11.8, prefill of 512 tokens over fp32 keys, 14/2 heads,
 // none before them 11.0 / 11.0 (the worst), 512 13.9 / 13.2.  Heads beyond it: 1 x 8192 71.5 / 42.4, 12 x 768 13.5 / 11.9.  bf16
