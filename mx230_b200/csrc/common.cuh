@@ -681,12 +681,12 @@ __device__ __forceinline__ void rope_pair(float &x1, float &x2, float cs, float 
 // ---- maximum and minimum over the warp (NaN is passed over, as by fmaxf) ----
 __device__ __forceinline__ float warp_max(float v) {
     float r;
-    asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
     return r;
 }
 __device__ __forceinline__ float warp_min(float v) {
     float r;
-    asm("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
     return r;
 }
 
