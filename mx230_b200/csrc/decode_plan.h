@@ -48,13 +48,13 @@ inline DecodeSplit plan_splits(long long slots, long long groups, long long keys
 // fp32 cache, CTAs of eight warps that have an SM to themselves.  fit[c]: clusters of c such CTAs that the device holds at once,
 // by its own count: how many GPCs have room for another cluster of seven or eight does not follow from the number of SMs (148 of
 // them hold 15; as 16, or as 17 and 18 of seven, they took a second wave).  False: the four-warp plan.
-// us a call, position on the device, at 500 / 4000 / 32000 keys (with the tile loop that read q from shared memory; with q in registers
-// groups of 7 and 8 heads are a fifth to a third faster in either plan); four-warp CTAs, clusters of eight counted as 7/8 of the SMs, this:
-//   16/16 heads  5.8 12.0 45.7 |  6.9 12.7 58.4 | 5.3 11.5 45.8        32/8  5.7 12.6 28.8 |  4.7  8.8 43.9 | 5.3 10.7 27.7
-//   32/4         8.1 16.1 41.1 |  6.7 12.6 40.7 | 6.8 12.7 27.0        72/9  8.3 18.2 50.2 |  6.8 13.2 58.3 | 7.2 13.6 43.7
-// Unknown length, more than two query heads a group (where the arithmetic of a key counts beside its loads): clusters of eight that
-// leave a fifth of the SMs empty make way for smaller ones, up to 16 CTAs a group, the warps of the four-warp plan.  With one or
-// two heads eight CTAs are enough at every length (12/12 4.7 10.7 36.0 | 3.8 7.4 33.0, clusters of five 4.4 9.5 33.4).
+// us a call, position on the device, at 500 / 4000 / 16000 / 32000 keys; four-warp CTAs | eight-warp CTAs in one cluster of eight | this:
+//   12/12 heads  3.7  8.7 12.4 35.3 | 3.2 5.4 16.2 30.9 | as the second           32/8  3.8  9.0 12.1 25.8 | 3.4 6.3 15.7 28.7 | 3.8 8.3 12.6 24.6
+//   32/4         4.3 10.1 16.8 27.6 | 4.1 8.5 12.7 18.7 | as the second           72/9  4.7 12.1 22.5 39.6 | 4.2 8.5 23.1 41.7 | 4.6 9.4 18.5 31.6
+// (16 groups and more: the four-warp plan, 16/16 4.1 8.9 25.9 44.4.)  Unknown length, more than two query heads a group: clusters of
+// eight that leave a fifth of the SMs empty make way for smaller ones, up to 16 CTAs a group, the warps of the four-warp plan: up to
+// 8000 keys they lose to the cluster of eight, beyond them they win as much.  With one or two heads the cluster of eight stays: smaller
+// ones win at 16000 keys only (12/12 3.5 7.5 14.6 33.0, 16/8 3.6 7.5 10.9 24.2 against 3.2 5.5 12.9 24.9).
 inline bool plan_wide(DecodeSplit &P, const int *fit, long long groups, int heads, long long keys, int pass_keys) {
     const bool known = keys > 0;
     int c = known && keys <= 7LL * pass_keys ? (int)((keys + pass_keys - 1) / pass_keys) : 8;
