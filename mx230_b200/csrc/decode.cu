@@ -1700,9 +1700,10 @@ int launch_decode(mx230_handle *h, void *stream, DecodeParams P, int n_seq, int 
         P.cl_size = 1, P.cluster_keys = 0;
         P.max_clusters = (int)(n < 1 ? 1 : n > 256 ? 256 : n);
     } else {
-        // fp32 cache, few groups: CTAs of eight warps with an SM to themselves take half as many key tiles in turn (one sequence: 778
-        // keys, 14/2 heads 8.2 -> 7.2 us, 4001 keys, 32/4 heads 15.4 -> 13.6; token of 24 layers at 1000 341 -> 313).  Known
-        // sequences beyond one cluster's keys keep three CTAs of four warps per SM.
+        // fp32 cache, few groups: CTAs of eight warps with an SM to themselves take half as many key tiles in turn (host
+        // position, 14/2 heads, 800 keys 4.4 -> 4.1 us, 32/4 heads, 3900 keys 9.4 -> 8.1; at 500 keys, where they have one tile a warp,
+        // four-warp CTAs are the faster ones, 3.7 against 4.2).  Known sequences beyond one cluster's keys keep three CTAs of four warps
+        // per SM.
         DecodeSplit S;
         const bool few = !q8 && base_ctas * 8 <= h->sm_count && known_keys <= 4 * 8 * F32_WARPS_WIDE * FT_KEYS;
         P.wide = few && plan_wide(S, h->wide_fit, base_ctas, P.group, known_keys, F32_WARPS_WIDE * FT_KEYS);

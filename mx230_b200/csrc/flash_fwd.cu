@@ -1369,8 +1369,8 @@ flash_fwd_rows64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     if (warp == SOFT_WARPS + 1) mx::tmem_dealloc(tmem, TM_COLS);
 }
 
-// Largest |q|^2 |k|^2 scale^2 log2(e)^2 over the rows of a head of bf16 Q and K -> L[head][first row of every query tile],
-// where flash_fwd_kernel looks for it (its own scratch would be shared by the streams of a handle; L is the call's).  A
+// Largest |q|^2 |k|^2 scale^2 log2(e)^2 over the rows of a head of bf16 Q and K -> L[head][every 64th row], the first row
+// of an item or query tile in every form, where the forward looks for it (its own scratch would be shared by the streams of a handle; L is the call's).  A
 // cluster per head, eight threads per row; bound by the latency of its loads (24 heads of 2048 rows: about 4 us) or, from some
 // 20 MB on, by HBM.  A warp stops at the first pass that shows the head beyond the bound (what is left in L is then a part of
 // the product, beyond it as well).  Forward of heads beyond the bound, us a call, whole pass / stopping: 1 x 32768 rows
